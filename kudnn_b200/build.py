@@ -27,7 +27,8 @@ NVCC_FLAGS = [
     "-I", os.path.join(_ROOT, "include"),
 ]
 
-CUDA_SOURCES = ["linear_api.cu", "simt_gemm.cu", "gemv.cu", "tc_gemm.cu", "pack.cu", "static_scratch.cu", "peer.cu", "eltwise.cu", "eltwise_api.cu"]
+CUDA_SOURCES = ["linear_api.cu", "simt_gemm.cu", "gemv.cu", "tc_gemm.cu", "tc_inst_f32.cu", "tc_inst_f16.cu", "tc_inst_bf16.cu",
+                "tc_inst_s8.cu", "pack.cu", "static_scratch.cu", "peer.cu", "eltwise.cu", "eltwise_api.cu"]
 
 
 def _nvcc():
@@ -72,7 +73,9 @@ def build_cuda(verbose=False, force=False, ptxas_info=False):
         s = os.path.join(_CSRC, src)
         o = os.path.join(_BUILD, src.replace(".cu", ".o"))
         objs.append(o)
-        if force or not _newer(o, [s] + headers):
+        # the tensor-core kernel's own headers concern its own translation units only
+        deps = [h for h in headers if src.startswith("tc_") or not os.path.basename(h).startswith("tc_")]
+        if force or not _newer(o, [s] + deps):
             cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if ptxas_info else []) + ["-c", s, "-o", o]
             jobs.append(cmd)
     outputs = []
