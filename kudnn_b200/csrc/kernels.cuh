@@ -63,14 +63,21 @@ struct TcOperands {
     // batched problems: `batch` matrices per operand, a_bstride / b_bstride elements apart (0: every entry shares one)
     long long batch = 1, a_bstride = 0, b_bstride = 0;
 };
+// How the epilogue meets its tensors: every row 16 bytes at a time (and beta = 0), rows whose elements are contiguous but
+// start anywhere, or neither.
+enum class TcRows { kVectors, kContiguous, kOther };
 struct TcPlan {
-    int block_n;   // 128 or 256
+    int block_n;   // tile width: a multiple of 16 up to 256
     int stages;
     int grid;
     size_t smem_bytes;
     // split-K (splits > 1) for problems with far fewer tiles than SMs: the kernel is launched as clusters of
     // `splits` CTAs, grid = tiles * splits
     int splits, kb_per_split;
+    int a_rows;      // rows of the activation operand per copy (fewer than 128 only when the problem has fewer)
+    int ring_bytes;  // shared memory in front of the barriers
+    int vector_rows;  // 1: TcRows::kVectors
+    int via_smem;    // 1: one work item per CTA, the tile is finished from shared memory
     int pair;      // 1: clusters of two CTAs share 256 x block_n tiles (cta_group::2)
     int narrow_from;  // pair mode: tiles from this index on are processed as two pieces of half the width
     unsigned char tmap_a[128] __attribute__((aligned(64)));
@@ -83,7 +90,8 @@ const char *tc_unavailable_reason();
 cudaError_t tc_encode_kmajor(void *map128, const void *base, int kind, long long rows, long long k_total, long long ld_elems,
                              int box_rows);
 // with_staging: the launch writes output mirrors and needs the epilogue's row staging in shared memory
-cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm_count, bool with_staging, TcPlan *plan);
+cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm_count, bool with_staging, TcRows rows,
+                         TcPlan *plan);
 // wait_limit_cycles: SM cycles after which a device-side wait gives up (0 = the default of about two seconds);
 // skip_kblock: test hook for the timeout path, -1 = off (see TcParams::skip_kb).
 // bp: batch strides of the epilogue tensors (ignored unless ops.batch > 1)

@@ -166,6 +166,7 @@ struct kudnn_b200_linear_s {
     const void *plan_a = nullptr, *plan_b = nullptr;
     long long plan_m = 0;
     bool plan_staging = false;
+    kb::TcRows plan_rows = kb::TcRows::kOther;
     bool plan_valid = false;
 
     // kudnn_b200_linear_run_sharded: one child primitive per shard, each on its own device with its own copy (or
@@ -307,6 +308,26 @@ bool kmajor_ready(const void *p, int dtype, long long s_row, long long s_k, long
 {
     const int vec = 16 / kb::dtype_size(dtype);
     return s_k == 1 && aligned16(p) && (rows == 1 || s_row % vec == 0);
+}
+
+// How the tensor-core epilogue can read and write the rows of c, bias, res and out.
+kb::TcRows epilogue_rows(const kb::LinearProblem &pr)
+{
+    const kb::EpiParams &e = pr.epi;
+    auto vectors = [&](const void *p, int dtype, long long s_m, long long s_n, const long long (&sb)[3]) {
+        const long long vec = 16 / kb::dtype_size(dtype);
+        return p == nullptr ||
+               (s_n == 1 && aligned16(p) && s_m % vec == 0 && sb[0] % vec == 0 && sb[1] % vec == 0 && sb[2] % vec == 0);
+    };
+    const bool second = e.res_op != KUDNN_B200_RES_NONE;
+    if (e.beta == 0.0f && e.n % 8 == 0 && vectors(e.c, e.c_dtype, e.c_sm, e.c_sn, pr.batch.c_sb) &&
+        (e.has_bias == 0 || e.bias_sn == 0 || vectors(e.bias, e.bias_dtype, e.bias_sm, e.bias_sn, pr.batch.bias_sb)) &&
+        (!second || (vectors(e.res, e.res_dtype, e.res_sm, e.res_sn, pr.batch.res_sb) &&
+                     vectors(e.out, e.out_dtype, e.out_sm, e.out_sn, pr.batch.out_sb)))) {
+        return kb::TcRows::kVectors;
+    }
+    const bool contiguous = (e.c == nullptr || e.c_sn == 1) && (!second || (e.res_sn == 1 && e.out_sn == 1));
+    return contiguous ? kb::TcRows::kContiguous : kb::TcRows::kOther;
 }
 
 long long round_up(long long v, long long a)
@@ -525,7 +546,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.lda = k_pad;
             }
             if (!(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m && !h->plan_staging)) {
-                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, false, &h->tc_plan);
+                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, false, kb::TcRows::kOther, &h->tc_plan);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "tensor map encoding");
                 }
@@ -841,8 +862,10 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.a_bstride = shared ? 0 : per;
             }
             const bool staging = pr.epi.n_mirrors > 0;
-            if (nb > 1 || !(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m && h->plan_staging == staging)) {
-                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, staging, &h->tc_plan);
+            const kb::TcRows rows = epilogue_rows(pr);
+            if (nb > 1 || !(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m &&
+                            h->plan_staging == staging && h->plan_rows == rows)) {
+                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, staging, rows, &h->tc_plan);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "tensor map encoding");
                 }
@@ -850,6 +873,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 h->plan_b = ops.b;
                 h->plan_m = d.m;
                 h->plan_staging = staging;
+                h->plan_rows = rows;
                 h->plan_valid = nb == 1;
                 if (const char *dbg = std::getenv("KUDNN_B200_DEBUG")) {
                     if (*dbg != '\0' && *dbg != '0') {

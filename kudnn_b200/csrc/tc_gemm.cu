@@ -98,83 +98,174 @@ cudaError_t tc_encode_kmajor(void *map128, const void *base, int kind, long long
     return e;
 }
 
-cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm_count, bool with_staging, TcPlan *plan)
+namespace {
+
+int env_choice(const char *name)
+{
+    const char *v = std::getenv(name);
+    return v == nullptr || *v == '\0' ? -1 : std::atoi(v);
+}
+
+int pair_clusters_of(int kind, size_t smem)
+{
+    return kind == KUDNN_B200_F32   ? pair_clusters_kind<KUDNN_B200_F32>(smem)
+           : kind == KUDNN_B200_F16 ? pair_clusters_kind<KUDNN_B200_F16>(smem)
+           : kind == KUDNN_B200_S8  ? pair_clusters_kind<KUDNN_B200_S8>(smem)
+                                    : pair_clusters_kind<KUDNN_B200_BF16>(smem);
+}
+
+// Estimated SM cycles of a launch of single CTAs.  A k-block of a tile costs its MMAs (2 cycles per column whatever the
+// operand type) or its operand bytes (about 60 per cycle and SM), whichever is more.
+double single_cta_cycles(long long tiles, int splits, long long kb, int bn, int a_rows, bool via_smem, int sm_count)
+{
+    const double per_kb = std::max(2.0 * bn, 2.1 * (a_rows + bn));
+    const double area = static_cast<double>(a_rows) * bn;
+    // finished from shared memory, with contiguous stores; or straight from tensor memory, under the next tile's products.
+    // The other ranks' shares of a cut tile arrive at about 12 bytes per cycle.
+    if (via_smem) {
+        const double finish = 2500.0 + 0.04 * area + 0.2 * area / splits + (splits > 1 ? 1000.0 + area * 4 * (splits - 1) / splits / 12 : 0.0);
+        const long long waves = (tiles * splits + sm_count - 1) / sm_count;
+        return waves * (2500.0 + kb * per_kb + finish);
+    }
+    const double epilogue = 1000.0 + 0.35 * area;
+    const long long waves = (tiles + sm_count - 1) / sm_count;
+    return 2500.0 + waves * std::max(kb * per_kb, epilogue) + epilogue;
+}
+
+}  // namespace
+
+cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm_count, bool with_staging, TcRows rows,
+                         TcPlan *plan)
 {
     static_assert(sizeof(CUtensorMap) <= 128, "tensor map storage too small");
     if (!tc_available()) {
         return cudaErrorNotSupported;
     }
+    const bool ints = ops.kind == KUDNN_B200_S8;
+    const int width_step = ints ? 32 : 16;
     const long long tiles_m = (m + kBM - 1) / kBM;
-    const long long tiles256 = ops.batch * tiles_m * ((n + 255) / 256);
-    const int bn = (tiles256 >= sm_count || n > 128 * 64) ? 256 : 128;
-    const long long tiles = ops.batch * tiles_m * ((n + bn - 1) / bn);  // over all batch entries
-    if (tiles > (1ll << 30)) {
+    const int a_rows_single = static_cast<int>(m >= kBM ? kBM : (m + 7) / 8 * 8);
+    const int elems_per_row = kStageRowBytes / dtype_size(ops.kind);
+    const long long num_kb = (ops.k_total + elems_per_row - 1) / elems_per_row;
+    // Single-CTA shapes: every tile width that the MMA takes, with K whole or cut between the 2, 4 or 8 CTAs of a cluster
+    // (the rows of the tile are divided among them for the final pass).  Which of them is fastest follows from how the
+    // tiles fill the SMs: with one work item per CTA a tile is finished from shared memory; more items than SMs run
+    // persistently, the epilogue of one under the products of the next.  Kernel times: 64 x 11008 x 4096 in 86 CTAs of
+    // 128 x 128 with K cut in two 39 us, in the shape chosen here 20 us; 1027 x 4096 x 11008 in two waves of 128 x 128
+    // tiles 133 us, in one wave of 144 tiles of 128 x 256 71 us.
+    const int forced_splits = env_choice("KUDNN_B200_TC_SPLITS");
+    double best = 1e300;
+    int bn = 128;
+    long long splits = 1;
+    bool via_smem = false;
+    for (int w = width_step; w <= 256; w += width_step) {
+        if (w - width_step >= n) {
+            break;  // wider than the matrix
+        }
+        const long long tiles = ops.batch * tiles_m * ((n + w - 1) / w);
+        if (tiles > (1ll << 30)) {
+            continue;
+        }
+        for (int sp = 1; sp <= kMaxSplits; sp *= 2) {
+            if (sp > 1) {
+                // every split keeps at least two k-blocks and none is empty; a GPC's SMs do not divide into clusters of four
+                // and eight without a rest (33 and 15 of them fit 148 SMs, cudaOccupancyMaxActiveClusters)
+                const long long per = (num_kb + sp - 1) / sp;
+                const int room = sp == 8 ? sm_count * 30 / 37 : sp == 4 ? sm_count * 33 / 37 : sm_count;
+                if (ints || per < 2 || (num_kb + per - 1) / per != sp || (forced_splits < 0 && tiles * sp > room)) {
+                    continue;
+                }
+            }
+            if (forced_splits >= 1 && sp > forced_splits) {
+                continue;
+            }
+            const bool one_item = sp > 1 || (!ints && !with_staging && (tiles <= sm_count || rows == TcRows::kContiguous));
+            double cost = single_cta_cycles(tiles, sp, (num_kb + sp - 1) / sp, w, a_rows_single, one_item, sm_count);
+            if (forced_splits >= 1 && sp * 2 <= forced_splits && sp * 2 <= kMaxSplits) {
+                cost *= 1e6;  // taken only if no larger cut fits
+            }
+            if (cost < best) {
+                best = cost;
+                bn = w;
+                splits = sp;
+                via_smem = one_item;
+            }
+        }
+    }
+    if (best >= 1e300) {
         return cudaErrorInvalidValue;
     }
-    // CTA pairs for the large-problem shape (256-wide tiles): 256 x 256 tiles over clusters of two.  Not for launches
+    // CTA pairs: 256 x 256 tiles over clusters of two, where that is estimated to be faster.  Not for launches
     // that run for many milliseconds: those are limited by the board's power cap, and the pair shape, which needs
     // fewer cycles, draws enough more power per cycle to end up slower there (bf16 n = 28672, k = 8192, ms per call,
     // pair / single CTA: 4096 rows 1.385 / 1.396, 8192 rows 2.84 / 2.85, 16384 rows 6.10 / 5.96, 32768 rows
     // 13.3 / 12.4).
     const double flops = 2.0 * static_cast<double>(m) * static_cast<double>(n) * static_cast<double>(ops.k_total);
-    // batched launches use single CTAs
-    bool pair = bn == 256 && m > kBM && flops < 6.0e12 && ops.batch == 1;
-    if (const char *env = std::getenv("KUDNN_B200_TC_PAIR")) {
-        pair = pair && std::atoi(env) != 0;
-    }
-    int pair_clusters = 0;
+    // batched launches use single CTAs, and so do outputs that cannot be stored as vectors
+    bool pair = n > kBM && m > kBM && flops < 6.0e12 && ops.batch == 1 && (rows == TcRows::kVectors || ints) && forced_splits <= 1 &&
+                env_choice("KUDNN_B200_TC_PAIR") != 0;
+    const int pair_stages = with_staging ? 5 : 6;
+    plan->narrow_from = 0;
     if (pair) {
-        const size_t smem = static_cast<size_t>(with_staging ? 5 : 6) * (kABytes + 128 * kStageRowBytes) + 1024 + kTailBytes +
-                            (with_staging ? kStagingBytes : 0);
-        pair_clusters = ops.kind == KUDNN_B200_F32   ? pair_clusters_kind<KUDNN_B200_F32>(smem)
-                        : ops.kind == KUDNN_B200_F16 ? pair_clusters_kind<KUDNN_B200_F16>(smem)
-                        : ops.kind == KUDNN_B200_S8  ? pair_clusters_kind<KUDNN_B200_S8>(smem)
-                                                     : pair_clusters_kind<KUDNN_B200_BF16>(smem);
-        pair = pair_clusters > 0;
+        const long long pair_tiles = ((m + 2 * kBM - 1) / (2 * kBM)) * ((n + 255) / 256);
+        const long long guess = sm_count / 2;
+        const long long full = pair_tiles / guess, rem = pair_tiles % guess;
+        const double waves = full + (rem == 0 ? 0.0 : (full > 0 && 2 * rem <= guess ? 0.55 : 1.0));
+        const double epilogue = 1000.0 + 0.35 * kBM * 256;
+        const double cycles = 4000.0 + waves * std::max(num_kb * 640.0, epilogue) + epilogue;
+        pair = cycles < best || env_choice("KUDNN_B200_TC_PAIR") > 0;
+        int clusters = 0;
+        if (pair) {
+            clusters = pair_clusters_of(ops.kind, static_cast<size_t>(pair_stages) * (kABytes + 128 * kStageRowBytes) + 1024 +
+                                                      kTailBytes + (with_staging ? kStagingBytes : 0));
+            pair = clusters > 0;
+        }
+        if (pair) {
+            bn = 256;
+            splits = 1;
+            via_smem = false;
+            plan->grid = 2 * static_cast<int>(pair_tiles < clusters ? pair_tiles : clusters);
+            // Tiles left over after the last full wave: if they would keep at most half of the pairs busy, each of them
+            // is processed as two pieces of half the width, which shortens that wave to a little more than half.
+            const long long left = pair_tiles % clusters;
+            const bool narrow = pair_tiles > clusters && left > 0 && 2 * left <= clusters;
+            plan->narrow_from = static_cast<int>(narrow ? pair_tiles - left : pair_tiles);
+        }
     }
     plan->pair = pair ? 1 : 0;
-    plan->narrow_from = 0;
+    plan->vector_rows = rows == TcRows::kVectors ? 1 : 0;
     plan->block_n = bn;
-    plan->stages = ((bn == 256 && !pair) ? 4 : 6) - (with_staging ? 1 : 0);
-    // Split-K: with at most half the SMs busy and a long K, the CTAs of a cluster share a tile and cut K between
-    // them (2, 4 or 8 ways: the rows of the tile are divided among the ranks for the final pass).  Each split keeps
-    // at least four k-blocks so that the pipeline still fills, and no split may be empty.
-    const int elems_per_row = kStageRowBytes / dtype_size(ops.kind);
-    const long long num_kb = (ops.k_total + elems_per_row - 1) / elems_per_row;
-    long long splits = 1;
-    if (!pair && tiles * 2 <= sm_count && num_kb >= 8 && ops.kind != KUDNN_B200_S8) {
-        long long want = std::min<long long>(sm_count / tiles, num_kb / 4);
-        if (const char *env = std::getenv("KUDNN_B200_TC_SPLITS")) {
-            const long long v = std::atoll(env);
-            if (v >= 1 && v <= num_kb) {
-                want = v;
-            }
-        }
-        while (splits * 2 <= want && splits * 2 <= kMaxSplits) {
-            splits *= 2;
-        }
-        while (splits > 1 && (num_kb + (num_kb + splits - 1) / splits - 1) / ((num_kb + splits - 1) / splits) != splits) {
-            splits /= 2;
-        }
-    }
+    plan->via_smem = via_smem ? 1 : 0;
     plan->splits = static_cast<int>(splits);
     plan->kb_per_split = static_cast<int>((num_kb + splits - 1) / splits);
-    const long long items = tiles * splits;
-    plan->grid = splits > 1 ? static_cast<int>(items) : static_cast<int>(tiles < sm_count ? tiles : sm_count);
+    plan->a_rows = pair ? kBM : a_rows_single;
+    const long long tiles = ops.batch * tiles_m * ((n + bn - 1) / bn);  // over all batch entries
+    if (!pair) {
+        plan->grid = static_cast<int>(via_smem ? tiles * splits : std::min<long long>(tiles, sm_count));
+    }
     const int b_rows = pair ? bn / 2 : bn;  // rows of the weight operand one CTA loads per k-block
-    plan->smem_bytes = static_cast<size_t>(plan->stages) * (kABytes + b_rows * kStageRowBytes) + 1024 + kTailBytes +
-                       (with_staging ? kStagingBytes : 0);
+    const long long stage = static_cast<long long>(plan->a_rows + b_rows) * kStageRowBytes;
+    const long long fixed = 1024 + kTailBytes + (with_staging ? kStagingBytes : 0);
+    plan->stages = static_cast<int>(std::min<long long>((kSmemLimit - fixed) / stage, kMaxStages));
     if (pair) {
-        const long long pair_tiles = ((m + 2 * kBM - 1) / (2 * kBM)) * ((n + bn - 1) / bn);
-        plan->grid = 2 * static_cast<int>(pair_tiles < pair_clusters ? pair_tiles : pair_clusters);
-        // Tiles left over after the last full wave: if they would keep at most half of the pairs busy, each of them
-        // is processed as two pieces of half the width, which shortens that wave to a little more than half.
-        const long long rem = pair_tiles % pair_clusters;
-        bool narrow = pair_tiles > pair_clusters && rem > 0 && 2 * rem <= pair_clusters;
-        plan->narrow_from = static_cast<int>(narrow ? pair_tiles - rem : pair_tiles);
+        plan->stages = pair_stages;
+    } else if (via_smem) {
+        plan->stages = std::max(std::min(plan->stages, plan->kb_per_split), 2);
+    }
+    // the last stage's MMA reads 128 rows of A wherever the copy stopped, and a tile finished from shared memory lies
+    // there as fp32 with four columns of padding
+    long long ring = std::max(plan->stages * stage, (plan->stages - 1) * stage + kABytes);
+    if (via_smem) {
+        ring = std::max<long long>(ring, static_cast<long long>(plan->a_rows) * (bn + 4) * 4);
+    }
+    ring = (ring + 1023) / 1024 * 1024;
+    plan->ring_bytes = static_cast<int>(ring);
+    plan->smem_bytes = static_cast<size_t>(ring + fixed);
+    if (plan->smem_bytes > static_cast<size_t>(kSmemLimit)) {
+        return cudaErrorInvalidValue;
     }
     CUtensorMap ta, tb;
-    cudaError_t e = encode_kmajor(&ta, ops.a, ops.kind, m, ops.k_total, ops.lda, kBM, ops.batch, ops.a_bstride);
+    cudaError_t e = encode_kmajor(&ta, ops.a, ops.kind, m, ops.k_total, ops.lda, plan->a_rows, ops.batch, ops.a_bstride);
     if (e != cudaSuccess) {
         return e;
     }
@@ -209,7 +300,7 @@ cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams
     p.skip_kb = (plan.pair == 0 && plan.splits == 1) ? skip_kblock : -1;
     {
         const bool sixteen = ops.kind == KUDNN_B200_F16 || ops.kind == KUDNN_B200_BF16;
-        const bool light = sixteen && plan.splits == 1 && ops.batch == 1 && epi.n_mirrors == 0 && epi.beta == 0.0f &&
+        const bool light = sixteen && plan.via_smem == 0 && ops.batch == 1 && epi.n_mirrors == 0 && epi.beta == 0.0f &&
                            epi.res_op == KUDNN_B200_RES_NONE && epi.c_dtype == ops.kind &&
                            (epi.has_bias == 0 || epi.bias_dtype == ops.kind) &&
                            (epi.act == KUDNN_B200_ACT_NONE || epi.act == KUDNN_B200_ACT_RELU || epi.act == KUDNN_B200_ACT_SWISH);
@@ -230,6 +321,11 @@ cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams
     p.splits = plan.splits;
     p.kb_per_split = plan.kb_per_split;
     p.stages = plan.stages;
+    p.bn = plan.block_n;
+    p.a_rows = plan.a_rows;
+    p.ring_bytes = plan.ring_bytes;
+    p.via_smem = plan.via_smem;
+    p.vector_rows = plan.vector_rows;
     {
         // The A rows of one raster group are re-read for every tile column and should stay in L2 next to the
         // streaming weights: at most about 64 MB of them (16 tile rows of 256 x 8192 bf16).  Measured on the 32768-row

@@ -12,7 +12,7 @@ cudaError_t launch_kind<KB_TC_KIND>(const TcPlan &plan, const TcParams &p, cudaS
     if (plan.pair) {
         return launch_one<KB_TC_KIND, 256, true>(plan, p, stream);
     }
-    return plan.block_n == 256 ? launch_one<KB_TC_KIND, 256, false>(plan, p, stream)
+    return plan.block_n > 128 ? launch_one<KB_TC_KIND, 256, false>(plan, p, stream)
                                : launch_one<KB_TC_KIND, 128, false>(plan, p, stream);
 }
 

@@ -50,7 +50,8 @@ constexpr int kWarpStageBytes = 32 * 128;  // per epilogue warp: 32 rows x 128 b
 // after the stage ring: barriers and flags (256 bytes), the bias slices; then, if present, the output staging
 constexpr int kTailBytes = 256 + kEpiWarps * kWarpBiasFloats * 4;
 constexpr int kStagingBytes = kEpiWarps * kWarpStageBytes;  // only launches with output mirrors carry it (one stage less)
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 12;
+constexpr int kSmemLimit = 232448;  // bytes of shared memory a CTA can have
 
 struct TcParams {
     EpiParams epi;
@@ -63,6 +64,14 @@ struct TcParams {
     // each contracts over kb_per_split k-blocks, and the partial tiles are added through distributed shared memory
     int splits, kb_per_split;
     int stages;  // depth of the shared-memory ring
+    // Tile width (columns of the output, rows of the weight operand per k-block and tile; at most the kBN of the kernel)
+    // and the rows of the activation operand a k-block brings in.  With fewer than 128 rows of activations the copy is
+    // cut to them: the MMA still multiplies 128 rows, the rest being whatever follows in the ring, and the accumulator
+    // rows that come of it are never read.
+    int bn, a_rows;
+    int ring_bytes;  // bytes in front of the barriers: the stage ring, and room for one tile as fp32 if it is finished from there
+    int via_smem;    // one work item per CTA, finished from shared memory (finish_rows)
+    int vector_rows;  // every row of the epilogue's tensors can be read and written 16 bytes at a time, beta = 0
     int group_m;  // tile rows per raster group: consecutive work items walk down group_m tile rows, then one tile right
     // CTA pairs: work items [0, narrow_from) are whole 256 x BN tiles; each later tile is two items of half the width,
     // so that a last wave that would keep fewer than half the pairs busy is spread over twice as many
@@ -86,6 +95,30 @@ struct TcParams {
     int epi_warps;
 };
 
+
+// The epilogue's tensors for the current batch entry.  Everything else about them is read from the kernel's parameters
+// themselves: a reference that may also name a copy on the stack turns every such read into a load through a generic
+// address, which cost half of the time of an epilogue pass.
+struct EpiTensors {
+    void *c;
+    const void *bias;
+    const void *res;
+    void *out;
+};
+
+__device__ __forceinline__ EpiTensors epi_tensors(const TcParams &p, int batch)
+{
+    EpiTensors t = {p.epi.c, p.epi.bias, p.epi.res, p.epi.out};
+    if (p.batch > 1) {
+        long long idx[3];
+        batch_decompose(p.bp, batch, idx);
+        t.c = offset_ptr(t.c, p.epi.c_dtype, batch_offset(p.bp.c_sb, idx));
+        t.bias = offset_ptr(t.bias, p.epi.bias_dtype, batch_offset(p.bp.bias_sb, idx));
+        t.res = offset_ptr(t.res, p.epi.res_dtype, batch_offset(p.bp.res_sb, idx));
+        t.out = offset_ptr(t.out, p.epi.out_dtype, batch_offset(p.bp.out_sb, idx));
+    }
+    return t;
+}
 
 // ---- epilogue side-input / output access, 8 consecutive columns at a time ---------------------------------
 
@@ -179,7 +212,7 @@ __device__ __forceinline__ bool vec_ok(const void *base, int dtype, long long id
 // independent dependency chains: with three epilogue warps per scheduler, instruction-level parallelism is what
 // hides the arithmetic latency.
 template <int kAct, int kPrecise>
-__device__ __forceinline__ void epilogue_group8(const EpiParams &e, const uint32_t (&raw)[8], long long mi, long long ni)
+__device__ __forceinline__ void epilogue_group8(const EpiParams &e, const EpiTensors &t, const uint32_t (&raw)[8], long long mi, long long ni)
 {
     const int valid = (e.n - ni >= 8) ? 8 : static_cast<int>(e.n - ni);
     if (valid <= 0) {
@@ -193,9 +226,9 @@ __device__ __forceinline__ void epilogue_group8(const EpiParams &e, const uint32
         v[j] = e.alpha * __uint_as_float(raw[j]);
     }
     const long long ic = mi * e.c_sm + ni * e.c_sn;
-    const bool c_vec = full8 && vec_ok(e.c, ct, ic, e.c_sn);
+    const bool c_vec = full8 && vec_ok(t.c, ct, ic, e.c_sn);
     if (e.beta != 0.0f) {
-        load8(e.c, ct, ic, e.c_sn, c_vec, valid, side);
+        load8(t.c, ct, ic, e.c_sn, c_vec, valid, side);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             v[j] += e.beta * side[j];
@@ -203,7 +236,7 @@ __device__ __forceinline__ void epilogue_group8(const EpiParams &e, const uint32
     }
     if (e.has_bias) {
         const long long ib = mi * e.bias_sm + ni * e.bias_sn;
-        load8(e.bias, e.bias_dtype, ib, e.bias_sn, full8 && vec_ok(e.bias, e.bias_dtype, ib, e.bias_sn), valid, side);
+        load8(t.bias, e.bias_dtype, ib, e.bias_sn, full8 && vec_ok(t.bias, e.bias_dtype, ib, e.bias_sn), valid, side);
     }
     if (e.half_chain != 0) {
 #pragma unroll
@@ -266,15 +299,15 @@ __device__ __forceinline__ void epilogue_group8(const EpiParams &e, const uint32
             }
         }
     }
-    if (e.c != nullptr) {
-        store8(e.c, ct, ic, e.c_sn, c_vec, valid, v);
+    if (t.c != nullptr) {
+        store8(t.c, ct, ic, e.c_sn, c_vec, valid, v);
         for (int i = 0; i < e.n_mirrors; ++i) {
-            store8(static_cast<char *>(e.c) + e.c_delta[i], ct, ic, e.c_sn, c_vec, valid, v);
+            store8(static_cast<char *>(t.c) + e.c_delta[i], ct, ic, e.c_sn, c_vec, valid, v);
         }
     }
     if (e.res_op != KUDNN_B200_RES_NONE) {
         const long long ir = mi * e.res_sm + ni * e.res_sn;
-        load8(e.res, e.res_dtype, ir, e.res_sn, full8 && vec_ok(e.res, e.res_dtype, ir, e.res_sn), valid, side);
+        load8(t.res, e.res_dtype, ir, e.res_sn, full8 && vec_ok(t.res, e.res_dtype, ir, e.res_sn), valid, side);
         if (e.res_op == KUDNN_B200_RES_IDENTICAL) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -304,10 +337,10 @@ __device__ __forceinline__ void epilogue_group8(const EpiParams &e, const uint32
             }
         }
         const long long io = mi * e.out_sm + ni * e.out_sn;
-        const bool out_vec = full8 && vec_ok(e.out, ot, io, e.out_sn);
-        store8(e.out, ot, io, e.out_sn, out_vec, valid, v);
+        const bool out_vec = full8 && vec_ok(t.out, ot, io, e.out_sn);
+        store8(t.out, ot, io, e.out_sn, out_vec, valid, v);
         for (int i = 0; i < e.n_mirrors; ++i) {
-            store8(static_cast<char *>(e.out) + e.out_delta[i], ot, io, e.out_sn, out_vec, valid, v);
+            store8(static_cast<char *>(t.out) + e.out_delta[i], ot, io, e.out_sn, out_vec, valid, v);
         }
     }
 }
@@ -389,43 +422,124 @@ __device__ __forceinline__ void round_rne8(float (&v)[8])
     }
 }
 
-// Arithmetic of the fast form of epilogue_group8 (beta == 0, side inputs contiguous along the row and 16-byte
-// aligned at this group, all 8 columns in range), first half: v receives the 8 values of c, exactly representable
-// in c's type.
-// kDt: element type of c, bias, res and out when they all equal the kernel's input type (the common case: every
-// type test below is then decided at compile time), or -1 when the types are read from the descriptor.
-template <int kAct, int kDt>
-__device__ __forceinline__ void compute_c8_fast(const EpiParams &e, const uint32_t (&raw)[8], const RowPointers &rp,
-                                                int byte_off_bias, int g, float (&v)[8])
+// ---- the chain on packed 16-bit values: the element type is kDt throughout, two values share a register wherever they are
+// exact in it, and a rounding is one conversion per pair.  Same arithmetic as chain8 / combine8.
+template <int kDt>
+__device__ __forceinline__ uint4 pack8_rne(const float (&v)[8])
 {
-    const int ct = kDt > 0 ? kDt : e.c_dtype;
-    float side[8];
+    unsigned w[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        v[j] = __uint_as_float(raw[j]);
-    }
-    if (e.alpha != 1.0f) {  // multiplying by exactly 1 changes nothing, so the common case skips the pass
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            v[j] *= e.alpha;
+    for (int j = 0; j < 4; ++j) {
+        if (kDt == KUDNN_B200_BF16) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            w[j] = *reinterpret_cast<const unsigned *>(&h);
+        } else {
+            const __half2 h = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+            w[j] = *reinterpret_cast<const unsigned *>(&h);
         }
     }
-    if (rp.bias_mode == 3) {
-        const float4 b0 = *reinterpret_cast<const float4 *>(rp.bias_smem + g * 8);
-        const float4 b1 = *reinterpret_cast<const float4 *>(rp.bias_smem + g * 8 + 4);
-        side[0] = b0.x; side[1] = b0.y; side[2] = b0.z; side[3] = b0.w;
-        side[4] = b1.x; side[5] = b1.y; side[6] = b1.z; side[7] = b1.w;
-    } else if (rp.bias_mode == 1) {
-        load8_vec(rp.bias + byte_off_bias, kDt > 0 ? kDt : e.bias_dtype, side);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <int kDt>
+__device__ __forceinline__ void unpack8(const uint4 &p, float (&v)[8])
+{
+    const unsigned w[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (kDt == KUDNN_B200_BF16) {
+            v[2 * j] = __uint_as_float(w[j] << 16);
+            v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+        } else {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[j]));
+            v[2 * j] = f.x;
+            v[2 * j + 1] = f.y;
+        }
+    }
+}
+
+template <int kAct, int kDt>
+__device__ __forceinline__ uint4 chain8_packed(const EpiParams &e, bool has_bias, const float (&side)[8], float (&v)[8])
+{
+    uint4 w;
+    if (kDt == KUDNN_B200_F16 && e.half_chain != 0) {
+        w = pack8_rne<kDt>(v);
+        if (has_bias) {
+            unpack8<kDt>(w, v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] += side[j];
+            }
+            w = pack8_rne<kDt>(v);
+        }
+    } else {
+        if (has_bias) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] += side[j];
+            }
+        }
+        w = pack8_rne<kDt>(v);
+    }
+    if (kAct == KUDNN_B200_ACT_NONE) {
+        return w;
+    }
+    unpack8<kDt>(w, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        v[j] = activation<false>(v[j], kAct, e.act_alpha);
+    }
+    if (kDt == KUDNN_B200_F16) {
+        return pack8_rne<kDt>(v);
+    }
+    if (kAct == KUDNN_B200_ACT_RELU && e.act_alpha != 0.0f) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = relu_bf16_overflow(v[j]);
+        }
+    }
+    // bf16: the upper halves of two values as they are
+    return make_uint4(__byte_perm(__float_as_uint(v[0]), __float_as_uint(v[1]), 0x7632),
+                      __byte_perm(__float_as_uint(v[2]), __float_as_uint(v[3]), 0x7632),
+                      __byte_perm(__float_as_uint(v[4]), __float_as_uint(v[5]), 0x7632),
+                      __byte_perm(__float_as_uint(v[6]), __float_as_uint(v[7]), 0x7632));
+}
+
+template <int kDt>
+__device__ __forceinline__ uint4 combine8_packed(const EpiParams &e, const uint4 &c, const uint4 &res)
+{
+    float v[8], side[8];
+    unpack8<kDt>(c, v);
+    unpack8<kDt>(res, side);
+    if (e.res_op == KUDNN_B200_RES_IDENTICAL) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] += side[j];
+        }
+    } else if (e.res_op == KUDNN_B200_RES_EXT) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = fmaf(side[j], e.gamma, v[j]);
+        }
     } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            side[j] = rp.bias_scalar;
+            v[j] *= side[j];
         }
     }
+    return pack8_rne<kDt>(v);
+}
+
+// The post-GEMM chain up to c for 8 values: v holds accumulators and receives values exactly representable in c's type.
+// kDt: element type of c, bias, res and out when they all equal the kernel's input type (the common case: every
+// type test below is then decided at compile time), or -1 when the types are read from the descriptor.
+template <int kAct, int kDt>
+__device__ __forceinline__ void chain8(const EpiParams &e, bool has_bias, const float (&side)[8], float (&v)[8])
+{
+    const int ct = kDt > 0 ? kDt : e.c_dtype;
     if (ct == KUDNN_B200_F16 && e.half_chain != 0) {
         round_rne8<KUDNN_B200_F16>(v);
-        if (rp.bias_mode != 0) {
+        if (has_bias) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 v[j] += side[j];
@@ -433,7 +547,7 @@ __device__ __forceinline__ void compute_c8_fast(const EpiParams &e, const uint32
             round_rne8<KUDNN_B200_F16>(v);
         }
     } else {
-        if (rp.bias_mode != 0) {
+        if (has_bias) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 v[j] += side[j];
@@ -475,12 +589,51 @@ __device__ __forceinline__ void compute_c8_fast(const EpiParams &e, const uint32
     }
 }
 
-// Second half: v holds the values of c and is replaced by those of the second output (c (+) res).
+// The accumulators of a group (times alpha) and its bias values.
 template <int kDt>
-__device__ __forceinline__ void compute_out8_fast(const EpiParams &e, const RowPointers &rp, int byte_off_res, float (&v)[8])
+__device__ __forceinline__ void fetch_c8(const EpiParams &e, const uint32_t (&raw)[8], const RowPointers &rp, int byte_off_bias,
+                                         int g, float (&v)[8], float (&side)[8])
+{
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        v[j] = __uint_as_float(raw[j]);
+    }
+    if (e.alpha != 1.0f) {  // multiplying by exactly 1 changes nothing, so the common case skips the pass
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] *= e.alpha;
+        }
+    }
+    if (rp.bias_mode == 3) {
+        const float4 b0 = *reinterpret_cast<const float4 *>(rp.bias_smem + g * 8);
+        const float4 b1 = *reinterpret_cast<const float4 *>(rp.bias_smem + g * 8 + 4);
+        side[0] = b0.x; side[1] = b0.y; side[2] = b0.z; side[3] = b0.w;
+        side[4] = b1.x; side[5] = b1.y; side[6] = b1.z; side[7] = b1.w;
+    } else if (rp.bias_mode == 1) {
+        load8_vec(rp.bias + byte_off_bias, kDt > 0 ? kDt : e.bias_dtype, side);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            side[j] = rp.bias_scalar;
+        }
+    }
+}
+
+// Arithmetic of the fast form of epilogue_group8 (beta == 0, side inputs contiguous along the row and 16-byte
+// aligned at this group, all 8 columns in range), first half: v receives the 8 values of c.
+template <int kAct, int kDt>
+__device__ __forceinline__ void compute_c8_fast(const EpiParams &e, const uint32_t (&raw)[8], const RowPointers &rp,
+                                                int byte_off_bias, int g, float (&v)[8])
 {
     float side[8];
-    load8_vec(rp.res + byte_off_res, kDt > 0 ? kDt : e.res_dtype, side);
+    fetch_c8<kDt>(e, raw, rp, byte_off_bias, g, v, side);
+    chain8<kAct, kDt>(e, rp.bias_mode != 0, side, v);
+}
+
+// Second half: v holds the values of c and is replaced by those of the second output (c (+) res).
+template <int kDt>
+__device__ __forceinline__ void combine8(const EpiParams &e, const float (&side)[8], float (&v)[8])
+{
     if (e.res_op == KUDNN_B200_RES_IDENTICAL) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -503,6 +656,14 @@ __device__ __forceinline__ void compute_out8_fast(const EpiParams &e, const RowP
     } else if (ot == KUDNN_B200_BF16) {
         round_rne8<KUDNN_B200_BF16>(v);
     }
+}
+
+template <int kDt>
+__device__ __forceinline__ void compute_out8_fast(const EpiParams &e, const RowPointers &rp, int byte_off_res, float (&v)[8])
+{
+    float side[8];
+    load8_vec(rp.res + byte_off_res, kDt > 0 ? kDt : e.res_dtype, side);
+    combine8<kDt>(e, side, v);
 }
 
 // Fast form of epilogue_group8: same arithmetic, no address arithmetic beyond pointer bumps, one 16-byte (fp32: two)
@@ -576,6 +737,15 @@ __device__ __forceinline__ uint4 epilogue_group8_packed(const EpiParams &e, cons
                                                         int byte_off_bias, int byte_off_res, int g)
 {
     float v[8];
+    if constexpr (kDt == KUDNN_B200_F16 || kDt == KUDNN_B200_BF16) {
+        float side[8];
+        fetch_c8<kDt>(e, raw, rp, byte_off_bias, g, v, side);
+        uint4 w = chain8_packed<kAct, kDt>(e, rp.bias_mode != 0, side, v);
+        if (rp.c == nullptr) {
+            w = combine8_packed<kDt>(e, w, *reinterpret_cast<const uint4 *>(rp.res + byte_off_res));
+        }
+        return w;
+    }
     compute_c8_fast<kAct, kDt>(e, raw, rp, byte_off_bias, g, v);
     int dt = kDt > 0 ? kDt : e.c_dtype;
     if (rp.c == nullptr) {
@@ -680,7 +850,7 @@ __device__ __noinline__ void epilogue_rows_coalesced(const EpiParams &e, uint32_
 // Row-base pointers for the vector path of the epilogue.  Returns whether that path applies to the `groups` groups
 // of 8 columns starting at (mi, n0): whole groups inside n, no beta term, every tensor involved contiguous along n
 // and 16-byte aligned there.
-__device__ __forceinline__ bool setup_row_pointers(const EpiParams &e, bool row_ok, long long mi, long long n0, int groups,
+__device__ __forceinline__ bool setup_row_pointers(const EpiParams &e, const EpiTensors &t, bool row_ok, long long mi, long long n0, int groups,
                                                    RowPointers &rp)
 {
     rp.c = nullptr;
@@ -692,43 +862,43 @@ __device__ __forceinline__ bool setup_row_pointers(const EpiParams &e, bool row_
     rp.bias_smem = nullptr;
     bool fast = row_ok && e.beta == 0.0f && (n0 + static_cast<long long>(groups) * 8 <= e.n);
     if (fast) {
-        if (e.c != nullptr) {
+        if (t.c != nullptr) {
             const long long ic = mi * e.c_sm + n0 * e.c_sn;
-            fast = fast && row_contiguous_aligned(e.c, e.c_dtype, ic, e.c_sn);
-            rp.c = static_cast<char *>(e.c) + ic * dtype_size(e.c_dtype);
+            fast = fast && row_contiguous_aligned(t.c, e.c_dtype, ic, e.c_sn);
+            rp.c = static_cast<char *>(t.c) + ic * dtype_size(e.c_dtype);
         }
         if (e.has_bias) {
             const long long ib = mi * e.bias_sm + n0 * e.bias_sn;
             if (e.bias_sn == 0) {
                 rp.bias_mode = 2;
-                rp.bias_scalar = load_as_f32(e.bias, e.bias_dtype, ib);
+                rp.bias_scalar = load_as_f32(t.bias, e.bias_dtype, ib);
             } else {
                 rp.bias_mode = 1;
-                fast = fast && row_contiguous_aligned(e.bias, e.bias_dtype, ib, e.bias_sn);
-                rp.bias = static_cast<const char *>(e.bias) + ib * dtype_size(e.bias_dtype);
+                fast = fast && row_contiguous_aligned(t.bias, e.bias_dtype, ib, e.bias_sn);
+                rp.bias = static_cast<const char *>(t.bias) + ib * dtype_size(e.bias_dtype);
             }
         }
         if (e.res_op != KUDNN_B200_RES_NONE) {
             const long long ir = mi * e.res_sm + n0 * e.res_sn;
             const long long io = mi * e.out_sm + n0 * e.out_sn;
-            fast = fast && row_contiguous_aligned(e.res, e.res_dtype, ir, e.res_sn) &&
-                   row_contiguous_aligned(e.out, e.out_dtype, io, e.out_sn);
-            rp.res = static_cast<const char *>(e.res) + ir * dtype_size(e.res_dtype);
-            rp.out = static_cast<char *>(e.out) + io * dtype_size(e.out_dtype);
+            fast = fast && row_contiguous_aligned(t.res, e.res_dtype, ir, e.res_sn) &&
+                   row_contiguous_aligned(t.out, e.out_dtype, io, e.out_sn);
+            rp.res = static_cast<const char *>(t.res) + ir * dtype_size(e.res_dtype);
+            rp.out = static_cast<char *>(t.out) + io * dtype_size(e.out_dtype);
         }
     }
     return fast;
 }
 
 template <int kAct, int kDt>
-__device__ __forceinline__ void epilogue_row(const EpiParams &e, uint32_t taddr, bool row_ok, long long mi, long long n0,
+__device__ __forceinline__ void epilogue_row(const EpiParams &e, const EpiTensors &t, uint32_t taddr, bool row_ok, long long mi, long long n0,
                                              int groups, const float *staged_bias, unsigned char *stage, int lane)
 {
     if (groups <= 0) {
         return;
     }
     RowPointers rp;
-    const bool fast = setup_row_pointers(e, row_ok, mi, n0, groups, rp);
+    const bool fast = setup_row_pointers(e, t, row_ok, mi, n0, groups, rp);
     if (staged_bias != nullptr && rp.bias_mode == 1) {
         rp.bias_mode = 3;
         rp.bias_smem = staged_bias;
@@ -778,21 +948,21 @@ __device__ __forceinline__ void epilogue_row(const EpiParams &e, uint32_t taddr,
         } else if (fast) {
             epilogue_group8_fast<kAct, kDt>(e, cur, rp, g * step_c, g * step_bias, g * step_res, g * step_out, g);
         } else if (row_ok) {
-            epilogue_group8<kAct, (kDt < 0 ? -1 : (kDt == KUDNN_B200_F32 ? 1 : 0))>(e, cur, mi, n0 + g * 8);
+            epilogue_group8<kAct, (kDt < 0 ? -1 : (kDt == KUDNN_B200_F32 ? 1 : 0))>(e, t, cur, mi, n0 + g * 8);
         }
     }
 }
 
 // 8-bit integer products: the accumulator holds exact 32-bit sums; c = acc (+ bias, 32-bit integers), clamped to the
 // 32-bit range like the general kernel does.  alpha = 1 and beta = 0 (the host sends anything else elsewhere).
-__device__ __forceinline__ void epilogue_row_int(const EpiParams &e, uint32_t taddr, bool row_ok, long long mi, long long n0,
+__device__ __forceinline__ void epilogue_row_int(const EpiParams &e, const EpiTensors &t, uint32_t taddr, bool row_ok, long long mi, long long n0,
                                                  int groups)
 {
     if (groups <= 0) {
         return;
     }
-    int *crow = static_cast<int *>(e.c) + (row_ok ? mi * e.c_sm + n0 * e.c_sn : 0);
-    const int *brow = e.has_bias ? static_cast<const int *>(e.bias) + (row_ok ? mi * e.bias_sm + n0 * e.bias_sn : 0) : nullptr;
+    int *crow = static_cast<int *>(t.c) + (row_ok ? mi * e.c_sm + n0 * e.c_sn : 0);
+    const int *brow = e.has_bias ? static_cast<const int *>(t.bias) + (row_ok ? mi * e.bias_sm + n0 * e.bias_sn : 0) : nullptr;
     const bool vec = row_ok && e.c_sn == 1 && (reinterpret_cast<uintptr_t>(crow) & 15u) == 0;
     uint32_t next[8], cur[8];
     tmem_load_8_issue(taddr, next);
@@ -864,14 +1034,13 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_smem_addr, uint32
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "r"(remote)
-                 : "memory");
+                 : "r"(remote));
     return v;
 }
 
 // Copies `groups` groups of 8 accumulator columns of this thread's row from TMEM to `dst` (shared memory).  The
 // loads are issued three groups at a time before the wait.
-__device__ __forceinline__ void dump_partial_row(uint32_t taddr, float *dst, int groups)
+__device__ __forceinline__ void dump_partial_row(uint32_t taddr, float *dst, int groups, bool row_ok)
 {
     for (int g0 = 0; g0 < groups; g0 += 3) {
         uint32_t r[3][8];
@@ -886,61 +1055,364 @@ __device__ __forceinline__ void dump_partial_row(uint32_t taddr, float *dst, int
         for (int u = 0; u < 3; ++u) {
             if (g0 + u < groups) {
                 tmem_load_wait(r[u]);
-                float4 *out = reinterpret_cast<float4 *>(dst + (g0 + u) * 8);
-                out[0] = make_float4(__uint_as_float(r[u][0]), __uint_as_float(r[u][1]), __uint_as_float(r[u][2]),
-                                     __uint_as_float(r[u][3]));
-                out[1] = make_float4(__uint_as_float(r[u][4]), __uint_as_float(r[u][5]), __uint_as_float(r[u][6]),
-                                     __uint_as_float(r[u][7]));
+                if (row_ok) {
+                    float4 *out = reinterpret_cast<float4 *>(dst + (g0 + u) * 8);
+                    out[0] = make_float4(__uint_as_float(r[u][0]), __uint_as_float(r[u][1]), __uint_as_float(r[u][2]),
+                                         __uint_as_float(r[u][3]));
+                    out[1] = make_float4(__uint_as_float(r[u][4]), __uint_as_float(r[u][5]), __uint_as_float(r[u][6]),
+                                         __uint_as_float(r[u][7]));
+                }
             }
         }
     }
 }
 
-// The epilogue threads of cluster rank `rank` finish rows [rank * 128 / splits, (rank + 1) * 128 / splits) of the tile.
-template <int kAct, int kDt, int kBN>
-__device__ __forceinline__ void finish_split_rows(const EpiParams &e, const float *part, int splits, uint32_t rank, int tm,
-                                                  int tn, int m, int n, int epi_tid)
+__device__ __forceinline__ float ld_cluster_f1(uint32_t local_smem_addr, uint32_t rank)
 {
-    constexpr int kPitch = kBN + 4;
-    constexpr int kGroups = kBN / 8;
-    const int rows_per = kBM / splits;
-    const uint32_t part_addr = smem_u32(part);
-    for (int u = epi_tid; u < rows_per * kGroups; u += kEpiWarps * 32) {
-        const int r_local = u / kGroups, g = u - r_local * kGroups;
-        const int row = static_cast<int>(rank) * rows_per + r_local;
-        const long long mi = static_cast<long long>(tm) * kBM + row;
-        const long long ni = static_cast<long long>(tn) * kBN + g * 8;
-        if (mi >= m || ni >= n) {
-            continue;
-        }
-        const uint32_t addr = part_addr + static_cast<uint32_t>((row * kPitch + g * 8) * 4);
-        float4 lo[kMaxSplits], hi[kMaxSplits];
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_smem_addr), "r"(rank));
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote));
+    return v;
+}
+
+// v = the 8 values at this place of the tile, added over the ranks' shared memories in rank order.
+__device__ __forceinline__ void add_ranks(uint32_t addr, int splits, float (&v)[8])
+{
+    float4 lo[kMaxSplits], hi[kMaxSplits];
 #pragma unroll
-        for (int s = 0; s < kMaxSplits; ++s) {
-            if (s < splits) {
-                lo[s] = ld_cluster_f4(addr, static_cast<uint32_t>(s));
-                hi[s] = ld_cluster_f4(addr + 16, static_cast<uint32_t>(s));
+    for (int s = 0; s < kMaxSplits; ++s) {
+        if (s < splits) {
+            lo[s] = ld_cluster_f4(addr, static_cast<uint32_t>(s));
+            hi[s] = ld_cluster_f4(addr + 16, static_cast<uint32_t>(s));
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        v[j] = 0.0f;
+    }
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s) {
+        if (s < splits) {
+            v[0] += lo[s].x; v[1] += lo[s].y; v[2] += lo[s].z; v[3] += lo[s].w;
+            v[4] += hi[s].x; v[5] += hi[s].y; v[6] += hi[s].z; v[7] += hi[s].w;
+        }
+    }
+}
+
+__device__ __forceinline__ void ld_tile8(uint32_t addr, float (&v)[8])
+{
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(addr + 16));
+}
+
+// ---- finishing a tile that lies in shared memory as fp32: one CTA's own, or the partial tiles of a cluster, added in rank
+// order.  Rank `rank` of the cluster takes `rows` rows from row0.  Bound by the instructions of the chain and by the remote
+// reads (about 25 bytes per ns and SM): threads of a row hold neighbouring groups of 8 columns, so that all accesses of a
+// warp are contiguous, and a thread keeps its columns (and their bias) and walks down the rows.  Against one thread per row
+// straight from the accumulator, kernel times: 60 x 2560 x 1024 16.4 -> 10.1 us, 333 x 3008 x 2056 with GELU 33 -> 16 us,
+// with rows that start anywhere (n = 3001) 46 -> 19 us.
+
+// Any element types; rows of 16-byte vectors; both outputs, mirrors and alpha as they come.
+template <int kAct, int kDt>
+__device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTensors &t, const float *part, int bn, int splits,
+                                                int row0, int rows, int tm, int tn, int n, int tid)
+{
+    const int groups = bn / 8;
+    const int step = kEpiWarps * 32 / groups;  // rows the CTA covers per pass
+    int r = tid / groups;
+    const int g = tid - r * groups;
+    const int ni = tn * bn + g * 8;
+    if (r >= step || ni >= n) {
+        return;
+    }
+    const int ct = kDt > 0 ? kDt : e.c_dtype, bt = kDt > 0 ? kDt : e.bias_dtype;
+    const int rt = kDt > 0 ? kDt : e.res_dtype, ot = kDt > 0 ? kDt : e.out_dtype;
+    const long long m0 = static_cast<long long>(tm) * kBM + row0 + r;
+    // byte addresses of this thread's piece of the row, and their advance per pass
+    char *c = t.c == nullptr ? nullptr : static_cast<char *>(t.c) + (m0 * e.c_sm + ni) * dtype_size(ct);
+    const bool second = e.res_op != KUDNN_B200_RES_NONE;
+    const char *res = static_cast<const char *>(t.res) + (m0 * e.res_sm + ni) * dtype_size(rt);
+    char *out = static_cast<char *>(t.out) + (m0 * e.out_sm + ni) * dtype_size(ot);
+    const long long c_step = e.c_sm * dtype_size(ct) * step;
+    const long long res_step = e.res_sm * dtype_size(rt) * step, out_step = e.out_sm * dtype_size(ot) * step;
+    const bool has_bias = e.has_bias != 0;
+    float side[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    auto fetch_bias = [&](long long mi) {
+        const char *bias = static_cast<const char *>(t.bias) + (mi * e.bias_sm + (e.bias_sn != 0 ? ni : 0)) * dtype_size(bt);
+        if (e.bias_sn != 0) {
+            load8_vec(bias, bt, side);
+        } else {
+            const float b = load_as_f32(bias, bt, 0);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                side[j] = b;
             }
         }
-        float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    };
+    if (has_bias && e.bias_sm == 0) {
+        fetch_bias(0);
+    }
+    const int pitch = (bn + 4) * 4;
+    uint32_t addr = smem_u32(part) + static_cast<uint32_t>((row0 + r) * pitch + g * 32);
+    for (long long mi = m0; r < rows; r += step, mi += step) {
+        float v[8];
+        if (splits == 1) {
+            ld_tile8(addr, v);
+        } else {
+            add_ranks(addr, splits, v);
+        }
+        addr += static_cast<uint32_t>(step * pitch);
+        float rs[8];
+        if (second) {
+            load8_vec(res, rt, rs);
+            res += res_step;
+        }
+        if (has_bias && e.bias_sm != 0) {
+            fetch_bias(mi);
+        }
+        if (e.alpha != 1.0f) {
 #pragma unroll
-        for (int s = 0; s < kMaxSplits; ++s) {
-            if (s < splits) {
-                acc[0] += lo[s].x; acc[1] += lo[s].y; acc[2] += lo[s].z; acc[3] += lo[s].w;
-                acc[4] += hi[s].x; acc[5] += hi[s].y; acc[6] += hi[s].z; acc[7] += hi[s].w;
+            for (int j = 0; j < 8; ++j) {
+                v[j] *= e.alpha;
             }
         }
-        uint32_t raw[8];
+        chain8<kAct, kDt>(e, has_bias, side, v);
+        if (c != nullptr) {
+            store8_vec(c, ct, v);
+            for (int i = 0; i < e.n_mirrors; ++i) {
+                store8_vec(c + e.c_delta[i], ct, v);
+            }
+            c += c_step;
+        }
+        if (second) {
+            combine8<kDt>(e, rs, v);
+            store8_vec(out, ot, v);
+            for (int i = 0; i < e.n_mirrors; ++i) {
+                store8_vec(out + e.out_delta[i], ot, v);
+            }
+            out += out_step;
+        }
+    }
+}
+
+// The usual case: 16-bit types throughout, one output (kSecond: out, else c), alpha = 1, beta = 0, a bias that is the same for
+// every row, no mirrors.  kRagged: the rows are contiguous but start anywhere; the finished values go back to this thread's
+// place in shared memory and leave from there, every store instruction covering 128 consecutive bytes of a row.
+template <int kAct, int kDt, bool kSecond, bool kSplit, bool kRagged>
+__device__ __forceinline__ void finish_rows_lean(const EpiParams &e, const EpiTensors &t, float *part, int bn, int splits,
+                                                 int row0, int rows, int tm, int tn, int n, int tid)
+{
+    const int groups = bn / 8;
+    const int step = kEpiWarps * 32 / groups;  // rows the CTA covers per pass
+    int r = tid / groups;
+    const int g = tid - r * groups;
+    const int ni = tn * bn + g * 8;
+    const int valid = n - ni < 8 ? n - ni : 8;
+    const bool works = r < step && valid > 0;
+    const long long m0 = static_cast<long long>(tm) * kBM + row0;
+    const int pitch = (bn + 4) * 4;
+    char *dst = kSecond ? static_cast<char *>(t.out) : static_cast<char *>(t.c);
+    const long long dst_pitch = (kSecond ? e.out_sm : e.c_sm) * 2;
+    if (works) {
+        const bool has_bias = e.has_bias != 0;
+        float side[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (has_bias) {
+            if (e.bias_sn == 1 && !kRagged) {
+                load8_vec(static_cast<const char *>(t.bias) + static_cast<long long>(ni) * 2, kDt, side);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    side[j] = j < valid ? load_as_f32(t.bias, kDt, (ni + j) * e.bias_sn) : 0.0f;
+                }
+            }
+        }
+        const char *res = static_cast<const char *>(t.res) + ((m0 + r) * e.res_sm + ni) * 2;
+        char *piece = dst + (m0 + r) * dst_pitch + static_cast<long long>(ni) * 2;
+        const long long res_step = e.res_sm * 2 * step, piece_step = dst_pitch * step;
+        uint32_t addr = smem_u32(part) + static_cast<uint32_t>((row0 + r) * pitch + g * 32);
+#pragma unroll 2
+        for (; r < rows; r += step) {
+            uint4 rs = make_uint4(0u, 0u, 0u, 0u);
+            if (kSecond && !kRagged) {
+                rs = *reinterpret_cast<const uint4 *>(res);
+            } else if (kSecond) {
+                unsigned h[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    h[j] = j < valid ? reinterpret_cast<const unsigned short *>(res)[j] : 0u;
+                }
+                rs = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+            }
+            res += res_step;
+            float v[8];
+            if (kSplit) {
+                add_ranks(addr, splits, v);
+            } else {
+                ld_tile8(addr, v);
+            }
+            uint4 w = chain8_packed<kAct, kDt>(e, has_bias, side, v);
+            if (kSecond) {
+                w = combine8_packed<kDt>(e, w, rs);
+            }
+            if (kRagged) {
+                // rows row0 .. row0 + rows of this CTA's copy are read by this rank alone, and these 32 bytes by this thread
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+            } else {
+                *reinterpret_cast<uint4 *>(piece) = w;
+                piece += piece_step;
+            }
+            addr += static_cast<uint32_t>(step * pitch);
+        }
+    }
+    if (kRagged) {
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+        const int left = n - tn * bn;
+        const int cols = left < bn ? left : bn;
+        const unsigned char *tile = reinterpret_cast<const unsigned char *>(part) + row0 * pitch;
+        auto value = [&](int row, int col) {
+            return static_cast<unsigned>(*reinterpret_cast<const unsigned short *>(tile + row * pitch + (col >> 3) * 32 + (col & 7) * 2));
+        };
+        for (int row = tid >> 5; row < rows; row += kEpiWarps) {
+            unsigned short *line = reinterpret_cast<unsigned short *>(dst + (m0 + row) * dst_pitch) + static_cast<long long>(tn) * bn;
+            const int head = static_cast<int>((reinterpret_cast<uintptr_t>(line) >> 1) & 1u);  // columns before a 4-byte boundary
+            if ((tid & 31) < head) {
+                line[0] = static_cast<unsigned short>(value(row, 0));
+            }
+            for (int col = head + 2 * (tid & 31); col < cols; col += 64) {
+                if (col + 1 < cols) {
+                    *reinterpret_cast<unsigned *>(line + col) = value(row, col) | (value(row, col + 1) << 16);
+                } else {
+                    line[col] = static_cast<unsigned short>(value(row, col));
+                }
+            }
+        }
+    }
+}
+
+// Everything else (any strides, beta): a warp takes a row and a lane the columns lane, lane + 32, ..., so that narrow accesses
+// of a warp are contiguous where the rows are.
+template <int kAct, int kDt>
+__device__ __forceinline__ void finish_rows_any(const EpiParams &e, const EpiTensors &t, const float *part, int bn, int splits,
+                                                int row0, int rows, int tm, int tn, int n, int tid)
+{
+    const int lane = tid & 31;
+    const int ct = kDt > 0 ? kDt : e.c_dtype, bt = kDt > 0 ? kDt : e.bias_dtype;
+    const int rt = kDt > 0 ? kDt : e.res_dtype, ot = kDt > 0 ? kDt : e.out_dtype;
+    const long long n0 = static_cast<long long>(tn) * bn + lane;
+    const int left = n - tn * bn;
+    const int cols = left < bn ? left : bn;  // columns of this tile that exist
+    const bool has_bias = e.has_bias != 0;
+    float side[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    auto fetch_bias = [&](long long mi) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            raw[j] = __float_as_uint(acc[j]);
+            if (lane + 32 * j < cols) {
+                side[j] = load_as_f32(t.bias, bt, mi * e.bias_sm + (n0 + 32 * j) * e.bias_sn);
+            }
         }
-        RowPointers rp;
-        if (setup_row_pointers(e, true, mi, ni, 1, rp)) {
-            epilogue_group8_fast<kAct, kDt>(e, raw, rp, 0, 0, 0, 0, 0);
-        } else {
-            epilogue_group8<kAct, (kDt < 0 ? -1 : (kDt == KUDNN_B200_F32 ? 1 : 0))>(e, raw, mi, ni);
+    };
+    if (has_bias && e.bias_sm == 0) {
+        fetch_bias(0);
+    }
+    const int pitch = (bn + 4) * 4;
+    for (int r = tid >> 5; r < rows; r += kEpiWarps) {
+        const long long mi = static_cast<long long>(tm) * kBM + row0 + r;
+        const uint32_t addr = smem_u32(part) + static_cast<uint32_t>((row0 + r) * pitch + lane * 4);
+        float v[8], rs[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = rs[j] = 0.0f;
         }
+        for (int s = 0; s < splits; ++s) {
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                x[j] = lane + 32 * j < cols ? ld_cluster_f1(addr + 128 * j, static_cast<uint32_t>(s)) : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] += x[j];
+            }
+        }
+        if (e.res_op != KUDNN_B200_RES_NONE) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (lane + 32 * j < cols) {
+                    rs[j] = load_as_f32(t.res, rt, mi * e.res_sm + (n0 + 32 * j) * e.res_sn);
+                }
+            }
+        }
+        if (has_bias && e.bias_sm != 0) {
+            fetch_bias(mi);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] *= e.alpha;
+        }
+        if (e.beta != 0.0f) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (lane + 32 * j < cols) {
+                    v[j] += e.beta * load_as_f32(t.c, ct, mi * e.c_sm + (n0 + 32 * j) * e.c_sn);
+                }
+            }
+        }
+        chain8<kAct, kDt>(e, has_bias, side, v);
+        if (t.c != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (lane + 32 * j < cols) {
+                    store_exact_mirrored(t.c, ct, mi * e.c_sm + (n0 + 32 * j) * e.c_sn, v[j], e.n_mirrors, e.c_delta);
+                }
+            }
+        }
+        if (e.res_op != KUDNN_B200_RES_NONE) {
+            combine8<kDt>(e, rs, v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (lane + 32 * j < cols) {
+                    store_exact_mirrored(t.out, ot, mi * e.out_sm + (n0 + 32 * j) * e.out_sn, v[j], e.n_mirrors, e.out_delta);
+                }
+            }
+        }
+    }
+}
+
+template <int kAct, int kDt>
+__device__ __forceinline__ void finish_rows(const EpiParams &e, const EpiTensors &t, bool vector_rows, float *part, int bn,
+                                            int splits, uint32_t rank, int tm, int tn, int m, int n, int tid)
+{
+    // the tile's rows, shared out evenly between the ranks
+    const int tile_rows = m - tm * kBM < kBM ? m - tm * kBM : kBM;
+    const int per_rank = (tile_rows + splits - 1) / splits;
+    const int row0 = static_cast<int>(rank) * per_rank;
+    const int rows = tile_rows - row0 < per_rank ? tile_rows - row0 : per_rank;
+    if constexpr (kDt == KUDNN_B200_F16 || kDt == KUDNN_B200_BF16) {
+        const bool second = e.res_op != KUDNN_B200_RES_NONE;
+        const bool contiguous = second ? e.out_sn == 1 && e.res_sn == 1 : e.c_sn == 1;
+        if (e.alpha == 1.0f && e.beta == 0.0f && e.n_mirrors == 0 && e.bias_sm == 0 && (t.c == nullptr) == second && contiguous) {
+#define KB_FINISH(SECOND, SPLIT, RAGGED) \
+    finish_rows_lean<kAct, kDt, SECOND, SPLIT, RAGGED>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid)
+            if (vector_rows) {
+                if (second) {
+                    splits > 1 ? KB_FINISH(true, true, false) : KB_FINISH(true, false, false);
+                } else {
+                    splits > 1 ? KB_FINISH(false, true, false) : KB_FINISH(false, false, false);
+                }
+            } else if (second) {
+                KB_FINISH(true, true, true);
+            } else {
+                KB_FINISH(false, true, true);
+            }
+#undef KB_FINISH
+            return;
+        }
+    }
+    if (vector_rows) {
+        finish_rows_vec<kAct, kDt>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
+    } else {
+        finish_rows_any<kAct, kDt>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
     }
 }
 
@@ -957,16 +1429,16 @@ __device__ __forceinline__ void decode_item(const TcParams &p, int item, int &ti
         batch = unit / p.num_tiles;
         tile = unit - batch * p.num_tiles;
         n_off = 0;
-        width = kBN;
+        width = p.bn;
     } else if (item < p.narrow_from) {
         tile = item;
         n_off = 0;
-        width = kBN;
+        width = p.bn;
     } else {
         const int j = item - p.narrow_from;
         tile = p.narrow_from + (j >> 1);
-        n_off = (j & 1) * (kBN / 2);
-        width = kBN / 2;
+        n_off = (j & 1) * (p.bn / 2);
+        width = p.bn / 2;
     }
 }
 
@@ -979,10 +1451,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     tc_linear_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                      const __grid_constant__ TcParams p)
 {
-    constexpr int kBRows = kPair ? kBN / 2 : kBN;  // rows of B this CTA loads per k-block
-    constexpr int kBBytes = kBRows * kStageRowBytes;
-    constexpr int kStageBytes = kABytes + kBBytes;
-    const int kStages = p.stages;  // 3-6, what fits beside the tail (and the output staging when mirrors are written)
+    // bytes of A, and of A and B, that this CTA loads per k-block
+    const int a_bytes = p.a_rows * kStageRowBytes;
+    const int stage_bytes = a_bytes + (kPair ? p.bn / 2 : p.bn) * kStageRowBytes;
+    const int kStages = p.stages;  // what fits beside the tail (and the output staging when mirrors are written)
     constexpr int kTmemCols = 2 * kBN;
     constexpr int kElemsPerRow = (kKind == KUDNN_B200_F32) ? 32 : (kKind == KUDNN_B200_S8 ? 128 : 64);  // per 128-byte k-block row
 
@@ -990,7 +1462,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // stage buffers need 1024-byte alignment for the 128-byte swizzle pattern
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023u) &
                                                             ~static_cast<uintptr_t>(1023u));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kStages * kStageBytes);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + p.ring_bytes);
     uint64_t *full_bar = bars;
     uint64_t *empty_bar = bars + kMaxStages;
     uint64_t *tmem_full = bars + 2 * kMaxStages;
@@ -1001,6 +1473,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
+    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_bar + s, 1);
@@ -1035,6 +1508,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();  // nothing before this line reads or writes global memory
     // work items: tiles (x splits) over CTAs, or pair tiles over clusters of two
     const uint32_t pair_rank = kPair ? cluster_rank() : 0u;
     const int first_item = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
@@ -1067,28 +1541,28 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         alive = false;
                         break;
                     }
-                    unsigned char *sa = smem + stage * kStageBytes;
-                    unsigned char *sb = sa + kABytes;
+                    unsigned char *sa = smem + stage * stage_bytes;
+                    unsigned char *sb = sa + a_bytes;
                     if (kb == p.skip_kb && blockIdx.x == 0 && item == first_item) {
                         // test hook: this stage is never filled
                     } else if (kPair) {
                         // both CTAs' bytes are counted on the leader's barrier; only the leader announces them
                         if (pair_rank == 0) {
-                            mbar_expect_tx(full_bar + stage, 2 * kStageBytes);
+                            mbar_expect_tx(full_bar + stage, 2 * stage_bytes);
                         }
                         const uint32_t leader_bar = map_to_rank(smem_u32(full_bar + stage), 0u);
                         tma_load_2d_pair(sa, &tmap_a, leader_bar, kb * kElemsPerRow, tm * kBM);
                         // this CTA's half of the piece's B rows (a narrow piece uses the first half of the box only)
                         tma_load_2d_pair(sb, &tmap_b, leader_bar, kb * kElemsPerRow,
-                                         tn * kBN + n_off + static_cast<int>(pair_rank) * (width / 2));
+                                         tn * p.bn + n_off + static_cast<int>(pair_rank) * (width / 2));
                     } else {
-                        mbar_expect_tx(full_bar + stage, kStageBytes);
+                        mbar_expect_tx(full_bar + stage, stage_bytes);
                         if (p.batch > 1) {
                             tma_load_3d(sa, &tmap_a, full_bar + stage, kb * kElemsPerRow, tm * kBM, p.a_bz != 0 ? batch : 0);
-                            tma_load_3d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * kBN, p.b_bz != 0 ? batch : 0);
+                            tma_load_3d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * p.bn, p.b_bz != 0 ? batch : 0);
                         } else {
                             tma_load_2d(sa, &tmap_a, full_bar + stage, kb * kElemsPerRow, tm * kBM);
-                            tma_load_2d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * kBN);
+                            tma_load_2d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * p.bn);
                         }
                     }
                     if (++stage == kStages) {
@@ -1109,7 +1583,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             for (int item = first_item; alive && item < p.num_items; item += item_stride) {
                 int tile, n_off, width, batch, split;
                 decode_item<kPair, kBN>(p, item, tile, n_off, width, batch, split);
-                const uint32_t idesc = (width == kBN) ? p.idesc : p.idesc_narrow;
+                const uint32_t idesc = (width == p.bn) ? p.idesc : p.idesc_narrow;
                 const int kb_begin = split * p.kb_per_split;
                 const int kb_end = (kb_begin + p.kb_per_split < p.num_kb) ? kb_begin + p.kb_per_split : p.num_kb;
                 if (!mbar_wait(tmem_empty + acc, acc_phase ^ 1u, abort_flag, p.status, 2, p.wait_limit)) {
@@ -1123,9 +1597,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + stage * kStageBytes);
+                    const uint32_t sa = smem_u32(smem + stage * stage_bytes);
                     const uint64_t adesc = make_smem_desc(sa);
-                    const uint64_t bdesc = make_smem_desc(sa + kABytes);
+                    const uint64_t bdesc = make_smem_desc(sa + a_bytes);
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
                         // 32 bytes along k inside the swizzle row = 2 units of the 16-byte address field
@@ -1167,7 +1641,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const int quarter = warp & 3;  // TMEM lanes this warp may touch: [32 * quarter, 32 * quarter + 32)
         const int row_in_tile = quarter * 32 + lane;
         const int part = (warp - 2) / 4;  // warps sharing a quarter split the tile's columns between them
-        EpiParams e_batch;  // the epilogue tensors of the current batch entry (batched launches only)
         // the bias slices of the working warps share the space laid out for kEpiWarps slices of kWarpBiasFloats
         float *warp_bias = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(bars) + 256) +
                            (warp - 2) * (kEpiWarps * kWarpBiasFloats / p.epi_warps);
@@ -1183,10 +1656,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         for (int item = first_item; item < p.num_items; item += item_stride) {
             int tile, n_off, width, batch, split;
             decode_item<kPair, kBN>(p, item, tile, n_off, width, batch, split);
-            if (p.batch > 1) {
-                e_batch = epi_for_batch(p.epi, p.bp, batch);
-            }
-            const EpiParams &e = p.batch > 1 ? e_batch : p.epi;
+            const EpiTensors t = epi_tensors(p, batch);
+            const EpiParams &e = p.epi;
             const int per_group = p.group_m * p.tiles_n;
             const int group = tile / per_group;
             const int first_m = group * p.group_m;
@@ -1198,7 +1669,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const int kParts = p.epi_warps / 4;
             const int piece_groups = width / 8;
             const int g_begin = part * piece_groups / kParts, g_end = (part + 1) * piece_groups / kParts;
-            const long long n0 = static_cast<long long>(tn) * kBN + n_off + g_begin * 8;
+            const long long n0 = static_cast<long long>(tn) * p.bn + n_off + g_begin * 8;
             long long cols = p.n - n0;
             const long long part_cols = static_cast<long long>(g_end - g_begin) * 8;
             cols = cols < 0 ? 0 : (cols < part_cols ? cols : part_cols);
@@ -1210,7 +1681,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 __syncwarp();  // every lane is done with the previous tile's values
                 for (int i = lane; i < groups * 8; i += 32) {
                     const long long col = n0 + i;
-                    warp_bias[i] = col < p.n ? load_as_f32(e.bias, e.bias_dtype, col) : 0.0f;
+                    warp_bias[i] = col < p.n ? load_as_f32(t.bias, e.bias_dtype, col) : 0.0f;
                 }
                 __syncwarp();
                 staged_bias = warp_bias;
@@ -1219,7 +1690,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             // the warp-wide tensor-memory instructions below
             const bool arrived =
                 __all_sync(0xffffffffu, mbar_wait(tmem_full + acc, acc_phase, abort_flag, p.status, 4, p.wait_limit));
-            if (!arrived && p.splits == 1) {
+            if (!arrived && p.via_smem == 0) {
                 break;
             }
             tc_fence_after();
@@ -1228,13 +1699,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const uint32_t taddr_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                        static_cast<uint32_t>(acc * kBN);
             const uint32_t taddr_part = taddr_row + static_cast<uint32_t>(g_begin * 8);
-            if (kKind != KUDNN_B200_S8 && p.splits > 1) {
-                // partial tile -> this CTA's shared memory (the stage buffers: every load into them has landed and
-                // every MMA that read them has completed once the accumulator barrier has fired); it is added to
-                // the other ranks' tiles after the role branches, where all warps of the cluster meet
+            if (kKind != KUDNN_B200_S8 && p.via_smem != 0) {
+                // (partial) tile -> this CTA's shared memory (the stage buffers: every load into them has landed and
+                // every MMA that read them has completed once the accumulator barrier has fired); with split K it is
+                // added to the other ranks' tiles after the role branches, where all warps of the cluster meet
                 if (arrived) {
                     float *part = reinterpret_cast<float *>(smem);
-                    dump_partial_row(taddr_part, part + row_in_tile * (kBN + 4) + g_begin * 8, g_end - g_begin);
+                    dump_partial_row(taddr_part, part + row_in_tile * (p.bn + 4) + g_begin * 8, g_end - g_begin, row_ok);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
@@ -1244,7 +1715,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 break;  // one work item per CTA in this mode
             }
             if constexpr (kKind == KUDNN_B200_S8) {
-                epilogue_row_int(e, taddr_part, row_ok, mi, n0, groups);
+                epilogue_row_int(e, t, taddr_part, row_ok, mi, n0, groups);
             } else {
                 // All output-side tensors in the kernel's input type (the usual case): the epilogue variants with the
                 // element type fixed at compile time.  Any other mix, or a rarer activation: the variant that reads the
@@ -1254,19 +1725,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 const int act_case = typed ? e.act : -1;
                 switch (act_case) {
                     case KUDNN_B200_ACT_NONE:
-                        epilogue_row<KUDNN_B200_ACT_NONE, kKind>(e, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
+                        epilogue_row<KUDNN_B200_ACT_NONE, kKind>(e, t, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
                         break;
                     case KUDNN_B200_ACT_RELU:
-                        epilogue_row<KUDNN_B200_ACT_RELU, kKind>(e, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
+                        epilogue_row<KUDNN_B200_ACT_RELU, kKind>(e, t, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
                         break;
                     case KUDNN_B200_ACT_SWISH:
-                        epilogue_row<KUDNN_B200_ACT_SWISH, kKind>(e, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
+                        epilogue_row<KUDNN_B200_ACT_SWISH, kKind>(e, t, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
                         break;
                     case KUDNN_B200_ACT_GELU_TANH:
-                        epilogue_row<KUDNN_B200_ACT_GELU_TANH, kKind>(e, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
+                        epilogue_row<KUDNN_B200_ACT_GELU_TANH, kKind>(e, t, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
                         break;
                     default:
-                        epilogue_row<-1, -1>(e, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
+                        epilogue_row<-1, -1>(e, t, taddr_part, row_ok, mi, n0, groups, staged_bias, warp_stage, lane);
                         break;
                 }
             }
@@ -1287,10 +1758,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
 
     if constexpr (kKind != KUDNN_B200_S8) {  // integer launches never split K
-        if (p.splits > 1) {
-            // ------------------------------------------------------------------ split-K: add the cluster's partial tiles
+        if (p.via_smem != 0) {
+            // ------------------------------------------------------------------ finish the tile from shared memory
             __syncwarp();
-            cluster_sync_all();  // all partial tiles are in place (a hardware barrier over every thread of the cluster)
+            cluster_sync_all();  // all (partial) tiles are in place (a hardware barrier over every thread of the cluster)
             if (warp >= 2 && *abort_flag == 0) {
                 const int unit = static_cast<int>(blockIdx.x) / p.splits;
                 const int batch = unit / p.num_tiles;
@@ -1302,31 +1773,30 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 const int in_group = tile - group * per_group;
                 const int tm = first_m + in_group % gsize;
                 const int tn = in_group / gsize;
-                const float *part = reinterpret_cast<const float *>(smem);
-                EpiParams e_batch;
-                if (p.batch > 1) {
-                    e_batch = epi_for_batch(p.epi, p.bp, batch);
-                }
-                const EpiParams &e = p.batch > 1 ? e_batch : p.epi;
-                const uint32_t rank = cluster_rank();
+                float *part = reinterpret_cast<float *>(smem);
+                const EpiTensors t = epi_tensors(p, batch);
+                const uint32_t rank = p.splits > 1 ? cluster_rank() : 0u;
                 const int epi_tid = static_cast<int>(threadIdx.x) - 64;
-                const bool typed = e.c_dtype == kKind && (e.has_bias == 0 || e.bias_dtype == kKind) &&
-                                   (e.res_op == KUDNN_B200_RES_NONE || (e.res_dtype == kKind && e.out_dtype == kKind));
-                switch (typed ? e.act : -1) {
+                const bool typed = p.epi.c_dtype == kKind && (p.epi.has_bias == 0 || p.epi.bias_dtype == kKind) &&
+                                   (p.epi.res_op == KUDNN_B200_RES_NONE || (p.epi.res_dtype == kKind && p.epi.out_dtype == kKind));
+                switch (typed ? p.epi.act : -1) {
                     case KUDNN_B200_ACT_NONE:
-                        finish_split_rows<KUDNN_B200_ACT_NONE, kKind, kBN>(e, part, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_NONE, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     case KUDNN_B200_ACT_RELU:
-                        finish_split_rows<KUDNN_B200_ACT_RELU, kKind, kBN>(e, part, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_RELU, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     case KUDNN_B200_ACT_SWISH:
-                        finish_split_rows<KUDNN_B200_ACT_SWISH, kKind, kBN>(e, part, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_SWISH, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     case KUDNN_B200_ACT_GELU_TANH:
-                        finish_split_rows<KUDNN_B200_ACT_GELU_TANH, kKind, kBN>(e, part, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_GELU_TANH, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        break;
+                    case KUDNN_B200_ACT_GELU_ERF:
+                        finish_rows<KUDNN_B200_ACT_GELU_ERF, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     default:
-                        finish_split_rows<-1, -1, kBN>(e, part, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<-1, -1>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                 }
             }
@@ -1366,34 +1836,19 @@ template <int kKind, int kBN, bool kPair>
 cudaError_t launch_one(const TcPlan &plan, const TcParams &p, cudaStream_t stream)
 {
     auto kernel = tc_linear_kernel<kKind, kBN, kPair>;
-    cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem_bytes));
+    // the most a CTA can have, whatever this launch takes: the attribute belongs to the kernel, and other host threads may
+    // be launching it with other sizes
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     if (e != cudaSuccess) {
         return e;
     }
     CUtensorMap ta, tb;
     std::memcpy(&ta, plan.tmap_a, sizeof(ta));
     std::memcpy(&tb, plan.tmap_b, sizeof(tb));
-    const int cluster = kPair ? 2 : plan.splits;
-    if (cluster > 1) {
-        // split-K: the CTAs that share a tile form a cluster, blockIdx.x = tile * splits + rank;
-        // pair mode: clusters of two, blockIdx.x = 2 * cluster + rank
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(plan.grid), 1, 1);
-        cfg.blockDim = dim3(kTcThreads, 1, 1);
-        cfg.dynamicSmemBytes = plan.smem_bytes;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = static_cast<unsigned>(cluster);
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kernel, ta, tb, p);
-    }
-    kernel<<<plan.grid, kTcThreads, plan.smem_bytes, stream>>>(ta, tb, p);
-    return cudaGetLastError();
+    // split-K: the CTAs that share a tile form a cluster, blockIdx.x = tile * splits + rank;
+    // pair mode: clusters of two, blockIdx.x = 2 * cluster + rank
+    return launch_chained(kernel, dim3(static_cast<unsigned>(plan.grid)), dim3(kTcThreads), plan.smem_bytes, stream,
+                          static_cast<unsigned>(kPair ? 2 : plan.splits), ta, tb, p);
 }
 
 // How many clusters of two CTAs of the pair kernel the device runs at once (SMs pair up inside a GPC, so this can be
@@ -1402,8 +1857,7 @@ template <int kKind>
 int max_pair_clusters(size_t smem_bytes)
 {
     auto kernel = tc_linear_kernel<kKind, 256, true>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes)) !=
-        cudaSuccess) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess) {
         return 0;
     }
     cudaLaunchConfig_t cfg = {};
