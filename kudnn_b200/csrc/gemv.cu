@@ -53,6 +53,9 @@ struct GemvParams {
     const unsigned short *w_blk;
     int blk_kb;  // 64-k blocks per group
     int w8;      // MMA kernel: the weights are 8-bit integers (1 = signed, 2 = unsigned), the activations fp16
+    // The weights were pre-packed, so no kernel in front of this one on the stream writes them: the first of them are
+    // requested while that kernel still runs (see pdl_wait).
+    int w_stable;
     EpiParams epi;
 };
 
@@ -134,40 +137,96 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_fma_kernel(const Ge
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *xs = reinterpret_cast<float *>(smem_raw);  // [kM][kpad]
     const int kpad = p.kb * kBlockK;
-
-    for (int i = threadIdx.x; i < kM * kpad; i += kThreads) {
-        const int mi = i / kpad, kk = i - mi * kpad;
-        float v = 0.0f;
-        if (kk < p.k) {
-            v = load_as_f32(p.x, kXDtype, static_cast<long long>(mi) * p.x_ld + kk);
-        }
-        if (kInt8) {
-            // a lane's 16 activations of a k-block are four float4 reads; the q-th reads of the 32 lanes lie side by
-            // side (element lane * 16 + q * 4 + j of the block sits at (q * 32 + lane) * 4 + j): no bank conflicts
-            const int blk = kk / kBlockK, r = kk - blk * kBlockK;
-            const int ln = r / 16, q = (r % 16) / 4, j = r % 4;
-            xs[mi * kpad + blk * kBlockK + (q * 32 + ln) * 4 + j] = v;
-        } else {
-            xs[i] = v;
-        }
-    }
-    __syncthreads();
+    const int threads = static_cast<int>(blockDim.x);
 
     const int lane = threadIdx.x & 31;
-    const int warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    if (warp >= p.active_warps) {
-        return;
-    }
+    const int warp = blockIdx.x * (threads >> 5) + (threadIdx.x >> 5);
+    const bool active = warp < p.active_warps;
     long long f = static_cast<long long>(warp) * p.span;
     const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
     const char *wbase = static_cast<const char *>(p.w);
     const int esize = (kDtype == KUDNN_B200_F32) ? 4 : (kInt8 ? 1 : 2);
 
-    while (f < f_end) {
-        const long long row = f / p.kb;
-        const int kb0 = static_cast<int>(f - row * p.kb);
-        const int nb = static_cast<int>(((p.kb - kb0) < (f_end - f)) ? (p.kb - kb0) : (f_end - f));
+    // blocks kb0 + i .. of a row: this lane's 16 bytes of each of the kUnroll blocks, zeros past the piece and past k
+    auto load_batch = [&](uint4 (&wv)[kUnroll], long long row, int kb0, int i, int nb) {
         const char *wrow = wbase + (row * p.w_ld + static_cast<long long>(lane) * kVec) * esize;
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int kk = (kb0 + i + u) * kBlockK + lane * kVec;
+            wv[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (i + u < nb && kk < p.k) {
+                wv[u] = ld_stream_16(wrow + static_cast<long long>(kb0 + i + u) * kBlockK * esize);
+            }
+        }
+    };
+    auto piece_of = [&](long long at, long long &row, int &kb0) {
+        row = at / p.kb;
+        kb0 = static_cast<int>(at - row * p.kb);
+        return static_cast<int>(((p.kb - kb0) < (f_end - at)) ? (p.kb - kb0) : (f_end - at));
+    };
+
+    pdl_launch_dependents();
+    if (p.w_stable == 0) {
+        pdl_wait();
+    }
+    uint4 wv[kUnroll];
+    bool preloaded = active && f < f_end;
+    if (preloaded) {
+        long long row;
+        int kb0;
+        const int nb = piece_of(f, row, kb0);
+        load_batch(wv, row, kb0, 0, nb);
+    }
+    if (p.w_stable != 0) {
+        pdl_wait();
+    }
+
+    // activations -> shared memory as fp32, 16 bytes of them per thread and step
+    constexpr int kXVec = kXDtype == KUDNN_B200_F32 ? 4 : 8;
+    const int vec_per_row = kpad / kXVec;
+    for (int i = threadIdx.x; i < kM * vec_per_row; i += threads) {
+        const int mi = i / vec_per_row, kk = (i - mi * vec_per_row) * kXVec;
+        float v[kXVec];
+#pragma unroll
+        for (int j = 0; j < kXVec; ++j) {
+            v[j] = 0.0f;
+        }
+        if (kk < p.k) {  // k is a multiple of the vector
+            const uint4 raw = *reinterpret_cast<const uint4 *>(static_cast<const char *>(p.x) +
+                                                               (static_cast<long long>(mi) * p.x_ld + kk) * (16 / kXVec));
+            if (kXDtype == KUDNN_B200_F32) {
+                v[0] = __uint_as_float(raw.x);
+                v[1] = __uint_as_float(raw.y);
+                v[2] = __uint_as_float(raw.z);
+                v[3] = __uint_as_float(raw.w);
+            } else {
+                unpack2<kXDtype>(raw.x, v[0], v[1]);
+                unpack2<kXDtype>(raw.y, v[2], v[3]);
+                unpack2<kXDtype>(raw.z, v[4 % kXVec], v[5 % kXVec]);
+                unpack2<kXDtype>(raw.w, v[6 % kXVec], v[7 % kXVec]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kXVec / 4; ++q) {
+            int at = kk + q * 4;
+            if (kInt8) {
+                // a lane's 16 activations of a k-block are four float4 reads; the q-th reads of the 32 lanes lie side by
+                // side (element lane * 16 + q * 4 + j of the block sits at (q * 32 + lane) * 4 + j): no bank conflicts
+                const int blk = at / kBlockK, r = at - blk * kBlockK;
+                at = blk * kBlockK + (((r % 16) / 4) * 32 + r / 16) * 4;
+            }
+            *reinterpret_cast<float4 *>(xs + mi * kpad + at) = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+        }
+    }
+    __syncthreads();
+    if (!active) {
+        return;
+    }
+
+    while (f < f_end) {
+        long long row;
+        int kb0;
+        const int nb = piece_of(f, row, kb0);
 
         float acc[kM];
 #pragma unroll
@@ -175,15 +234,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_fma_kernel(const Ge
             acc[mi] = 0.0f;
         }
         for (int i = 0; i < nb; i += kUnroll) {
-            uint4 wv[kUnroll];
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                const int kk = (kb0 + i + u) * kBlockK + lane * kVec;
-                wv[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (i + u < nb && kk < p.k) {
-                    wv[u] = ld_stream_16(wrow + static_cast<long long>(kb0 + i + u) * kBlockK * esize);
-                }
+            if (!preloaded) {
+                load_batch(wv, row, kb0, i, nb);
             }
+            preloaded = false;
 #pragma unroll
             for (int u = 0; u < kUnroll; ++u) {
                 if (i + u < nb) {
@@ -381,12 +435,72 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
     const int chunk = blockIdx.x % p.ksplit;
     const int cta_in_chunk = blockIdx.x / p.ksplit;
     const int kc0 = chunk * p.kc;
+    const int threads = static_cast<int>(blockDim.x);
+
+    const int lane = threadIdx.x & 31;
+    const int gid = lane >> 2, tig = lane & 3;
+    const int warp = cta_in_chunk * (threads >> 5) + (threadIdx.x >> 5);
+    const bool active = warp < p.active_warps;
+    long long f = static_cast<long long>(warp) * p.span;
+    const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
+
+    // this lane's share of blocks kb0 + i .. of a group, zeros past the piece, the rows and k
+    auto load_batch = [&](uint4 (&wv)[kUnroll][kWide && kW8 == 0 ? 2 : 1], long long group, int kb0, int i, int nb) {
+        const long long wrow_idx = group * 8 + gid;
+        const bool row_ok = wrow_idx < p.n;
+        const unsigned short *wrow = static_cast<const unsigned short *>(p.w) + wrow_idx * p.w_ld + kc0 + tig * (kLaneBytes / 2);
+        const unsigned char *wrow8 = static_cast<const unsigned char *>(p.w) + wrow_idx * p.w_ld + kc0 + tig * 16;
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int kloc = (kb0 + i + u) * kBlockK;
+#pragma unroll
+            for (int h = 0; h < (kWide && kW8 == 0 ? 2 : 1); ++h) {
+                wv[u][h] = make_uint4(0u, 0u, 0u, 0u);
+                if (kW8 != 0) {
+                    if (i + u < nb && row_ok && (kc0 + kloc + tig * 16) < p.k) {
+                        wv[u][h] = ld_stream_16(wrow8 + kloc);
+                    }
+                } else if (p.w_blk != nullptr) {
+                    const int k_abs = kc0 + kloc + tig * (kLaneBytes / 2) + h * 8;
+                    if (i + u < nb && (k_abs >> 6) < p.blk_kb) {
+                        const int c = (k_abs & 63) >> 3;
+                        wv[u][h] = ld_stream_16(p.w_blk + (group * p.blk_kb + (k_abs >> 6)) * 512 + (c & 1) * 256 +
+                                                (gid * 4 + (c >> 1)) * 8);
+                    }
+                } else if (i + u < nb && row_ok && (kc0 + kloc + tig * (kLaneBytes / 2) + h * 8) < p.k) {
+                    wv[u][h] = ld_stream_16(wrow + kloc + h * 8);
+                }
+            }
+        }
+    };
+    auto piece_of = [&](long long at, long long &group, int &kb0) {
+        group = at / p.kb;
+        kb0 = static_cast<int>(at - group * p.kb);
+        return static_cast<int>(((p.kb - kb0) < (f_end - at)) ? (p.kb - kb0) : (f_end - at));
+    };
+
+    pdl_launch_dependents();
+    if (p.w_stable == 0) {
+        pdl_wait();
+    }
+    // the first weights are requested before anything else, so HBM is already busy while the activations load
+    uint4 wv[kUnroll][kWide && kW8 == 0 ? 2 : 1];
+    bool preloaded = active && f < f_end;
+    if (preloaded) {
+        long long group;
+        int kb0;
+        const int nb = piece_of(f, group, kb0);
+        load_batch(wv, group, kb0, 0, nb);
+    }
+    if (p.w_stable != 0) {
+        pdl_wait();
+    }
 
     // activations of this chunk -> shared memory (16-bit, zero padded in m and k)
     {
         const int vec_per_row = p.kc / 8;
         const unsigned short *xg = static_cast<const unsigned short *>(p.x);
-        for (int i = threadIdx.x; i < kRows * vec_per_row; i += kThreads) {
+        for (int i = threadIdx.x; i < kRows * vec_per_row; i += threads) {
             const int mi = i / vec_per_row, v = i - mi * vec_per_row;
             const int kk = kc0 + v * 8;
             uint4 val = make_uint4(0u, 0u, 0u, 0u);
@@ -397,53 +511,23 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
         }
     }
     __syncthreads();
-
-    const int lane = threadIdx.x & 31;
-    const int gid = lane >> 2, tig = lane & 3;
-    const int warp = cta_in_chunk * (kThreads / 32) + (threadIdx.x >> 5);
-    if (warp >= p.active_warps) {
+    if (!active) {
         return;
     }
-    long long f = static_cast<long long>(warp) * p.span;
-    const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
-    const unsigned short *wg = static_cast<const unsigned short *>(p.w);
     const unsigned char *xa_row = smem_raw + gid * row_bytes + tig * kLaneBytes;
     const unsigned char *xb_row = smem_raw + (gid + 8) * row_bytes + tig * kLaneBytes;
 
     while (f < f_end) {
-        const long long group = f / p.kb;
-        const int kb0 = static_cast<int>(f - group * p.kb);
-        const int nb = static_cast<int>(((p.kb - kb0) < (f_end - f)) ? (p.kb - kb0) : (f_end - f));
-        const long long wrow_idx = group * 8 + gid;
-        const bool row_ok = wrow_idx < p.n;
-        const unsigned short *wrow = wg + wrow_idx * p.w_ld + kc0 + tig * (kLaneBytes / 2);
-        const unsigned char *wrow8 = static_cast<const unsigned char *>(p.w) + wrow_idx * p.w_ld + kc0 + tig * 16;
+        long long group;
+        int kb0;
+        const int nb = piece_of(f, group, kb0);
 
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         for (int i = 0; i < nb; i += kUnroll) {
-            uint4 wv[kUnroll][kWide ? 2 : 1];
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                const int kloc = (kb0 + i + u) * kBlockK;
-#pragma unroll
-                for (int h = 0; h < (kWide ? 2 : 1); ++h) {
-                    wv[u][h] = make_uint4(0u, 0u, 0u, 0u);
-                    if (kW8 != 0) {
-                        if (h == 0 && i + u < nb && row_ok && (kc0 + kloc + tig * 16) < p.k) {
-                            wv[u][0] = ld_stream_16(wrow8 + kloc);
-                        }
-                    } else if (p.w_blk != nullptr) {
-                        const int k_abs = kc0 + kloc + tig * (kLaneBytes / 2) + h * 8;
-                        if (i + u < nb && (k_abs >> 6) < p.blk_kb) {
-                            const int c = (k_abs & 63) >> 3;
-                            wv[u][h] = ld_stream_16(p.w_blk + (group * p.blk_kb + (k_abs >> 6)) * 512 + (c & 1) * 256 +
-                                                    (gid * 4 + (c >> 1)) * 8);
-                        }
-                    } else if (i + u < nb && row_ok && (kc0 + kloc + tig * (kLaneBytes / 2) + h * 8) < p.k) {
-                        wv[u][h] = ld_stream_16(wrow + kloc + h * 8);
-                    }
-                }
+            if (!preloaded) {
+                load_batch(wv, group, kb0, i, nb);
             }
+            preloaded = false;
 #pragma unroll
             for (int u = 0; u < kUnroll; ++u) {
                 if (i + u < nb) {
@@ -512,7 +596,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) gemv_mma_staged_kernel(cons
     const int lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
     const int warp_in_cta = threadIdx.x >> 5;
-    const int warp = cta_in_chunk * (kStagedThreads / 32) + warp_in_cta;
+    const int warp = cta_in_chunk * (static_cast<int>(blockDim.x) >> 5) + warp_in_cta;
     const bool active = warp < p.active_warps;
     long long f = static_cast<long long>(warp) * p.span;
     const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
@@ -551,11 +635,18 @@ __global__ void __launch_bounds__(kStagedThreads, 1) gemv_mma_staged_kernel(cons
         return left >= 8 ? 8 : static_cast<int>(left);
     };
 
+    pdl_launch_dependents();
+    if (p.w_stable == 0) {
+        pdl_wait();
+    }
     // the first weight block is requested before anything else, so HBM is already busy while the activations load
     uint4 va[8], vb[8];
     if (active && f < f_end) {
         const long long group = f / p.kb;
         load_block(va, group * 8, rows_of(group), static_cast<int>(f - group * p.kb));
+    }
+    if (p.w_stable != 0) {
+        pdl_wait();
     }
 
     // Activations of this chunk -> shared memory.  Every thread issues eight 16-byte loads before it stores anything
@@ -566,11 +657,12 @@ __global__ void __launch_bounds__(kStagedThreads, 1) gemv_mma_staged_kernel(cons
         const int vec_per_row = p.kc / 8;
         const int total_vec = kRows * vec_per_row;
         const unsigned short *xg = static_cast<const unsigned short *>(p.x);
-        for (int base = threadIdx.x; base < total_vec; base += kStagedThreads * 8) {
+        const int threads = static_cast<int>(blockDim.x);
+        for (int base = threadIdx.x; base < total_vec; base += threads * 8) {
             uint4 xv[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const int i = base + u * kStagedThreads;
+                const int i = base + u * threads;
                 xv[u] = make_uint4(0u, 0u, 0u, 0u);
                 if (i < total_vec) {
                     const int mi = i / vec_per_row, vi = i - mi * vec_per_row;
@@ -582,7 +674,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) gemv_mma_staged_kernel(cons
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const int i = base + u * kStagedThreads;
+                const int i = base + u * threads;
                 if (i < total_vec) {
                     const int mi = i / vec_per_row, vi = i - mi * vec_per_row;
                     const int blk = vi >> 2, q = vi & 3;
@@ -698,45 +790,37 @@ int env_int(const char *name, int fallback)
     return std::atoi(v);
 }
 
-template <typename K>
-cudaError_t set_smem(K kernel, size_t bytes)
+// The shared-memory limit of a kernel is set to the same value by every launch, so that host threads cannot disturb each other.
+cudaError_t launch_gemv_kernel(void (*kernel)(GemvParams), const GemvParams &p, const GemvPlan &plan, cudaStream_t stream)
 {
-    if (bytes > 48 * 1024) {
-        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    if (plan.smem_bytes > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e != cudaSuccess) {
+            return e;
+        }
     }
-    return cudaSuccess;
+    return launch_chained(kernel, dim3(static_cast<unsigned>(plan.grid)), dim3(static_cast<unsigned>(plan.block)), plan.smem_bytes,
+                          stream, 1, p);
 }
 
 template <int kDtype, int kUnroll, int kThreads, int kMinBlocks>
 cudaError_t launch_fma_m(const GemvParams &p, const GemvPlan &plan, cudaStream_t stream)
 {
-#define KB_FMA_CASE(M)                                                                                            \
-    case M: {                                                                                                     \
-        auto kernel = gemv_fma_kernel<kDtype, M, kUnroll, kThreads, kMinBlocks>;                                  \
-        cudaError_t e = set_smem(kernel, plan.smem_bytes);                                                        \
-        if (e != cudaSuccess) return e;                                                                           \
-        kernel<<<plan.grid, plan.block, plan.smem_bytes, stream>>>(p);                                            \
-        break;                                                                                                    \
+    if (p.m == 1) {
+        return launch_gemv_kernel(gemv_fma_kernel<kDtype, 1, kUnroll, kThreads, kMinBlocks>, p, plan, stream);
     }
-    if constexpr (kDtype == KUDNN_B200_S8 || kDtype == KUDNN_B200_U8) {
-        // 8-bit weights take this kernel for a single activation row only
+    // 8-bit weights take this kernel for a single activation row only
+    if constexpr (kDtype != KUDNN_B200_S8 && kDtype != KUDNN_B200_U8) {
         switch (p.m) {
-            KB_FMA_CASE(1)
-            default:
-                return cudaErrorInvalidValue;
-        }
-    } else {
-        switch (p.m) {
-            KB_FMA_CASE(1)
-            KB_FMA_CASE(2)
-            KB_FMA_CASE(3)
-            KB_FMA_CASE(4)
-            default:
-                return cudaErrorInvalidValue;
+            case 2:
+                return launch_gemv_kernel(gemv_fma_kernel<kDtype, 2, kUnroll, kThreads, kMinBlocks>, p, plan, stream);
+            case 3:
+                return launch_gemv_kernel(gemv_fma_kernel<kDtype, 3, kUnroll, kThreads, kMinBlocks>, p, plan, stream);
+            case 4:
+                return launch_gemv_kernel(gemv_fma_kernel<kDtype, 4, kUnroll, kThreads, kMinBlocks>, p, plan, stream);
         }
     }
-#undef KB_FMA_CASE
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 template <int kDtype, int kUnroll, int kThreads, int kMinBlocks>
@@ -744,66 +828,38 @@ cudaError_t launch_mma_rows(const GemvParams &p, const GemvPlan &plan, cudaStrea
 {
     if (p.w8 != 0) {
         if constexpr (kDtype == KUDNN_B200_F16) {
-#define KB_W8_CASE(ROWS16, SIGN)                                                                                   \
-    {                                                                                                              \
-        auto kernel = gemv_mma_kernel<kDtype, ROWS16, true, kUnroll, kThreads, kMinBlocks, SIGN>;                    \
-        cudaError_t e = set_smem(kernel, plan.smem_bytes);                                                         \
-        if (e != cudaSuccess) return e;                                                                            \
-        kernel<<<plan.grid, plan.block, plan.smem_bytes, stream>>>(p);                                             \
-    }
+#define KB_W8_CASE(ROWS16, SIGN) \
+    launch_gemv_kernel(gemv_mma_kernel<kDtype, ROWS16, true, kUnroll, kThreads, kMinBlocks, SIGN>, p, plan, stream)
             if (p.m > 8) {
-                if (p.w8 == 1) KB_W8_CASE(true, 1) else KB_W8_CASE(true, 2)
-            } else {
-                if (p.w8 == 1) KB_W8_CASE(false, 1) else KB_W8_CASE(false, 2)
+                return p.w8 == 1 ? KB_W8_CASE(true, 1) : KB_W8_CASE(true, 2);
             }
+            return p.w8 == 1 ? KB_W8_CASE(false, 1) : KB_W8_CASE(false, 2);
 #undef KB_W8_CASE
-            return cudaGetLastError();
         } else {
             return cudaErrorInvalidValue;
         }
     }
     if (p.m > 8 && plan.wide != 0) {
         // three blocks (96 bytes per lane) in flight: 91.0 us against 91.7 us with two and 98.3 us with four (spills)
-        auto kernel = gemv_mma_kernel<kDtype, true, true, (kUnroll > 2 ? kUnroll * 3 / 4 : 1), kThreads, kMinBlocks>;
-        cudaError_t e = set_smem(kernel, plan.smem_bytes);
-        if (e != cudaSuccess) return e;
-        kernel<<<plan.grid, plan.block, plan.smem_bytes, stream>>>(p);
-    } else if (p.m > 8) {
-        auto kernel = gemv_mma_kernel<kDtype, true, false, kUnroll, kThreads, kMinBlocks>;
-        cudaError_t e = set_smem(kernel, plan.smem_bytes);
-        if (e != cudaSuccess) return e;
-        kernel<<<plan.grid, plan.block, plan.smem_bytes, stream>>>(p);
-    } else {
-        auto kernel = gemv_mma_kernel<kDtype, false, false, kUnroll, kThreads, kMinBlocks>;
-        cudaError_t e = set_smem(kernel, plan.smem_bytes);
-        if (e != cudaSuccess) return e;
-        kernel<<<plan.grid, plan.block, plan.smem_bytes, stream>>>(p);
+        return launch_gemv_kernel(gemv_mma_kernel<kDtype, true, true, (kUnroll > 2 ? kUnroll * 3 / 4 : 1), kThreads, kMinBlocks>, p,
+                                  plan, stream);
     }
-    return cudaGetLastError();
+    return p.m > 8 ? launch_gemv_kernel(gemv_mma_kernel<kDtype, true, false, kUnroll, kThreads, kMinBlocks>, p, plan, stream)
+                   : launch_gemv_kernel(gemv_mma_kernel<kDtype, false, false, kUnroll, kThreads, kMinBlocks>, p, plan, stream);
 }
 
 template <int kDtype>
 cudaError_t launch_mma_staged(const GemvParams &p, const GemvPlan &plan, cudaStream_t stream)
 {
-    if (p.m > 8) {
-        auto kernel = gemv_mma_staged_kernel<kDtype, true>;
-        cudaError_t e = set_smem(kernel, plan.smem_bytes);
-        if (e != cudaSuccess) return e;
-        kernel<<<plan.grid, plan.block, plan.smem_bytes, stream>>>(p);
-    } else {
-        auto kernel = gemv_mma_staged_kernel<kDtype, false>;
-        cudaError_t e = set_smem(kernel, plan.smem_bytes);
-        if (e != cudaSuccess) return e;
-        kernel<<<plan.grid, plan.block, plan.smem_bytes, stream>>>(p);
-    }
-    return cudaGetLastError();
+    return p.m > 8 ? launch_gemv_kernel(gemv_mma_staged_kernel<kDtype, true>, p, plan, stream)
+                   : launch_gemv_kernel(gemv_mma_staged_kernel<kDtype, false>, p, plan, stream);
 }
 
 // Launch shapes: threads per CTA / resident CTAs per SM the kernel is compiled for.
 struct GemvShape {
     int threads, min_blocks;
 };
-constexpr GemvShape kShapes[3] = {{512, 2}, {1024, 1}, {1024, 2}};
+constexpr GemvShape kShapes[2] = {{512, 2}, {1024, 1}};
 constexpr int kStagedShape = 3;  // GemvPlan::shape of the staged-feed MMA kernel
 
 template <int kDtype, bool kFma>
@@ -820,7 +876,6 @@ cudaError_t launch_shape(const GemvParams &p, const GemvPlan &plan, int shape, c
     switch (shape) {
         KB_SHAPE_CASE(0, 512, 2)
         KB_SHAPE_CASE(1, 1024, 1)
-        KB_SHAPE_CASE(2, 1024, 2)
         default:
             return cudaErrorInvalidValue;
     }
@@ -829,8 +884,60 @@ cudaError_t launch_shape(const GemvParams &p, const GemvPlan &plan, int shape, c
 
 }  // namespace
 
+// How `units` units (weight rows, or groups of 8 rows) of `blocks` blocks are cut between the warps of `ctas` CTAs: spans of
+// equal length, at least `min_span` blocks each, and as few warps per CTA as the spans need, so that a small matrix is
+// spread over all SMs.
+struct GemvCut {
+    long long span, active;
+    int warps_per_cta, slots;
+};
+
+GemvCut cut_units(long long units, long long blocks, int ctas, int warps, long long min_span)
+{
+    GemvCut c;
+    const long long total = units * blocks;
+    long long active = std::min<long long>(static_cast<long long>(ctas) * warps, total / min_span);
+    active = std::max<long long>(active, 1);
+    c.span = (total + active - 1) / active;
+    c.active = (total + c.span - 1) / c.span;
+    c.warps_per_cta = static_cast<int>(std::min<long long>(warps, (c.active + ctas - 1) / ctas));
+    c.slots = static_cast<int>((blocks + c.span - 1) / c.span) + 1;
+    return c;
+}
+
+// The number of K chunks of the MMA kernels.  More chunks shorten the stretch of the activations that every CTA copies to its
+// shared memory (about 40 bytes per ns and SM) and cost partial sums (512 bytes written and read per piece of a group):
+// estimated ns of both beside the stream of the weights.  Returns 0 when no chunk fits `budget`.
+int choose_ksplit(long long groups, long long k, long long block_k, int rows, long long block_bytes, int ctas_all, int ctas_per_sm,
+                  int warps, long long min_span, size_t budget)
+{
+    int best = 0;
+    double best_ns = 1e300;
+    for (int ks = 1; ks <= 64; ks = ks < 8 ? ks + 1 : ks + ks / 4) {
+        const long long kc = ((k + ks - 1) / ks + block_k - 1) / block_k * block_k;
+        if ((ks - 1) * kc >= k && ks > 1) {
+            continue;  // the last chunk would be empty
+        }
+        if (static_cast<size_t>(rows) * (kc * 2 + kMmaRowPadBytes) > budget || ctas_all / ks < 1) {
+            continue;
+        }
+        const long long kbc = kc / block_k;
+        const GemvCut c = cut_units(groups, kbc, ctas_all / ks, warps, min_span);
+        const double per_sm = static_cast<double>(c.span) * block_bytes * c.warps_per_cta * ctas_per_sm;
+        const double stream = std::max(per_sm / 40.0, static_cast<double>(groups) * kbc * ks * block_bytes / 5800.0);
+        const double fill = 500.0 + static_cast<double>(rows) * kc * 2 * ctas_per_sm / 40.0;
+        const double pieces = static_cast<double>(ks) * (groups + (c.span % kbc == 0 || kbc % c.span == 0 ? groups * ((kbc + c.span - 1) / c.span - 1) : c.active));
+        const double partials = ks == 1 && c.span % kbc == 0 ? 0.0 : 800.0 + pieces * 1024.0 / 5000.0;
+        if (stream + fill + partials < best_ns) {
+            best_ns = stream + fill + partials;
+            best = ks;
+        }
+    }
+    return best;
+}
+
 // Decides whether a problem can take a streaming kernel and how it is cut.  Pure host arithmetic.
-bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, GemvPlan *plan)
+bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fixed_scratch, GemvPlan *plan)
 {
     if (pr.batch_count != 1 || pr.m > 16 || pr.m < 1) {
         return false;
@@ -861,7 +968,6 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, GemvPla
         kernel = (dt == KUDNN_B200_F32 || pr.m <= 1) ? KUDNN_B200_KERNEL_GEMV_FMA : KUDNN_B200_KERNEL_GEMV_MMA;
     }
     plan->kernel = kernel;
-    int shape = -1;
     if (kernel == KUDNN_B200_KERNEL_GEMV_FMA) {
         if (pr.m > 4) {
             return false;
@@ -872,29 +978,21 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, GemvPla
         if (smem > max_smem) {
             return false;
         }
-        if (shape < 0 || shape > 2) {
-            shape = (smem <= 100 * 1024) ? 0 : 1;
-        }
-        if (smem > 100 * 1024) {
-            shape = 1;  // only one CTA fits per SM
-        }
-        const int threads = kShapes[shape].threads, warps = threads / 32;
-        const int grid = sm_count * kShapes[shape].min_blocks;
-        const long long total = pr.n * kb;
-        long long active = std::min<long long>(static_cast<long long>(grid) * warps, pr.n);  // keeps span >= kb
-        active = std::max<long long>(active, 1);
-        const long long span = (total + active - 1) / active;
-        active = (total + span - 1) / span;
+        const int shape = smem > 100 * 1024 ? 1 : 0;  // above 100 KB only one CTA fits per SM
+        const int warps = kShapes[shape].threads / 32;
+        const int ctas = sm_count * kShapes[shape].min_blocks;
+        // At least four blocks (2 KB) per warp.  With fixed scratch a row is not cut more than once.
+        const GemvCut c = cut_units(pr.n, kb, ctas, warps, fixed_scratch ? kb : 4);
         plan->shape = shape;
         plan->wide = 0;
-        plan->block = threads;
-        plan->grid = static_cast<int>((active + warps - 1) / warps);
+        plan->block = 32 * (fixed_scratch ? warps : c.warps_per_cta);
+        plan->grid = static_cast<int>((c.active + plan->block / 32 - 1) / (plan->block / 32));
         plan->ksplit = 1;
-        plan->active_warps = static_cast<int>(active);
-        plan->span = span;
-        plan->slots = 2;
+        plan->active_warps = static_cast<int>(c.active);
+        plan->span = c.span;
+        plan->slots = fixed_scratch ? 2 : c.slots;
         plan->smem_bytes = smem;
-        plan->partial_floats = pr.n * 2 * pr.m;
+        plan->partial_floats = pr.n * plan->slots * pr.m;
         plan->counter_count = pr.n;
         return true;
     }
@@ -911,66 +1009,74 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, GemvPla
     // off (0), KUDNN_B200_GEMV_WIDE=0 makes the fragment-shaped loads 16 bytes per lane.
     const int staged_env = env_int("KUDNN_B200_GEMV_STAGED", -1);
     const bool staged = !w8 && (staged_env < 0 ? (rows == 8 && pr.b_blocked != nullptr) : staged_env != 0);
-    if (staged && (shape < 0 || shape == kStagedShape)) {
+    const long long groups = (pr.n + 7) / 8;
+    // With fixed scratch: the fewest chunks that fit, and a group of rows cut at most once per chunk boundary.
+    auto finish_plan = [&](int shape, int ksplit, long long kc, long long block_k, int ctas, int warps, long long min_span, size_t smem) {
+        const long long kbc = kc / block_k;
+        GemvCut c = cut_units(groups, kbc, std::max(ctas / ksplit, 1), warps, fixed_scratch ? 1 : min_span);
+        if (fixed_scratch) {
+            const long long total = groups * kbc;
+            long long active = std::min<long long>(static_cast<long long>(std::max(ctas / ksplit, 1)) * warps, 2 * groups);
+            active = std::max<long long>(active, 1);
+            c.span = (total + active - 1) / active;
+            c.active = (total + c.span - 1) / c.span;
+            c.warps_per_cta = warps;
+            c.slots = static_cast<int>((kbc + c.span - 1) / c.span) + 1;
+        }
+        plan->shape = shape;
+        plan->block = 32 * c.warps_per_cta;
+        plan->grid = static_cast<int>((c.active + c.warps_per_cta - 1) / c.warps_per_cta) * ksplit;
+        plan->ksplit = ksplit;
+        plan->active_warps = static_cast<int>(c.active);
+        plan->span = c.span;
+        plan->slots = c.slots;
+        plan->smem_bytes = smem;
+        plan->partial_floats = groups * ksplit * plan->slots * 128;
+        plan->counter_count = groups;
+    };
+    auto chunk_len = [&](int parts, long long block_k) { return ((pr.k + parts - 1) / parts + block_k - 1) / block_k * block_k; };
+    auto fewest_chunks = [&](long long block_k, size_t budget) {
+        int ks = 1;
+        while (ks < 64 && static_cast<size_t>(rows) * (chunk_len(ks, block_k) * 2 + kMmaRowPadBytes) > budget) {
+            ks *= 2;
+        }
+        return ks;
+    };
+    if (staged) {
         // staged feed: 512 threads, one CTA per SM, blocks of 8 rows x 256 k
         const int warps = kStagedThreads / 32;
         const size_t staging = static_cast<size_t>(warps) * kStagedWarpBytes;
         const size_t budget = 225 * 1024 - staging;
-        int ksplit = 0;
-        auto chunk_len = [&](int parts) {
-            return ((pr.k + parts - 1) / parts + kStagedBlockK - 1) / kStagedBlockK * kStagedBlockK;
-        };
-        if (ksplit <= 0) {
-            ksplit = 1;
-            while (ksplit < 64 && static_cast<size_t>(rows) * (chunk_len(ksplit) * 2 + kMmaRowPadBytes) > budget) {
-                ksplit *= 2;
-            }
+        int ksplit = fixed_scratch ? 0
+                                   : choose_ksplit(groups, pr.k, kStagedBlockK, rows, 8 * kStagedBlockK * 2, sm_count, 1, warps, 1, budget);
+        if (ksplit == 0) {
+            ksplit = fewest_chunks(kStagedBlockK, budget);
         }
-        const long long kc = chunk_len(ksplit);
+        const long long kc = chunk_len(ksplit, kStagedBlockK);
         const size_t xbytes = static_cast<size_t>(rows) * (kc * 2 + kMmaRowPadBytes);
         if (xbytes <= budget) {
-            const int grid = std::max(sm_count / ksplit, 1) * ksplit;
-            const long long groups = (pr.n + 7) / 8;
-            const long long kbc = kc / kStagedBlockK;
-            const long long total = groups * kbc;
-            long long active = std::min<long long>(static_cast<long long>(grid / ksplit) * warps, 2 * groups);
-            active = std::max<long long>(active, 1);
-            const long long span = (total + active - 1) / active;
-            active = (total + span - 1) / span;
-            plan->shape = kStagedShape;
             plan->wide = 0;
-            plan->block = kStagedThreads;
-            plan->grid = static_cast<int>((active + warps - 1) / warps) * ksplit;
-            plan->ksplit = ksplit;
-            plan->active_warps = static_cast<int>(active);
-            plan->span = span;
-            plan->slots = static_cast<int>((kbc + span - 1) / span) + 1;
-            plan->smem_bytes = xbytes + staging;
-            plan->partial_floats = groups * ksplit * plan->slots * 128;
-            plan->counter_count = groups;
+            const int ctas = fixed_scratch ? std::max(sm_count / ksplit, 1) * ksplit : sm_count;
+            finish_plan(kStagedShape, ksplit, kc, kStagedBlockK, ctas, warps, 1, xbytes + staging);
             return true;
         }
     }
-    if (shape < 0 || shape > 2) {
-        // 16 activation rows: one 1024-thread CTA per SM leaves room for a longer K chunk (fewer partial sums)
-        shape = (rows == 16) ? 1 : 0;
-    }
+    // 16 activation rows: one 1024-thread CTA per SM leaves room for a longer K chunk (fewer partial sums)
+    int shape = (rows == 16) ? 1 : 0;
     const size_t smem_budget = (kShapes[shape].min_blocks == 2) ? 100 * 1024 : max_smem;
-    int ksplit = 0;
     // 16 activation rows: blocks of 64 k with 32 bytes per lane (see gemv_mma_kernel)
     const bool wide = w8 || (rows == 16 && env_int("KUDNN_B200_GEMV_WIDE", 1) != 0);
     const long long block_k = wide ? 64 : 32;
-    if (ksplit <= 0) {
-        ksplit = 1;
-        while (ksplit < 64) {
-            const long long kc = ((pr.k + ksplit - 1) / ksplit + block_k - 1) / block_k * block_k;
-            if (static_cast<size_t>(rows) * (kc * 2 + kMmaRowPadBytes) <= smem_budget) {
-                break;
-            }
-            ksplit *= 2;
-        }
+    const long long block_bytes = 8 * block_k * (w8 ? 1 : 2);
+    const int warps = kShapes[shape].threads / 32;
+    const long long min_span = 4096 / block_bytes;  // at least 4 KB of weights per warp
+    int ksplit = fixed_scratch ? 0
+                               : choose_ksplit(groups, pr.k, block_k, rows, block_bytes, sm_count * kShapes[shape].min_blocks,
+                                               kShapes[shape].min_blocks, warps, min_span, smem_budget);
+    if (ksplit == 0) {
+        ksplit = fewest_chunks(block_k, smem_budget);
     }
-    const long long kc = ((pr.k + ksplit - 1) / ksplit + block_k - 1) / block_k * block_k;
+    const long long kc = chunk_len(ksplit, block_k);
     const size_t smem = static_cast<size_t>(rows) * (kc * 2 + kMmaRowPadBytes);
     if (smem > max_smem) {
         return false;
@@ -978,27 +1084,10 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, GemvPla
     if (smem > 100 * 1024 && kShapes[shape].min_blocks == 2) {
         shape = 1;
     }
-    const int threads = kShapes[shape].threads, warps = threads / 32;
-    int grid = sm_count * kShapes[shape].min_blocks;
-    grid = std::max(grid / ksplit, 1) * ksplit;
-    const long long groups = (pr.n + 7) / 8;
-    const long long kbc = kc / block_k;
-    const long long total = groups * kbc;
-    long long active = std::min<long long>(static_cast<long long>(grid / ksplit) * warps, 2 * groups);
-    active = std::max<long long>(active, 1);
-    const long long span = (total + active - 1) / active;
-    active = (total + span - 1) / span;
     plan->wide = wide ? 1 : 0;
-    plan->shape = shape;
-    plan->block = threads;
-    plan->grid = static_cast<int>((active + warps - 1) / warps) * ksplit;
-    plan->ksplit = ksplit;
-    plan->active_warps = static_cast<int>(active);
-    plan->span = span;
-    plan->slots = static_cast<int>((kbc + span - 1) / span) + 1;
-    plan->smem_bytes = smem;
-    plan->partial_floats = groups * ksplit * plan->slots * 128;
-    plan->counter_count = groups;
+    const int ctas = sm_count * kShapes[shape].min_blocks;
+    finish_plan(shape, ksplit, kc, block_k, fixed_scratch ? std::max(ctas / ksplit, 1) * ksplit : ctas, kShapes[shape].threads / 32,
+                min_span, smem);
     return true;
 }
 
@@ -1022,6 +1111,7 @@ cudaError_t launch_gemv(const LinearProblem &pr, const GemvPlan &plan, const Gem
     p.partials = ws.partials;
     p.counters = ws.counters;
     p.epi = pr.epi;
+    p.w_stable = pr.b_stable ? 1 : 0;
     p.w_blk = plan.kernel == KUDNN_B200_KERNEL_GEMV_MMA ? static_cast<const unsigned short *>(pr.b_blocked) : nullptr;
     p.w8 = pr.b_dtype == KUDNN_B200_S8 ? 1 : (pr.b_dtype == KUDNN_B200_U8 ? 2 : 0);
     p.blk_kb = static_cast<int>(pr.b_blocked_kpad / 64);

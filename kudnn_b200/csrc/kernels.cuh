@@ -15,6 +15,7 @@ struct LinearProblem {
     // the weights once more in the decode-packed layout (see GemvParams::w_blk in gemv.cu), or null
     const void *b_blocked = nullptr;
     long long b_blocked_kpad = 0;
+    bool b_stable = false;  // b was pre-packed: no kernel on the stream writes it
     EpiParams epi;
     BatchParams batch;
     long long batch_count;
@@ -49,7 +50,8 @@ cudaError_t launch_simt(const LinearProblem &pr, cudaStream_t stream);
 cudaError_t launch_int_gemm(const LinearProblem &pr, cudaStream_t stream);
 
 // Streaming kernels for m <= 16 (2-D problems, K-contiguous operands).
-bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, GemvPlan *plan);
+// fixed_scratch: cut with the fewest partial sums (the caller's scratch does not grow)
+bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fixed_scratch, GemvPlan *plan);
 cudaError_t launch_gemv(const LinearProblem &pr, const GemvPlan &plan, const GemvWorkspace &ws, cudaStream_t stream);
 
 // Tensor-core kernel.  Operands must be K-major with 16-byte aligned rows; see tc_eligible().

@@ -599,8 +599,9 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             a8.b = w8;
             kb::LinearProblem p8;
             fill_problem(d8, a8, &p8);
+            p8.b_stable = packed8;
             kb::GemvPlan plan8;
-            if (kb::gemv_plan(p8, h->sm_count, forced8, &plan8)) {
+            if (kb::gemv_plan(p8, h->sm_count, forced8, false, &plan8)) {
                 kb::GemvWorkspace ws8;
                 rc = reserve_gemv_scratch(h, plan8.partial_floats, plan8.counter_count, stream, &ws8);
                 if (rc != KUDNN_B200_OK) {
@@ -687,6 +688,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
         pr.b = h->packed_raw;
         pr.b_sk = 1;
         pr.b_sn = h->packed_ld;
+        pr.b_stable = true;
         if (h->blocked_kpad > 0) {
             pr.b_blocked = h->b_blocked.ptr;
             pr.b_blocked_kpad = h->blocked_kpad;
@@ -697,7 +699,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
     if (two_d && d.m <= 16 &&
         (forced == KUDNN_B200_KERNEL_AUTO || forced == KUDNN_B200_KERNEL_GEMV_FMA || forced == KUDNN_B200_KERNEL_GEMV_MMA)) {
         kb::GemvPlan plan;
-        if (kb::gemv_plan(pr, h->sm_count, forced, &plan)) {
+        if (kb::gemv_plan(pr, h->sm_count, forced, false, &plan)) {
             kb::GemvWorkspace ws;
             rc = reserve_gemv_scratch(h, plan.partial_floats, plan.counter_count, stream, &ws);
             if (rc != KUDNN_B200_OK) {

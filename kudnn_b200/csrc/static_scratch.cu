@@ -171,7 +171,7 @@ extern "C" int kudnn_b200_linear_run_static_scratch(const kudnn_b200_linear_desc
     pr.batch_count = 1;
 
     kb::GemvPlan plan;
-    if (!kb::gemv_plan(pr, slot.sm_count, KUDNN_B200_KERNEL_AUTO, &plan)) {
+    if (!kb::gemv_plan(pr, slot.sm_count, KUDNN_B200_KERNEL_AUTO, true, &plan)) {
         return kb::set_last_error(KUDNN_B200_UNSUPPORTED,
                                   "static-scratch run: the streaming kernels need K-contiguous, 16-byte aligned a and b "
                                   "of one element type");
