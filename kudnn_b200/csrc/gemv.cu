@@ -68,6 +68,13 @@ __device__ __forceinline__ uint4 ld_stream_16(const void *p)
     return v;
 }
 
+// Orders this thread's accesses on both sides of a counter update.  __threadfence() is the sequentially consistent fence, which
+// costs more than the hand-over of partial sums needs.
+__device__ __forceinline__ void fence_acq_rel_gpu()
+{
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
+
 template <int kDtype>
 __device__ __forceinline__ void unpack2(unsigned w, float &lo, float &hi)
 {
@@ -316,10 +323,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_fma_kernel(const Ge
                 for (int mi = 0; mi < kM; ++mi) {
                     mine[mi] = acc[mi];
                 }
-                __threadfence();
+                fence_acq_rel_gpu();
                 const unsigned old = atomicAdd(p.counters + row, 1u);
                 if (old == static_cast<unsigned>(pieces - 1)) {
-                    __threadfence();
+                    fence_acq_rel_gpu();
                     const float *all = p.partials + row * p.slots * kM;
 #pragma unroll
                     for (int mi = 0; mi < kM; ++mi) {
@@ -377,7 +384,7 @@ __device__ __forceinline__ void mma_finish_group(const GemvParams &p, float (&ac
         const int slot = chunk * p.slots + (warp - w0);
         float *unit = p.partials + group * (static_cast<long long>(p.ksplit) * p.slots * 128);
         *reinterpret_cast<float4 *>(unit + slot * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        __threadfence();
+        fence_acq_rel_gpu();
         __syncwarp();
         unsigned old = 0u;
         if (lane == 0) {
@@ -385,15 +392,29 @@ __device__ __forceinline__ void mma_finish_group(const GemvParams &p, float (&ac
         }
         old = __shfl_sync(0xffffffffu, old, 0);
         if (old == static_cast<unsigned>(p.ksplit * pieces - 1)) {
-            __threadfence();
+            fence_acq_rel_gpu();
             float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            for (int c = 0; c < p.ksplit; ++c) {
-                for (int j = 0; j < pieces; ++j) {
-                    const float4 v = __ldcg(reinterpret_cast<const float4 *>(unit + (c * p.slots + j) * 128 + lane * 4));
-                    s[0] += v.x;
-                    s[1] += v.y;
-                    s[2] += v.z;
-                    s[3] += v.w;
+            // added in slot order, four loads in flight
+            const int count = p.ksplit * pieces;
+            for (int i0 = 0; i0 < count; i0 += 4) {
+                float4 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int i = i0 + u;
+                    v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (i < count) {
+                        const int c = i / pieces, j = i - c * pieces;
+                        v[u] = __ldcg(reinterpret_cast<const float4 *>(unit + (c * p.slots + j) * 128 + lane * 4));
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (i0 + u < count) {
+                        s[0] += v[u].x;
+                        s[1] += v[u].y;
+                        s[2] += v[u].z;
+                        s[3] += v[u].w;
+                    }
                 }
             }
             acc[0] = s[0];
@@ -906,8 +927,9 @@ GemvCut cut_units(long long units, long long blocks, int ctas, int warps, long l
 }
 
 // The number of K chunks of the MMA kernels.  More chunks shorten the stretch of the activations that every CTA copies to its
-// shared memory (about 40 bytes per ns and SM) and cost partial sums (512 bytes written and read per piece of a group):
-// estimated ns of both beside the stream of the weights.  Returns 0 when no chunk fits `budget`.
+// shared memory (about 40 bytes per ns and SM) and give every warp more pieces of a group to end: estimated ns of both beside
+// the stream of the weights.  Measured over 1 to 16 chunks, us: 16 x 28672 x 8192 84 with 2, 94 with 4, 127 with 8; 16 x 6144 x
+// 5888 24 / 21 / 22 / 21 with 1 / 2 / 4 / 6; 4 x 11008 x 4096 23 / 24 / 30 with 1 / 2 / 4.  Returns 0 when no chunk fits `budget`.
 int choose_ksplit(long long groups, long long k, long long block_k, int rows, long long block_bytes, int ctas_all, int ctas_per_sm,
                   int warps, long long min_span, size_t budget)
 {
@@ -926,8 +948,9 @@ int choose_ksplit(long long groups, long long k, long long block_k, int rows, lo
         const double per_sm = static_cast<double>(c.span) * block_bytes * c.warps_per_cta * ctas_per_sm;
         const double stream = std::max(per_sm / 40.0, static_cast<double>(groups) * kbc * ks * block_bytes / 5800.0);
         const double fill = 500.0 + static_cast<double>(rows) * kc * 2 * ctas_per_sm / 40.0;
-        const double pieces = static_cast<double>(ks) * (groups + (c.span % kbc == 0 || kbc % c.span == 0 ? groups * ((kbc + c.span - 1) / c.span - 1) : c.active));
-        const double partials = ks == 1 && c.span % kbc == 0 ? 0.0 : 800.0 + pieces * 1024.0 / 5000.0;
+        // pieces a warp ends: each stalls it for several microseconds (partial sums, fence, counter, the last one's additions)
+        const double pieces = static_cast<double>(groups) / c.active + (kbc % c.span == 0 || c.span % kbc == 0 ? 0.0 : 1.0);
+        const double partials = 6000.0 * std::max(pieces, 1.0);
         if (stream + fill + partials < best_ns) {
             best_ns = stream + fill + partials;
             best = ks;
