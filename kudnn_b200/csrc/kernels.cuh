@@ -108,6 +108,7 @@ struct PackBatch {
     long long count, n1, n2;
     long long sb[3];
     long long dst_batch;
+    long long rows = 0, row_slices = 1;  // filled in by the launcher of the row kernels
 };
 
 // Packing / conversion kernels.

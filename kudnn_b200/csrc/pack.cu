@@ -119,6 +119,83 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const float *src_base, 
     }
 }
 
+// ---- rows that are contiguous along k already (activations, per call): no transpose, one 16-byte piece of the packed row
+// per thread.  Bound by memory; the 32 x 32 transpose above reads and writes element by element and took 5 us for what
+// these finish in the shadow of the next kernel's launch.
+// kBytes-wide elements of one type; the source rows start anywhere.
+template <int kBytes>
+__global__ void __launch_bounds__(256) pack_rows_kernel(const void *src_base, long long k, long long s_row, void *dst_base, long long ldd,
+                                                        long long pieces, const PackBatch pb)
+{
+    constexpr int kVec = 16 / kBytes;
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long piece = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+    if (piece >= pieces) {
+        return;
+    }
+    const long long row = blockIdx.y + static_cast<long long>(gridDim.y) * (blockIdx.z % pb.row_slices);
+    const long long flat = blockIdx.z / pb.row_slices;
+    if (row >= pb.rows) {
+        return;
+    }
+    const unsigned char *src = static_cast<const unsigned char *>(src_base) + (src_batch_offset(pb, flat) + row * s_row + piece * kVec) * kBytes;
+    const long long left = (k - piece * kVec) * kBytes;  // bytes of this piece that exist
+    unsigned w[4] = {0u, 0u, 0u, 0u};
+    if (left >= 16 && (reinterpret_cast<uintptr_t>(src) & 3u) == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w[i] = reinterpret_cast<const unsigned *>(src)[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) {
+            if (i * kBytes < left) {
+                const unsigned v = kBytes == 2 ? reinterpret_cast<const unsigned short *>(src)[i] : src[i];
+                w[i * kBytes / 4] |= v << (8 * (i * kBytes % 4));
+            }
+        }
+    }
+    reinterpret_cast<uint4 *>(static_cast<unsigned char *>(dst_base) + (flat * pb.dst_batch + row * ldd) * kBytes)[piece] =
+        make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// fp32 rows -> TF32 planes, four columns per thread
+__global__ void __launch_bounds__(256) split_rows_kernel(const float *src_base, long long k, long long s_row, float *dst_base,
+                                                         long long ldd, long long k_pad, int is_weight, const PackBatch pb)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long kk = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 4;
+    const long long row = blockIdx.y + static_cast<long long>(gridDim.y) * (blockIdx.z % pb.row_slices);
+    const long long flat = blockIdx.z / pb.row_slices;
+    if (kk >= k_pad || row >= pb.rows) {
+        return;
+    }
+    const float *src = src_base + src_batch_offset(pb, flat) + row * s_row + kk;
+    float v[4];
+    if (kk + 4 <= k && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+        const float4 x = *reinterpret_cast<const float4 *>(src);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = kk + i < k ? src[i] : 0.0f;
+        }
+    }
+    float hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        hi[i] = to_tf32(v[i]);
+        lo[i] = to_tf32(v[i] - hi[i]);
+    }
+    const float4 h = make_float4(hi[0], hi[1], hi[2], hi[3]), l = make_float4(lo[0], lo[1], lo[2], lo[3]);
+    float *dst = dst_base + flat * pb.dst_batch + row * ldd + kk;
+    *reinterpret_cast<float4 *>(dst) = is_weight ? h : l;
+    *reinterpret_cast<float4 *>(dst + k_pad) = is_weight ? l : h;
+    *reinterpret_cast<float4 *>(dst + 2 * k_pad) = h;
+}
+
 // one thread per 16-byte chunk of the destination
 __global__ void __launch_bounds__(256) pack_blocks_kernel(const unsigned short *src, long long rows, long long k, long long ld,
                                                           uint4 *dst, long long nkb, long long total_chunks)
@@ -156,13 +233,39 @@ cudaError_t launch_pack_blocks(const void *src, long long rows, long long k, lon
     return cudaGetLastError();
 }
 
+namespace {
+
+// Grid of the row kernels: 256 pieces x a row x (batch entry, slice of 65535 rows); false when it does not fit.
+bool row_grid(long long pieces, long long rows, PackBatch *pb, dim3 *grid)
+{
+    const long long y = rows < 65535 ? rows : 65535;
+    const long long slices = (rows + y - 1) / y;
+    if (slices * pb->count > 65535) {
+        return false;
+    }
+    pb->rows = rows;
+    pb->row_slices = slices;
+    *grid = dim3(static_cast<unsigned>((pieces + 255) / 256), static_cast<unsigned>(y), static_cast<unsigned>(slices * pb->count));
+    return true;
+}
+
+}  // namespace
+
 cudaError_t launch_pack_kmajor(const void *src, int src_dtype, long long rows, long long k, long long s_row,
                                long long s_k, void *dst, int dst_dtype, long long ldd, long long k_pad,
                                cudaStream_t stream, const PackBatch *batch)
 {
     const PackBatch one = {1, 1, 1, {0, 0, 0}, 0};
     const PackBatch &pb = batch != nullptr ? *batch : one;
-    dim3 grid(static_cast<unsigned>((rows + 31) / 32), static_cast<unsigned>((k_pad + 31) / 32), static_cast<unsigned>(pb.count));
+    dim3 grid;
+    const int es = dtype_size(dst_dtype), vec = 16 / es;
+    PackBatch by_row = pb;
+    if (s_k == 1 && src_dtype == dst_dtype && es < 4 && k_pad % vec == 0 && ldd % vec == 0 && pb.dst_batch % vec == 0 &&
+        (reinterpret_cast<uintptr_t>(dst) & 15u) == 0 && row_grid(k_pad / vec, rows, &by_row, &grid)) {
+        return es == 2 ? launch_chained(pack_rows_kernel<2>, grid, dim3(256), 0, stream, 1, src, k, s_row, dst, ldd, k_pad / vec, by_row)
+                       : launch_chained(pack_rows_kernel<1>, grid, dim3(256), 0, stream, 1, src, k, s_row, dst, ldd, k_pad / vec, by_row);
+    }
+    grid = dim3(static_cast<unsigned>((rows + 31) / 32), static_cast<unsigned>((k_pad + 31) / 32), static_cast<unsigned>(pb.count));
     if (grid.y > 65535 || pb.count > 65535) {
         return cudaErrorInvalidValue;
     }
@@ -175,7 +278,14 @@ cudaError_t launch_split_tf32(const void *src, long long rows, long long k, long
 {
     const PackBatch one = {1, 1, 1, {0, 0, 0}, 0};
     const PackBatch &pb = batch != nullptr ? *batch : one;
-    dim3 grid(static_cast<unsigned>((rows + 31) / 32), static_cast<unsigned>((k_pad + 31) / 32), static_cast<unsigned>(pb.count));
+    dim3 grid;
+    PackBatch by_row = pb;
+    if (s_k == 1 && k_pad % 4 == 0 && ldd % 4 == 0 && pb.dst_batch % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0 &&
+        row_grid(k_pad / 4, rows, &by_row, &grid)) {
+        return launch_chained(split_rows_kernel, grid, dim3(256), 0, stream, 1, static_cast<const float *>(src), k, s_row, dst, ldd, k_pad,
+                              is_weight, by_row);
+    }
+    grid = dim3(static_cast<unsigned>((rows + 31) / 32), static_cast<unsigned>((k_pad + 31) / 32), static_cast<unsigned>(pb.count));
     if (grid.y > 65535 || pb.count > 65535) {
         return cudaErrorInvalidValue;
     }

@@ -56,6 +56,140 @@ __device__ __forceinline__ void epilogue_int(const EpiParams &p, int acc, long l
     c[ic] = static_cast<int>(r);
 }
 
+// ---- the same product for problems of few tiles, where latency counts: 32 x 32 outputs per CTA, and K cut between four
+// groups of 64 threads.  A group advances 16 k at a time on its own (a named barrier), with the next step's operands on
+// their way to registers while the current one is multiplied; the four partial sums are added in group order, and each of
+// the 256 threads finishes four outputs.  Bound by the round trips to memory: one per 64 k, one for the side inputs.
+constexpr int kSmallTile = 32;
+constexpr int kSmallGroups = 4;
+constexpr int kSmallPitch = kSmallTile + 4;
+
+__global__ void __launch_bounds__(256) simt_small_kernel(const SimtParams p)
+{
+    __shared__ __align__(16) float sa[kSmallGroups][kStepK][kSmallPitch];
+    __shared__ __align__(16) float sb[kSmallGroups][kStepK][kSmallPitch];
+    __shared__ __align__(16) float sums[kSmallGroups][kSmallTile][kSmallPitch];
+
+    const int tid = threadIdx.x;
+    const int group = tid / 64, t = tid % 64;
+    const int tx = t % 8, ty = t / 8;
+    const long long m0 = static_cast<long long>(blockIdx.y) * kSmallTile;
+    const long long n0 = static_cast<long long>(blockIdx.x) * kSmallTile;
+
+    pdl_launch_dependents();
+    long long bidx[3];
+    batch_decompose(p.batch, blockIdx.z, bidx);
+    const void *a = offset_ptr(p.a, p.a_dtype, batch_offset(p.batch.a_sb, bidx));
+    const void *b = offset_ptr(p.b, p.b_dtype, batch_offset(p.batch.b_sb, bidx));
+    pdl_wait();
+
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            acc[i][j] = 0.0f;
+        }
+    }
+
+    // this thread's 8 elements of each operand per step: the walk order follows whichever stride is unit
+    const bool a_by_k = p.a_sk == 1, b_by_k = p.b_sk == 1;
+    const int a_r = a_by_k ? t / kStepK : t % kSmallTile, a_k = a_by_k ? t % kStepK : t / kSmallTile;
+    const int b_r = b_by_k ? t / kStepK : t % kSmallTile, b_k = b_by_k ? t % kStepK : t / kSmallTile;
+    const int a_dr = a_by_k ? 64 / kStepK : 0, a_dk = a_by_k ? 0 : 64 / kSmallTile;
+    const int b_dr = b_by_k ? 64 / kStepK : 0, b_dk = b_by_k ? 0 : 64 / kSmallTile;
+    float va[8], vb[8];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const long long ra = m0 + a_r + e * a_dr, ka = k0 + a_k + e * a_dk;
+            const long long rb = n0 + b_r + e * b_dr, kb = k0 + b_k + e * b_dk;
+            va[e] = ra < p.m && ka < p.k ? load_as_f32(a, p.a_dtype, ra * p.a_sm + ka * p.a_sk) : 0.0f;
+            vb[e] = rb < p.n && kb < p.k ? load_as_f32(b, p.b_dtype, rb * p.b_sn + kb * p.b_sk) : 0.0f;
+        }
+    };
+    int k0 = group * kStepK;
+    if (k0 < p.k) {
+        fetch(k0);
+    }
+    for (; k0 < p.k; k0 += kSmallGroups * kStepK) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            sa[group][a_k + e * a_dk][a_r + e * a_dr] = va[e];
+            sb[group][b_k + e * b_dk][b_r + e * b_dr] = vb[e];
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory");
+        if (k0 + kSmallGroups * kStepK < p.k) {
+            fetch(k0 + kSmallGroups * kStepK);
+        }
+#pragma unroll
+        for (int kk = 0; kk < kStepK; ++kk) {
+            const float4 av = *reinterpret_cast<const float4 *>(&sa[group][kk][ty * 4]);
+            const float4 bv = *reinterpret_cast<const float4 *>(&sb[group][kk][tx * 4]);
+            const float x[4] = {av.x, av.y, av.z, av.w}, y[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+                }
+            }
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory");
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        *reinterpret_cast<float4 *>(&sums[group][ty * 4 + i][tx * 4]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+    __syncthreads();
+
+    const int row = tid / 8, col = (tid % 8) * 4;
+    const long long mi = m0 + row;
+    if (mi >= p.m || n0 + col >= p.n) {
+        return;
+    }
+    const EpiParams &e = p.epi;
+    void *c = offset_ptr(e.c, e.c_dtype, batch_offset(p.batch.c_sb, bidx));
+    const void *bias = offset_ptr(e.bias, e.bias_dtype, batch_offset(p.batch.bias_sb, bidx));
+    const void *res = offset_ptr(e.res, e.res_dtype, batch_offset(p.batch.res_sb, bidx));
+    void *out = offset_ptr(e.out, e.out_dtype, batch_offset(p.batch.out_sb, bidx));
+    float old[4], bv[4], rv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const long long ni = n0 + col + j;
+        old[j] = bv[j] = rv[j] = 0.0f;
+        if (ni < p.n) {
+            if (e.beta != 0.0f && c != nullptr) {
+                old[j] = load_as_f32(c, e.c_dtype, mi * e.c_sm + ni * e.c_sn);
+            }
+            if (e.has_bias) {
+                bv[j] = load_as_f32(bias, e.bias_dtype, mi * e.bias_sm + ni * e.bias_sn);
+            }
+            if (e.res_op != KUDNN_B200_RES_NONE) {
+                rv[j] = load_as_f32(res, e.res_dtype, mi * e.res_sm + ni * e.res_sn);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const long long ni = n0 + col + j;
+        if (ni < p.n) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int g = 0; g < kSmallGroups; ++g) {
+                sum += sums[g][row][col + j];
+            }
+            const EpiResult r = finish_element(e, sum, old[j], bv[j], rv[j]);
+            if (c != nullptr) {
+                store_exact_mirrored(c, e.c_dtype, mi * e.c_sm + ni * e.c_sn, r.c, e.n_mirrors, e.c_delta);
+            }
+            if (e.res_op != KUDNN_B200_RES_NONE) {
+                store_exact_mirrored(out, e.out_dtype, mi * e.out_sm + ni * e.out_sn, r.out, e.n_mirrors, e.out_delta);
+            }
+        }
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) simt_linear_kernel(const SimtParams p)
 {
@@ -194,6 +328,19 @@ static cudaError_t launch_general(const LinearProblem &pr, cudaStream_t stream, 
         // so a slice start is folded into the outermost batch stride only when it divides evenly
         if (z0 != 0) {
             return cudaErrorInvalidValue;
+        }
+        // Few tiles: the small kernel (times of a call in a chain, us, small / large tiles: 113 x 198 x 246 18.5 / 60.6, 21 x 512 x 23
+        // 7.4 / 24.2, both fp32 with SiLU).  From two waves of 64 x 64 tiles on, their four times lower operand traffic counts.
+        const long long large_tiles = ((pr.n + kTile - 1) / kTile) * ((pr.m + kTile - 1) / kTile) * nbatch;
+        const long long small_rows = (pr.m + kSmallTile - 1) / kSmallTile;
+        if (!integer && large_tiles < 2 * 148 && small_rows <= 65535) {
+            const dim3 small_grid(static_cast<unsigned>((pr.n + kSmallTile - 1) / kSmallTile), static_cast<unsigned>(small_rows),
+                                  static_cast<unsigned>(nbatch));
+            cudaError_t e = launch_chained(simt_small_kernel, small_grid, dim3(256), 0, stream, 1, p);
+            if (e != cudaSuccess) {
+                return e;
+            }
+            continue;
         }
         dim3 grid(static_cast<unsigned>((pr.n + kTile - 1) / kTile), static_cast<unsigned>((pr.m + kTile - 1) / kTile),
                   static_cast<unsigned>(nbatch < 65535 ? nbatch : 65535));
