@@ -513,6 +513,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             if (packed) {
                 ops.b = h->packed_ptr;
                 ops.ldb = h->packed_ld;
+                ops.b_stable = true;
             } else if (kmajor_ready(args.b, d.b_dtype, d.b_sn, d.b_sk, d.n)) {
                 ops.b = args.b;
                 ops.ldb = d.b_sn;
@@ -726,7 +727,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
     const bool tc_types = d.a_dtype == d.b_dtype;
     // fp32 takes two launches there (the activations are split first): 76 x 1562 x 73 with GELU, 8.7e6 products, 23 us against
     // 10 us on the general kernel; 31 x 1817 x 151, 8.5e6, 13.6 against 12.4 us
-    const double tc_from = d.a_dtype == KUDNN_B200_F32 ? 16.0e6 : 8.0e6;
+    const double tc_from = d.a_dtype == KUDNN_B200_F32 && nb == 1 ? 16.0e6 : 8.0e6;
     const bool tc_worth = static_cast<double>(d.m) * d.n * d.k * static_cast<double>(nb) >= tc_from && d.k >= 32;
     const bool tc_batch_ok = nb == 1 || (nb <= 65535 && pr.epi.n_mirrors == 0);
     if (tc_batch_ok && tc_types && (forced == KUDNN_B200_KERNEL_TC || (forced == KUDNN_B200_KERNEL_AUTO && tc_worth))) {
@@ -800,6 +801,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.b = h->packed_ptr;
                 ops.ldb = h->packed_ld;
                 ops.k_total = h->packed_ktotal;
+                ops.b_stable = true;
             } else if (!f32 && kmajor_ready(args.b, d.b_dtype, d.b_sn, d.b_sk, d.n) && flat_stride(d.b_sb, &bstride)) {
                 ops.b = args.b;
                 ops.ldb = d.b_sn;

@@ -202,7 +202,7 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     // 13.3 / 12.4).
     const double flops = 2.0 * static_cast<double>(m) * static_cast<double>(n) * static_cast<double>(ops.k_total);
     // batched launches use single CTAs, and so do outputs that cannot be stored as vectors
-    bool pair = n > kBM && m > kBM && flops < 6.0e12 && ops.batch == 1 && (rows == TcRows::kVectors || ints) && forced_splits <= 1 &&
+    bool pair = n > kBM && m > kBM && (flops < 6.0e12 || env_choice("KUDNN_B200_TC_PAIR") > 0) && ops.batch == 1 && (rows == TcRows::kVectors || ints) && forced_splits <= 1 &&
                 env_choice("KUDNN_B200_TC_PAIR") != 0;
     const int pair_stages = with_staging ? 5 : 6;
     plan->narrow_from = 0;
@@ -322,6 +322,7 @@ cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams
     p.kb_per_split = plan.kb_per_split;
     p.stages = plan.stages;
     p.bn = plan.block_n;
+    p.b_stable = ops.b_stable ? 1 : 0;
     p.a_rows = plan.a_rows;
     p.ring_bytes = plan.ring_bytes;
     p.via_smem = plan.via_smem;

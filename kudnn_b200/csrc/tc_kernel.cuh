@@ -70,6 +70,7 @@ struct TcParams {
     // rows that come of it are never read.
     int bn, a_rows;
     int ring_bytes;  // bytes in front of the barriers: the stage ring, and room for one tile as fp32 if it is finished from there
+    int b_stable;  // the weights were pre-packed: the first of them are loaded while the previous kernel still runs
     int via_smem;    // one work item per CTA, finished from shared memory (finish_rows)
     int vector_rows;  // every row of the epilogue's tensors can be read and written 16 bytes at a time, beta = 0
     int group_m;  // tile rows per raster group: consecutive work items walk down group_m tile rows, then one tile right
@@ -1508,7 +1509,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_wait();  // nothing before this line reads or writes global memory
     // work items: tiles (x splits) over CTAs, or pair tiles over clusters of two
     const uint32_t pair_rank = kPair ? cluster_rank() : 0u;
     const int first_item = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
@@ -1519,6 +1519,39 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
+            // Pre-packed weights of the first work item fill the ring before the previous kernel has ended.  The stages are
+            // announced in full; the activations join them below.
+            int early = 0;
+            if (p.b_stable != 0 && p.skip_kb < 0 && first_item < p.num_items) {
+                int tile, n_off, width, batch, split;
+                decode_item<kPair, kBN>(p, first_item, tile, n_off, width, batch, split);
+                const int kb_begin = split * p.kb_per_split;
+                const int kb_end = (kb_begin + p.kb_per_split < p.num_kb) ? kb_begin + p.kb_per_split : p.num_kb;
+                const int per_group = p.group_m * p.tiles_n;
+                const int first_m = tile / per_group * p.group_m;
+                const int gsize = (p.tiles_m - first_m < p.group_m) ? (p.tiles_m - first_m) : p.group_m;
+                const int row = (tile % per_group) / gsize * p.bn;
+                early = kb_end - kb_begin < kStages ? kb_end - kb_begin : kStages;
+                for (int i = 0; i < early; ++i) {
+                    unsigned char *sb = smem + i * stage_bytes + a_bytes;
+                    const int x = (kb_begin + i) * kElemsPerRow;
+                    if (kPair) {
+                        if (pair_rank == 0) {
+                            mbar_expect_tx(full_bar + i, 2 * stage_bytes);
+                        }
+                        tma_load_2d_pair(sb, &tmap_b, map_to_rank(smem_u32(full_bar + i), 0u), x,
+                                         row + n_off + static_cast<int>(pair_rank) * (width / 2));
+                    } else {
+                        mbar_expect_tx(full_bar + i, stage_bytes);
+                        if (p.batch > 1) {
+                            tma_load_3d(sb, &tmap_b, full_bar + i, x, row, p.b_bz != 0 ? batch : 0);
+                        } else {
+                            tma_load_2d(sb, &tmap_b, full_bar + i, x, row);
+                        }
+                    }
+                }
+            }
+            pdl_wait();
             int stage = 0;
             uint32_t phase = 0;
             bool alive = true;
@@ -1547,24 +1580,33 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         // test hook: this stage is never filled
                     } else if (kPair) {
                         // both CTAs' bytes are counted on the leader's barrier; only the leader announces them
-                        if (pair_rank == 0) {
+                        if (pair_rank == 0 && early == 0) {
                             mbar_expect_tx(full_bar + stage, 2 * stage_bytes);
                         }
                         const uint32_t leader_bar = map_to_rank(smem_u32(full_bar + stage), 0u);
                         tma_load_2d_pair(sa, &tmap_a, leader_bar, kb * kElemsPerRow, tm * kBM);
                         // this CTA's half of the piece's B rows (a narrow piece uses the first half of the box only)
-                        tma_load_2d_pair(sb, &tmap_b, leader_bar, kb * kElemsPerRow,
-                                         tn * p.bn + n_off + static_cast<int>(pair_rank) * (width / 2));
+                        if (early == 0) {
+                            tma_load_2d_pair(sb, &tmap_b, leader_bar, kb * kElemsPerRow,
+                                             tn * p.bn + n_off + static_cast<int>(pair_rank) * (width / 2));
+                        }
                     } else {
-                        mbar_expect_tx(full_bar + stage, stage_bytes);
+                        if (early == 0) {
+                            mbar_expect_tx(full_bar + stage, stage_bytes);
+                        }
                         if (p.batch > 1) {
                             tma_load_3d(sa, &tmap_a, full_bar + stage, kb * kElemsPerRow, tm * kBM, p.a_bz != 0 ? batch : 0);
-                            tma_load_3d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * p.bn, p.b_bz != 0 ? batch : 0);
+                            if (early == 0) {
+                                tma_load_3d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * p.bn, p.b_bz != 0 ? batch : 0);
+                            }
                         } else {
                             tma_load_2d(sa, &tmap_a, full_bar + stage, kb * kElemsPerRow, tm * kBM);
-                            tma_load_2d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * p.bn);
+                            if (early == 0) {
+                                tma_load_2d(sb, &tmap_b, full_bar + stage, kb * kElemsPerRow, tn * p.bn);
+                            }
                         }
                     }
+                    early = early > 0 ? early - 1 : 0;
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1u;
@@ -1638,6 +1680,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
     } else if (warp < 2 + p.epi_warps) {
         // ------------------------------------------------------------------ epilogue warps
+        pdl_wait();
         const int quarter = warp & 3;  // TMEM lanes this warp may touch: [32 * quarter, 32 * quarter + 32)
         const int row_in_tile = quarter * 32 + lane;
         const int part = (warp - 2) / 4;  // warps sharing a quarter split the tile's columns between them
