@@ -506,9 +506,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
     if (p.w_stable == 0) {
         pdl_wait();
     }
-    // the first weights are requested before anything else, so HBM is already busy while the activations load
+    // The first weights are requested before anything else, so HBM is already busy while the activations load.  Not 8-bit ones:
+    // the loop that takes them over is slower by more than that gains (4 x 28672 x 8192 61.8 against 63.0 us).
+    constexpr bool kEarly = kW8 == 0;
     uint4 wv[kUnroll][kWide && kW8 == 0 ? 2 : 1];
-    bool preloaded = active && f < f_end;
+    bool preloaded = kEarly && active && f < f_end;
     if (preloaded) {
         long long group;
         int kb0;
@@ -547,7 +549,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
 
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         for (int i = 0; i < nb; i += kUnroll) {
-            if (!preloaded) {
+            if (!kEarly || !preloaded) {
                 load_batch(wv, group, kb0, i, nb);
             }
             preloaded = false;
