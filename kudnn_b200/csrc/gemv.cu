@@ -370,12 +370,14 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], unsigned a0, unsigned a
 // y[gid + 8][...] in acc[2..3].  A group that one warp covered alone goes straight to the epilogue; otherwise the
 // partial tile goes to the warp's slot and the last arrival adds all slots in slot order, kInFlight loads at a time (four where
 // the kernel has the registers: 4 x 28672 x 8192 with two chunks 79.4 -> 78.7 us; one where they cost a spill, 84 against 85 us).
-template <int kInFlight>
+// kSwap: the weights are the 16-row operand; the lane holds y[2*tig + {0,1}][n0] in acc[0..1] and [..][n0 + 8] in acc[2..3]
+// with n0 = group * 16 + gid.
+template <int kInFlight, bool kSwap = false>
 __device__ __forceinline__ void mma_finish_group(const GemvParams &p, float (&acc)[4], long long group, int chunk, int warp,
                                                  int lane)
 {
     const int gid = lane >> 2, tig = lane & 3;
-    const long long n0 = group * 8 + tig * 2;
+    const long long n0 = kSwap ? group * 16 + gid : group * 8 + tig * 2;
     const long long first_blk = group * p.kb;
     const int w0 = static_cast<int>(first_blk / p.span);
     const int w1 = static_cast<int>((first_blk + p.kb - 1) / p.span);
@@ -432,8 +434,8 @@ __device__ __forceinline__ void mma_finish_group(const GemvParams &p, float (&ac
     if (finish) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int mi = gid + ((e >= 2) ? 8 : 0);
-            const long long ni = n0 + (e & 1);
+            const int mi = kSwap ? tig * 2 + (e & 1) : gid + ((e >= 2) ? 8 : 0);
+            const long long ni = kSwap ? n0 + ((e >= 2) ? 8 : 0) : n0 + (e & 1);
             if (mi < p.m && ni < p.n) {
                 epilogue_scalar(p.epi, acc[e], mi, ni);
             }
@@ -445,7 +447,10 @@ __device__ __forceinline__ void mma_finish_group(const GemvParams &p, float (&ac
 // kWide: a block is 8 rows x 64 k and a lane loads 32 consecutive bytes of its row (two 16-byte loads), feeding four
 // MMAs; a warp instruction then touches 8 rows x 128 bytes instead of 8 x 64, which HBM serves about 5 % faster.
 // kW8 (1 signed, 2 unsigned; with kWide and fp16): the weights are 8-bit integers read as they are, 16 bytes = 16 values
-// of a row per lane and block, and widened to fp16 in registers; the activations are laid out as for kWide.
+// of a row per lane and block, and widened to fp16 in registers; the activations are laid out as for kWide.  With up to 8
+// activation rows the operands change places: 16 weight rows are the M = 16 operand and the activations the N = 8 one, so
+// that an MMA multiplies 256 weights instead of 128.  At half the bytes per weight the rate of mma.sync was the limit:
+// 4 x 28672 x 8192 61.8 -> 52.5 us.
 template <int kDtype, bool kRows16, bool kWide, int kUnroll, int kThreads, int kMinBlocks, int kW8 = 0>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const GemvParams p)
 {
@@ -453,6 +458,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
     constexpr int kRows = kRows16 ? 16 : 8;
     constexpr int kBlockK = kWide ? 64 : 32;
     constexpr int kLaneBytes = kWide ? 32 : 16;
+    constexpr bool kSwap = kW8 != 0 && !kRows16;
+    constexpr int kLoads = kSwap || (kWide && kW8 == 0) ? 2 : 1;  // 16-byte loads per lane and block
     // row pitch of the activations in shared memory: the skew keeps the 8 lanes of a 16-byte load phase on distinct banks
     const int row_bytes = p.kc * 2 + (kWide ? 16 : kMmaRowPadBytes);
     const int chunk = blockIdx.x % p.ksplit;
@@ -468,7 +475,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
     const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
 
     // this lane's share of blocks kb0 + i .. of a group, zeros past the piece, the rows and k
-    auto load_batch = [&](uint4 (&wv)[kUnroll][kWide && kW8 == 0 ? 2 : 1], long long group, int kb0, int i, int nb) {
+    auto load_batch = [&](uint4 (&wv)[kUnroll][kLoads], long long group, int kb0, int i, int nb) {
         const long long wrow_idx = group * 8 + gid;
         const bool row_ok = wrow_idx < p.n;
         const unsigned short *wrow = static_cast<const unsigned short *>(p.w) + wrow_idx * p.w_ld + kc0 + tig * (kLaneBytes / 2);
@@ -477,9 +484,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
         for (int u = 0; u < kUnroll; ++u) {
             const int kloc = (kb0 + i + u) * kBlockK;
 #pragma unroll
-            for (int h = 0; h < (kWide && kW8 == 0 ? 2 : 1); ++h) {
+            for (int h = 0; h < kLoads; ++h) {
                 wv[u][h] = make_uint4(0u, 0u, 0u, 0u);
-                if (kW8 != 0) {
+                if (kSwap) {
+                    const long long row = group * 16 + gid + 8 * h;
+                    if (i + u < nb && row < p.n && (kc0 + kloc + tig * 16) < p.k) {
+                        wv[u][h] = ld_stream_16(static_cast<const unsigned char *>(p.w) + row * p.w_ld + kc0 + tig * 16 + kloc);
+                    }
+                } else if (kW8 != 0) {
                     if (i + u < nb && row_ok && (kc0 + kloc + tig * 16) < p.k) {
                         wv[u][h] = ld_stream_16(wrow8 + kloc);
                     }
@@ -509,7 +521,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
     // The first weights are requested before anything else, so HBM is already busy while the activations load.  Not 8-bit ones:
     // the loop that takes them over is slower by more than that gains (4 x 28672 x 8192 61.8 against 63.0 us).
     constexpr bool kEarly = kW8 == 0;
-    uint4 wv[kUnroll][kWide && kW8 == 0 ? 2 : 1];
+    uint4 wv[kUnroll][kLoads];
     bool preloaded = kEarly && active && f < f_end;
     if (preloaded) {
         long long group;
@@ -564,7 +576,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
                         if (kRows16) {
                             xb = *reinterpret_cast<const uint4 *>(xb_row + kloc * 2 + h * 16);
                         }
-                        if (kW8 != 0) {
+                        if (kSwap) {
+                            // words 2h and 2h + 1 of both rows' 16 values; xa holds the activations that meet them
+                            unsigned l0, l1, h0, h1;
+                            unpack4_i8_h2<kW8 == 1>(h == 0 ? wv[u][0].x : wv[u][0].z, l0, l1);
+                            unpack4_i8_h2<kW8 == 1>(h == 0 ? wv[u][kLoads - 1].x : wv[u][kLoads - 1].z, h0, h1);
+                            mma_16816<kDtype>(acc, l0, h0, l1, h1, xa.x, xa.y);
+                            unpack4_i8_h2<kW8 == 1>(h == 0 ? wv[u][0].y : wv[u][0].w, l0, l1);
+                            unpack4_i8_h2<kW8 == 1>(h == 0 ? wv[u][kLoads - 1].y : wv[u][kLoads - 1].w, h0, h1);
+                            mma_16816<kDtype>(acc, l0, h0, l1, h1, xa.z, xa.w);
+                        } else if (kW8 != 0) {
                             // values 8h .. 8h + 7 of the lane's 16: two words of the one load
                             unsigned c0, c1, c2, c3;
                             unpack4_i8_h2<kW8 == 1>(h == 0 ? wv[u][0].x : wv[u][0].z, c0, c1);
@@ -580,7 +601,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
             }
         }
 
-        mma_finish_group<1>(p, acc, group, chunk, warp, lane);
+        mma_finish_group<1, kSwap>(p, acc, group, chunk, warp, lane);
         f += nb;
     }
 }
@@ -854,7 +875,9 @@ cudaError_t launch_mma_rows(const GemvParams &p, const GemvPlan &plan, cudaStrea
     if (p.w8 != 0) {
         if constexpr (kDtype == KUDNN_B200_F16) {
 #define KB_W8_CASE(ROWS16, SIGN) \
-    launch_gemv_kernel(gemv_mma_kernel<kDtype, ROWS16, true, kUnroll, kThreads, kMinBlocks, SIGN>, p, plan, stream)
+    launch_gemv_kernel(gemv_mma_kernel<kDtype, ROWS16, true, (ROWS16 ? kUnroll : kSwapUnroll), kThreads, kMinBlocks, SIGN>, p, plan, stream)
+            // one block (two loads per lane) at a time: 4 x 28672 x 8192 52.5 us, with two, three and four 54.0, 60.2, 58.2
+            constexpr int kSwapUnroll = 1;
             if (p.m > 8) {
                 return p.w8 == 1 ? KB_W8_CASE(true, 1) : KB_W8_CASE(true, 2);
             }
@@ -1036,7 +1059,8 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
     // off (0), KUDNN_B200_GEMV_WIDE=0 makes the fragment-shaped loads 16 bytes per lane.
     const int staged_env = env_int("KUDNN_B200_GEMV_STAGED", -1);
     const bool staged = !w8 && (staged_env < 0 ? (rows == 8 && pr.b_blocked != nullptr) : staged_env != 0);
-    const long long groups = (pr.n + 7) / 8;
+    const bool swapped = w8 && rows == 8;  // groups of 16 weight rows (see gemv_mma_kernel)
+    const long long groups = swapped ? (pr.n + 15) / 16 : (pr.n + 7) / 8;
     // With fixed scratch: the fewest chunks that fit, and a group of rows cut at most once per chunk boundary.
     auto finish_plan = [&](int shape, int ksplit, long long kc, long long block_k, int ctas, int warps, long long min_span, size_t smem) {
         const long long kbc = kc / block_k;
@@ -1060,6 +1084,14 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
         plan->smem_bytes = smem;
         plan->partial_floats = groups * ksplit * plan->slots * 128;
         plan->counter_count = groups;
+        if (fixed_scratch && swapped) {
+            // what groups of 8 rows would take, so that the same problems fit the fixed scratch whatever the group
+            const long long eighths = (pr.n + 7) / 8, total = eighths * kbc;
+            const long long active = std::max<long long>(std::min<long long>(static_cast<long long>(std::max(ctas / ksplit, 1)) * warps, 2 * eighths), 1);
+            const long long span = (total + active - 1) / active;
+            plan->partial_floats = std::max<long long>(plan->partial_floats, eighths * ksplit * ((kbc + span - 1) / span + 1) * 128);
+            plan->counter_count = eighths;
+        }
     };
     auto chunk_len = [&](int parts, long long block_k) { return ((pr.k + parts - 1) / parts + block_k - 1) / block_k * block_k; };
     auto fewest_chunks = [&](long long block_k, size_t budget) {
@@ -1094,7 +1126,7 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
     // 16 activation rows: blocks of 64 k with 32 bytes per lane (see gemv_mma_kernel)
     const bool wide = w8 || (rows == 16 && env_int("KUDNN_B200_GEMV_WIDE", 1) != 0);
     const long long block_k = wide ? 64 : 32;
-    const long long block_bytes = 8 * block_k * (w8 ? 1 : 2);
+    const long long block_bytes = (swapped ? 16 : 8) * block_k * (w8 ? 1 : 2);
     const int warps = kShapes[shape].threads / 32;
     const long long min_span = 4096 / block_bytes;  // at least 4 KB of weights per warp
     int ksplit = fixed_scratch ? 0
@@ -1175,7 +1207,7 @@ cudaError_t launch_gemv(const LinearProblem &pr, const GemvPlan &plan, const Gem
     const long long kc = ((pr.k + plan.ksplit - 1) / plan.ksplit + block_k - 1) / block_k * block_k;
     p.kc = static_cast<int>(kc);
     p.kb = static_cast<int>(kc / block_k);
-    p.total = ((pr.n + 7) / 8) * p.kb;
+    p.total = (w8 && pr.m <= 8 ? (pr.n + 15) / 16 : (pr.n + 7) / 8) * p.kb;
     if (pr.a_dtype == KUDNN_B200_F16) {
         return launch_shape<KUDNN_B200_F16, false>(p, plan, plan.shape, stream);
     }
