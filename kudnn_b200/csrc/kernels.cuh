@@ -15,7 +15,7 @@ struct LinearProblem {
     // the weights once more in the decode-packed layout (see GemvParams::w_blk in gemv.cu), or null
     const void *b_blocked = nullptr;
     long long b_blocked_kpad = 0;
-    bool b_stable = false;  // b was pre-packed: no kernel on the stream writes it
+    bool b_stable = false;  // b is a pre-packed copy: no kernel on the stream writes it
     EpiParams epi;
     BatchParams batch;
     long long batch_count;
@@ -64,7 +64,7 @@ struct TcOperands {
     int a_signed = 1, b_signed = 1;  // kind _S8 only: whether each operand holds signed values
     // batched problems: `batch` matrices per operand, a_bstride / b_bstride elements apart (0: every entry shares one)
     long long batch = 1, a_bstride = 0, b_bstride = 0;
-    bool b_stable = false;  // b was pre-packed: no kernel on the stream writes it
+    bool b_stable = false;  // b is a pre-packed copy: no kernel on the stream writes it
 };
 // How the epilogue meets its tensors: every row 16 bytes at a time (and beta = 0), rows whose elements are contiguous but
 // start anywhere, or neither.

@@ -310,6 +310,13 @@ bool kmajor_ready(const void *p, int dtype, long long s_row, long long s_k, long
     return s_k == 1 && aligned16(p) && (rows == 1 || s_row % vec == 0);
 }
 
+// Whether the packed weights are a copy that only pre-packing writes (and waits for).  Weights used in place are the caller's:
+// a kernel in front of a run may still be writing them, so nothing of them is read ahead of that kernel's end.
+bool owns_packed(const Handle *h)
+{
+    return h->packed_ptr != nullptr && h->packed_ptr == h->b_packed.ptr;
+}
+
 // How the tensor-core epilogue can read and write the rows of c, bias, res and out.
 kb::TcRows epilogue_rows(const kb::LinearProblem &pr)
 {
@@ -513,7 +520,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             if (packed) {
                 ops.b = h->packed_ptr;
                 ops.ldb = h->packed_ld;
-                ops.b_stable = true;
+                ops.b_stable = owns_packed(h);
             } else if (kmajor_ready(args.b, d.b_dtype, d.b_sn, d.b_sk, d.n)) {
                 ops.b = args.b;
                 ops.ldb = d.b_sn;
@@ -600,7 +607,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             a8.b = w8;
             kb::LinearProblem p8;
             fill_problem(d8, a8, &p8);
-            p8.b_stable = packed8;
+            p8.b_stable = packed8 && owns_packed(h);
             kb::GemvPlan plan8;
             if (kb::gemv_plan(p8, h->sm_count, forced8, false, &plan8)) {
                 kb::GemvWorkspace ws8;
@@ -689,7 +696,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
         pr.b = h->packed_raw;
         pr.b_sk = 1;
         pr.b_sn = h->packed_ld;
-        pr.b_stable = true;
+        pr.b_stable = owns_packed(h) || h->blocked_kpad > 0;
         if (h->blocked_kpad > 0) {
             pr.b_blocked = h->b_blocked.ptr;
             pr.b_blocked_kpad = h->blocked_kpad;
@@ -801,7 +808,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.b = h->packed_ptr;
                 ops.ldb = h->packed_ld;
                 ops.k_total = h->packed_ktotal;
-                ops.b_stable = true;
+                ops.b_stable = owns_packed(h);
             } else if (!f32 && kmajor_ready(args.b, d.b_dtype, d.b_sn, d.b_sk, d.n) && flat_stride(d.b_sb, &bstride)) {
                 ops.b = args.b;
                 ops.ldb = d.b_sn;

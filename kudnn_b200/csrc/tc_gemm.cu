@@ -179,7 +179,9 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
             if (forced_splits >= 1 && sp > forced_splits) {
                 continue;
             }
-            const bool one_item = sp > 1 || (!ints && !with_staging && (tiles <= sm_count || rows == TcRows::kContiguous));
+            // (an output whose rows are not contiguous, column by column for one, leaves from the accumulator with a thread per row)
+            const bool one_item = sp > 1 || (!ints && !with_staging && rows != TcRows::kOther &&
+                                             (tiles <= sm_count || rows == TcRows::kContiguous));
             double cost = single_cta_cycles(tiles, sp, (num_kb + sp - 1) / sp, w, a_rows_single, one_item, sm_count);
             if (forced_splits >= 1 && sp * 2 <= forced_splits && sp * 2 <= kMaxSplits) {
                 cost *= 1e6;  // taken only if no larger cut fits
