@@ -1,0 +1,102 @@
+"""The launch shapes that depend on the problem's size: tile widths and K cuts of the tensor-core kernel with the tile finished
+from shared memory, the general kernel for few tiles, row packing, and the cuts of the streaming kernels.  Sizes sit at the
+edges: one row or column over a tile, rows that start anywhere, K shorter than a block, the last group of weight rows
+incomplete."""
+import numpy as np
+import pytest
+import torch
+
+import kudnn_b200 as kb
+from oracle import ko
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(cuda_device, kernel, **case):
+    case = dict(dict(x_dist="normal", w_std=0.05, seed=17), **case)
+    prepack = case.pop("prepack", False)
+    desc, arrays, c = helpers.build_case(case)
+    ref_c, ref_o = helpers.run_oracle(desc, arrays, c, acc=ko.ACC_F64)
+    got_c, got_o, used = helpers.run_gpu(desc, arrays, c, cuda_device, prepack=prepack)
+    assert used == kernel
+    if c["want_c"]:
+        helpers.compare(got_c, ref_c, desc.c_dtype)
+    if desc.res_op != kb.RES_NONE:
+        helpers.compare(got_o, ref_o, desc.out_dtype)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("m,n,k", [(17, 2561, 1030), (129, 1040, 2050), (333, 3001, 264), (257, 48, 4104), (24, 19208, 72)])
+@pytest.mark.parametrize("act,res_op", [(kb.ACT_GELU_ERF, kb.RES_NONE), (kb.ACT_NONE, kb.RES_IDENTICAL)])
+@pytest.mark.parametrize("layout", ["BA", "AB"])
+def test_tile_widths_and_cuts(cuda_device, dtype, m, n, k, act, res_op, layout):
+    _run(cuda_device, kb.KERNEL_TC, m=m, n=n, k=k, dtype=dtype, bias="row", act=act, res_op=res_op, b_layout=layout,
+         prepack=n % 2 == 0)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("splits", ["1", "2", "4", "8"])
+@pytest.mark.parametrize("n", [130, 136])
+@pytest.mark.parametrize("bias", ["row", "full"])
+def test_every_cut_of_k(cuda_device, monkeypatch, dtype, splits, n, bias):
+    monkeypatch.setenv("KUDNN_B200_TC_SPLITS", splits)
+    _run(cuda_device, kb.KERNEL_TC, m=133, n=n, k=1100, dtype=dtype, bias=bias, act=kb.ACT_SWISH, res_op=kb.RES_NONE)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("m,n,k", [(33, 65, 1), (31, 33, 15), (113, 198, 246), (64, 1600, 65), (18, 17, 300)])
+@pytest.mark.parametrize("layout", ["BA", "AB"])
+def test_few_tiles_on_the_general_kernel(cuda_device, dtype, m, n, k, layout):
+    _run(cuda_device, kb.KERNEL_SIMT, m=m, n=n, k=k, dtype=dtype, bias="row", act=kb.ACT_SWISH, res_op=kb.RES_IDENTICAL, b_layout=layout)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1000, 8200), (1, 70, 16384), (3, 520, 4104), (8, 1003, 6152), (9, 2000, 5896), (16, 24, 8192)])
+@pytest.mark.parametrize("prepack", [False, True])
+def test_streaming_cuts(cuda_device, m, n, k, prepack):
+    kernel = kb.KERNEL_GEMV_FMA if m == 1 else kb.KERNEL_GEMV_MMA
+    _run(cuda_device, kernel, m=m, n=n, k=k, dtype="bf16", bias="row", act=kb.ACT_SWISH, res_op=kb.RES_NONE, prepack=prepack)
+
+
+@pytest.mark.parametrize("wcode", [kb.S8, kb.U8])
+@pytest.mark.parametrize("m", [2, 7, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(15, 8208), (1003, 1040), (2464, 5264)])
+def test_streaming_8_bit_weights(cuda_device, wcode, m, n, k):
+    rng = np.random.default_rng(5)
+    x = ko.to_storage(rng.standard_normal((1, m, k), dtype=np.float32), kb.F16)
+    lo, hi = (-128, 128) if wcode == kb.S8 else (0, 256)
+    arrays = {"a": x, "b": rng.integers(lo, hi, (1, n, k)).astype(ko.np_dtype(wcode))}
+    desc = kb.make_desc(m, n, k, kb.F16, b_dtype=wcode)
+    c = helpers.case_defaults(dict(m=m, n=n, k=k, res_op=kb.RES_NONE))
+    ref, _ = helpers.run_oracle(desc, arrays, c, acc=ko.ACC_F64)
+    for prepack in (False, True):
+        got, _, used = helpers.run_gpu(desc, arrays, c, cuda_device, prepack=prepack)
+        assert used == kb.KERNEL_GEMV_MMA
+        helpers.compare(got, ref, desc.c_dtype)
+
+
+def test_chained_calls_read_each_others_results(cuda_device):
+    """Layers whose input is the previous layer's output, across the kernels that may start before it has ended."""
+    rng = np.random.default_rng(9)
+    stream = torch.cuda.current_stream().cuda_stream
+    for m in (1, 4, 12, 40, 300):
+        width = 512
+        ws = [torch.from_numpy(rng.standard_normal((width, width), dtype=np.float32) / width ** 0.5).to(cuda_device, torch.bfloat16)
+              for _ in range(6)]
+        lins = [kb.Linear(kb.make_desc(m, width, width, kb.BF16)) for _ in ws]
+        for lin, w in zip(lins, ws):
+            lin.prepack(w, stream=stream)
+        x = torch.from_numpy(rng.standard_normal((m, width), dtype=np.float32)).to(cuda_device, torch.bfloat16)
+        want = x.float()
+        for w in ws:
+            want = (want @ w.float().T).to(torch.bfloat16).float()
+        for _ in range(20):
+            bufs = [torch.full((m, width), float("nan"), device=cuda_device, dtype=torch.bfloat16) for _ in ws]
+            src = x
+            for lin, w, dst in zip(lins, ws, bufs):
+                lin.run(src, w, dst, stream=stream)
+                src = dst
+            # six roundings to 8 significant bits, each at most 2^-8 of a value of order one, and what they grow to
+            assert torch.allclose(src.float(), want, atol=6 * 2.0 ** -8 * 4, rtol=2.0 ** -6)
+        for lin in lins:
+            lin.close()
