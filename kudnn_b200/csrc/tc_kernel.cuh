@@ -6,7 +6,7 @@
 //
 // Shape of one CTA (320 threads, persistent over output tiles, one CTA per SM):
 //   warp 0       producer: one lane issues the TMA loads of the A tile [128 x 128 B] and the B tile [rows x 128 B]
-//                of every k-block into the ring (4 to 6 stages), 128-byte swizzle, completion on an mbarrier
+//                of every k-block into the ring (2 to 12 stages), 128-byte swizzle, completion on an mbarrier
 //   warp 1       one lane issues tcgen05.mma (K = 32 bytes per instruction, four per k-block) into one of two TMEM
 //                accumulators and commits to the stage's "empty" barrier / the tile's "full" barrier; the warp also
 //                owns TMEM allocation
@@ -14,9 +14,9 @@
 //                split the columns) 8 columns at a time, applies the post-GEMM chain and stores 16 or 32 bytes per
 //                tensor straight from registers (with output mirrors: 128-byte row pieces collected in shared memory); the
 //                second accumulator lets this overlap the next tile's main loop
-// Three launch shapes (tc_make_plan): clusters of two CTAs on 256 x 256 tiles with cta_group::2 MMAs (large
-// problems), single CTAs on 128 x 256 / 128 x 128 tiles, and clusters of 2-8 CTAs that cut K of one 128 x 128 tile
-// and add their partial tiles through distributed shared memory (few tiles, long K).
+// Launch shapes (tc_make_plan picks by estimated time): clusters of two CTAs on 256 x 256 tiles with cta_group::2 MMAs;
+// persistent single CTAs on 128 x bn tiles, bn a multiple of 16 up to 256; and single CTAs, or clusters of 2-8 that cut K of
+// one tile, with one work item each, whose tile is finished from (distributed) shared memory.
 // Operands are K-major ([rows, k], k contiguous).  16-bit inputs run as kind::f16 with fp32 accumulation.  fp32
 // inputs run as kind::tf32 on split planes: x = hi + lo with hi = tf32(x), and the packed operands
 // A' = [a_lo | a_hi | a_hi], B' = [b_hi | b_lo | b_hi] make one pass over 3k compute a_lo.b_hi + a_hi.b_lo + a_hi.b_hi.
