@@ -2,6 +2,7 @@
 #include "tc_kernel.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -106,12 +107,29 @@ int env_choice(const char *name)
     return v == nullptr || *v == '\0' ? -1 : std::atoi(v);
 }
 
-int pair_clusters_of(int kind, size_t smem)
+// The driver is asked once per device, kind and shared-memory size: the query takes several microseconds, and a plan is made
+// for every call whose activations lie at a new address.
+int pair_clusters_of(int kind, bool with_staging, size_t smem)
 {
-    return kind == KUDNN_B200_F32   ? pair_clusters_kind<KUDNN_B200_F32>(smem)
-           : kind == KUDNN_B200_F16 ? pair_clusters_kind<KUDNN_B200_F16>(smem)
-           : kind == KUDNN_B200_S8  ? pair_clusters_kind<KUDNN_B200_S8>(smem)
-                                    : pair_clusters_kind<KUDNN_B200_BF16>(smem);
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices][8][2];  // clusters + 1; 0 = not asked yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    std::atomic<int> *slot = dev < kDevices && kind < 8 ? &known[dev][kind][with_staging ? 1 : 0] : nullptr;
+    if (slot != nullptr && slot->load() > 0) {
+        return slot->load() - 1;
+    }
+    const int clusters = kind == KUDNN_B200_F32   ? pair_clusters_kind<KUDNN_B200_F32>(smem)
+                         : kind == KUDNN_B200_F16 ? pair_clusters_kind<KUDNN_B200_F16>(smem)
+                         : kind == KUDNN_B200_S8  ? pair_clusters_kind<KUDNN_B200_S8>(smem)
+                                                  : pair_clusters_kind<KUDNN_B200_BF16>(smem);
+    if (slot != nullptr && clusters > 0) {  // a failed query is asked again
+        slot->store(clusters + 1);
+    }
+    return clusters;
 }
 
 // Estimated SM cycles of a launch of single CTAs.  A k-block of a tile costs its MMAs (2 cycles per column whatever the
@@ -218,7 +236,7 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
         pair = cycles < best || env_choice("KUDNN_B200_TC_PAIR") > 0;
         int clusters = 0;
         if (pair) {
-            clusters = pair_clusters_of(ops.kind, static_cast<size_t>(pair_stages) * (kABytes + 128 * kStageRowBytes) + 1024 +
+            clusters = pair_clusters_of(ops.kind, with_staging, static_cast<size_t>(pair_stages) * (kABytes + 128 * kStageRowBytes) + 1024 +
                                                       kTailBytes + (with_staging ? kStagingBytes : 0));
             pair = clusters > 0;
         }

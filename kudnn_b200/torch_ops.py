@@ -54,6 +54,16 @@ def clear_cache():
         lin.close()
 
 
+def _run(x, x2, weight, bias, act, act_alpha, res2, res_op, gamma, m, n, k, out):
+    lin = _handle(m, n, k, x2, weight, bias, act, act_alpha, res2, res_op)
+    stream = torch.cuda.current_stream(x.device).cuda_stream
+    b = None if bias is None else bias.data_ptr()
+    if res_op != capi.RES_NONE:
+        lin.run(x2.data_ptr(), weight.data_ptr(), None, b, res2.data_ptr(), out.data_ptr(), gamma=gamma, stream=stream)
+    else:
+        lin.run(x2.data_ptr(), weight.data_ptr(), out.data_ptr(), b, stream=stream)
+
+
 @torch.library.custom_op("kudnn_b200::linear", mutates_args=(), device_types="cuda")
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = 0,
            act_alpha: float = 1.0, residual: Optional[torch.Tensor] = None, res_op: int = 0,
@@ -79,13 +89,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         if residual is None or residual.shape != out.shape or residual.dtype != x.dtype:
             raise ValueError("kudnn_b200::linear: residual must have the output's shape and type")
         res2 = residual.contiguous()
-    with torch.cuda.device(x.device):
-        lin = _handle(m, n, k, x2, weight, bias, act, act_alpha, res2, res_op)
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        if res_op != capi.RES_NONE:
-            lin.run(x2, weight, None, bias, res2, out, gamma=gamma, stream=stream)
-        else:
-            lin.run(x2, weight, out, bias, stream=stream)
+    if x.device.index == torch.cuda.current_device():
+        _run(x, x2, weight, bias, act, act_alpha, res2, res_op, gamma, m, n, k, out)
+    else:
+        with torch.cuda.device(x.device):
+            _run(x, x2, weight, bias, act, act_alpha, res2, res_op, gamma, m, n, k, out)
     return out
 
 
