@@ -11,6 +11,7 @@ import collections
 from typing import Optional
 
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from . import capi
 
@@ -21,28 +22,31 @@ ACTIVATIONS = {None: capi.ACT_NONE, "none": capi.ACT_NONE, "relu": capi.ACT_RELU
 RESIDUALS = {None: capi.RES_NONE, "none": capi.RES_NONE, "add": capi.RES_IDENTICAL, "ext": capi.RES_EXT,
              "mul": capi.RES_ELTWISE_MUL}
 
-# Created primitives, keyed by everything the descriptor holds plus the weight's address (a primitive pre-packs the
-# weights it first sees and recognises them by pointer).  Bounded: the oldest handle is destroyed when full.
+# Created primitives, keyed by everything the descriptor holds plus the weight's storage, address and version (a primitive
+# pre-packs the weights it first sees and recognises them by pointer).  The weak reference kept beside a primitive holds
+# the storage's identity, not its memory: as long as it exists no other storage has that identity, so weights that are
+# allocated later where freed ones were never meet their packed copy.  Bounded: the oldest handle is destroyed when full.
 _HANDLES = collections.OrderedDict()
 _MAX_HANDLES = 128
 
 
 def _handle(m, n, k, x, weight, bias, act, act_alpha, residual, res_op):
     code = _DTYPES[x.dtype]
-    key = (x.device.index, m, n, k, code, x.stride(-2) if x.dim() > 1 else k, weight.data_ptr(), weight.stride(0),
+    storage = weight.untyped_storage()
+    key = (x.device.index, m, n, k, code, x.stride(-2) if x.dim() > 1 else k, storage._cdata, weight.data_ptr(), weight.stride(0),
            weight.stride(1), weight._version, None if bias is None else _DTYPES[bias.dtype], act, act_alpha, res_op)
-    lin = _HANDLES.get(key)
-    if lin is not None:
+    entry = _HANDLES.get(key)
+    if entry is not None:
         _HANDLES.move_to_end(key)
-        return lin
+        return entry[0]
     desc = capi.make_desc(m, n, k, code, a_strides=(k, 1), b_strides=(weight.stride(1), weight.stride(0)),
                           has_bias=bias is not None, bias_dtype=None if bias is None else _DTYPES[bias.dtype], act=act,
                           act_alpha=act_alpha, res_op=res_op)
     lin = capi.Linear(desc)
     lin.prepack(weight, stream=torch.cuda.current_stream(x.device).cuda_stream)
-    _HANDLES[key] = lin
+    _HANDLES[key] = (lin, StorageWeakRef(storage))
     while len(_HANDLES) > _MAX_HANDLES:
-        _, old = _HANDLES.popitem(last=False)
+        _, (old, _) = _HANDLES.popitem(last=False)
         old.close()
     return lin
 
@@ -50,7 +54,7 @@ def _handle(m, n, k, x, weight, bias, act, act_alpha, residual, res_op):
 def clear_cache():
     """Destroys every cached primitive (and the packed weight copies they own)."""
     while _HANDLES:
-        _, lin = _HANDLES.popitem()
+        _, (lin, _) = _HANDLES.popitem()
         lin.close()
 
 

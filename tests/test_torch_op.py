@@ -1,5 +1,8 @@
 """The torch.library operator kudnn_b200::linear and the nn.Linear drop-in module (kudnn_b200/torch_ops.py): the
 documented PyTorch integration point of the reference (docs/zh/KuDNN_development_guide.md:1748-1775) on this side."""
+import collections
+import types
+
 import numpy as np
 import pytest
 import torch
@@ -18,6 +21,47 @@ def test_fake_implementation_propagates_shapes_without_a_device():
     assert y.shape == (3, 7, 96) and y.dtype == torch.bfloat16 and y.device.type == "meta"
     r = torch.empty(3, 7, 96, dtype=torch.bfloat16, device="meta")
     assert torch.ops.kudnn_b200.linear(x, w, None, 0, 1.0, r, kb.RES_IDENTICAL).shape == (3, 7, 96)
+
+
+class _RecordedLinear:
+    """Stands in for a primitive: remembers the weights it packed."""
+
+    def __init__(self, desc):
+        self.closed = False
+
+    def prepack(self, b, stream=None):
+        self.weights = b.clone()
+
+    def close(self):
+        self.closed = True
+
+
+@pytest.fixture
+def recorded_handles(monkeypatch):
+    monkeypatch.setattr(torch_ops.capi, "Linear", _RecordedLinear)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: types.SimpleNamespace(cuda_stream=1))
+    monkeypatch.setattr(torch_ops, "_HANDLES", collections.OrderedDict())
+
+    def handle(weight, m=4):
+        x = torch.zeros(m, weight.shape[1])
+        return torch_ops._handle(m, weight.shape[0], weight.shape[1], x, weight, None, 0, 1.0, None, 0)
+
+    return handle
+
+
+def test_weights_where_freed_ones_were_are_packed_again(recorded_handles):
+    memory = np.zeros((8, 16), dtype=np.float32)
+    first = torch.from_numpy(memory)
+    old = recorded_handles(first)
+    assert recorded_handles(first) is old and recorded_handles(first[:]) is old
+    where = first.data_ptr()
+    del first
+    memory[:] = 1.0
+    second = torch.from_numpy(memory)
+    assert second.data_ptr() == where and second._version == 0
+    assert torch.equal(recorded_handles(second).weights, second)
+    second.add_(1.0)
+    assert torch.equal(recorded_handles(second).weights, second)
 
 
 def _oracle(x, w, b, act, res, res_op):
