@@ -127,10 +127,11 @@ KUDNN_B200_API int kudnn_b200_linear_prepack(kudnn_b200_linear_t handle, const v
 KUDNN_B200_API int kudnn_b200_linear_unpack(kudnn_b200_linear_t handle);
 
 /* Execute with DEVICE pointers on `cuda_stream` (a cudaStream_t, NULL = default stream); asynchronous.
- * A handle owns device scratch (split-K partial sums and arrival counters, packed activations, the status block)
- * that all of its runs share: the handle's lock serialises the host side only, so runs of ONE handle must not overlap
- * on the GPU.  Keep a handle on one stream at a time; kudnn_b200_linear_clone gives every further stream a handle of
- * its own.
+ * Runs of one handle on different streams may overlap on the GPU: the packed weights are only read, and the handle keeps
+ * device scratch (split-K partial sums and arrival counters, packed activations) for every stream it is used on, at most
+ * sixteen (a further one waits for the device and takes over the scratch used longest ago).  Runs that are captured into
+ * a CUDA graph get scratch of their own per capture, so graphs may be replayed beside other runs and each other; the
+ * handle must outlive them, and re-packing needs all of its runs to have ended.
  * Replaces GemmImpl::Run / LinearActivationLayerFWDImpl::Run / LinearResFWDImpl::Run
  * (src/dnn/src/kudnn_gemm.cpp:859-877, kudnn_linear_activationlayer.cpp:40-56, kudnn_linear_res.cpp:184-202). */
 KUDNN_B200_API int kudnn_b200_linear_run(kudnn_b200_linear_t handle, const kudnn_b200_linear_args *args,

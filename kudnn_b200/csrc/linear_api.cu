@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -81,6 +82,13 @@ cudaError_t device_malloc(void **ptr, size_t bytes)
     return cudaMalloc(ptr, bytes);
 }
 
+// While it exists, this thread may allocate and free although a stream is being captured: neither becomes part of the graph.
+struct CaptureRelaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CaptureRelaxed() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~CaptureRelaxed() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 struct DeviceBuffer {
     void *ptr = nullptr;
     size_t bytes = 0;
@@ -89,6 +97,7 @@ struct DeviceBuffer {
         if (need <= bytes) {
             return cudaSuccess;
         }
+        CaptureRelaxed relaxed;
         if (ptr != nullptr) {
             cudaFree(ptr);
             ptr = nullptr;
@@ -109,6 +118,29 @@ struct DeviceBuffer {
         bytes = 0;
     }
 };
+
+// What the launches of one stream write besides their outputs.  Kernels of different streams may run at the same time, so
+// every stream that a handle is used on has its own, and so has every captured graph, whichever stream replays it.
+struct StreamScratch {
+    unsigned long long stream_id = 0;  // cudaStreamGetId: unlike the stream's address never given to another stream; in a graph
+                                       // the address of the captured stream
+    unsigned long long capture_id = 0;                // 0: not part of a graph
+    std::shared_ptr<std::atomic<bool>> graph_alive;   // cleared when the graph that holds launches on this scratch is gone
+    unsigned long long last_use = 0;
+    bool counters_clear = false;  // the arrival counters are zero, or will be when the next launch on the stream starts
+    DeviceBuffer partials, counters;  // split-K partial sums and arrival counters of the streaming kernels
+    DeviceBuffer a;                   // packed activations
+    DeviceBuffer b;                   // packed weights (when not pre-packed)
+    DeviceBuffer q;                   // 8-bit weights widened to fp16 (when not pre-packed)
+    void release()
+    {
+        for (DeviceBuffer *buf : {&partials, &counters, &a, &b, &q}) {
+            buf->release();
+        }
+    }
+};
+// Streams a handle keeps scratch for; one more, and the one used longest ago gives its memory back.
+constexpr size_t kMaxScratchStreams = 16;
 
 }  // namespace
 
@@ -141,16 +173,12 @@ struct kudnn_b200_linear_s {
     // device-side waits: limit in SM cycles (0 = default) and the timeout test hook (kudnn_b200_debug_set_wait)
     long long wait_limit = 0;
     int skip_kblock = -1;
-    cudaStream_t counters_stream = nullptr;  // stream the arrival counters were last zeroed or used on
-    bool counters_dirty = false;             // a kernel that gave up may have left arrival counters set
 
     DeviceBuffer status;        // kb::DeviceStatus
-    DeviceBuffer gemv_partials, gemv_counters;
-    DeviceBuffer a_scratch;     // per-call packed activations
-    DeviceBuffer b_scratch;     // per-call packed weights (when not pre-packed)
+    std::vector<std::unique_ptr<StreamScratch>> scratch;
+    unsigned long long scratch_uses = 0;
     DeviceBuffer b_packed;      // pre-packed weights
     DeviceBuffer b_blocked;     // decode-shaped handles: the weights once more in 8-row x 64-k blocks
-    DeviceBuffer q_scratch;     // 8-bit weights widened to fp16 per call (when not pre-packed)
     DeviceBuffer stage[6];      // host-pointer staging: a, b, c, bias, res, out
 
     // pre-pack state
@@ -437,35 +465,124 @@ bool collapse_batch(const kudnn_b200_linear_desc &d, kudnn_b200_linear_desc *out
     return true;
 }
 
+void graph_gone(void *claim)
+{
+    auto *alive = static_cast<std::shared_ptr<std::atomic<bool>> *>(claim);
+    (*alive)->store(false);
+    delete alive;
+}
+
+// The scratch for launches on `stream`.  A stream that is being captured gets one that belongs to the graph: it is reused
+// only after the graph, every executable made from it and their last run are gone.
+int scratch_for(Handle *h, cudaStream_t stream, StreamScratch **out)
+{
+    unsigned long long stream_id = 0, capture_id = 0;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        (void)cudaGetLastError();  // the launch will fail and say why
+    }
+    cudaGraph_t graph = nullptr;
+    if (status == cudaStreamCaptureStatusActive) {
+        const cudaGraphNode_t *nodes = nullptr;
+        const cudaGraphEdgeData *edges = nullptr;
+        size_t count = 0;
+        cudaError_t e = cudaStreamGetCaptureInfo_v3(stream, &status, &capture_id, &graph, &nodes, &edges, &count);
+        if (e != cudaSuccess) {
+            return fail_cuda(e, "stream capture");
+        }
+        stream_id = reinterpret_cast<uintptr_t>(stream);  // a stream has no id to ask for while it is captured
+    } else if (cudaStreamGetId(stream, &stream_id) != cudaSuccess) {
+        (void)cudaGetLastError();
+    }
+    StreamScratch *free_slot = nullptr, *oldest = nullptr;
+    size_t streams = 0;
+    for (auto &sc : h->scratch) {
+        if (sc->stream_id == stream_id && sc->capture_id == capture_id && (graph == nullptr || sc->graph_alive->load())) {
+            sc->last_use = ++h->scratch_uses;
+            *out = sc.get();
+            return KUDNN_B200_OK;
+        }
+        if (sc->capture_id != 0) {
+            if (graph != nullptr && free_slot == nullptr && !sc->graph_alive->load()) {
+                free_slot = sc.get();
+            }
+        } else {
+            streams += 1;
+            if (oldest == nullptr || sc->last_use < oldest->last_use) {
+                oldest = sc.get();
+            }
+        }
+    }
+    if (graph == nullptr && streams >= kMaxScratchStreams) {
+        cudaError_t e = cudaDeviceSynchronize();
+        if (e != cudaSuccess) {
+            return fail_cuda(e, "scratch of another stream");
+        }
+        oldest->release();
+        free_slot = oldest;
+    }
+    std::shared_ptr<std::atomic<bool>> *claim = nullptr;
+    try {
+        if (free_slot == nullptr) {
+            h->scratch.emplace_back(new StreamScratch());
+            free_slot = h->scratch.back().get();
+        }
+        free_slot->graph_alive = std::make_shared<std::atomic<bool>>(false);
+        if (graph != nullptr) {
+            claim = new std::shared_ptr<std::atomic<bool>>(free_slot->graph_alive);
+        }
+    } catch (const std::bad_alloc &) {
+        return fail(KUDNN_B200_ALLOC_FAILED, "out of host memory");
+    }
+    free_slot->stream_id = stream_id;
+    free_slot->capture_id = capture_id;
+    free_slot->last_use = ++h->scratch_uses;
+    free_slot->counters_clear = false;
+    if (graph != nullptr) {
+        cudaUserObject_t object;
+        cudaError_t e = cudaUserObjectCreate(&object, claim, graph_gone, 1, cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess) {
+            delete claim;
+            return fail_cuda(e, "stream capture");
+        }
+        e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+        if (e != cudaSuccess) {
+            (void)cudaUserObjectRelease(object, 1);
+            return fail_cuda(e, "stream capture");
+        }
+        free_slot->graph_alive->store(true);
+    }
+    *out = free_slot;
+    return KUDNN_B200_OK;
+}
+
 // Split-K scratch of the streaming kernels: partial sums and arrival counters, grown on demand.
-int reserve_gemv_scratch(Handle *h, long long partial_floats, long long counter_count, cudaStream_t stream,
+int reserve_gemv_scratch(StreamScratch *sc, long long partial_floats, long long counter_count, cudaStream_t stream,
                          kb::GemvWorkspace *ws)
 {
-    cudaError_t e = h->gemv_partials.reserve(static_cast<size_t>(partial_floats) * sizeof(float));
+    cudaError_t e = sc->partials.reserve(static_cast<size_t>(partial_floats) * sizeof(float));
     if (e != cudaSuccess) {
         return fail_cuda(e, "streaming-kernel scratch");
     }
-    const bool grow = h->gemv_counters.bytes < static_cast<size_t>(counter_count) * sizeof(unsigned);
-    if (grow) {
-        e = h->gemv_counters.reserve(static_cast<size_t>(counter_count) * sizeof(unsigned));
+    if (sc->counters.bytes < static_cast<size_t>(counter_count) * sizeof(unsigned)) {
+        sc->counters_clear = false;
+        e = sc->counters.reserve(static_cast<size_t>(counter_count) * sizeof(unsigned));
         if (e != cudaSuccess) {
             return fail_cuda(e, "streaming-kernel counters");
         }
     }
-    // The kernels leave the counters at zero, so they are cleared only when they are new, after a run that gave
-    // up, or when the caller moved to another stream (the clear is then ordered in front of this launch).
-    if (grow || h->counters_dirty || h->counters_stream != stream) {
-        e = cudaMemsetAsync(h->gemv_counters.ptr, 0, h->gemv_counters.bytes, stream);
+    // The kernels leave the counters at zero, so they are cleared only when they are new or after a run that gave up.
+    if (!sc->counters_clear) {
+        e = cudaMemsetAsync(sc->counters.ptr, 0, sc->counters.bytes, stream);
         if (e != cudaSuccess) {
             return fail_cuda(e, "streaming-kernel counters");
         }
-        h->counters_dirty = false;
-        h->counters_stream = stream;
+        sc->counters_clear = true;
     }
-    ws->partials = static_cast<float *>(h->gemv_partials.ptr);
-    ws->counters = static_cast<unsigned *>(h->gemv_counters.ptr);
-    ws->partial_floats = static_cast<long long>(h->gemv_partials.bytes / sizeof(float));
-    ws->counter_count = static_cast<long long>(h->gemv_counters.bytes / sizeof(unsigned));
+    ws->partials = static_cast<float *>(sc->partials.ptr);
+    ws->counters = static_cast<unsigned *>(sc->counters.ptr);
+    ws->partial_floats = static_cast<long long>(sc->partials.bytes / sizeof(float));
+    ws->counter_count = static_cast<long long>(sc->counters.bytes / sizeof(unsigned));
     return KUDNN_B200_OK;
 }
 
@@ -491,6 +608,11 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
         return fail(KUDNN_B200_BAD_ARGUMENTS, "run: beta != 0 needs c");
     }
     int rc = ensure_device(h);
+    if (rc != KUDNN_B200_OK) {
+        return rc;
+    }
+    StreamScratch *sc = nullptr;
+    rc = scratch_for(h, stream, &sc);
     if (rc != KUDNN_B200_OK) {
         return rc;
     }
@@ -525,32 +647,32 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.b = args.b;
                 ops.ldb = d.b_sn;
             } else {
-                cudaError_t e = h->b_scratch.reserve(static_cast<size_t>(d.n) * k_pad);
+                cudaError_t e = sc->b.reserve(static_cast<size_t>(d.n) * k_pad);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "packed weights");
                 }
-                e = kb::launch_pack_kmajor(args.b, d.b_dtype, d.n, d.k, d.b_sn, d.b_sk, h->b_scratch.ptr, d.b_dtype, k_pad, k_pad, stream);
+                e = kb::launch_pack_kmajor(args.b, d.b_dtype, d.n, d.k, d.b_sn, d.b_sk, sc->b.ptr, d.b_dtype, k_pad, k_pad, stream);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "weight pack kernel");
                 }
                 launches += 1;
-                ops.b = h->b_scratch.ptr;
+                ops.b = sc->b.ptr;
                 ops.ldb = k_pad;
             }
             if (kmajor_ready(args.a, d.a_dtype, d.a_sm, d.a_sk, d.m)) {
                 ops.a = args.a;
                 ops.lda = d.a_sm;
             } else {
-                cudaError_t e = h->a_scratch.reserve(static_cast<size_t>(d.m) * k_pad);
+                cudaError_t e = sc->a.reserve(static_cast<size_t>(d.m) * k_pad);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "packed activations");
                 }
-                e = kb::launch_pack_kmajor(args.a, d.a_dtype, d.m, d.k, d.a_sm, d.a_sk, h->a_scratch.ptr, d.a_dtype, k_pad, k_pad, stream);
+                e = kb::launch_pack_kmajor(args.a, d.a_dtype, d.m, d.k, d.a_sm, d.a_sk, sc->a.ptr, d.a_dtype, k_pad, k_pad, stream);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "activation pack kernel");
                 }
                 launches += 1;
-                ops.a = h->a_scratch.ptr;
+                ops.a = sc->a.ptr;
                 ops.lda = k_pad;
             }
             if (!(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m && !h->plan_staging)) {
@@ -611,7 +733,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             kb::GemvPlan plan8;
             if (kb::gemv_plan(p8, h->sm_count, forced8, false, &plan8)) {
                 kb::GemvWorkspace ws8;
-                rc = reserve_gemv_scratch(h, plan8.partial_floats, plan8.counter_count, stream, &ws8);
+                rc = reserve_gemv_scratch(sc, plan8.partial_floats, plan8.counter_count, stream, &ws8);
                 if (rc != KUDNN_B200_OK) {
                     return rc;
                 }
@@ -636,16 +758,16 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 return fail(KUDNN_B200_UNSUPPORTED, "8-bit weights of batched problems are not supported");
             }
             const long long k_pad = round_up(d.k, 8);
-            cudaError_t e = h->q_scratch.reserve(static_cast<size_t>(d.n) * k_pad * 2);
+            cudaError_t e = sc->q.reserve(static_cast<size_t>(d.n) * k_pad * 2);
             if (e != cudaSuccess) {
                 return fail_cuda(e, "widened weights");
             }
-            e = kb::launch_pack_kmajor(w8, d.b_dtype, d.n, d.k, w8_sn, w8_sk, h->q_scratch.ptr, KUDNN_B200_F16, k_pad, k_pad, stream);
+            e = kb::launch_pack_kmajor(w8, d.b_dtype, d.n, d.k, w8_sn, w8_sk, sc->q.ptr, KUDNN_B200_F16, k_pad, k_pad, stream);
             if (e != cudaSuccess) {
                 return fail_cuda(e, "weight widening kernel");
             }
             dq.b_sn = k_pad;
-            aq.b = h->q_scratch.ptr;
+            aq.b = sc->q.ptr;
         }
         const int rcq = run_device(h, dq, aq, stream);
         if (rcq == KUDNN_B200_OK && aq.b != args.b) {
@@ -709,7 +831,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
         kb::GemvPlan plan;
         if (kb::gemv_plan(pr, h->sm_count, forced, false, &plan)) {
             kb::GemvWorkspace ws;
-            rc = reserve_gemv_scratch(h, plan.partial_floats, plan.counter_count, stream, &ws);
+            rc = reserve_gemv_scratch(sc, plan.partial_floats, plan.counter_count, stream, &ws);
             if (rc != KUDNN_B200_OK) {
                 return rc;
             }
@@ -817,11 +939,11 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             } else if (nb == 1) {
                 long long ld = 0, kt = 0;
                 const void *raw = nullptr;
-                rc = pack_weights(h, args.b, &h->b_scratch, false, stream, &ld, &kt, &raw, &launches);
+                rc = pack_weights(h, args.b, &sc->b, false, stream, &ld, &kt, &raw, &launches);
                 if (rc != KUDNN_B200_OK) {
                     return rc;
                 }
-                ops.b = h->b_scratch.ptr;
+                ops.b = sc->b.ptr;
                 ops.ldb = ld;
                 ops.k_total = kt;
             } else {
@@ -829,20 +951,20 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 const long long k_pad = round_up(d.k, f32 ? 32 : 8);
                 const long long pitch = f32 ? 3 * k_pad : k_pad;
                 const long long per = d.n * pitch;
-                cudaError_t e = h->b_scratch.reserve(static_cast<size_t>(shared ? 1 : nb) * per * es);
+                cudaError_t e = sc->b.reserve(static_cast<size_t>(shared ? 1 : nb) * per * es);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "packed weights");
                 }
                 const kb::PackBatch pb = pack_batch(d.b_sb, shared, per);
-                e = f32 ? kb::launch_split_tf32(args.b, d.n, d.k, d.b_sn, d.b_sk, static_cast<float *>(h->b_scratch.ptr), pitch,
+                e = f32 ? kb::launch_split_tf32(args.b, d.n, d.k, d.b_sn, d.b_sk, static_cast<float *>(sc->b.ptr), pitch,
                                                 k_pad, 1, stream, &pb)
-                        : kb::launch_pack_kmajor(args.b, d.b_dtype, d.n, d.k, d.b_sn, d.b_sk, h->b_scratch.ptr, d.b_dtype, pitch,
+                        : kb::launch_pack_kmajor(args.b, d.b_dtype, d.n, d.k, d.b_sn, d.b_sk, sc->b.ptr, d.b_dtype, pitch,
                                                  k_pad, stream, &pb);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "weight pack kernel");
                 }
                 launches += 1;
-                ops.b = h->b_scratch.ptr;
+                ops.b = sc->b.ptr;
                 ops.ldb = pitch;
                 ops.k_total = f32 ? 3 * k_pad : d.k;
                 ops.b_bstride = shared ? 0 : per;
@@ -858,20 +980,20 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 const long long k_pad = round_up(d.k, f32 ? 32 : 8);
                 const long long pitch = f32 ? 3 * k_pad : k_pad;
                 const long long per = d.m * pitch;
-                cudaError_t e = h->a_scratch.reserve(static_cast<size_t>(shared ? 1 : nb) * per * es);
+                cudaError_t e = sc->a.reserve(static_cast<size_t>(shared ? 1 : nb) * per * es);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "packed activations");
                 }
                 const kb::PackBatch pb = pack_batch(d.a_sb, shared, per);
-                e = f32 ? kb::launch_split_tf32(args.a, d.m, d.k, d.a_sm, d.a_sk, static_cast<float *>(h->a_scratch.ptr), pitch,
+                e = f32 ? kb::launch_split_tf32(args.a, d.m, d.k, d.a_sm, d.a_sk, static_cast<float *>(sc->a.ptr), pitch,
                                                 k_pad, 0, stream, &pb)
-                        : kb::launch_pack_kmajor(args.a, d.a_dtype, d.m, d.k, d.a_sm, d.a_sk, h->a_scratch.ptr, d.a_dtype, pitch,
+                        : kb::launch_pack_kmajor(args.a, d.a_dtype, d.m, d.k, d.a_sm, d.a_sk, sc->a.ptr, d.a_dtype, pitch,
                                                  k_pad, stream, &pb);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "activation pack kernel");
                 }
                 launches += 1;
-                ops.a = h->a_scratch.ptr;
+                ops.a = sc->a.ptr;
                 ops.lda = pitch;
                 ops.a_bstride = shared ? 0 : per;
             }
@@ -994,7 +1116,9 @@ int read_status(Handle *h)
     }
     if (st.code != kb::kErrNone) {
         cudaMemset(h->status.ptr, 0, sizeof(st));
-        h->counters_dirty = true;
+        for (auto &sc : h->scratch) {
+            sc->counters_clear = false;  // a kernel that gave up may have left arrival counters set
+        }
         return fail(KUDNN_B200_TIMEOUT, "device-side wait gave up (site %d, block %d)", st.where, st.block);
     }
     return KUDNN_B200_OK;
@@ -1240,13 +1364,11 @@ int kudnn_b200_linear_destroy(kudnn_b200_linear_t h)
             cur = -1;
         }
         h->status.release();
-        h->gemv_partials.release();
-        h->gemv_counters.release();
-        h->a_scratch.release();
-        h->b_scratch.release();
+        for (auto &sc : h->scratch) {
+            sc->release();
+        }
         h->b_packed.release();
         h->b_blocked.release();
-        h->q_scratch.release();
         for (auto &s : h->stage) {
             s.release();
         }
@@ -1831,8 +1953,11 @@ int64_t kudnn_b200_linear_workspace_bytes(kudnn_b200_linear_t h)
     if (h == nullptr) {
         return 0;
     }
-    return static_cast<int64_t>(h->gemv_partials.bytes + h->gemv_counters.bytes + h->a_scratch.bytes + h->b_scratch.bytes +
-                                h->b_packed.bytes + h->b_blocked.bytes);
+    size_t bytes = h->b_packed.bytes + h->b_blocked.bytes;
+    for (const auto &sc : h->scratch) {
+        bytes += sc->partials.bytes + sc->counters.bytes + sc->a.bytes + sc->b.bytes;
+    }
+    return static_cast<int64_t>(bytes);
 }
 
 int kudnn_b200_shard_range(int64_t total, int nparts, int part, int64_t align, int64_t *begin, int64_t *count)

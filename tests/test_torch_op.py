@@ -113,3 +113,41 @@ def test_operator_passes_opcheck(cuda_device):
     torch.library.opcheck(torch.ops.kudnn_b200.linear.default, (x, w, b, kb.ACT_RELU, 0.0),
                           test_utils=("test_schema", "test_faketensor"))
     torch_ops.clear_cache()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,dtype", [(200, 520, 1024, torch.float32), (1, 700, 4104, torch.bfloat16), (4, 1003, 6152, torch.bfloat16),
+                                         (60, 512, 1030, torch.float16)])
+def test_one_layer_on_two_streams_and_in_graphs(cuda_device, m, n, k, dtype):
+    """Scratch (split activations, partial sums and counters, packed rows) is written by every call; calls on different
+    streams and replays of different graphs overlap."""
+    torch.manual_seed(11)
+    mod = torch_ops.Linear.from_torch(torch.nn.Linear(k, n, device=cuda_device, dtype=dtype), act="silu")
+    xs = [torch.randn(m, k, device=cuda_device, dtype=dtype) for _ in range(4)]
+    with torch.no_grad():
+        want = [mod(x) for x in xs]
+        torch.cuda.synchronize()
+        streams = [torch.cuda.Stream() for _ in range(4)]
+        outs = [[], [], [], []]
+        for _ in range(40):
+            for i in range(2):
+                with torch.cuda.stream(streams[i]):
+                    outs[i].append(mod(xs[i]))
+        torch.cuda.synchronize()
+        graphs = []
+        for i in (2, 3):
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[-1]):
+                outs[i] += [mod(xs[i]) for _ in range(8)]
+        for out in outs[2] + outs[3]:
+            out.zero_()
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for i in range(4):
+                with torch.cuda.stream(streams[i]):
+                    graphs[i - 2].replay() if i >= 2 else outs[i].append(mod(xs[i]))
+        torch.cuda.synchronize()
+    for got, ref in zip(outs, want):
+        assert all(torch.equal(y, ref) for y in got)
+    del graphs
+    torch_ops.clear_cache()
