@@ -249,6 +249,10 @@ KUDNN_B200_API int kudnn_b200_peer_buffer_destroy(void *dev_ptr);
 KUDNN_B200_API int kudnn_b200_debug_set_wait(kudnn_b200_linear_t handle, long long wait_limit_cycles, int skip_kblock);
 KUDNN_B200_API int kudnn_b200_debug_fail_allocation(int nth);
 
+/* How many captures (one per stream captured) hold launches of this handle in graphs that still exist: while it is not 0
+ * the handle must not be destroyed. */
+KUDNN_B200_API int kudnn_b200_linear_graphs(kudnn_b200_linear_t handle);
+
 /* Introspection used by tests and the benchmark. */
 KUDNN_B200_API int kudnn_b200_linear_force_kernel(kudnn_b200_linear_t handle, int kernel);
 KUDNN_B200_API int kudnn_b200_linear_last_kernel(kudnn_b200_linear_t handle);

@@ -66,7 +66,7 @@ EXPORTS = [
     "kudnn_b200_peer_buffer_open", "kudnn_b200_peer_buffer_close", "kudnn_b200_peer_buffer_destroy",
     "kudnn_b200_linear_unpack", "kudnn_b200_debug_set_wait", "kudnn_b200_debug_fail_allocation",
     "kudnn_b200_linear_run_sharded", "kudnn_b200_activation_validate", "kudnn_b200_activation_run", "kudnn_b200_rmsnorm_validate", "kudnn_b200_rmsnorm_run",
-    "kudnn_b200_linear_set_multicast",
+    "kudnn_b200_linear_set_multicast", "kudnn_b200_linear_graphs",
 ]
 
 _lib = None
@@ -114,6 +114,7 @@ def library():
     lib.kudnn_b200_linear_force_kernel.argtypes = [vp, i32]
     lib.kudnn_b200_linear_last_kernel.argtypes = [vp]
     lib.kudnn_b200_linear_last_launches.argtypes = [vp]
+    lib.kudnn_b200_linear_graphs.argtypes = [vp]
     lib.kudnn_b200_linear_workspace_bytes.argtypes = [vp]
     lib.kudnn_b200_linear_workspace_bytes.restype = i64
     lib.kudnn_b200_shard_range.argtypes = [i64, i32, i32, i64, ctypes.POINTER(i64), ctypes.POINTER(i64)]
@@ -331,6 +332,11 @@ class Linear:
     @property
     def last_launches(self):
         return self._lib.kudnn_b200_linear_last_launches(self._h)
+
+    @property
+    def graphs(self):
+        """Captures whose CUDA graphs still exist and hold launches of this primitive."""
+        return self._lib.kudnn_b200_linear_graphs(self._h)
 
     @property
     def workspace_bytes(self):

@@ -112,6 +112,7 @@ struct DeviceBuffer {
     void release()
     {
         if (ptr != nullptr) {
+            CaptureRelaxed relaxed;
             cudaFree(ptr);
         }
         ptr = nullptr;
@@ -1946,6 +1947,19 @@ int kudnn_b200_linear_last_kernel(kudnn_b200_linear_t h)
 int kudnn_b200_linear_last_launches(kudnn_b200_linear_t h)
 {
     return h == nullptr ? 0 : h->last_launches;
+}
+
+int kudnn_b200_linear_graphs(kudnn_b200_linear_t h)
+{
+    if (h == nullptr) {
+        return 0;
+    }
+    std::lock_guard<std::mutex> guard(h->lock);
+    int count = 0;
+    for (const auto &sc : h->scratch) {
+        count += sc->capture_id != 0 && sc->graph_alive->load() ? 1 : 0;
+    }
+    return count;
 }
 
 int64_t kudnn_b200_linear_workspace_bytes(kudnn_b200_linear_t h)

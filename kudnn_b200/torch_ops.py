@@ -8,6 +8,7 @@ tracing and ``torch.compile`` graph capture see the right output without touchin
 libkudnn_b200.so; torch supplies the tensors, the current stream and the output allocation.
 """
 import collections
+import threading
 from typing import Optional
 
 import torch
@@ -25,9 +26,11 @@ RESIDUALS = {None: capi.RES_NONE, "none": capi.RES_NONE, "add": capi.RES_IDENTIC
 # Created primitives, keyed by everything the descriptor holds plus the weight's storage, address and version (a primitive
 # pre-packs the weights it first sees and recognises them by pointer).  The weak reference kept beside a primitive holds
 # the storage's identity, not its memory: as long as it exists no other storage has that identity, so weights that are
-# allocated later where freed ones were never meet their packed copy.  Bounded: the oldest handle is destroyed when full.
+# allocated later where freed ones were never meet their packed copy.  Bounded: when full, the primitive used longest ago is
+# dropped, and destroyed when no call of another thread uses it any more; one whose launches a CUDA graph holds stays.
 _HANDLES = collections.OrderedDict()
 _MAX_HANDLES = 128
+_LOCK = threading.Lock()
 
 
 def _handle(m, n, k, x, weight, bias, act, act_alpha, residual, res_op):
@@ -35,27 +38,31 @@ def _handle(m, n, k, x, weight, bias, act, act_alpha, residual, res_op):
     storage = weight.untyped_storage()
     key = (x.device.index, m, n, k, code, x.stride(-2) if x.dim() > 1 else k, storage._cdata, weight.data_ptr(), weight.stride(0),
            weight.stride(1), weight._version, None if bias is None else _DTYPES[bias.dtype], act, act_alpha, res_op)
-    entry = _HANDLES.get(key)
-    if entry is not None:
-        _HANDLES.move_to_end(key)
-        return entry[0]
-    desc = capi.make_desc(m, n, k, code, a_strides=(k, 1), b_strides=(weight.stride(1), weight.stride(0)),
-                          has_bias=bias is not None, bias_dtype=None if bias is None else _DTYPES[bias.dtype], act=act,
-                          act_alpha=act_alpha, res_op=res_op)
-    lin = capi.Linear(desc)
-    lin.prepack(weight, stream=torch.cuda.current_stream(x.device).cuda_stream)
-    _HANDLES[key] = (lin, StorageWeakRef(storage))
-    while len(_HANDLES) > _MAX_HANDLES:
-        _, (old, _) = _HANDLES.popitem(last=False)
-        old.close()
-    return lin
+    with _LOCK:
+        entry = _HANDLES.get(key)
+        if entry is not None:
+            _HANDLES.move_to_end(key)
+            return entry[0]
+        desc = capi.make_desc(m, n, k, code, a_strides=(k, 1), b_strides=(weight.stride(1), weight.stride(0)),
+                              has_bias=bias is not None, bias_dtype=None if bias is None else _DTYPES[bias.dtype], act=act,
+                              act_alpha=act_alpha, res_op=res_op)
+        lin = capi.Linear(desc)
+        lin.prepack(weight, stream=torch.cuda.current_stream(x.device).cuda_stream)
+        if len(_HANDLES) >= _MAX_HANDLES:
+            oldest = next((old for old, (other, _) in _HANDLES.items() if other.graphs == 0), None)
+            if oldest is not None:
+                del _HANDLES[oldest]
+        _HANDLES[key] = (lin, StorageWeakRef(storage))
+        return lin
 
 
 def clear_cache():
-    """Destroys every cached primitive (and the packed weight copies they own)."""
-    while _HANDLES:
-        _, (lin, _) = _HANDLES.popitem()
-        lin.close()
+    """Destroys every cached primitive (and the packed weight copies they own); graphs that hold calls of the operator
+    must not be replayed afterwards."""
+    with _LOCK:
+        while _HANDLES:
+            _, (lin, _) = _HANDLES.popitem()
+            lin.close()
 
 
 def _run(x, x2, weight, bias, act, act_alpha, res2, res_op, gamma, m, n, k, out):

@@ -27,7 +27,7 @@ class _RecordedLinear:
     """Stands in for a primitive: remembers the weights it packed."""
 
     def __init__(self, desc):
-        self.closed = False
+        self.closed, self.graphs = False, 0
 
     def prepack(self, b, stream=None):
         self.weights = b.clone()
@@ -62,6 +62,17 @@ def test_weights_where_freed_ones_were_are_packed_again(recorded_handles):
     assert torch.equal(recorded_handles(second).weights, second)
     second.add_(1.0)
     assert torch.equal(recorded_handles(second).weights, second)
+
+
+def test_a_full_cache_keeps_primitives_that_graphs_use(recorded_handles, monkeypatch):
+    monkeypatch.setattr(torch_ops, "_MAX_HANDLES", 3)
+    weight = torch.zeros(8, 16)
+    first = [recorded_handles(weight, m) for m in (1, 2, 3)]
+    first[0].graphs = 1
+    fourth = recorded_handles(weight, 4)
+    assert [recorded_handles(weight, m) for m in (1, 3, 4)] == [first[0], first[2], fourth]
+    assert not any(lin.closed for lin in first)  # a caller may be about to run the one that was dropped
+    assert recorded_handles(weight, 2) is not first[1]
 
 
 def _oracle(x, w, b, act, res, res_op):
@@ -149,5 +160,8 @@ def test_one_layer_on_two_streams_and_in_graphs(cuda_device, m, n, k, dtype):
         torch.cuda.synchronize()
     for got, ref in zip(outs, want):
         assert all(torch.equal(y, ref) for y in got)
+    (lin, _), = torch_ops._HANDLES.values()
+    assert lin.graphs == 2
     del graphs
+    torch.cuda.synchronize()
     torch_ops.clear_cache()
