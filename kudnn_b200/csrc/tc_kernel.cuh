@@ -1617,6 +1617,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         if (lane == 0 && pair_rank == 0) {  // in a pair, the leader issues for both CTAs
+            // the limit of the waits below counts from here: no stage is complete while the previous kernel runs, because its
+            // activations are loaded after that
+            pdl_wait();
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;

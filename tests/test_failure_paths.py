@@ -39,6 +39,34 @@ def test_bounded_wait_runs_out_and_the_handle_recovers(cuda_device):
     assert lin.last_kernel == kb.KERNEL_TC
 
 
+@pytest.mark.parametrize("m,n,k,prepack", [(256, 256, 256, False), (512, 2048, 256, True)])
+def test_the_wait_limit_does_not_count_the_kernel_in_front(cuda_device, m, n, k, prepack):
+    """A launch that is set up while a long kernel still runs on a few SMs waits for that one outside its limited waits."""
+    case = dict(m=m, n=n, k=k, dtype="bf16", b_layout="AB", bias="row", x_dist="normal", w_std=0.05, seed=73)
+    desc, arrays, c = helpers.build_case(case)
+    ref_c, _ = helpers.run_oracle(desc, arrays, c)
+    d = {key: helpers._to_torch(v, cuda_device) for key, v in arrays.items()}
+    y = torch.zeros((m, n), dtype=torch.int16, device=cuda_device)
+    stream = torch.cuda.current_stream().cuda_stream
+    lin = kb.Linear(desc)
+    lin.force_kernel(kb.KERNEL_TC)
+    if prepack:
+        lin.prepack(d["b"], stream=stream)
+    lin.run(d["a"], d["b"], y, d["bias"], stream=stream)
+    # one CTA that walks 400000 k: several milliseconds, while the limit is about one
+    slow = kb.Linear(kb.make_desc(32, 32, 400000, kb.F32))
+    slow.force_kernel(kb.KERNEL_SIMT)
+    x = torch.zeros((32, 400000), device=cuda_device)
+    out = torch.zeros((32, 32), device=cuda_device)
+    lin.debug_set_wait(2_000_000, -1)
+    y.zero_()
+    for _ in range(2):
+        slow.run(x, x, out, stream=stream)
+        lin.run(d["a"], d["b"], y, d["bias"], stream=stream)
+    lin.check(stream=stream)
+    helpers.compare(helpers._from_torch(y).reshape(ref_c.shape), ref_c, desc.c_dtype)
+
+
 def test_device_allocation_failure_is_reported_and_survived(cuda_device):
     case = dict(m=4, n=1000, k=1032, dtype="bf16", bias="row", x_dist="normal", w_std=0.05, seed=72)
     desc, arrays, c = helpers.build_case(case)
