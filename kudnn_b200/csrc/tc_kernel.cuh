@@ -1474,7 +1474,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_bar + s, 1);
@@ -1501,6 +1500,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                          : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+        // Only now may the next kernel's CTAs start: the allocation waits for as long as another CTA holds the columns, and a
+        // successor that got in front of a CTA of this launch would itself be waiting for this launch to end.
+        pdl_launch_dependents();
     }
     tc_fence_before();
     __syncthreads();

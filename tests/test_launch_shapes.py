@@ -100,3 +100,23 @@ def test_chained_calls_read_each_others_results(cuda_device):
             assert torch.allclose(src.float(), want, atol=6 * 2.0 ** -8 * 4, rtol=2.0 ** -6)
         for lin in lins:
             lin.close()
+
+
+@pytest.mark.parametrize("m", [40, 300])
+def test_chained_integer_products(cuda_device, m):
+    """Integer tiles of up to 128 columns leave room for two CTAs on an SM: those of consecutive launches share its tensor memory."""
+    rng = np.random.default_rng(10)
+    stream = torch.cuda.current_stream().cuda_stream
+    n, k = 3000, 1040
+    a = torch.from_numpy(rng.integers(-128, 128, (4, m, k)).astype(np.int8)).to(cuda_device)
+    b = torch.from_numpy(rng.integers(-128, 128, (k, n)).astype(np.int8)).to(cuda_device)
+    want = (a.double() @ b.double()).to(torch.int32)
+    desc = kb.make_desc(m, n, k, kb.S8, c_dtype=kb.S32, b_strides=(n, 1))
+    lin = kb.Linear(desc)
+    lin.prepack(b, stream=stream)
+    got = torch.zeros((60, m, n), dtype=torch.int32, device=cuda_device)
+    for i in range(60):
+        lin.run(a[i % 4], b, got[i], stream=stream)
+    lin.check(stream=stream)
+    assert lin.last_kernel == kb.KERNEL_TC
+    assert all(torch.equal(got[i], want[i % 4]) for i in range(60))
