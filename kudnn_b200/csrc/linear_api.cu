@@ -235,14 +235,16 @@ int ensure_device(Handle *h)
     if (h->device != -1) {
         return fail(KUDNN_B200_BAD_ARGUMENTS, "handle was first used on device %d, current device is %d", h->device, dev);
     }
-    cudaDeviceProp prop;
-    e = cudaGetDeviceProperties(&prop, dev);
+    // three attributes rather than cudaGetDeviceProperties, which takes tens of milliseconds: every new handle comes here
+    int major = 0, minor = 0, sm_count = 0;
+    e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) {
-        return fail_cuda(e, "cudaGetDeviceProperties");
+        return fail_cuda(e, "device attributes");
     }
-    if (prop.major != 10) {
-        return fail(KUDNN_B200_NO_DEVICE, "device %d is sm_%d%d; this library carries sm_100a code only", dev, prop.major,
-                    prop.minor);
+    if (major != 10) {
+        return fail(KUDNN_B200_NO_DEVICE, "device %d is sm_%d%d; this library carries sm_100a code only", dev, major, minor);
     }
     e = h->status.reserve(sizeof(kb::DeviceStatus));
     if (e != cudaSuccess) {
@@ -253,7 +255,7 @@ int ensure_device(Handle *h)
         return fail_cuda(e, "status block");
     }
     h->device = dev;
-    h->sm_count = prop.multiProcessorCount;
+    h->sm_count = sm_count;
     return KUDNN_B200_OK;
 }
 
