@@ -1170,8 +1170,8 @@ cudaError_t launch_gemv(const LinearProblem &pr, const GemvPlan &plan, const Gem
     p.partials = ws.partials;
     p.counters = ws.counters;
     p.epi = pr.epi;
-    p.w_stable = pr.b_stable ? 1 : 0;
     p.w_blk = plan.kernel == KUDNN_B200_KERNEL_GEMV_MMA ? static_cast<const unsigned short *>(pr.b_blocked) : nullptr;
+    p.w_stable = pr.b_stable || p.w_blk != nullptr ? 1 : 0;  // the decode-packed copy is always the handle's own
     p.w8 = pr.b_dtype == KUDNN_B200_S8 ? 1 : (pr.b_dtype == KUDNN_B200_U8 ? 2 : 0);
     p.blk_kb = static_cast<int>(pr.b_blocked_kpad / 64);
     const bool w8 = pr.b_dtype == KUDNN_B200_S8 || pr.b_dtype == KUDNN_B200_U8;

@@ -821,7 +821,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
         pr.b = h->packed_raw;
         pr.b_sk = 1;
         pr.b_sn = h->packed_ld;
-        pr.b_stable = owns_packed(h) || h->blocked_kpad > 0;
+        pr.b_stable = owns_packed(h);
         if (h->blocked_kpad > 0) {
             pr.b_blocked = h->b_blocked.ptr;
             pr.b_blocked_kpad = h->blocked_kpad;

@@ -120,3 +120,26 @@ def test_chained_integer_products(cuda_device, m):
     lin.check(stream=stream)
     assert lin.last_kernel == kb.KERNEL_TC
     assert all(torch.equal(got[i], want[i % 4]) for i in range(60))
+
+
+@pytest.mark.parametrize("kernel,m", [(kb.KERNEL_GEMV_FMA, 1), (kb.KERNEL_GEMV_FMA, 3), (kb.KERNEL_TC, 40)])
+def test_weights_in_place_are_read_after_the_kernel_that_writes_them(cuda_device, kernel, m):
+    """Rows used where the caller keeps them are not requested early, whatever other copy a primitive has."""
+    rng = np.random.default_rng(12)
+    stream = torch.cuda.current_stream().cuda_stream
+    n, k = 1024, 512
+    parts = torch.from_numpy(rng.standard_normal((20, n, 64), dtype=np.float32)).to(cuda_device, torch.bfloat16)
+    mix = torch.from_numpy(rng.standard_normal((k, 64), dtype=np.float32) / 8).to(cuda_device, torch.bfloat16)
+    x = torch.from_numpy(rng.standard_normal((m, k), dtype=np.float32)).to(cuda_device, torch.bfloat16)
+    w = torch.zeros((n, k), device=cuda_device, dtype=torch.bfloat16)
+    y = torch.zeros((20, m, n), device=cuda_device, dtype=torch.bfloat16)
+    writer, reader = kb.Linear(kb.make_desc(n, k, 64, kb.BF16)), kb.Linear(kb.make_desc(m, n, k, kb.BF16))
+    reader.force_kernel(kernel)
+    reader.prepack(w, stream=stream)
+    for i in range(20):
+        writer.run(parts[i], mix, w, stream=stream)
+        reader.run(x, w, y[i], stream=stream)
+    for i in range(20):
+        want = x.float() @ (parts[i].float() @ mix.float().T).to(torch.bfloat16).float().T
+        # one rounding of the result, and weights that round the other way (2^-8 of each of the 512 terms, added as a random walk)
+        assert torch.allclose(y[i].float(), want, atol=2.0 ** -8 * 512 ** 0.5, rtol=2.0 ** -8)
