@@ -39,6 +39,7 @@ struct GemvParams {
     int kc;            // chunk length in k (MMA kernel), multiple of 32
     int ksplit;
     int active_warps;  // per chunk
+    int work_warps;    // warps of a CTA that take a span; the others only help to copy the activations
     long long span;
     long long total;   // blocks per chunk
     int slots;         // slots per unit per chunk
@@ -147,8 +148,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_fma_kernel(const Ge
     const int threads = static_cast<int>(blockDim.x);
 
     const int lane = threadIdx.x & 31;
-    const int warp = blockIdx.x * (threads >> 5) + (threadIdx.x >> 5);
-    const bool active = warp < p.active_warps;
+    const int warp_in_cta = threadIdx.x >> 5;
+    const int warp = blockIdx.x * p.work_warps + warp_in_cta;
+    const bool active = warp_in_cta < p.work_warps && warp < p.active_warps;
     long long f = static_cast<long long>(warp) * p.span;
     const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
     const char *wbase = static_cast<const char *>(p.w);
@@ -469,8 +471,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) gemv_mma_kernel(const Ge
 
     const int lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
-    const int warp = cta_in_chunk * (threads >> 5) + (threadIdx.x >> 5);
-    const bool active = warp < p.active_warps;
+    const int warp_in_cta = threadIdx.x >> 5;
+    const int warp = cta_in_chunk * p.work_warps + warp_in_cta;
+    const bool active = warp_in_cta < p.work_warps && warp < p.active_warps;
     long long f = static_cast<long long>(warp) * p.span;
     const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
 
@@ -642,8 +645,8 @@ __global__ void __launch_bounds__(kStagedThreads, 1) gemv_mma_staged_kernel(cons
     const int lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
     const int warp_in_cta = threadIdx.x >> 5;
-    const int warp = cta_in_chunk * (static_cast<int>(blockDim.x) >> 5) + warp_in_cta;
-    const bool active = warp < p.active_warps;
+    const int warp = cta_in_chunk * p.work_warps + warp_in_cta;
+    const bool active = warp_in_cta < p.work_warps && warp < p.active_warps;
     long long f = static_cast<long long>(warp) * p.span;
     const long long f_end = (f + p.span < p.total) ? f + p.span : p.total;
     const unsigned short *wg = static_cast<const unsigned short *>(p.w);
@@ -933,8 +936,10 @@ cudaError_t launch_shape(const GemvParams &p, const GemvPlan &plan, int shape, c
 }  // namespace
 
 // How `units` units (weight rows, or groups of 8 rows) of `blocks` blocks are cut between the warps of `ctas` CTAs: spans of
-// equal length, at least `min_span` blocks each, and as few warps per CTA as the spans need, so that a small matrix is
-// spread over all SMs.
+// equal length, at least `min_span` blocks each, and as few working warps per CTA as the spans need, so that a small matrix is
+// spread over all SMs.  With min_span = blocks a warp has at least one whole unit, which it ends without a hand-over.  Longer
+// spans at a time when warps are idle only lengthen the chain of a warp (us per call, one unit / at least 4 KB per warp: 2 x
+// 9000 x 32 bf16 5.0 / 20.8, 12 x 200 x 32 4.2 / 12.2), and shorter ones cost a hand-over (4 x 209 x 1152 fp32 7.0 / 12.5).
 struct GemvCut {
     long long span, active;
     int warps_per_cta, slots;
@@ -953,16 +958,24 @@ GemvCut cut_units(long long units, long long blocks, int ctas, int warps, long l
     return c;
 }
 
+// Threads of a CTA: its working warps, and enough others that a thread copies at most two vectors of the activations (a single
+// warp per CTA took 8 us longer for 4 x 16 x 8192 fp32), but not more (512 threads against 224, 2 x 2048 x 512 fp32 7.3 / 6.1 us).
+int cta_threads(int work_warps, long long x_vectors, int limit)
+{
+    const long long copy = (x_vectors / 2 + 31) / 32 * 32;
+    return static_cast<int>(std::min<long long>(std::max<long long>(32 * work_warps, copy), limit));
+}
+
 // The number of K chunks of the MMA kernels.  More chunks shorten the stretch of the activations that every CTA copies to its
-// shared memory (about 40 bytes per ns and SM) and give every warp more pieces of a group to end: estimated ns of both beside
-// the stream of the weights.  Measured over 1 to 16 chunks, us: 16 x 28672 x 8192 84 with 2, 94 with 4, 127 with 8; 16 x 6144 x
+// shared memory (about 40 bytes per ns and SM) and the chain of loads of a warp (block_ns for a block), and give every warp more
+// pieces of a group to end: estimated ns of all three beside the stream of the weights.  Measured over 1 to 16 chunks, us: 16 x 28672 x 8192 84 with 2, 94 with 4, 127 with 8; 16 x 6144 x
 // 5888 24 / 21 / 22 / 21 with 1 / 2 / 4 / 6; 4 x 11008 x 4096 23 / 24 / 30 with 1 / 2 / 4.  Returns 0 when no chunk fits `budget`.
-int choose_ksplit(long long groups, long long k, long long block_k, int rows, long long block_bytes, int ctas_all, int ctas_per_sm,
-                  int warps, long long min_span, size_t budget)
+int choose_ksplit(long long groups, long long k, long long block_k, int rows, long long block_bytes, double block_ns, double slot_ns, int ctas_all,
+                  int ctas_per_sm, int warps, size_t budget)
 {
     int best = 0;
     double best_ns = 1e300;
-    for (int ks = 1; ks <= 64; ks = ks < 8 ? ks + 1 : ks + ks / 4) {
+    for (const int ks : {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64}) {
         const long long kc = ((k + ks - 1) / ks + block_k - 1) / block_k * block_k;
         if ((ks - 1) * kc >= k && ks > 1) {
             continue;  // the last chunk would be empty
@@ -971,13 +984,19 @@ int choose_ksplit(long long groups, long long k, long long block_k, int rows, lo
             continue;
         }
         const long long kbc = kc / block_k;
-        const GemvCut c = cut_units(groups, kbc, ctas_all / ks, warps, min_span);
+        if (ks > 1 && kbc * block_bytes < 4096) {
+            continue;  // a warp's piece of a group is worth a hand-over from about 4 KB on
+        }
+        const GemvCut c = cut_units(groups, kbc, ctas_all / ks, warps, kbc);
         const double per_sm = static_cast<double>(c.span) * block_bytes * c.warps_per_cta * ctas_per_sm;
-        const double stream = std::max(per_sm / 40.0, static_cast<double>(groups) * kbc * ks * block_bytes / 5800.0);
+        const double stream = std::max(std::max(per_sm / 40.0, static_cast<double>(groups) * kbc * ks * block_bytes / 5800.0),
+                                       c.span * block_ns);
         const double fill = 500.0 + static_cast<double>(rows) * kc * 2 * ctas_per_sm / 40.0;
-        // pieces a warp ends: each stalls it for several microseconds (partial sums, fence, counter, the last one's additions)
-        const double pieces = static_cast<double>(groups) / c.active + (kbc % c.span == 0 || c.span % kbc == 0 ? 0.0 : 1.0);
-        const double partials = 6000.0 * std::max(pieces, 1.0);
+        // pieces a warp ends: each stalls it for several microseconds (partial sums, fence, counter, the last one's additions of
+        // all chunks), a whole group for less
+        const bool whole = kbc % c.span == 0 || c.span % kbc == 0;
+        const double pieces = static_cast<double>(groups) / c.active + (whole ? 0.0 : 1.0);
+        const double partials = (ks == 1 && whole ? 3000.0 : 6000.0 + slot_ns * ks) * std::max(pieces, 1.0);
         if (stream + fill + partials < best_ns) {
             best_ns = stream + fill + partials;
             best = ks;
@@ -1031,12 +1050,27 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
         const int shape = smem > 100 * 1024 ? 1 : 0;  // above 100 KB only one CTA fits per SM
         const int warps = kShapes[shape].threads / 32;
         const int ctas = sm_count * kShapes[shape].min_blocks;
-        // At least four blocks (2 KB) per warp.  With fixed scratch a row is not cut more than once.
-        const GemvCut c = cut_units(pr.n, kb, ctas, warps, fixed_scratch ? kb : 4);
+        // Whole rows, or rows cut 4, 8 or 16 ways where the chain of a warp's loads (ns per block, measured on 16 to 1024 rows
+        // of K up to 32768) is longer than the hand-over that the cut costs: 16 x 16384 bf16, one activation row, 10.9 us whole,
+        // 7.2 in 16 parts; 200 x 8192 fp32 8.1 and 6.3; 512 x 2048 fp32 5.2 whole.  With fixed scratch a row is not cut more than once.
+        const double block_ns = w8 ? 250.0 : dt == KUDNN_B200_F32 ? 110.0 * pr.m : 180.0 * pr.m;
+        GemvCut c = cut_units(pr.n, kb, ctas, warps, kb);
+        if (!fixed_scratch) {
+            double best = c.span * block_ns;
+            for (int parts = 4; parts <= 16; parts *= 2) {
+                const GemvCut cut = cut_units(pr.n, kb, ctas, warps, (kb + parts - 1) / parts);
+                const double ns = cut.span * block_ns + (2000.0 + 120.0 * parts) * pr.m;
+                if (cut.span < c.span && ns < best) {
+                    best = ns;
+                    c = cut;
+                }
+            }
+        }
         plan->shape = shape;
         plan->wide = 0;
-        plan->block = 32 * (fixed_scratch ? warps : c.warps_per_cta);
-        plan->grid = static_cast<int>((c.active + plan->block / 32 - 1) / (plan->block / 32));
+        plan->work_warps = fixed_scratch ? warps : c.warps_per_cta;
+        plan->block = cta_threads(plan->work_warps, pr.m * kb * block_k / (dt == KUDNN_B200_F32 ? 4 : 8), 32 * warps);
+        plan->grid = static_cast<int>((c.active + plan->work_warps - 1) / plan->work_warps);
         plan->ksplit = 1;
         plan->active_warps = static_cast<int>(c.active);
         plan->span = c.span;
@@ -1062,9 +1096,9 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
     const bool swapped = w8 && rows == 8;  // groups of 16 weight rows (see gemv_mma_kernel)
     const long long groups = swapped ? (pr.n + 15) / 16 : (pr.n + 7) / 8;
     // With fixed scratch: the fewest chunks that fit, and a group of rows cut at most once per chunk boundary.
-    auto finish_plan = [&](int shape, int ksplit, long long kc, long long block_k, int ctas, int warps, long long min_span, size_t smem) {
+    auto finish_plan = [&](int shape, int ksplit, long long kc, long long block_k, int ctas, int warps, size_t smem) {
         const long long kbc = kc / block_k;
-        GemvCut c = cut_units(groups, kbc, std::max(ctas / ksplit, 1), warps, fixed_scratch ? 1 : min_span);
+        GemvCut c = cut_units(groups, kbc, std::max(ctas / ksplit, 1), warps, kbc);
         if (fixed_scratch) {
             const long long total = groups * kbc;
             long long active = std::min<long long>(static_cast<long long>(std::max(ctas / ksplit, 1)) * warps, 2 * groups);
@@ -1075,7 +1109,8 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
             c.slots = static_cast<int>((kbc + c.span - 1) / c.span) + 1;
         }
         plan->shape = shape;
-        plan->block = 32 * c.warps_per_cta;
+        plan->work_warps = c.warps_per_cta;
+        plan->block = cta_threads(plan->work_warps, rows * kc / 8, 32 * warps);
         plan->grid = static_cast<int>((c.active + c.warps_per_cta - 1) / c.warps_per_cta) * ksplit;
         plan->ksplit = ksplit;
         plan->active_warps = static_cast<int>(c.active);
@@ -1107,7 +1142,7 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
         const size_t staging = static_cast<size_t>(warps) * kStagedWarpBytes;
         const size_t budget = 225 * 1024 - staging;
         int ksplit = fixed_scratch ? 0
-                                   : choose_ksplit(groups, pr.k, kStagedBlockK, rows, 8 * kStagedBlockK * 2, sm_count, 1, warps, 1, budget);
+                                   : choose_ksplit(groups, pr.k, kStagedBlockK, rows, 8 * kStagedBlockK * 2, 1000.0, 80.0, sm_count, 1, warps, budget);
         if (ksplit == 0) {
             ksplit = fewest_chunks(kStagedBlockK, budget);
         }
@@ -1116,7 +1151,7 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
         if (xbytes <= budget) {
             plan->wide = 0;
             const int ctas = fixed_scratch ? std::max(sm_count / ksplit, 1) * ksplit : sm_count;
-            finish_plan(kStagedShape, ksplit, kc, kStagedBlockK, ctas, warps, 1, xbytes + staging);
+            finish_plan(kStagedShape, ksplit, kc, kStagedBlockK, ctas, warps, xbytes + staging);
             return true;
         }
     }
@@ -1128,10 +1163,10 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
     const long long block_k = wide ? 64 : 32;
     const long long block_bytes = (swapped ? 16 : 8) * block_k * (w8 ? 1 : 2);
     const int warps = kShapes[shape].threads / 32;
-    const long long min_span = 4096 / block_bytes;  // at least 4 KB of weights per warp
+    const double block_ns = w8 ? (rows == 16 ? 300.0 : 700.0) : wide ? 900.0 : 400.0;
     int ksplit = fixed_scratch ? 0
-                               : choose_ksplit(groups, pr.k, block_k, rows, block_bytes, sm_count * kShapes[shape].min_blocks,
-                                               kShapes[shape].min_blocks, warps, min_span, smem_budget);
+                               : choose_ksplit(groups, pr.k, block_k, rows, block_bytes, block_ns, 250.0, sm_count * kShapes[shape].min_blocks,
+                                               kShapes[shape].min_blocks, warps, smem_budget);
     if (ksplit == 0) {
         ksplit = fewest_chunks(block_k, smem_budget);
     }
@@ -1146,7 +1181,7 @@ bool gemv_plan(const LinearProblem &pr, int sm_count, int forced_kernel, bool fi
     plan->wide = wide ? 1 : 0;
     const int ctas = sm_count * kShapes[shape].min_blocks;
     finish_plan(shape, ksplit, kc, block_k, fixed_scratch ? std::max(ctas / ksplit, 1) * ksplit : ctas, kShapes[shape].threads / 32,
-                min_span, smem);
+                smem);
     return true;
 }
 
@@ -1164,6 +1199,7 @@ cudaError_t launch_gemv(const LinearProblem &pr, const GemvPlan &plan, const Gem
     p.n = static_cast<int>(pr.n);
     p.k = static_cast<int>(pr.k);
     p.ksplit = plan.ksplit;
+    p.work_warps = plan.work_warps;
     p.active_warps = plan.active_warps;
     p.span = plan.span;
     p.slots = plan.slots;

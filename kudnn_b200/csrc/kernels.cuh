@@ -32,6 +32,7 @@ struct GemvWorkspace {
 struct GemvPlan {
     int kernel;         // KUDNN_B200_KERNEL_GEMV_FMA / _MMA
     int grid, block;    // launch shape
+    int work_warps;     // warps of a CTA that take a span; the others only help to copy the activations
     int shape;          // index of the compiled (threads, CTAs per SM) variant
     int ksplit;         // K chunks (MMA kernel)
     int wide;           // MMA kernel with fragment-shaped loads: 1 = blocks of 64 k, 32 bytes per lane

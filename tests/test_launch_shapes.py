@@ -51,16 +51,23 @@ def test_few_tiles_on_the_general_kernel(cuda_device, dtype, m, n, k, layout):
     _run(cuda_device, kb.KERNEL_SIMT, m=m, n=n, k=k, dtype=dtype, bias="row", act=kb.ACT_SWISH, res_op=kb.RES_IDENTICAL, b_layout=layout)
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 1000, 8200), (1, 70, 16384), (3, 520, 4104), (8, 1003, 6152), (9, 2000, 5896), (16, 24, 8192)])
+@pytest.mark.parametrize("m,n,k", [(1, 1000, 8200), (1, 70, 16384), (3, 520, 4104), (8, 1003, 6152), (9, 2000, 5896), (16, 24, 8192),
+                                   (2, 9001, 32), (5, 7, 40), (12, 200, 72), (1, 20000, 264), (1, 3, 32), (8, 28003, 1040)])
 @pytest.mark.parametrize("prepack", [False, True])
 def test_streaming_cuts(cuda_device, m, n, k, prepack):
     kernel = kb.KERNEL_GEMV_FMA if m == 1 else kb.KERNEL_GEMV_MMA
     _run(cuda_device, kernel, m=m, n=n, k=k, dtype="bf16", bias="row", act=kb.ACT_SWISH, res_op=kb.RES_NONE, prepack=prepack)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 5000, 516), (2, 9001, 36), (4, 209, 1156), (3, 70, 8196), (1, 300, 20484)])
+@pytest.mark.parametrize("prepack", [False, True])
+def test_streaming_cuts_fp32(cuda_device, m, n, k, prepack):
+    _run(cuda_device, kb.KERNEL_GEMV_FMA, m=m, n=n, k=k, dtype="f32", bias="row", act=kb.ACT_SWISH, res_op=kb.RES_IDENTICAL, prepack=prepack)
+
+
 @pytest.mark.parametrize("wcode", [kb.S8, kb.U8])
-@pytest.mark.parametrize("m", [2, 7, 8, 9, 16])
-@pytest.mark.parametrize("n,k", [(15, 8208), (1003, 1040), (2464, 5264)])
+@pytest.mark.parametrize("m", [1, 2, 7, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(15, 8208), (1003, 1040), (2464, 5264), (9001, 48)])
 def test_streaming_8_bit_weights(cuda_device, wcode, m, n, k):
     rng = np.random.default_rng(5)
     x = ko.to_storage(rng.standard_normal((1, m, k), dtype=np.float32), kb.F16)
@@ -71,7 +78,7 @@ def test_streaming_8_bit_weights(cuda_device, wcode, m, n, k):
     ref, _ = helpers.run_oracle(desc, arrays, c, acc=ko.ACC_F64)
     for prepack in (False, True):
         got, _, used = helpers.run_gpu(desc, arrays, c, cuda_device, prepack=prepack)
-        assert used == kb.KERNEL_GEMV_MMA
+        assert used == (kb.KERNEL_GEMV_FMA if m == 1 else kb.KERNEL_GEMV_MMA)
         helpers.compare(got, ref, desc.c_dtype)
 
 
