@@ -1123,7 +1123,7 @@ __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTen
     const int step = kEpiWarps * 32 / groups;  // rows the CTA covers per pass
     int r = tid / groups;
     const int g = tid - r * groups;
-    const int ni = tn * bn + g * 8;
+    const long long ni = static_cast<long long>(tn) * bn + g * 8;  // the last tile may end past the 32-bit range
     if (r >= step || ni >= n) {
         return;
     }
@@ -1208,8 +1208,8 @@ __device__ __forceinline__ void finish_rows_lean(const EpiParams &e, const EpiTe
     const int step = kEpiWarps * 32 / groups;  // rows the CTA covers per pass
     int r = tid / groups;
     const int g = tid - r * groups;
-    const int ni = tn * bn + g * 8;
-    const int valid = n - ni < 8 ? n - ni : 8;
+    const long long ni = static_cast<long long>(tn) * bn + g * 8;  // the last tile may end past the 32-bit range
+    const int valid = n - ni < 8 ? static_cast<int>(n - ni) : 8;
     const bool works = r < step && valid > 0;
     const long long m0 = static_cast<long long>(tm) * kBM + row0;
     const int pitch = (bn + 4) * 4;
@@ -1268,8 +1268,8 @@ __device__ __forceinline__ void finish_rows_lean(const EpiParams &e, const EpiTe
     }
     if (kRagged) {
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-        const int left = n - tn * bn;
-        const int cols = left < bn ? left : bn;
+        const long long left = n - static_cast<long long>(tn) * bn;
+        const int cols = left < bn ? static_cast<int>(left) : bn;
         const unsigned char *tile = reinterpret_cast<const unsigned char *>(part) + row0 * pitch;
         auto value = [&](int row, int col) {
             return static_cast<unsigned>(*reinterpret_cast<const unsigned short *>(tile + row * pitch + (col >> 3) * 32 + (col & 7) * 2));
@@ -1301,8 +1301,8 @@ __device__ __forceinline__ void finish_rows_any(const EpiParams &e, const EpiTen
     const int ct = kDt > 0 ? kDt : e.c_dtype, bt = kDt > 0 ? kDt : e.bias_dtype;
     const int rt = kDt > 0 ? kDt : e.res_dtype, ot = kDt > 0 ? kDt : e.out_dtype;
     const long long n0 = static_cast<long long>(tn) * bn + lane;
-    const int left = n - tn * bn;
-    const int cols = left < bn ? left : bn;  // columns of this tile that exist
+    const long long left = n - static_cast<long long>(tn) * bn;
+    const int cols = left < bn ? static_cast<int>(left) : bn;  // columns of this tile that exist
     const bool has_bias = e.has_bias != 0;
     float side[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     auto fetch_bias = [&](long long mi) {
