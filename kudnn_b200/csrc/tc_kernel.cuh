@@ -1123,8 +1123,9 @@ __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTen
     const int step = kEpiWarps * 32 / groups;  // rows the CTA covers per pass
     int r = tid / groups;
     const int g = tid - r * groups;
-    const long long ni = static_cast<long long>(tn) * bn + g * 8;  // the last tile may end past the 32-bit range
-    if (r >= step || ni >= n) {
+    const unsigned col = static_cast<unsigned>(tn) * bn + g * 8;  // the last tile may end past the range of an int
+    const int ni = static_cast<int>(col);
+    if (r >= step || col >= static_cast<unsigned>(n)) {
         return;
     }
     const int ct = kDt > 0 ? kDt : e.c_dtype, bt = kDt > 0 ? kDt : e.bias_dtype;
@@ -1208,8 +1209,9 @@ __device__ __forceinline__ void finish_rows_lean(const EpiParams &e, const EpiTe
     const int step = kEpiWarps * 32 / groups;  // rows the CTA covers per pass
     int r = tid / groups;
     const int g = tid - r * groups;
-    const long long ni = static_cast<long long>(tn) * bn + g * 8;  // the last tile may end past the 32-bit range
-    const int valid = n - ni < 8 ? static_cast<int>(n - ni) : 8;
+    const unsigned col = static_cast<unsigned>(tn) * bn + g * 8;  // the last tile may end past the range of an int
+    const int ni = static_cast<int>(col);
+    const int valid = col >= static_cast<unsigned>(n) ? 0 : (n - ni < 8 ? n - ni : 8);
     const bool works = r < step && valid > 0;
     const long long m0 = static_cast<long long>(tm) * kBM + row0;
     const int pitch = (bn + 4) * 4;
@@ -1500,9 +1502,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                          : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
-        // Only now may the next kernel's CTAs start: the allocation waits for as long as another CTA holds the columns, and a
-        // successor that got in front of a CTA of this launch would itself be waiting for this launch to end.
-        pdl_launch_dependents();
     }
     tc_fence_before();
     __syncthreads();
@@ -1685,6 +1684,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
     } else if (warp < 2 + p.epi_warps) {
         // ------------------------------------------------------------------ epilogue warps
+        // Only now, with this CTA's tensor memory allocated, may the next kernel's CTAs start: the allocation waits for as long as
+        // another CTA holds the columns, and a successor that got in front of a CTA of this launch would itself be waiting for
+        // this launch to end.
+        pdl_launch_dependents();
         pdl_wait();
         const int quarter = warp & 3;  // TMEM lanes this warp may touch: [32 * quarter, 32 * quarter + 32)
         const int row_in_tile = quarter * 32 + lane;
