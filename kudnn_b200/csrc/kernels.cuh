@@ -67,9 +67,9 @@ struct TcOperands {
     long long batch = 1, a_bstride = 0, b_bstride = 0;
     bool b_stable = false;  // b is a pre-packed copy: no kernel on the stream writes it
 };
-// How the epilogue meets its tensors: every row 16 bytes at a time (and beta = 0), rows whose elements are contiguous but
-// start anywhere, or neither.
-enum class TcRows { kVectors, kContiguous, kOther };
+// How the epilogue meets its tensors: every row 16 bytes at a time; the same but for the last columns, n being no multiple of 8;
+// rows whose elements are contiguous but start anywhere; or neither.
+enum class TcRows { kVectors, kAligned, kContiguous, kOther };
 struct TcPlan {
     int block_n;   // tile width: a multiple of 16 up to 256
     int stages;
@@ -80,7 +80,7 @@ struct TcPlan {
     int splits, kb_per_split;
     int a_rows;      // rows of the activation operand per copy (fewer than 128 only when the problem has fewer)
     int ring_bytes;  // shared memory in front of the barriers
-    int vector_rows;  // 1: TcRows::kVectors
+    TcRows rows;
     int via_smem;    // 1: one work item per CTA, the tile is finished from shared memory
     int pair;      // 1: clusters of two CTAs share 256 x block_n tiles (cta_group::2)
     int narrow_from;  // pair mode: tiles from this index on are processed as two pieces of half the width

@@ -358,11 +358,11 @@ kb::TcRows epilogue_rows(const kb::LinearProblem &pr)
                (s_n == 1 && aligned16(p) && s_m % vec == 0 && sb[0] % vec == 0 && sb[1] % vec == 0 && sb[2] % vec == 0);
     };
     const bool second = e.res_op != KUDNN_B200_RES_NONE;
-    if (e.beta == 0.0f && e.n % 8 == 0 && vectors(e.c, e.c_dtype, e.c_sm, e.c_sn, pr.batch.c_sb) &&
+    if (vectors(e.c, e.c_dtype, e.c_sm, e.c_sn, pr.batch.c_sb) &&
         (e.has_bias == 0 || e.bias_sn == 0 || vectors(e.bias, e.bias_dtype, e.bias_sm, e.bias_sn, pr.batch.bias_sb)) &&
         (!second || (vectors(e.res, e.res_dtype, e.res_sm, e.res_sn, pr.batch.res_sb) &&
                      vectors(e.out, e.out_dtype, e.out_sm, e.out_sn, pr.batch.out_sb)))) {
-        return kb::TcRows::kVectors;
+        return e.n % 8 == 0 ? kb::TcRows::kVectors : kb::TcRows::kAligned;
     }
     const bool contiguous = (e.c == nullptr || e.c_sn == 1) && (!second || (e.res_sn == 1 && e.out_sn == 1));
     return contiguous ? kb::TcRows::kContiguous : kb::TcRows::kOther;

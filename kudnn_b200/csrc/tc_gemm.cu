@@ -221,9 +221,13 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     // pair / single CTA: 4096 rows 1.385 / 1.396, 8192 rows 2.84 / 2.85, 16384 rows 6.10 / 5.96, 32768 rows
     // 13.3 / 12.4).
     const double flops = 2.0 * static_cast<double>(m) * static_cast<double>(n) * static_cast<double>(ops.k_total);
-    // batched launches use single CTAs, and so do outputs that cannot be stored as vectors
-    bool pair = n > kBM && m > kBM && (flops < 6.0e12 || env_choice("KUDNN_B200_TC_PAIR") > 0) && ops.batch == 1 && (rows == TcRows::kVectors || ints) && forced_splits <= 1 &&
-                env_choice("KUDNN_B200_TC_PAIR") != 0;
+    // Batched launches use single CTAs.
+    bool pair = n > kBM && m > kBM && (flops < 6.0e12 || env_choice("KUDNN_B200_TC_PAIR") > 0) && ops.batch == 1 &&
+                forced_splits <= 1 && env_choice("KUDNN_B200_TC_PAIR") != 0;
+    // Cycles the epilogue takes per value: a thread's row leaves 16 bytes at a time, or value by value, rows side by side for one
+    // output (column by column) or scattered.  4096 x 4603 x 2304, pair against single CTAs: bf16 379 and 130 us, fp32, whose
+    // products take six times as long, 414 and 427 us.
+    const double per_value = ints || rows == TcRows::kVectors || rows == TcRows::kAligned ? 0.35 : rows == TcRows::kContiguous ? 4.3 : 2.5;
     const int pair_stages = with_staging ? 5 : 6;
     plan->narrow_from = 0;
     if (pair) {
@@ -231,7 +235,7 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
         const long long guess = sm_count / 2;
         const long long full = pair_tiles / guess, rem = pair_tiles % guess;
         const double waves = full + (rem == 0 ? 0.0 : (full > 0 && 2 * rem <= guess ? 0.55 : 1.0));
-        const double epilogue = 1000.0 + 0.35 * kBM * 256;
+        const double epilogue = 1000.0 + per_value * kBM * 256;
         const double cycles = 4000.0 + waves * std::max(num_kb * 640.0, epilogue) + epilogue;
         pair = cycles < best || env_choice("KUDNN_B200_TC_PAIR") > 0;
         int clusters = 0;
@@ -253,7 +257,7 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
         }
     }
     plan->pair = pair ? 1 : 0;
-    plan->vector_rows = rows == TcRows::kVectors ? 1 : 0;
+    plan->rows = rows;
     plan->block_n = bn;
     plan->via_smem = via_smem ? 1 : 0;
     plan->splits = static_cast<int>(splits);
@@ -346,7 +350,7 @@ cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams
     p.a_rows = plan.a_rows;
     p.ring_bytes = plan.ring_bytes;
     p.via_smem = plan.via_smem;
-    p.vector_rows = plan.vector_rows;
+    p.rows = plan.rows;
     {
         // The A rows of one raster group are re-read for every tile column and should stay in L2 next to the
         // streaming weights: at most about 64 MB of them (16 tile rows of 256 x 8192 bf16).  Measured on the 32768-row

@@ -72,7 +72,7 @@ struct TcParams {
     int ring_bytes;  // bytes in front of the barriers: the stage ring, and room for one tile as fp32 if it is finished from there
     int b_stable;  // the weights were pre-packed: the first of them are loaded while the previous kernel still runs
     int via_smem;    // one work item per CTA, finished from shared memory (finish_rows)
-    int vector_rows;  // every row of the epilogue's tensors can be read and written 16 bytes at a time, beta = 0
+    TcRows rows;  // how a tile finished from shared memory meets the epilogue's tensors
     int group_m;  // tile rows per raster group: consecutive work items walk down group_m tile rows, then one tile right
     // CTA pairs: work items [0, narrow_from) are whole 256 x BN tiles; each later tile is two items of half the width,
     // so that a last wave that would keep fewer than half the pairs busy is spread over twice as many
@@ -1114,7 +1114,35 @@ __device__ __forceinline__ void ld_tile8(uint32_t addr, float (&v)[8])
 // straight from the accumulator, kernel times: 60 x 2560 x 1024 16.4 -> 10.1 us, 333 x 3008 x 2056 with GELU 33 -> 16 us,
 // with rows that start anywhere (n = 3001) 46 -> 19 us.
 
-// Any element types; rows of 16-byte vectors; both outputs, mirrors and alpha as they come.
+// Eight values of a row as one or two vectors, or the `valid` values that exist one by one.
+__device__ __forceinline__ void load_piece(const char *p, int dt, int valid, float (&v)[8])
+{
+    if (valid == 8) {
+        load8_vec(p, dt, v);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = j < valid ? load_as_f32(p, dt, j) : 0.0f;
+        }
+    }
+}
+
+__device__ __forceinline__ void store_piece(char *p, int dt, int valid, const float (&v)[8])
+{
+    if (valid == 8) {
+        store8_vec(p, dt, v);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j < valid) {
+                store_exact(p, dt, j, v[j]);
+            }
+        }
+    }
+}
+
+// Any element types; rows of 16-byte vectors, of which the last may be cut short by n (kAligned); both outputs, mirrors, alpha
+// and beta as they come.
 template <int kAct, int kDt>
 __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTensors &t, const float *part, int bn, int splits,
                                                 int row0, int rows, int tm, int tn, int n, int tid)
@@ -1130,6 +1158,7 @@ __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTen
     }
     const int ct = kDt > 0 ? kDt : e.c_dtype, bt = kDt > 0 ? kDt : e.bias_dtype;
     const int rt = kDt > 0 ? kDt : e.res_dtype, ot = kDt > 0 ? kDt : e.out_dtype;
+    const int valid = n - ni < 8 ? static_cast<int>(n - ni) : 8;
     const long long m0 = static_cast<long long>(tm) * kBM + row0 + r;
     // byte addresses of this thread's piece of the row, and their advance per pass
     char *c = t.c == nullptr ? nullptr : static_cast<char *>(t.c) + (m0 * e.c_sm + ni) * dtype_size(ct);
@@ -1143,7 +1172,7 @@ __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTen
     auto fetch_bias = [&](long long mi) {
         const char *bias = static_cast<const char *>(t.bias) + (mi * e.bias_sm + (e.bias_sn != 0 ? ni : 0)) * dtype_size(bt);
         if (e.bias_sn != 0) {
-            load8_vec(bias, bt, side);
+            load_piece(bias, bt, valid, side);
         } else {
             const float b = load_as_f32(bias, bt, 0);
 #pragma unroll
@@ -1167,7 +1196,7 @@ __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTen
         addr += static_cast<uint32_t>(step * pitch);
         float rs[8];
         if (second) {
-            load8_vec(res, rt, rs);
+            load_piece(res, rt, valid, rs);
             res += res_step;
         }
         if (has_bias && e.bias_sm != 0) {
@@ -1179,19 +1208,27 @@ __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTen
                 v[j] *= e.alpha;
             }
         }
+        if (e.beta != 0.0f) {
+            float old[8];
+            load_piece(c, ct, valid, old);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] += e.beta * old[j];
+            }
+        }
         chain8<kAct, kDt>(e, has_bias, side, v);
         if (c != nullptr) {
-            store8_vec(c, ct, v);
+            store_piece(c, ct, valid, v);
             for (int i = 0; i < e.n_mirrors; ++i) {
-                store8_vec(c + e.c_delta[i], ct, v);
+                store_piece(c + e.c_delta[i], ct, valid, v);
             }
             c += c_step;
         }
         if (second) {
             combine8<kDt>(e, rs, v);
-            store8_vec(out, ot, v);
+            store_piece(out, ot, valid, v);
             for (int i = 0; i < e.n_mirrors; ++i) {
-                store8_vec(out + e.out_delta[i], ot, v);
+                store_piece(out + e.out_delta[i], ot, valid, v);
             }
             out += out_step;
         }
@@ -1293,7 +1330,7 @@ __device__ __forceinline__ void finish_rows_lean(const EpiParams &e, const EpiTe
     }
 }
 
-// Everything else (any strides, beta): a warp takes a row and a lane the columns lane, lane + 32, ..., so that narrow accesses
+// Everything else (any strides): a warp takes a row and a lane the columns lane, lane + 32, ..., so that narrow accesses
 // of a warp are contiguous where the rows are.
 template <int kAct, int kDt>
 __device__ __forceinline__ void finish_rows_any(const EpiParams &e, const EpiTensors &t, const float *part, int bn, int splits,
@@ -1383,7 +1420,7 @@ __device__ __forceinline__ void finish_rows_any(const EpiParams &e, const EpiTen
 }
 
 template <int kAct, int kDt>
-__device__ __forceinline__ void finish_rows(const EpiParams &e, const EpiTensors &t, bool vector_rows, float *part, int bn,
+__device__ __forceinline__ void finish_rows(const EpiParams &e, const EpiTensors &t, TcRows kind, float *part, int bn,
                                             int splits, uint32_t rank, int tm, int tn, int m, int n, int tid)
 {
     // the tile's rows, shared out evenly between the ranks
@@ -1397,7 +1434,7 @@ __device__ __forceinline__ void finish_rows(const EpiParams &e, const EpiTensors
         if (e.alpha == 1.0f && e.beta == 0.0f && e.n_mirrors == 0 && e.bias_sm == 0 && (t.c == nullptr) == second && contiguous) {
 #define KB_FINISH(SECOND, SPLIT, RAGGED) \
     finish_rows_lean<kAct, kDt, SECOND, SPLIT, RAGGED>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid)
-            if (vector_rows) {
+            if (kind == TcRows::kVectors) {
                 if (second) {
                     splits > 1 ? KB_FINISH(true, true, false) : KB_FINISH(true, false, false);
                 } else {
@@ -1412,7 +1449,7 @@ __device__ __forceinline__ void finish_rows(const EpiParams &e, const EpiTensors
             return;
         }
     }
-    if (vector_rows) {
+    if (kind == TcRows::kVectors || kind == TcRows::kAligned) {
         finish_rows_vec<kAct, kDt>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
     } else {
         finish_rows_any<kAct, kDt>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
@@ -1832,22 +1869,22 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                    (p.epi.res_op == KUDNN_B200_RES_NONE || (p.epi.res_dtype == kKind && p.epi.out_dtype == kKind));
                 switch (typed ? p.epi.act : -1) {
                     case KUDNN_B200_ACT_NONE:
-                        finish_rows<KUDNN_B200_ACT_NONE, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_NONE, kKind>(p.epi, t, p.rows, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     case KUDNN_B200_ACT_RELU:
-                        finish_rows<KUDNN_B200_ACT_RELU, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_RELU, kKind>(p.epi, t, p.rows, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     case KUDNN_B200_ACT_SWISH:
-                        finish_rows<KUDNN_B200_ACT_SWISH, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_SWISH, kKind>(p.epi, t, p.rows, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     case KUDNN_B200_ACT_GELU_TANH:
-                        finish_rows<KUDNN_B200_ACT_GELU_TANH, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_GELU_TANH, kKind>(p.epi, t, p.rows, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     case KUDNN_B200_ACT_GELU_ERF:
-                        finish_rows<KUDNN_B200_ACT_GELU_ERF, kKind>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<KUDNN_B200_ACT_GELU_ERF, kKind>(p.epi, t, p.rows, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                     default:
-                        finish_rows<-1, -1>(p.epi, t, p.vector_rows != 0, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
+                        finish_rows<-1, -1>(p.epi, t, p.rows, part, p.bn, p.splits, rank, tm, tn, p.m, p.n, epi_tid);
                         break;
                 }
             }

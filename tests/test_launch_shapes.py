@@ -150,3 +150,42 @@ def test_weights_in_place_are_read_after_the_kernel_that_writes_them(cuda_device
         want = x.float() @ (parts[i].float() @ mix.float().T).to(torch.bfloat16).float().T
         # one rounding of the result, and weights that round the other way (2^-8 of each of the 512 terms, added as a random walk)
         assert torch.allclose(y[i].float(), want, atol=2.0 ** -8 * 512 ** 0.5, rtol=2.0 ** -8)
+
+
+@pytest.mark.parametrize("dtype,ctype", [("bf16", "bf16"), ("f16", "f16"), ("f32", "f32"), ("bf16", "f32")])
+@pytest.mark.parametrize("n", [136, 132, 131, 129])
+@pytest.mark.parametrize("m,pairs", [(133, False), (20, False), (300, True)])
+@pytest.mark.parametrize("beta,both", [(0.5, False), (0.5, True), (0.0, True)])
+def test_rows_of_vectors_with_beta_and_a_cut_last_column(cuda_device, monkeypatch, dtype, ctype, n, m, pairs, beta, both):
+    """c is read and written, rows start on 16 bytes and end inside a vector: nothing beyond column n is touched."""
+    if pairs:
+        monkeypatch.setenv("KUDNN_B200_TC_PAIR", "1")
+    td = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
+    code = {"f32": kb.F32, "f16": kb.F16, "bf16": kb.BF16}
+    k, gen = 520, torch.Generator(device=cuda_device)
+    gen.manual_seed(21)
+
+    def draw(*shape, dt=td[dtype], std=1.0):
+        return (torch.randn(shape, generator=gen, device=cuda_device) * std).to(dt)
+
+    vec = 16 // td[ctype].itemsize
+    pitch = (n + vec - 1) // vec * vec
+    a, w, bias = draw(m, k), draw(n, k, std=0.05), draw(n, dt=td[ctype])
+    c, res, out = (draw(m, pitch, dt=td[ctype]) for _ in range(3))
+    c0, out0 = c.clone(), out.clone()
+    desc = kb.make_desc(m, n, k, code[dtype], c_dtype=code[ctype], has_bias=True, bias_dtype=code[ctype], act=kb.ACT_RELU, act_alpha=0.0,
+                        res_op=kb.RES_IDENTICAL if both else kb.RES_NONE, res_dtype=code[ctype], out_dtype=code[ctype],
+                        c_strides=(pitch, 1), res_strides=(pitch, 1), out_strides=(pitch, 1))
+    lin = kb.Linear(desc)
+    lin.force_kernel(kb.KERNEL_TC)
+    lin.run(a, w, c, bias, res if both else None, out if both else None, beta=beta, stream=torch.cuda.current_stream().cuda_stream)
+    lin.check(stream=torch.cuda.current_stream().cuda_stream)
+    want = (a.double() @ w.double().T + beta * c0[:, :n].double() + bias.double()).relu()
+    # 16-bit results: a rounding after the bias and one after the second operator.  fp32: up to 195 additions to an accumulator of
+    # up to 6, each cut at 2^-23 of it, as a random walk (10^-5)
+    eps = {"bf16": 2.0 ** -8, "f16": 2.0 ** -11, "f32": 2.0 ** -16}[ctype]
+    assert torch.allclose(c[:, :n].double(), want, rtol=3 * eps, atol=4 * eps)
+    assert torch.equal(c[:, n:], c0[:, n:])
+    if both:
+        assert torch.allclose(out[:, :n].double(), want + res[:, :n].double(), rtol=3 * eps, atol=8 * eps)
+        assert torch.equal(out[:, n:], out0[:, n:])
