@@ -46,9 +46,9 @@ struct GemvPlan {
 // Records the calling thread's last error text and returns `code`.
 int set_last_error(int code, const char *message);
 
-cudaError_t launch_simt(const LinearProblem &pr, cudaStream_t stream);
+cudaError_t launch_simt(const LinearProblem &pr, int sm_count, cudaStream_t stream);
 // 8-bit integer operands (S8 / U8), 32-bit integer result and bias: exact sums
-cudaError_t launch_int_gemm(const LinearProblem &pr, cudaStream_t stream);
+cudaError_t launch_int_gemm(const LinearProblem &pr, int sm_count, cudaStream_t stream);
 
 // Streaming kernels for m <= 16 (2-D problems, K-contiguous operands).
 // fixed_scratch: cut with the fewest partial sums (the caller's scratch does not grow)

@@ -704,7 +704,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
         if (ip.batch_count > 65535) {
             return fail(KUDNN_B200_UNSUPPORTED, "more than 65535 batch entries");
         }
-        cudaError_t e = kb::launch_int_gemm(ip, stream);
+        cudaError_t e = kb::launch_int_gemm(ip, h->sm_count, stream);
         if (e != cudaSuccess) {
             return fail_cuda(e, "integer kernel launch");
         }
@@ -857,9 +857,10 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
     // apart (or are one shared matrix); anything else is packed first, all entries in one launch.
     const long long nb = pr.batch_count;
     const bool tc_types = d.a_dtype == d.b_dtype;
-    // fp32 takes two launches there (the activations are split first): 76 x 1562 x 73 with GELU, 8.7e6 products, 23 us against
-    // 10 us on the general kernel; 31 x 1817 x 151, 8.5e6, 13.6 against 12.4 us
-    const double tc_from = d.a_dtype == KUDNN_B200_F32 && nb == 1 ? 16.0e6 : 8.0e6;
+    // fp32 takes two launches there (the activations are split first), the general kernel 2 us per 64 k.  Times of both in us, 64
+    // rows, 8 to 16 million products: k = 64 10-15 and 8, 128 10-16 and 11, 192 12 and 14, 256 10-12 and 15-16, 512 11 and 24;
+    // 24 x 64 x 8192 43 and 264.
+    const double tc_from = d.a_dtype == KUDNN_B200_F32 && nb == 1 && d.k < 256 ? 16.0e6 : 8.0e6;
     const bool tc_worth = static_cast<double>(d.m) * d.n * d.k * static_cast<double>(nb) >= tc_from && d.k >= 32;
     const bool tc_batch_ok = nb == 1 || (nb <= 65535 && pr.epi.n_mirrors == 0);
     if (tc_batch_ok && tc_types && (forced == KUDNN_B200_KERNEL_TC || (forced == KUDNN_B200_KERNEL_AUTO && tc_worth))) {
@@ -1042,7 +1043,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
     if (pr.batch_count > 65535) {
         return fail(KUDNN_B200_UNSUPPORTED, "more than 65535 batch entries");
     }
-    cudaError_t e = kb::launch_simt(pr, stream);
+    cudaError_t e = kb::launch_simt(pr, h->sm_count, stream);
     if (e != cudaSuccess) {
         return fail_cuda(e, "general kernel launch");
     }

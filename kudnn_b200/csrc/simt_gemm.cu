@@ -293,19 +293,19 @@ __global__ void __launch_bounds__(256) simt_linear_kernel(const SimtParams p)
 
 }  // namespace
 
-static cudaError_t launch_general(const LinearProblem &pr, cudaStream_t stream, bool integer);
+static cudaError_t launch_general(const LinearProblem &pr, int sm_count, cudaStream_t stream, bool integer);
 
-cudaError_t launch_simt(const LinearProblem &pr, cudaStream_t stream)
+cudaError_t launch_simt(const LinearProblem &pr, int sm_count, cudaStream_t stream)
 {
-    return launch_general(pr, stream, false);
+    return launch_general(pr, sm_count, stream, false);
 }
 
-cudaError_t launch_int_gemm(const LinearProblem &pr, cudaStream_t stream)
+cudaError_t launch_int_gemm(const LinearProblem &pr, int sm_count, cudaStream_t stream)
 {
-    return launch_general(pr, stream, true);
+    return launch_general(pr, sm_count, stream, true);
 }
 
-static cudaError_t launch_general(const LinearProblem &pr, cudaStream_t stream, bool integer)
+static cudaError_t launch_general(const LinearProblem &pr, int sm_count, cudaStream_t stream, bool integer)
 {
     SimtParams p;
     p.a = pr.a;
@@ -333,7 +333,7 @@ static cudaError_t launch_general(const LinearProblem &pr, cudaStream_t stream, 
         // 7.4 / 24.2, both fp32 with SiLU).  From two waves of 64 x 64 tiles on, their four times lower operand traffic counts.
         const long long large_tiles = ((pr.n + kTile - 1) / kTile) * ((pr.m + kTile - 1) / kTile) * nbatch;
         const long long small_rows = (pr.m + kSmallTile - 1) / kSmallTile;
-        if (!integer && large_tiles < 2 * 148 && small_rows <= 65535) {
+        if (!integer && large_tiles < 2 * sm_count && small_rows <= 65535) {
             const dim3 small_grid(static_cast<unsigned>((pr.n + kSmallTile - 1) / kSmallTile), static_cast<unsigned>(small_rows),
                                   static_cast<unsigned>(nbatch));
             cudaError_t e = launch_chained(simt_small_kernel, small_grid, dim3(256), 0, stream, 1, p);

@@ -51,6 +51,12 @@ def test_few_tiles_on_the_general_kernel(cuda_device, dtype, m, n, k, layout):
     _run(cuda_device, kb.KERNEL_SIMT, m=m, n=n, k=k, dtype=dtype, bias="row", act=kb.ACT_SWISH, res_op=kb.RES_IDENTICAL, b_layout=layout)
 
 
+@pytest.mark.parametrize("m,n,k,kernel", [(24, 64, 8192, kb.KERNEL_TC), (17, 256, 2000, kb.KERNEL_TC), (128, 256, 256, kb.KERNEL_TC),
+                                          (128, 512, 200, kb.KERNEL_SIMT), (76, 1562, 73, kb.KERNEL_SIMT)])
+def test_small_fp32_goes_by_the_length_of_k(cuda_device, m, n, k, kernel):
+    _run(cuda_device, kernel, m=m, n=n, k=k, dtype="f32", bias="row", act=kb.ACT_RELU, act_alpha=0.0, res_op=kb.RES_NONE)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1000, 8200), (1, 70, 16384), (3, 520, 4104), (8, 1003, 6152), (9, 2000, 5896), (16, 24, 8192),
                                    (2, 9001, 32), (5, 7, 40), (12, 200, 72), (1, 20000, 264), (1, 3, 32), (8, 28003, 1040)])
 @pytest.mark.parametrize("prepack", [False, True])
