@@ -289,9 +289,10 @@ __device__ __forceinline__ void epilogue_scalar(const EpiParams &p, float acc, l
 }
 
 // ---- programmatic dependent launch
-// Every kernel of the library lets the next one on its stream be set up while it still runs, and waits for its predecessor
-// before it touches memory that the predecessor may write; what it does earlier (barriers, tensor memory, descriptors)
-// depends on no kernel.  Takes 2-4 us off a call that follows another one.
+// The tensor-core kernel, the streaming kernels, simt_small_kernel, pack_rows_kernel and split_rows_kernel let the next kernel
+// on their stream be set up while they still run, and wait for their predecessor before they touch memory that it may write;
+// what they do earlier (barriers, tensor memory, descriptors, weights in copies that the handle owns) depends on no kernel.  The
+// other kernels of the library do neither.  Takes 2-4 us off a call that follows another one.
 __device__ __forceinline__ void pdl_launch_dependents()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -11,14 +11,15 @@
 // buffer, bumps the unit's arrival counter, and the warp that arrives last adds the slots in slot order (so the
 // result does not depend on timing) and runs the fused epilogue.  Counters return to zero before the kernel ends.
 //
-//   FMA kernel  m <= 4, fp32 / fp16 / bf16.  Lane l of a warp owns k = 8l..8l+7 (16-bit) of every block of a row,
-//               accumulates with fp32 FMA against the activations held in shared memory as fp32, and a
+//   FMA kernel  m <= 4, fp32 / fp16 / bf16; m = 1 on 8-bit weights.  Lane l of a warp owns k = 8l..8l+7 (16-bit) of
+//               every block of a row, accumulates with fp32 FMA against the activations held in shared memory as fp32, and a
 //               warp-shuffle tree folds the 32 lanes when the row (or the span) ends.
 //   MMA kernel  m <= 16, fp16 / bf16.  A block is 8 rows x 32 k; the 16 bytes a lane loads feed two
 //               mma.sync.m16n8k16 (activations as the 16-row operand, zero padded), fp32 accumulators.  The
 //               contraction index inside a block is permuted identically for both operands so a lane's 16 bytes
 //               are consecutive in memory.  K is additionally cut into `ksplit` chunks across CTAs so the
-//               activation chunk fits shared memory.
+//               activation chunk fits shared memory.  8-bit weights with up to 8 activation rows: groups of 16 weight
+//               rows, which are then the 16-row operand, and the activations the 8-column one.
 #include "kernels.cuh"
 
 #include <algorithm>

@@ -1,13 +1,15 @@
 // General Linear kernel: any element strides, any of the three float storage types per tensor, any size,
-// leading batch dimensions with broadcast.  fp32 FMA accumulation in ascending k.  The same kernel with 32-bit integer
+// leading batch dimensions with broadcast.  fp32 FMA accumulation, in ascending k (large tiles) or in four interleaved parts
+// that are added in order (few tiles).  The kernel of large tiles with 32-bit integer
 // accumulators is the 8-bit integer product <s8|u8, s8|u8, s32, s32> of the reference
 // (src/dnn/src/kudnn_gemm.cpp:259-334): exact sums, an optional s32 bias, no post-operation.  It covers the shapes the
 // tensor-core and streaming kernels decline (rows that are not 16-byte aligned, tiny problems, transposed
 // activations) and serves as the on-device cross-check of the fast kernels.
 //
 // Work decomposition: one CTA per 64x64 output tile per batch entry, 256 threads, 4x4 outputs per thread,
-// k advanced 16 at a time through shared memory.  The role of this kernel in the reference is the batched loop
-// around the BLAS call, src/dnn/src/kudnn_gemm.cpp:710-824.
+// k advanced 16 at a time through shared memory; with fewer than two waves of such tiles 32x32 outputs per CTA
+// (simt_small_kernel).  The role of these kernels in the reference is the batched loop around the BLAS call,
+// src/dnn/src/kudnn_gemm.cpp:710-824.
 #include "kernels.cuh"
 
 namespace kb {
