@@ -39,9 +39,11 @@ def test_tile_widths_and_cuts(cuda_device, dtype, m, n, k, act, res_op, layout):
 @pytest.mark.parametrize("splits", ["1", "2", "4", "8"])
 @pytest.mark.parametrize("n", [130, 136])
 @pytest.mark.parametrize("bias", ["row", "full"])
-def test_every_cut_of_k(cuda_device, monkeypatch, dtype, splits, n, bias):
+def test_every_cut_of_k(cuda_device, monkeypatch, capfd, dtype, splits, n, bias):
     monkeypatch.setenv("KUDNN_B200_TC_SPLITS", splits)
-    _run(cuda_device, kb.KERNEL_TC, m=133, n=n, k=1100, dtype=dtype, bias=bias, act=kb.ACT_SWISH, res_op=kb.RES_NONE)
+    monkeypatch.setenv("KUDNN_B200_DEBUG", "1")
+    _run(cuda_device, kb.KERNEL_TC, m=133, n=n, k=1500, dtype=dtype, bias=bias, act=kb.ACT_SWISH, res_op=kb.RES_NONE)
+    assert "k splits %s," % splits in capfd.readouterr().err
 
 
 @pytest.mark.parametrize("dtype", ["bf16", "f16", "f32"])
@@ -88,31 +90,47 @@ def test_streaming_8_bit_weights(cuda_device, wcode, m, n, k):
         helpers.compare(got, ref, desc.c_dtype)
 
 
-def test_chained_calls_read_each_others_results(cuda_device):
-    """Layers whose input is the previous layer's output, across the kernels that may start before it has ended."""
+# rows, width, whether the CTA pairs are asked for, what the plan must say (None: another kernel)
+_CHAINS = [(1, 512, False, None), (4, 512, False, None), (12, 512, False, None), (33, 72, False, None), (40, 512, False, "128 x"),
+           (300, 512, False, "128 x"), (300, 1030, False, "128 x"), (300, 512, True, "256 (CTA pair)"), (300, 1030, True, "256 (CTA pair)")]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("owned", [False, True])
+@pytest.mark.parametrize("m,width,pairs,plan", _CHAINS)
+def test_chained_calls_read_each_others_results(cuda_device, monkeypatch, capfd, dtype, owned, m, width, pairs, plan):
+    """Layers whose input is the previous layer's output, across the kernels that may start before it has ended: packed and split
+    activations, and weights in a packed copy (owned: stored [k, n]; fp32 always), the first of which are loaded early."""
+    if pairs and width == 1030:
+        width = 1032  # rows that are no vectors are left to single CTAs at this size
+    if pairs:
+        monkeypatch.setenv("KUDNN_B200_TC_PAIR", "1")
+    monkeypatch.setenv("KUDNN_B200_DEBUG", "1")
     rng = np.random.default_rng(9)
     stream = torch.cuda.current_stream().cuda_stream
-    for m in (1, 4, 12, 40, 300):
-        width = 512
-        ws = [torch.from_numpy(rng.standard_normal((width, width), dtype=np.float32) / width ** 0.5).to(cuda_device, torch.bfloat16)
-              for _ in range(6)]
-        lins = [kb.Linear(kb.make_desc(m, width, width, kb.BF16)) for _ in ws]
-        for lin, w in zip(lins, ws):
-            lin.prepack(w, stream=stream)
-        x = torch.from_numpy(rng.standard_normal((m, width), dtype=np.float32)).to(cuda_device, torch.bfloat16)
-        want = x.float()
-        for w in ws:
-            want = (want @ w.float().T).to(torch.bfloat16).float()
-        for _ in range(20):
-            bufs = [torch.full((m, width), float("nan"), device=cuda_device, dtype=torch.bfloat16) for _ in ws]
-            src = x
-            for lin, w, dst in zip(lins, ws, bufs):
-                lin.run(src, w, dst, stream=stream)
-                src = dst
-            # six roundings to 8 significant bits, each at most 2^-8 of a value of order one, and what they grow to
-            assert torch.allclose(src.float(), want, atol=6 * 2.0 ** -8 * 4, rtol=2.0 ** -6)
-        for lin in lins:
-            lin.close()
+    code = kb.BF16 if dtype == torch.bfloat16 else kb.F32
+    ws = [torch.from_numpy(rng.standard_normal((width, width), dtype=np.float32) / width ** 0.5).to(cuda_device, dtype) for _ in range(6)]
+    lins = [kb.Linear(kb.make_desc(m, width, width, code, b_strides=(width, 1) if owned else (1, width))) for _ in ws]
+    for lin, w in zip(lins, ws):
+        lin.prepack(w, stream=stream)
+    x = torch.from_numpy(rng.standard_normal((m, width), dtype=np.float32)).to(cuda_device, dtype)
+    want = x.double()
+    for w in ws:
+        want = (want @ (w.double() if owned else w.double().T)).to(dtype).double()
+    # six roundings to 8 significant bits, each at most 2^-8 of a value of order one, and what they grow to; fp32: sums of up to
+    # 1032 products whose errors of 2^-22 (three TF32 products) add as a random walk, in six layers
+    atol, rtol = (6 * 2.0 ** -8 * 4, 2.0 ** -6) if dtype == torch.bfloat16 else (6 * 2.0 ** -22 * 1032 ** 0.5 * 4, 2.0 ** -16)
+    for _ in range(20):
+        bufs = [torch.full((m, width), float("nan"), device=cuda_device, dtype=dtype) for _ in ws]
+        src = x
+        for lin, w, dst in zip(lins, ws, bufs):
+            lin.run(src, w, dst, stream=stream)
+            src = dst
+        assert torch.allclose(src.double(), want, atol=atol, rtol=rtol)
+    said = capfd.readouterr().err
+    assert plan is None or plan in said
+    for lin in lins:
+        lin.close()
 
 
 @pytest.mark.parametrize("m", [40, 300])
