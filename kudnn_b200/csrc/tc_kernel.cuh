@@ -1143,7 +1143,7 @@ __device__ __forceinline__ void store_piece(char *p, int dt, int valid, const fl
 
 // Any element types; rows of 16-byte vectors, of which the last may be cut short by n (kAligned); both outputs, mirrors, alpha
 // and beta as they come.
-template <int kAct, int kDt>
+template <int kAct, int kDt, bool kCut>
 __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTensors &t, const float *part, int bn, int splits,
                                                 int row0, int rows, int tm, int tn, int n, int tid)
 {
@@ -1158,7 +1158,7 @@ __device__ __forceinline__ void finish_rows_vec(const EpiParams &e, const EpiTen
     }
     const int ct = kDt > 0 ? kDt : e.c_dtype, bt = kDt > 0 ? kDt : e.bias_dtype;
     const int rt = kDt > 0 ? kDt : e.res_dtype, ot = kDt > 0 ? kDt : e.out_dtype;
-    const int valid = n - ni < 8 ? static_cast<int>(n - ni) : 8;
+    const int valid = kCut && n - ni < 8 ? n - ni : 8;  // known to be 8 without the cut, so that the loads of a row go out together
     const long long m0 = static_cast<long long>(tm) * kBM + row0 + r;
     // byte addresses of this thread's piece of the row, and their advance per pass
     char *c = t.c == nullptr ? nullptr : static_cast<char *>(t.c) + (m0 * e.c_sm + ni) * dtype_size(ct);
@@ -1449,8 +1449,10 @@ __device__ __forceinline__ void finish_rows(const EpiParams &e, const EpiTensors
             return;
         }
     }
-    if (kind == TcRows::kVectors || kind == TcRows::kAligned) {
-        finish_rows_vec<kAct, kDt>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
+    if (kind == TcRows::kVectors) {
+        finish_rows_vec<kAct, kDt, false>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
+    } else if (kind == TcRows::kAligned) {
+        finish_rows_vec<kAct, kDt, true>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
     } else {
         finish_rows_any<kAct, kDt>(e, t, part, bn, splits, row0, rows, tm, tn, n, tid);
     }
