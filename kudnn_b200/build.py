@@ -28,7 +28,7 @@ NVCC_FLAGS = [
 ]
 
 CUDA_SOURCES = ["linear_api.cu", "simt_gemm.cu", "gemv.cu", "tc_gemm.cu", "tc_inst_f32.cu", "tc_inst_f16.cu", "tc_inst_bf16.cu",
-                "tc_inst_s8.cu", "pack.cu", "static_scratch.cu", "peer.cu", "eltwise.cu", "eltwise_api.cu"]
+                "tc_inst_s8.cu", "tc_wide_f16.cu", "tc_wide_bf16.cu", "pack.cu", "static_scratch.cu", "peer.cu", "eltwise.cu", "eltwise_api.cu"]
 
 
 def _nvcc():
@@ -73,8 +73,9 @@ def build_cuda(verbose=False, force=False, ptxas_info=False):
         s = os.path.join(_CSRC, src)
         o = os.path.join(_BUILD, src.replace(".cu", ".o"))
         objs.append(o)
-        # the tensor-core kernel's own headers concern its own translation units only
-        deps = [h for h in headers if src.startswith("tc_") or not os.path.basename(h).startswith("tc_")]
+        # the tensor-core kernels' own headers concern their own translation units only
+        unused = "tc_wide" if src.startswith("tc_inst_") else "tc_inst" if src.startswith("tc_") else "tc_"
+        deps = [h for h in headers if not os.path.basename(h).startswith(unused)]
         if force or not _newer(o, [s] + deps):
             cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if ptxas_info else []) + ["-c", s, "-o", o]
             jobs.append(cmd)

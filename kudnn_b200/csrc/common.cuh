@@ -151,16 +151,35 @@ __device__ __forceinline__ void store_exact_mirrored(void *base, int dtype, long
     }
 }
 
-// 1 / (1 + exp(t)); the reference clamps the exponent argument to [-87, 87]
-// (src/dnn/src/kernels/vml/vml_sve_la_sigmoid.h:39-48).
-template <bool kPrecise>
-__device__ __forceinline__ float sigmoid_neg(float t)
+// 2^t and 1 / v as the hardware gives them (about 2 and 1 units in the last place), denormals as zero
+__device__ __forceinline__ float ex2_approx(float t)
 {
-    // No explicit clamp is needed: beyond +87 the exponential overflows to +inf and the quotient is 0, beyond -87 it
-    // underflows and the quotient is 1, which are the reference's clamped values (a denormal instead of 0 in the
-    // sliver 87 < t < 88.7).  Branch-free, so eight of these interleave in the epilogues.
-    return kPrecise ? (1.0f / (1.0f + expf(t))) : __fdividef(1.0f, 1.0f + __expf(t));
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
+    return r;
 }
+__device__ __forceinline__ float rcp_approx(float v)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// 1 / (1 + 2^t)
+__device__ __forceinline__ float sigmoid_neg2(float t)
+{
+    // Branch-free and without a clamp: beyond t = 126 the quotient is 0, far below it 1, which are the values of the
+    // reference's clamp of the exponent (src/dnn/src/kernels/vml/vml_sve_la_sigmoid.h:39-48).  Denormals as zero change nothing
+    // here: a power that small vanishes beside the 1.
+    return rcp_approx(1.0f + ex2_approx(t));
+}
+// 1 / (1 + exp(t)), libm grade
+__device__ __forceinline__ float sigmoid_neg_precise(float t)
+{
+    return 1.0f / (1.0f + expf(t));
+}
+
+constexpr float kLog2E = 1.4426950408889634f;
 
 // kPrecise selects libm-grade exp/erf (fp32 outputs); otherwise the fast hardware approximations, whose error
 // (about 1e-6 relative) is far below one unit of a 16-bit result.
@@ -171,19 +190,16 @@ __device__ __forceinline__ float activation(float x, int act, float alpha)
         case KUDNN_B200_ACT_RELU:
             return (x <= 0.0f) ? x * alpha : x;
         case KUDNN_B200_ACT_SWISH:
-            return x * sigmoid_neg<kPrecise>(-(x * alpha));
+            return x * (kPrecise ? sigmoid_neg_precise(-(x * alpha)) : sigmoid_neg2(x * (-alpha * kLog2E)));
         case KUDNN_B200_ACT_SIGMOID:
-            return sigmoid_neg<kPrecise>(-x);
+            return kPrecise ? sigmoid_neg_precise(-x) : sigmoid_neg2(x * -kLog2E);
         case KUDNN_B200_ACT_TANH:
             return tanhf(x);
         case KUDNN_B200_ACT_GELU_TANH: {
-            // src/dnn/src/kernels/vml/gelu_tanh/vml_sve_la_gelu_tanh.h:22-39, tanh as vml_sve_la_tanh.h:116-142:
-            // y (1 - y^2 / 3) below 0.05, 1 - 2 / (1 + exp(2y)) otherwise; both evaluated, one selected
             const float y = (1.0f + x * x * 0.044715f) * x * 0.7978845608f;
             const float small = y * (1.0f - y * y * (1.0f / 3.0f));
             const float yc = fminf(y, 40.0f);  // exp(2 * 40) is finite; tanh is 1 to fp32 precision long before
-            const float e = kPrecise ? expf(yc + yc) : __expf(yc + yc);
-            const float big = kPrecise ? (1.0f - 2.0f / (1.0f + e)) : (1.0f - __fdividef(2.0f, 1.0f + e));
+            const float big = kPrecise ? 1.0f - 2.0f / (1.0f + expf(yc + yc)) : 1.0f - 2.0f * sigmoid_neg2(yc * (2.0f * kLog2E));
             const float th = (fabsf(y) < 0.05f) ? small : big;
             return (1.0f + th) * 0.5f * x;
         }

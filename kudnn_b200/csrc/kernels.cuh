@@ -84,8 +84,11 @@ struct TcPlan {
     int via_smem;    // 1: one work item per CTA, the tile is finished from shared memory
     int pair;      // 1: clusters of two CTAs share 256 x block_n tiles (cta_group::2)
     int narrow_from;  // pair mode: tiles from this index on are processed as two pieces of half the width
+    int wide;        // 1: CTA pairs on 256 x 512 tiles (tc_wide.cuh)
+    int wide_whole, wide_half, wide_items;  // its work items: whole tiles, halves, and all including the quarters
     unsigned char tmap_a[128] __attribute__((aligned(64)));
     unsigned char tmap_b[128] __attribute__((aligned(64)));
+    unsigned char tmap_b64[128] __attribute__((aligned(64)));  // wide: 64 rows of the weights, for quarters
 };
 bool tc_available();
 const char *tc_unavailable_reason();
@@ -94,8 +97,10 @@ const char *tc_unavailable_reason();
 cudaError_t tc_encode_kmajor(void *map128, const void *base, int kind, long long rows, long long k_total, long long ld_elems,
                              int box_rows);
 // with_staging: the launch writes output mirrors and needs the epilogue's row staging in shared memory
+// wide_ok: the kernel of 256 x 512 tiles takes this epilogue (tc_wide_takes)
 cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm_count, bool with_staging, TcRows rows,
-                         TcPlan *plan);
+                         bool wide_ok, TcPlan *plan);
+bool tc_wide_takes(const TcOperands &ops, const EpiParams &epi, TcRows rows);
 // wait_limit_cycles: SM cycles after which a device-side wait gives up (0 = the default of about two seconds);
 // skip_kblock: test hook for the timeout path, -1 = off (see TcParams::skip_kb).
 // bp: batch strides of the epilogue tensors (ignored unless ops.batch > 1)

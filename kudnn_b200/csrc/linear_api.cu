@@ -196,6 +196,7 @@ struct kudnn_b200_linear_s {
     long long plan_m = 0;
     bool plan_staging = false;
     kb::TcRows plan_rows = kb::TcRows::kOther;
+    bool plan_wide_ok = false;
     bool plan_valid = false;
 
     // kudnn_b200_linear_run_sharded: one child primitive per shard, each on its own device with its own copy (or
@@ -679,7 +680,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.lda = k_pad;
             }
             if (!(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m && !h->plan_staging)) {
-                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, false, kb::TcRows::kOther, &h->tc_plan);
+                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, false, kb::TcRows::kOther, false, &h->tc_plan);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "tensor map encoding");
                 }
@@ -1003,9 +1004,10 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             }
             const bool staging = pr.epi.n_mirrors > 0;
             const kb::TcRows rows = epilogue_rows(pr);
+            const bool wide_ok = kb::tc_wide_takes(ops, pr.epi, rows);
             if (nb > 1 || !(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m &&
-                            h->plan_staging == staging && h->plan_rows == rows)) {
-                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, staging, rows, &h->tc_plan);
+                            h->plan_staging == staging && h->plan_rows == rows && h->plan_wide_ok == wide_ok)) {
+                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, staging, rows, wide_ok, &h->tc_plan);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "tensor map encoding");
                 }
@@ -1014,13 +1016,14 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 h->plan_m = d.m;
                 h->plan_staging = staging;
                 h->plan_rows = rows;
+                h->plan_wide_ok = wide_ok;
                 h->plan_valid = nb == 1;
                 if (const char *dbg = std::getenv("KUDNN_B200_DEBUG")) {
                     if (*dbg != '\0' && *dbg != '0') {
                         std::fprintf(stderr, "kudnn_b200: tensor-core plan batch=%lld m=%lld n=%lld k=%lld: tile %s x %d, %d stages, "
                                              "grid %d, k splits %d, narrow tail from tile %d, %zu bytes of shared memory\n",
                                      nb, static_cast<long long>(d.m), static_cast<long long>(d.n), static_cast<long long>(d.k),
-                                     h->tc_plan.pair ? "256 (CTA pair)" : "128", h->tc_plan.block_n, h->tc_plan.stages,
+                                     h->tc_plan.pair ? "256 (CTA pair)" : "128", h->tc_plan.wide ? 512 : h->tc_plan.block_n, h->tc_plan.stages,
                                      h->tc_plan.grid, h->tc_plan.splits, h->tc_plan.pair ? h->tc_plan.narrow_from : -1, h->tc_plan.smem_bytes);
                     }
                 }

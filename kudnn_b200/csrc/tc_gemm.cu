@@ -1,5 +1,5 @@
 // Host side of the tensor-core Linear kernel (tc_kernel.cuh): tensor maps, launch plans, launch parameters.
-#include "tc_kernel.cuh"
+#include "tc_wide.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -134,7 +134,7 @@ int pair_clusters_of(int kind, bool with_staging, size_t smem)
 
 // Estimated SM cycles of a launch of single CTAs.  A k-block of a tile costs its MMAs (2 cycles per column whatever the
 // operand type) or its operand bytes (about 60 per cycle and SM), whichever is more.
-double single_cta_cycles(long long tiles, int splits, long long kb, int bn, int a_rows, bool via_smem, int sm_count)
+double single_cta_cycles(long long tiles, int splits, long long kb, int bn, int a_rows, bool via_smem, int sm_count, double per_value = 0.35)
 {
     const double per_kb = std::max(2.0 * bn, 2.1 * (a_rows + bn));
     const double area = static_cast<double>(a_rows) * bn;
@@ -145,15 +145,68 @@ double single_cta_cycles(long long tiles, int splits, long long kb, int bn, int 
         const long long waves = (tiles * splits + sm_count - 1) / sm_count;
         return waves * (2500.0 + kb * per_kb + finish);
     }
-    const double epilogue = 1000.0 + 0.35 * area;
+    const double epilogue = 1000.0 + per_value * area;
     const long long waves = (tiles + sm_count - 1) / sm_count;
     return 2500.0 + waves * std::max(kb * per_kb, epilogue) + epilogue;
 }
 
+// Estimated SM cycles of the kernel of 256 x 512 tiles on `pairs` CTA pairs, and how its work is cut: the whole tiles of the last
+// wave, which would keep only some of the pairs busy, become halves, and the halves of a last wave quarters.
+double wide_cycles(long long m, long long n, long long kb, int pairs, TcPlan *plan)
+{
+    // A k-block costs 1024 cycles of MMAs in a whole tile (measured 1.85 times the 640 of a pair's 256 x 256 tile in
+    // tc_kernel.cuh, in launches that fill the GPU), and in a half or a quarter what six stages in flight bring in; where K is
+    // short the epilogue is the longer part.
+    const double whole_cost = std::max(kb * 1200.0, 16000.0), half_cost = std::max(kb * 740.0, 9000.0);
+    const double quarter_cost = std::max(kb * 670.0, 6000.0);
+    const long long tiles_m = (m + 255) / 256, columns = (n + 255) / 256;
+    const long long tiles = tiles_m * (columns / 2), odd = tiles_m * (columns % 2);
+    const int forced = env_choice("KUDNN_B200_TC_WIDE");
+    double best = 1e300;
+    for (const long long whole : {tiles, tiles / pairs * pairs, 0ll}) {
+        const long long halves = 2 * (tiles - whole) + odd;
+        for (const long long cut : {0ll, (whole + halves) % pairs, halves}) {
+            if (cut > halves || (forced >= 1 && forced <= 3 && (whole != (forced == 1 ? tiles : 0) || cut != (forced == 3 ? halves : 0)))) {
+                continue;
+            }
+            // item i falls to pair i modulo their number: pair j has X / pairs of the first X, and one more if j < X % pairs, so that
+            // only these pairs can be the busiest
+            const long long ends[3] = {whole, whole + halves - cut, whole + halves + cut};
+            double longest = 0.0;
+            for (const long long pair : {0ll, ends[0] % pairs, ends[1] % pairs, ends[2] % pairs}) {
+                long long count[3];
+                for (int i = 0; i < 3; ++i) {
+                    count[i] = ends[i] / pairs + (pair < ends[i] % pairs ? 1 : 0);
+                }
+                longest = std::max(longest, whole_cost * count[0] + half_cost * (count[1] - count[0]) + quarter_cost * (count[2] - count[1]));
+            }
+            if (longest < best) {
+                best = longest;
+                plan->wide_whole = static_cast<int>(whole);
+                plan->wide_half = static_cast<int>(halves - cut);
+                plan->wide_items = static_cast<int>(whole + halves + cut);
+            }
+        }
+    }
+    return 20000.0 + best;  // start, and the last epilogue
+}
+
 }  // namespace
 
+bool tc_wide_takes(const TcOperands &ops, const EpiParams &epi, TcRows rows)
+{
+    const int kind = ops.kind;
+    const bool second = epi.res_op != KUDNN_B200_RES_NONE;
+    return (kind == KUDNN_B200_F16 || kind == KUDNN_B200_BF16) && ops.batch == 1 && rows == TcRows::kVectors && epi.n_mirrors == 0 &&
+           epi.beta == 0.0f && (epi.c == nullptr) == second && epi.c_dtype == kind &&
+           (epi.has_bias == 0 || (epi.bias_dtype == kind && epi.bias_sm == 0)) &&
+           (!second || (epi.res_dtype == kind && epi.out_dtype == kind)) &&
+           (epi.act == KUDNN_B200_ACT_NONE || epi.act == KUDNN_B200_ACT_RELU || epi.act == KUDNN_B200_ACT_SWISH ||
+            epi.act == KUDNN_B200_ACT_GELU_TANH);
+}
+
 cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm_count, bool with_staging, TcRows rows,
-                         TcPlan *plan)
+                         bool wide_ok, TcPlan *plan)
 {
     static_assert(sizeof(CUtensorMap) <= 128, "tensor map storage too small");
     if (!tc_available()) {
@@ -230,6 +283,10 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     const double per_value = ints || rows == TcRows::kVectors || rows == TcRows::kAligned ? 0.35 : rows == TcRows::kContiguous ? 4.3 : 2.5;
     const int pair_stages = with_staging ? 5 : 6;
     plan->narrow_from = 0;
+    // What the shape chosen so far is held against the kernel of 512-column tiles with: the same estimate, but with what a value
+    // of its epilogue takes where K is too short to cover it (2048 rows against 1024, n = 9216, k = 256: 10 to 12 us per tile).
+    constexpr double kNarrowPerValue = 0.55;
+    double narrow_cycles = via_smem ? best : single_cta_cycles(ops.batch * tiles_m * ((n + bn - 1) / bn), 1, num_kb, bn, a_rows_single, false, sm_count, kNarrowPerValue);
     if (pair) {
         const long long pair_tiles = ((m + 2 * kBM - 1) / (2 * kBM)) * ((n + 255) / 256);
         const long long guess = sm_count / 2;
@@ -238,6 +295,9 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
         const double epilogue = 1000.0 + per_value * kBM * 256;
         const double cycles = 4000.0 + waves * std::max(num_kb * 640.0, epilogue) + epilogue;
         pair = cycles < best || env_choice("KUDNN_B200_TC_PAIR") > 0;
+        if (pair) {
+            narrow_cycles = 4000.0 + waves * std::max(num_kb * 640.0, kNarrowPerValue * kBM * 256) + kNarrowPerValue * kBM * 256;
+        }
         int clusters = 0;
         if (pair) {
             clusters = pair_clusters_of(ops.kind, with_staging, static_cast<size_t>(pair_stages) * (kABytes + 128 * kStageRowBytes) + 1024 +
@@ -254,6 +314,20 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
             const long long left = pair_tiles % clusters;
             const bool narrow = pair_tiles > clusters && left > 0 && 2 * left <= clusters;
             plan->narrow_from = static_cast<int>(narrow ? pair_tiles - left : pair_tiles);
+        }
+    }
+    plan->wide = 0;
+    const int forced_wide = env_choice("KUDNN_B200_TC_WIDE");
+    if (wide_ok && m > kBM && forced_splits <= 1 && forced_wide != 0 && (env_choice("KUDNN_B200_TC_PAIR") < 0 || forced_wide > 0) &&
+        m < (1ll << 31) - 512 && n < (1ll << 31) - 512 && ((m + 255) / 256) * ((n + 127) / 128) < (1ll << 30)) {
+        const int clusters = pair_clusters_of(ops.kind, with_staging, kWideSmem);
+        if (clusters > 0 && (wide_cycles(m, n, num_kb, clusters, plan) < narrow_cycles || forced_wide > 0)) {
+            plan->wide = 1;
+            pair = true;
+            bn = 256;
+            splits = 1;
+            via_smem = false;
+            plan->grid = 2 * std::min(plan->wide_items, clusters);
         }
     }
     plan->pair = pair ? 1 : 0;
@@ -284,7 +358,7 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     }
     ring = (ring + 1023) / 1024 * 1024;
     plan->ring_bytes = static_cast<int>(ring);
-    plan->smem_bytes = static_cast<size_t>(ring + fixed);
+    plan->smem_bytes = plan->wide ? kWideSmem : static_cast<size_t>(ring + fixed);
     if (plan->smem_bytes > static_cast<size_t>(kSmemLimit)) {
         return cudaErrorInvalidValue;
     }
@@ -299,13 +373,69 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     }
     std::memcpy(plan->tmap_a, &ta, sizeof(ta));
     std::memcpy(plan->tmap_b, &tb, sizeof(tb));
-    return cudaSuccess;
+    if (plan->wide) {
+        e = encode_kmajor(&tb, ops.b, ops.kind, n, ops.k_total, ops.ldb, 64, ops.batch, ops.b_bstride);
+        std::memcpy(plan->tmap_b64, &tb, sizeof(tb));
+    }
+    return e;
 }
+
+namespace {
+
+// The A rows of one raster group are re-read for every tile column and should stay in L2 next to the
+// streaming weights: at most about 64 MB of them (16 tile rows of 256 x 8192 bf16).  Measured on the 32768-row
+// layer, ms per call for 8 / 12 / 16 tile rows per group: 13.05 / 12.84 / 12.72; DRAM traffic is the same
+// within 3 % (the wave's working set exceeds what L2 retains either way).
+int raster_group(const TcOperands &ops, int tile_rows)
+{
+    const long long tile_bytes = static_cast<long long>(tile_rows) * ops.k_total * dtype_size(ops.kind);
+    const long long gm = (64ll << 20) / (tile_bytes > 0 ? tile_bytes : 1);
+    return static_cast<int>(gm < 2 ? 2 : (gm > kMaxGroupM ? kMaxGroupM : gm));
+}
+
+cudaError_t launch_wide(const TcOperands &ops, const TcPlan &plan, const EpiParams &epi, long long m, long long n,
+                        DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles)
+{
+    if (!tc_wide_takes(ops, epi, plan.rows)) {
+        return cudaErrorInvalidValue;  // the plan was made for another epilogue
+    }
+    WideParams p;
+    p.epi = epi;
+    p.m = static_cast<int>(m);
+    p.n = static_cast<int>(n);
+    const int elems_per_row = kStageRowBytes / dtype_size(ops.kind);
+    p.num_kb = static_cast<int>((ops.k_total + elems_per_row - 1) / elems_per_row);
+    p.tiles_m = static_cast<int>((m + 255) / 256);
+    p.tiles_w = static_cast<int>((n + 255) / 256 / 2);
+    p.group_m = raster_group(ops, 2 * kBM);
+    p.n_whole = plan.wide_whole;
+    p.n_half = plan.wide_half;
+    p.num_items = plan.wide_items;
+    p.idesc = make_idesc(ops.kind, 256, 2 * kBM);
+    p.idesc_quarter = make_idesc(ops.kind, 128, 2 * kBM);
+    p.b_stable = ops.b_stable ? 1 : 0;
+    p.status = status;
+    p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimitCycles;
+    // the output, written in boxes of 32 rows x 128 bytes
+    const bool second = epi.res_op != KUDNN_B200_RES_NONE;
+    CUtensorMap out;
+    const cudaError_t e = encode_kmajor(&out, second ? epi.out : epi.c, ops.kind, m, n, second ? epi.out_sm : epi.c_sm, 32);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    return ops.kind == KUDNN_B200_F16 ? launch_wide_kind<KUDNN_B200_F16>(plan, &out, p, stream)
+                                      : launch_wide_kind<KUDNN_B200_BF16>(plan, &out, p, stream);
+}
+
+}  // namespace
 
 cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams &epi, long long m, long long n,
                       DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles, int skip_kblock,
                       const BatchParams *bp)
 {
+    if (plan.wide) {
+        return launch_wide(ops, plan, epi, m, n, status, stream, wait_limit_cycles);
+    }
     TcParams p;
     p.epi = epi;
     p.batch = static_cast<int>(ops.batch);
@@ -351,16 +481,7 @@ cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams
     p.ring_bytes = plan.ring_bytes;
     p.via_smem = plan.via_smem;
     p.rows = plan.rows;
-    {
-        // The A rows of one raster group are re-read for every tile column and should stay in L2 next to the
-        // streaming weights: at most about 64 MB of them (16 tile rows of 256 x 8192 bf16).  Measured on the 32768-row
-        // layer, ms per call for 8 / 12 / 16 tile rows per group: 13.05 / 12.84 / 12.72; DRAM traffic is the same
-        // within 3 % (the wave's working set exceeds what L2 retains either way).
-        const long long tile_bytes = static_cast<long long>(tile_rows) * ops.k_total * dtype_size(ops.kind);
-        long long gm = (64ll << 20) / (tile_bytes > 0 ? tile_bytes : 1);
-        gm = gm < 2 ? 2 : (gm > kMaxGroupM ? kMaxGroupM : gm);
-        p.group_m = static_cast<int>(gm);
-    }
+    p.group_m = raster_group(ops, tile_rows);
     p.num_items = plan.pair ? plan.narrow_from + 2 * (p.num_tiles - plan.narrow_from)
                             : p.num_tiles * plan.splits * static_cast<int>(ops.batch);
     p.narrow_from = plan.pair ? plan.narrow_from : p.num_tiles;

@@ -459,32 +459,34 @@ __device__ __forceinline__ void unpack8(const uint4 &p, float (&v)[8])
     }
 }
 
-template <int kAct, int kDt>
-__device__ __forceinline__ uint4 chain8_packed(const EpiParams &e, bool has_bias, const float (&side)[8], float (&v)[8])
+// up to the activation: bias and rounding
+template <int kDt>
+__device__ __forceinline__ uint4 round8_packed(const EpiParams &e, bool has_bias, const float (&side)[8], float (&v)[8])
 {
-    uint4 w;
     if (kDt == KUDNN_B200_F16 && e.half_chain != 0) {
-        w = pack8_rne<kDt>(v);
-        if (has_bias) {
-            unpack8<kDt>(w, v);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                v[j] += side[j];
-            }
-            w = pack8_rne<kDt>(v);
+        const uint4 w = pack8_rne<kDt>(v);
+        if (!has_bias) {
+            return w;
         }
-    } else {
-        if (has_bias) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                v[j] += side[j];
-            }
-        }
-        w = pack8_rne<kDt>(v);
+        unpack8<kDt>(w, v);
     }
+    if (has_bias) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] += side[j];
+        }
+    }
+    return pack8_rne<kDt>(v);
+}
+
+// the activation on rounded values
+template <int kAct, int kDt>
+__device__ __forceinline__ uint4 act8_packed(const EpiParams &e, const uint4 &w)
+{
     if (kAct == KUDNN_B200_ACT_NONE) {
         return w;
     }
+    float v[8];
     unpack8<kDt>(w, v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -506,18 +508,36 @@ __device__ __forceinline__ uint4 chain8_packed(const EpiParams &e, bool has_bias
                       __byte_perm(__float_as_uint(v[6]), __float_as_uint(v[7]), 0x7632));
 }
 
+template <int kAct, int kDt>
+__device__ __forceinline__ uint4 chain8_packed(const EpiParams &e, bool has_bias, const float (&side)[8], float (&v)[8])
+{
+    return act8_packed<kAct, kDt>(e, round8_packed<kDt>(e, has_bias, side, v));
+}
+
+// The sum (product) of two 16-bit values rounded to 16 bits, two at a time.  Rounding the fp32 sum (product) would give the same:
+// fp32 has more than twice their bits and two.
+template <int kDt>
+__device__ __forceinline__ unsigned add2_packed(unsigned a, unsigned b)
+{
+    unsigned r;
+    if (kDt == KUDNN_B200_BF16) {
+        asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    } else {
+        asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    }
+    return r;
+}
+
 template <int kDt>
 __device__ __forceinline__ uint4 combine8_packed(const EpiParams &e, const uint4 &c, const uint4 &res)
 {
+    if (e.res_op == KUDNN_B200_RES_IDENTICAL) {
+        return make_uint4(add2_packed<kDt>(c.x, res.x), add2_packed<kDt>(c.y, res.y), add2_packed<kDt>(c.z, res.z), add2_packed<kDt>(c.w, res.w));
+    }
     float v[8], side[8];
     unpack8<kDt>(c, v);
     unpack8<kDt>(res, side);
-    if (e.res_op == KUDNN_B200_RES_IDENTICAL) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            v[j] += side[j];
-        }
-    } else if (e.res_op == KUDNN_B200_RES_EXT) {
+    if (e.res_op == KUDNN_B200_RES_EXT) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             v[j] = fmaf(side[j], e.gamma, v[j]);

@@ -213,3 +213,55 @@ def test_rows_of_vectors_with_beta_and_a_cut_last_column(cuda_device, monkeypatc
     if both:
         assert torch.allclose(out[:, :n].double(), want + res[:, :n].double(), rtol=3 * eps, atol=8 * eps)
         assert torch.equal(out[:, n:], out0[:, n:])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cut,m,n,k", [("1", 129, 512, 64), ("1", 300, 1288, 200), ("1", 1027, 776, 1096), ("2", 257, 520, 8), ("2", 513, 1032, 328),
+                                       ("3", 300, 264, 456), ("3", 2000, 1160, 136), (None, 2500, 9992, 264)])
+@pytest.mark.parametrize("act,res_op,bias,alpha", [(kb.ACT_NONE, kb.RES_NONE, None, 1.0), (kb.ACT_RELU, kb.RES_IDENTICAL, "row", 1.0),
+                                                   (kb.ACT_SWISH, kb.RES_NONE, "row", 1.0), (kb.ACT_GELU_TANH, kb.RES_EXT, "one", 1.0),
+                                                   (kb.ACT_NONE, kb.RES_ELTWISE_MUL, "row", 0.75), (kb.ACT_SWISH, kb.RES_IDENTICAL, None, 0.75)])
+def test_wide_tiles_equal_the_narrow_ones(cuda_device, monkeypatch, capfd, dtype, cut, m, n, k, act, res_op, bias, alpha):
+    """Tiles of 512 columns, whole (1), in halves (2), in quarters (3) and as planned, against the tiles of 256: the same products
+    in the same order.  Rows and columns past the tiles' edges, a tile whose second half is empty, outputs and residuals with a
+    pitch, one call after the other on the same stream."""
+    stream = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(31)
+
+    def draw(*shape, std=1.0):
+        return (torch.randn(shape, generator=gen, device=cuda_device) * std).to(dtype)
+
+    code = kb.BF16 if dtype == torch.bfloat16 else kb.F16
+    pitch, res_pitch = n + 8, n + 24
+    second = res_op != kb.RES_NONE
+    owned = k % 16 == 8  # weights stored [k, n]: packed into a copy whose first rows are loaded early
+    xs, w, res = [draw(m, k), draw(m, k)], draw(*((k, n) if owned else (n, k)), std=0.05), draw(m, res_pitch)
+    side = draw(n) if bias == "row" else draw(1) if bias == "one" else None
+    desc = kb.make_desc(m, n, k, code, b_strides=(n, 1) if owned else None, has_bias=bias is not None,
+                        bias_strides=(0, 0) if bias == "one" else None, act=act, act_alpha=0.25,
+                        res_op=res_op, c_strides=(pitch, 1), res_strides=(res_pitch, 1), out_strides=(pitch, 1))
+    monkeypatch.setenv("KUDNN_B200_DEBUG", "1")
+    got = []
+    for wide in ("0", cut):
+        for name, value in (("KUDNN_B200_TC_WIDE", wide), ("KUDNN_B200_TC_PAIR", "1" if wide == "0" else None)):
+            monkeypatch.delenv(name, raising=False) if value is None else monkeypatch.setenv(name, value)
+        lin = kb.Linear(desc)
+        lin.force_kernel(kb.KERNEL_TC)
+        lin.prepack(w, stream=stream)
+        ys = [torch.full((m, pitch), 7.0, device=cuda_device, dtype=dtype) for _ in xs]
+        for x, y in zip(xs, ys):
+            lin.run(x, w, None if second else y, side, res if second else None, y if second else None, alpha=alpha, gamma=0.5, stream=stream)
+        lin.check(stream=stream)
+        said = capfd.readouterr().err
+        assert ("256 (CTA pair) x 512" in said) == (wide != "0")
+        got.append(ys)
+        lin.close()
+    for a, b in zip(*got):
+        assert bool((b[:, n:] == 7.0).all())
+        if alpha == 1.0:
+            assert torch.equal(a, b)
+        else:
+            # alpha * acc + bias is rounded once here and twice there: one unit of the 16-bit value, carried through the chain
+            eps = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
+            assert torch.allclose(a.float(), b.float(), rtol=2 * eps, atol=2 * eps)
