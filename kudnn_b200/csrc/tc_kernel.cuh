@@ -490,7 +490,7 @@ __device__ __forceinline__ uint4 act8_packed(const EpiParams &e, const uint4 &w)
     unpack8<kDt>(w, v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        v[j] = activation<false>(v[j], kAct, e.act_alpha);
+        v[j] = kAct == KUDNN_B200_ACT_GELU_TANH ? gelu_tanh_sigmoid(v[j]) : activation<false>(v[j], kAct, e.act_alpha);
     }
     if (kDt == KUDNN_B200_F16) {
         return pack8_rne<kDt>(v);
