@@ -104,9 +104,10 @@ bool tc_wide_takes(const TcOperands &ops, const EpiParams &epi, TcRows rows);
 // wait_limit_cycles: SM cycles after which a device-side wait gives up (0 = the default of about two seconds);
 // skip_kblock: test hook for the timeout path, -1 = off (see TcParams::skip_kb).
 // bp: batch strides of the epilogue tensors (ignored unless ops.batch > 1)
+// run_if: the kernel leaves at once when *run_if is 0
 cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams &epi, long long m, long long n,
                       DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles = 0, int skip_kblock = -1,
-                      const BatchParams *bp = nullptr);
+                      const BatchParams *bp = nullptr, const int *run_if = nullptr);
 
 // Batched packing: `count` matrices; entry `flat` of the source starts sb[0] * i0 + sb[1] * i1 + sb[2] * i2 elements
 // into the tensor, (i0, i1, i2) the decomposition of flat over the extents (.., n1, n2); entry `flat` of the packed
@@ -133,6 +134,25 @@ cudaError_t launch_pack_blocks(const void *src, long long rows, long long k, lon
 cudaError_t launch_split_tf32(const void *src, long long rows, long long k, long long s_row, long long s_k, float *dst,
                               long long ldd, long long k_pad, int is_weight, cudaStream_t stream,
                               const PackBatch *batch = nullptr);
+
+// The TF32 split of contiguous activation rows, by few CTAs and only if *run_if is not 0.
+cudaError_t launch_split_tf32_if(const int *run_if, const void *src, long long rows, long long k, long long s_row, float *dst, long long ldd,
+                                 long long k_pad, int sm_count, cudaStream_t stream);
+
+// fp32 operands as two planes of fp16 (tc_planes.cuh): rows of k_pad / 64 blocks of [64 hi | 64 lo], a scale per row, and a byte per
+// row that is set where the planes do not carry the row.
+struct PlanesOperand {
+    unsigned short *planes;
+    float *scale;
+    unsigned char *flags;
+};
+// contiguous rows of 16-byte aligned fp32, row pitch s_row elements; k_pad is a multiple of 64
+cudaError_t launch_split_half(const void *src, long long rows, long long k, long long s_row, const PlanesOperand &dst, long long k_pad,
+                              cudaStream_t stream);
+bool planes_take(const EpiParams &epi);
+// *fallback becomes 1 if any row of a is marked: nothing of c is written then.
+cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long long k_pad, const EpiParams &epi, long long m, long long n,
+                          int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles);
 
 // Stand-alone element-wise activation and RMS normalisation (eltwise.cu); device pointers.
 cudaError_t launch_activation(const void *src, int src_dtype, void *dst, int dst_dtype, long long count, int act, float alpha,

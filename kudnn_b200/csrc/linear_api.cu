@@ -133,9 +133,10 @@ struct StreamScratch {
     DeviceBuffer a;                   // packed activations
     DeviceBuffer b;                   // packed weights (when not pre-packed)
     DeviceBuffer q;                   // 8-bit weights widened to fp16 (when not pre-packed)
+    DeviceBuffer planes;              // fp32 activations as fp16 planes, with their scales and marks
     void release()
     {
-        for (DeviceBuffer *buf : {&partials, &counters, &a, &b, &q}) {
+        for (DeviceBuffer *buf : {&partials, &counters, &a, &b, &q, &planes}) {
             buf->release();
         }
     }
@@ -180,6 +181,7 @@ struct kudnn_b200_linear_s {
     unsigned long long scratch_uses = 0;
     DeviceBuffer b_packed;      // pre-packed weights
     DeviceBuffer b_blocked;     // decode-shaped handles: the weights once more in 8-row x 64-k blocks
+    DeviceBuffer b_planes;      // fp32: the weights once more as fp16 planes (tc_planes.cuh), for large products
     DeviceBuffer stage[6];      // host-pointer staging: a, b, c, bias, res, out
 
     // pre-pack state
@@ -189,6 +191,8 @@ struct kudnn_b200_linear_s {
     const void *packed_raw = nullptr;  // K-major copy in the original element type (what the other kernels read)
     long long packed_ld = 0, packed_ktotal = 0;
     long long blocked_kpad = 0;  // columns per row of b_blocked (k rounded up to 256); 0 = no blocked copy
+
+    long long planes_kpad = 0;   // columns per row of b_planes (k rounded up to 64); 0 = no planes
 
     // tensor-map cache of the last tensor-core launch
     kb::TcPlan tc_plan;
@@ -424,6 +428,41 @@ int pack_weights(Handle *h, const void *b_dev, DeviceBuffer *buf, bool with_raw,
         *raw = buf->ptr;
     }
     return KUDNN_B200_OK;
+}
+
+// Rows of fp16 planes in one buffer: the planes, a scale per row, a mark per row, and a word for the launches that depend on the marks.
+kb::PlanesOperand planes_in(void *base, long long rows, long long k_pad, int **word = nullptr)
+{
+    kb::PlanesOperand p;
+    unsigned char *at = static_cast<unsigned char *>(base);
+    p.planes = reinterpret_cast<unsigned short *>(at);
+    at += rows * 2 * k_pad * 2;
+    p.scale = reinterpret_cast<float *>(at);
+    at += rows * 4;
+    if (word != nullptr) {
+        *word = reinterpret_cast<int *>(at);
+    }
+    p.flags = at + 16;
+    return p;
+}
+
+size_t planes_bytes(long long rows, long long k_pad)
+{
+    return static_cast<size_t>(rows) * (2 * k_pad * 2 + 4 + 1) + 16;
+}
+
+// Whether an fp32 product is worth the planes: they take half of the time of the TF32 form and two more launches, 4 us.  Times of
+// both in us: 512 x 1152 x 1152 23.4 and 24.4, 676 x 1280 x 1152 33 and 31, 1024 x 1152 x 1152 31 and 26, 1195 x 2816 x 1472 66 and
+// 38, 4096 x 4608 x 2304 350 and 185, x 64 57 and 37.  With fewer than 20 tiles of 256 x 256 most pairs would be idle, where the TF32 form cuts K:
+// 741 x 1280 x 2816 48 and 51, 620 x 1280 x 4736 60 and 65.
+bool planes_worth(const kudnn_b200_linear_desc &d)
+{
+    const char *forced = std::getenv("KUDNN_B200_TC_PLANES");
+    if (forced != nullptr && *forced != '\0') {
+        return *forced != '0';
+    }
+    const long long tiles = ((d.m + 255) / 256) * ((d.n + 255) / 256);
+    return tiles >= 20 && d.k >= 64 && static_cast<double>(d.m) * d.n * d.k >= 1.0e9;
 }
 
 // A batched problem whose weights are shared by all batch entries and whose other tensors are laid out so that
@@ -974,12 +1013,40 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.k_total = f32 ? 3 * k_pad : d.k;
                 ops.b_bstride = shared ? 0 : per;
             }
+            // fp32, large and pre-packed: fp16 planes, unless a row asks for the TF32 planes, which the device decides
+            const int *run_if = nullptr;
+            if (f32 && use_packed && two_d && h->planes_kpad > 0 && kmajor_ready(args.a, d.a_dtype, d.a_sm, d.a_sk, d.m) && kb::planes_take(pr.epi)) {
+                const long long kp = h->planes_kpad, k32 = round_up(d.k, 32);
+                cudaError_t e = sc->planes.reserve(planes_bytes(d.m, kp));
+                if (e == cudaSuccess) e = sc->a.reserve(static_cast<size_t>(d.m) * 3 * k32 * 4);
+                if (e != cudaSuccess) {
+                    return fail_cuda(e, "packed activations");
+                }
+                int *word = nullptr;
+                const kb::PlanesOperand pa = planes_in(sc->planes.ptr, d.m, kp, &word), pb = planes_in(h->b_planes.ptr, d.n, kp);
+                e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
+                if (e == cudaSuccess) {
+                    e = kb::launch_planes(pa, pb, kp, pr.epi, d.m, d.n, word, static_cast<kb::DeviceStatus *>(h->status.ptr), h->sm_count, stream,
+                                          h->wait_limit);
+                }
+                if (e == cudaSuccess) {
+                    e = kb::launch_split_tf32_if(word, args.a, d.m, d.k, d.a_sm, static_cast<float *>(sc->a.ptr), 3 * k32, k32, h->sm_count, stream);
+                }
+                if (e != cudaSuccess) {
+                    return fail_cuda(e, "fp16 planes launch");
+                }
+                launches += 3;
+                run_if = word;
+            }
             // activations
             long long astride = 0;
             if (!f32 && kmajor_ready(args.a, d.a_dtype, d.a_sm, d.a_sk, d.m) && flat_stride(d.a_sb, &astride)) {
                 ops.a = args.a;
                 ops.lda = d.a_sm;
                 ops.a_bstride = astride;
+            } else if (run_if != nullptr) {
+                ops.a = sc->a.ptr;
+                ops.lda = 3 * round_up(d.k, 32);
             } else {
                 const bool shared = all_shared(d.a_sb);
                 const long long k_pad = round_up(d.k, f32 ? 32 : 8);
@@ -1030,7 +1097,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             }
             cudaError_t e = kb::launch_tc(ops, h->tc_plan, pr.epi, d.m, d.n,
                                           static_cast<kb::DeviceStatus *>(h->status.ptr), stream, h->wait_limit,
-                                          h->skip_kblock, &pr.batch);
+                                          h->skip_kblock, &pr.batch, run_if);
             if (e != cudaSuccess) {
                 return fail_cuda(e, "tensor-core kernel launch");
             }
@@ -1376,6 +1443,7 @@ int kudnn_b200_linear_destroy(kudnn_b200_linear_t h)
         }
         h->b_packed.release();
         h->b_blocked.release();
+        h->b_planes.release();
         for (auto &s : h->stage) {
             s.release();
         }
@@ -1466,6 +1534,7 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
         return KUDNN_B200_OK;
     }
     h->packed_int8 = false;
+    h->planes_kpad = 0;
     if (is_int8_dtype(d.b_dtype) && d.m <= 16 && d.k % 16 == 0) {
         // fp16 activations, 8-bit weights, decode shapes: the streaming kernels read the 8-bit values themselves.
         // K-major rows with a pitch of a multiple of 16 bytes: the caller's device buffer if it is so, else a copy.
@@ -1518,6 +1587,28 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
         h->packed_raw = raw;
         h->packed_ld = ld;
         h->packed_ktotal = kt;
+    }
+    // Large fp32 products get the weights as fp16 planes too, if the planes carry every row
+    if (d.b_dtype == KUDNN_B200_F32 && planes_worth(d)) {
+        const long long kp = round_up(d.k, 64);
+        e = h->b_planes.reserve(planes_bytes(d.n, kp));
+        if (e != cudaSuccess) {
+            return fail_cuda(e, "weight planes");
+        }
+        const kb::PlanesOperand pb = planes_in(h->b_planes.ptr, d.n, kp);
+        e = kb::launch_split_half(h->packed_raw, d.n, d.k, h->packed_ld, pb, kp, stream);
+        std::vector<unsigned char> marks(static_cast<size_t>(d.n));
+        if (e == cudaSuccess) e = cudaMemcpyAsync(marks.data(), pb.flags, marks.size(), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) {
+            return fail_cuda(e, "weight planes");
+        }
+        if (std::all_of(marks.begin(), marks.end(), [](unsigned char f) { return f == 0; })) {
+            h->planes_kpad = kp;
+        }
+    }
+    if (h->planes_kpad == 0) {
+        h->b_planes.release();
     }
     // Decode-shaped primitives (m <= 16, 16-bit types) stream the whole weight matrix on every call: they get a
     // second copy in blocks of 8 rows x 64 k, the unit their MMA kernels read, so that a warp's loads are one
@@ -1920,10 +2011,12 @@ int kudnn_b200_linear_unpack(kudnn_b200_linear_t h)
     h->packed_raw = nullptr;
     h->packed_ld = h->packed_ktotal = 0;
     h->blocked_kpad = 0;
+    h->planes_kpad = 0;
     h->plan_valid = false;
     if (h->device >= 0) {
         h->b_packed.release();
         h->b_blocked.release();
+        h->b_planes.release();
     }
     return KUDNN_B200_OK;
 }
@@ -1973,9 +2066,9 @@ int64_t kudnn_b200_linear_workspace_bytes(kudnn_b200_linear_t h)
     if (h == nullptr) {
         return 0;
     }
-    size_t bytes = h->b_packed.bytes + h->b_blocked.bytes;
+    size_t bytes = h->b_packed.bytes + h->b_blocked.bytes + h->b_planes.bytes;
     for (const auto &sc : h->scratch) {
-        bytes += sc->partials.bytes + sc->counters.bytes + sc->a.bytes + sc->b.bytes;
+        bytes += sc->partials.bytes + sc->counters.bytes + sc->a.bytes + sc->b.bytes + sc->planes.bytes;
     }
     return static_cast<int64_t>(bytes);
 }

@@ -196,6 +196,137 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *src_base, 
     *reinterpret_cast<float4 *>(dst + 2 * k_pad) = h;
 }
 
+// The same split of activation rows by CTAs that walk over the rows, and only if *run_if is not 0: the launch that otherwise leaves
+// at once has to be small.
+__global__ void __launch_bounds__(256) split_rows_if_kernel(const int *run_if, const float *src_base, long long rows, long long k, long long s_row,
+                                                            float *dst_base, long long ldd, long long k_pad)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    if (*run_if == 0) {
+        return;
+    }
+    for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+        const float *src = src_base + row * s_row;
+        float *dst = dst_base + row * ldd;
+        for (long long kk = threadIdx.x; kk < k_pad; kk += 256) {
+            const float v = kk < k ? src[kk] : 0.0f;
+            const float hi = to_tf32(v);
+            dst[kk] = to_tf32(v - hi);
+            dst[k_pad + kk] = hi;
+            dst[2 * k_pad + kk] = hi;
+        }
+    }
+}
+
+// fp32 rows -> two planes of fp16 (see tc_planes.cuh): a CTA per row, eight columns per thread and step.  Bound by memory: the row
+// is read once (rows of up to 8192 columns stay in registers between the search for the largest element and the conversion) and as
+// many bytes are written.
+constexpr int kSplitThreads = 128, kSplitHeld = 8;
+
+__global__ void __launch_bounds__(kSplitThreads) split_half_kernel(const float *src_base, long long k, long long s_row, unsigned short *planes,
+                                                                   float *scales, unsigned char *flags, long long k_pad)
+{
+    __shared__ unsigned most[kSplitThreads / 32], least[kSplitThreads / 32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long row = blockIdx.x;
+    const float *src = src_base + row * s_row;
+    const int pieces = static_cast<int>(k_pad / 8);
+    auto fetch = [&](int piece, float (&v)[8]) {
+        const long long kk = static_cast<long long>(piece) * 8;
+        if (piece < pieces && kk + 8 <= k) {
+            const float4 x = *reinterpret_cast<const float4 *>(src + kk), y = *reinterpret_cast<const float4 *>(src + kk + 4);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                v[i] = piece < pieces && kk + i < k ? src[kk + i] : 0.0f;
+            }
+        }
+    };
+    // the largest magnitude and the smallest that is not zero, as bit patterns
+    unsigned mx = 0u, mn = 0xffffffffu;
+    auto look = [&](const float (&v)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const unsigned u = __float_as_uint(v[i]) & 0x7fffffffu;
+            mx = mx > u ? mx : u;
+            mn = u != 0u && u < mn ? u : mn;
+        }
+    };
+    float held[kSplitHeld][8];
+    const bool holds = pieces <= kSplitThreads * kSplitHeld;
+    if (holds) {
+#pragma unroll
+        for (int j = 0; j < kSplitHeld; ++j) {
+            if (j * kSplitThreads < pieces) {
+                fetch(j * kSplitThreads + static_cast<int>(threadIdx.x), held[j]);
+                look(held[j]);
+            }
+        }
+    } else {
+        for (int piece = static_cast<int>(threadIdx.x); piece < pieces; piece += kSplitThreads) {
+            fetch(piece, held[0]);
+            look(held[0]);
+        }
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    if ((threadIdx.x & 31) == 0) {
+        most[threadIdx.x >> 5] = mx;
+        least[threadIdx.x >> 5] = mn;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kSplitThreads / 32; ++w) {
+        mx = most[w] > mx ? most[w] : mx;
+        mn = least[w] < mn ? least[w] : mn;
+    }
+    const int exponent = static_cast<int>(mx >> 23) - 127;
+    const bool in_range = mx == 0u || (exponent >= -100 && exponent < 64);
+    // 2^(14 - exponent) and its inverse
+    const float up = mx == 0u || !in_range ? 1.0f : __uint_as_float(static_cast<unsigned>(127 + 14 - exponent) << 23);
+    const float down = mx == 0u || !in_range ? 1.0f : __uint_as_float(static_cast<unsigned>(127 - 14 + exponent) << 23);
+    if (threadIdx.x == 0) {
+        scales[row] = down;
+        flags[row] = !in_range || (mn != 0xffffffffu && __uint_as_float(mn) * up < 0x1p-20f) ? 1 : 0;
+    }
+    unsigned short *dst = planes + row * 2 * k_pad;
+    auto put = [&](int piece, const float (&v)[8]) {
+        if (piece >= pieces) {
+            return;
+        }
+        unsigned hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float x = v[2 * i] * up, y = v[2 * i + 1] * up;
+            const __half2 h = __floats2half2_rn(x, y);
+            const float2 back = __half22float2(h);
+            const __half2 l = __floats2half2_rn((x - back.x) * 2048.0f, (y - back.y) * 2048.0f);
+            hi[i] = *reinterpret_cast<const unsigned *>(&h);
+            lo[i] = *reinterpret_cast<const unsigned *>(&l);
+        }
+        uint4 *at = reinterpret_cast<uint4 *>(dst + (piece >> 3) * 128 + (piece & 7) * 8);
+        at[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        at[8] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    };
+    if (holds) {
+#pragma unroll
+        for (int j = 0; j < kSplitHeld; ++j) {
+            if (j * kSplitThreads < pieces) {
+                put(j * kSplitThreads + static_cast<int>(threadIdx.x), held[j]);
+            }
+        }
+    } else {
+        for (int piece = static_cast<int>(threadIdx.x); piece < pieces; piece += kSplitThreads) {
+            fetch(piece, held[0]);
+            put(piece, held[0]);
+        }
+    }
+}
+
 // one thread per 16-byte chunk of the destination
 __global__ void __launch_bounds__(256) pack_blocks_kernel(const unsigned short *src, long long rows, long long k, long long ld,
                                                           uint4 *dst, long long nkb, long long total_chunks)
@@ -292,6 +423,21 @@ cudaError_t launch_split_tf32(const void *src, long long rows, long long k, long
     split_tf32_kernel<<<grid, 256, 0, stream>>>(static_cast<const float *>(src), rows, k, s_row, s_k, dst, ldd, k_pad,
                                                 is_weight, pb);
     return cudaGetLastError();
+}
+
+cudaError_t launch_split_tf32_if(const int *run_if, const void *src, long long rows, long long k, long long s_row, float *dst, long long ldd,
+                                 long long k_pad, int sm_count, cudaStream_t stream)
+{
+    const long long grid = rows < 4ll * sm_count ? rows : 4ll * sm_count;
+    return launch_chained(split_rows_if_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, stream, 1, run_if, static_cast<const float *>(src),
+                          rows, k, s_row, dst, ldd, k_pad);
+}
+
+cudaError_t launch_split_half(const void *src, long long rows, long long k, long long s_row, const PlanesOperand &dst, long long k_pad,
+                              cudaStream_t stream)
+{
+    return launch_chained(split_half_kernel, dim3(static_cast<unsigned>(rows)), dim3(kSplitThreads), 0, stream, 1, static_cast<const float *>(src), k,
+                          s_row, dst.planes, dst.scale, dst.flags, k_pad);
 }
 
 }  // namespace kb

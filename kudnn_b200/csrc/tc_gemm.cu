@@ -431,13 +431,14 @@ cudaError_t launch_wide(const TcOperands &ops, const TcPlan &plan, const EpiPara
 
 cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams &epi, long long m, long long n,
                       DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles, int skip_kblock,
-                      const BatchParams *bp)
+                      const BatchParams *bp, const int *run_if)
 {
     if (plan.wide) {
-        return launch_wide(ops, plan, epi, m, n, status, stream, wait_limit_cycles);
+        return run_if != nullptr ? cudaErrorInvalidValue : launch_wide(ops, plan, epi, m, n, status, stream, wait_limit_cycles);
     }
     TcParams p;
     p.epi = epi;
+    p.run_if = run_if;
     p.batch = static_cast<int>(ops.batch);
     p.a_bz = ops.a_bstride != 0 ? 1 : 0;
     p.b_bz = ops.b_bstride != 0 ? 1 : 0;

@@ -72,6 +72,7 @@ struct TcParams {
     int ring_bytes;  // bytes in front of the barriers: the stage ring, and room for one tile as fp32 if it is finished from there
     int b_stable;  // the weights were pre-packed: the first of them are loaded while the previous kernel still runs
     int via_smem;    // one work item per CTA, finished from shared memory (finish_rows)
+    const int *run_if;  // if not null: nothing is done when it points to 0
     TcRows rows;  // how a tile finished from shared memory meets the epilogue's tensors
     int group_m;  // tile rows per raster group: consecutive work items walk down group_m tile rows, then one tile right
     // CTA pairs: work items [0, narrow_from) are whole 256 x BN tiles; each later tile is two items of half the width,
@@ -1535,6 +1536,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
+    if (p.run_if != nullptr) {
+        pdl_wait();
+        if (*p.run_if == 0) {
+            return;  // every CTA reads the same
+        }
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_bar + s, 1);

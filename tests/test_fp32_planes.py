@@ -1,0 +1,97 @@
+"""fp32 products as planes of fp16: the error bound of the split over tile edges, and rows that the planes do not carry, which the
+device sends to the TF32 form, also in a captured graph."""
+import pytest
+import torch
+
+import kudnn_b200 as kb
+
+pytestmark = pytest.mark.gpu
+
+_ACTS = {kb.ACT_NONE: lambda v: v, kb.ACT_RELU: torch.relu, kb.ACT_SWISH: torch.nn.functional.silu,
+         kb.ACT_GELU_TANH: lambda v: torch.nn.functional.gelu(v, approximate="tanh")}
+
+
+def _layer(monkeypatch, planes, m, n, k, w, owned=False, **desc):
+    monkeypatch.setenv("KUDNN_B200_TC_PLANES", planes)
+    lin = kb.Linear(kb.make_desc(m, n, k, kb.F32, b_strides=(n, 1) if owned else None, **desc))
+    lin.force_kernel(kb.KERNEL_TC)
+    lin.prepack(w, stream=torch.cuda.current_stream().cuda_stream)
+    return lin
+
+
+def _draw(device, *shape):
+    gen = torch.Generator(device=device)
+    gen.manual_seed(sum(shape))
+    return torch.randn(shape, generator=gen, device=device)
+
+
+@pytest.mark.parametrize("m,n,k,owned", [(1, 4, 8, False), (255, 260, 64, True), (257, 128, 68, False), (300, 1032, 1100, True), (2600, 1028, 72, False),
+                                         (130, 300, 8200, False), (1024, 2500, 704, True)])
+@pytest.mark.parametrize("act,bias,alpha", [(kb.ACT_NONE, False, 1.0), (kb.ACT_RELU, True, 1.0), (kb.ACT_SWISH, True, 0.5), (kb.ACT_GELU_TANH, False, 1.0)])
+def test_error_of_the_planes(cuda_device, monkeypatch, m, n, k, owned, act, bias, alpha):
+    stream = torch.cuda.current_stream().cuda_stream
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, *((k, n) if owned else (n, k))) * 0.02
+    # rows of very different size, and one of zeros: each has its own scale
+    a *= torch.pow(2.0, torch.randint(-40, 20, (m, 1), device=cuda_device)).float()
+    a[m // 2] = 0.0
+    side = _draw(cuda_device, n) if bias else None
+    lin = _layer(monkeypatch, "1", m, n, k, w, owned, has_bias=bias, act=act, act_alpha=0.0 if act == kb.ACT_RELU else 1.0, c_strides=(n + 4, 1))
+    c = torch.full((m, n + 4), 7.0, device=cuda_device)
+    for _ in range(2):
+        lin.run(a, w, c, side, alpha=alpha, stream=stream)
+    lin.check(stream=stream)
+    assert lin.last_launches == 4
+    w64 = w.double() if owned else w.double().T
+    pre = alpha * (a.double() @ w64) + (side.double() if bias else 0.0)
+    want = _ACTS[act](pre)
+    # each operand is carried to 2^-22, the product of the low parts (2^-22) is left out, and k / 16 additions to an accumulator, three
+    # per step, each cut at 2^-23 of a partial sum; the activations' slope is at most 1.13
+    size = alpha * (a.double().abs() @ w64.abs()) + (side.double().abs() if bias else 0.0)
+    bound = 1.13 * (3 * 2.0 ** -22 + (k / 16 * 3 + 4) * 2.0 ** -23) * size + 2.0 ** -22 * want.abs()
+    assert bool(((c[:, :n].double() - want).abs() <= bound).all())
+    assert bool((c[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("where,value", [((0, 0), float("inf")), ((3, 5), 1e-20), ((699, 999), float("nan")), ((5, 7), 1e30), ((699, slice(None)), 1e-40)])
+def test_rows_the_planes_do_not_carry(cuda_device, monkeypatch, where, value):
+    m, n, k = 700, 1000, 1000
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    marked = a.clone()
+    marked[where] = value
+    want = []
+    planes, tf32 = (_layer(monkeypatch, p, m, n, k, w) for p in "10")
+    for x in (a, marked):
+        c = torch.empty((m, n), device=cuda_device)
+        tf32.run(x, w, c, stream=torch.cuda.current_stream().cuda_stream)
+        want.append(c)
+    c, x = torch.empty((m, n), device=cuda_device), a.clone()
+    planes.run(x, w, c, stream=torch.cuda.current_stream().cuda_stream)  # scratch exists before the capture
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        planes.run(x, w, c, stream=torch.cuda.current_stream().cuda_stream)
+    for source, ref, exact in ((a, want[0], False), (marked, want[1], True), (a, want[0], False)):
+        x.copy_(source)
+        graph.replay()
+        torch.cuda.synchronize()
+        # the same launches on the TF32 planes, bit by bit; or two forms, each within 2^-20 (|a| |w|)
+        if exact:
+            assert torch.equal(c.nan_to_num(1.5), ref.nan_to_num(1.5))
+        else:
+            assert bool(((c - ref).abs() <= 2.0 ** -16 * (source.abs() @ w.abs().T)).all()) and not torch.equal(c, ref)
+    assert planes.last_launches == 4 and tf32.last_launches == 2
+    planes.check()
+
+
+@pytest.mark.parametrize("value", [float("inf"), 1e-25, 1e25])
+def test_weights_the_planes_do_not_carry(cuda_device, monkeypatch, value):
+    m, n, k = 300, 520, 328
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    w[519, 327] = value
+    outs = []
+    for planes in "01":
+        lin = _layer(monkeypatch, planes, m, n, k, w)
+        outs.append(torch.empty((m, n), device=cuda_device))
+        lin.run(a, w, outs[-1], stream=torch.cuda.current_stream().cuda_stream)
+        lin.check()
+        assert lin.last_launches == 2
+    assert torch.equal(outs[0].nan_to_num(1.5), outs[1].nan_to_num(1.5))
