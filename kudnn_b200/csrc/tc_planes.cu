@@ -10,7 +10,8 @@ using namespace tc;
 bool planes_take(const EpiParams &epi)
 {
     return epi.n_mirrors == 0 && epi.beta == 0.0f && epi.c != nullptr && epi.res_op == KUDNN_B200_RES_NONE &&
-           epi.c_dtype == KUDNN_B200_F32 && epi.c_sn == 1 && epi.c_sm % 4 == 0 && (reinterpret_cast<uintptr_t>(epi.c) & 15u) == 0 &&
+           // (a TMA store does not clip inside 16 bytes)
+           epi.n % 4 == 0 && epi.c_dtype == KUDNN_B200_F32 && epi.c_sn == 1 && epi.c_sm % 4 == 0 && (reinterpret_cast<uintptr_t>(epi.c) & 15u) == 0 &&
            (epi.has_bias == 0 || (epi.bias_dtype == KUDNN_B200_F32 && epi.bias_sm == 0)) &&
            (epi.act == KUDNN_B200_ACT_NONE || epi.act == KUDNN_B200_ACT_RELU || epi.act == KUDNN_B200_ACT_SWISH ||
             epi.act == KUDNN_B200_ACT_GELU_TANH);
