@@ -28,7 +28,7 @@ NVCC_FLAGS = [
 ]
 
 CUDA_SOURCES = ["linear_api.cu", "simt_gemm.cu", "gemv.cu", "tc_gemm.cu", "tc_inst_f32.cu", "tc_inst_f16.cu", "tc_inst_bf16.cu",
-                "tc_inst_s8.cu", "tc_wide_f16.cu", "tc_wide_bf16.cu", "tc_planes.cu", "pack.cu", "static_scratch.cu", "peer.cu", "eltwise.cu", "eltwise_api.cu"]
+                "tc_inst_s8.cu", "tc_wide_f16.cu", "tc_wide_bf16.cu", "tc_wide_s8.cu", "tc_planes.cu", "pack.cu", "static_scratch.cu", "peer.cu", "eltwise.cu", "eltwise_api.cu"]
 
 
 def _nvcc():

@@ -629,6 +629,20 @@ int reserve_gemv_scratch(StreamScratch *sc, long long partial_floats, long long 
     return KUDNN_B200_OK;
 }
 
+// The launch shape of the tensor-core kernel, where KUDNN_B200_DEBUG asks for it.
+void print_plan(const Handle *h, long long nb, const kudnn_b200_linear_desc &d)
+{
+    const char *dbg = std::getenv("KUDNN_B200_DEBUG");
+    if (dbg == nullptr || *dbg == '\0' || *dbg == '0') {
+        return;
+    }
+    std::fprintf(stderr, "kudnn_b200: tensor-core plan batch=%lld m=%lld n=%lld k=%lld: tile %s x %d, %d stages, "
+                         "grid %d, k splits %d, narrow tail from tile %d, %zu bytes of shared memory\n",
+                 nb, static_cast<long long>(d.m), static_cast<long long>(d.n), static_cast<long long>(d.k),
+                 h->tc_plan.pair ? "256 (CTA pair)" : "128", h->tc_plan.wide ? 512 : h->tc_plan.block_n, h->tc_plan.stages,
+                 h->tc_plan.grid, h->tc_plan.splits, h->tc_plan.pair ? h->tc_plan.narrow_from : -1, h->tc_plan.smem_bytes);
+}
+
 // `d_in` is the handle's descriptor, or a copy of it restricted to a block of rows (host-pointer pipeline)
 int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_linear_args &args, cudaStream_t stream)
 {
@@ -718,8 +732,9 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 ops.a = sc->a.ptr;
                 ops.lda = k_pad;
             }
-            if (!(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m && !h->plan_staging)) {
-                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, false, kb::TcRows::kOther, false, &h->tc_plan);
+            const bool wide_ok = kb::tc_wide_takes(ops, ip.epi, kb::TcRows::kOther);
+            if (!(h->plan_valid && h->plan_a == ops.a && h->plan_b == ops.b && h->plan_m == d.m && !h->plan_staging && h->plan_wide_ok == wide_ok)) {
+                cudaError_t e = kb::tc_make_plan(ops, d.m, d.n, h->sm_count, false, kb::TcRows::kOther, wide_ok, &h->tc_plan);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "tensor map encoding");
                 }
@@ -727,7 +742,9 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 h->plan_b = ops.b;
                 h->plan_m = d.m;
                 h->plan_staging = false;
+                h->plan_wide_ok = wide_ok;
                 h->plan_valid = true;
+                print_plan(h, 1, d);
             }
             cudaError_t e = kb::launch_tc(ops, h->tc_plan, ip.epi, d.m, d.n, static_cast<kb::DeviceStatus *>(h->status.ptr), stream,
                                           h->wait_limit, -1, nullptr);
@@ -1085,15 +1102,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 h->plan_rows = rows;
                 h->plan_wide_ok = wide_ok;
                 h->plan_valid = nb == 1;
-                if (const char *dbg = std::getenv("KUDNN_B200_DEBUG")) {
-                    if (*dbg != '\0' && *dbg != '0') {
-                        std::fprintf(stderr, "kudnn_b200: tensor-core plan batch=%lld m=%lld n=%lld k=%lld: tile %s x %d, %d stages, "
-                                             "grid %d, k splits %d, narrow tail from tile %d, %zu bytes of shared memory\n",
-                                     nb, static_cast<long long>(d.m), static_cast<long long>(d.n), static_cast<long long>(d.k),
-                                     h->tc_plan.pair ? "256 (CTA pair)" : "128", h->tc_plan.wide ? 512 : h->tc_plan.block_n, h->tc_plan.stages,
-                                     h->tc_plan.grid, h->tc_plan.splits, h->tc_plan.pair ? h->tc_plan.narrow_from : -1, h->tc_plan.smem_bytes);
-                    }
-                }
+                print_plan(h, nb, d);
             }
             cudaError_t e = kb::launch_tc(ops, h->tc_plan, pr.epi, d.m, d.n,
                                           static_cast<kb::DeviceStatus *>(h->status.ptr), stream, h->wait_limit,

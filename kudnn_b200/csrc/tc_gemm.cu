@@ -61,6 +61,7 @@ cudaError_t encode_kmajor(CUtensorMap *map, const void *base, int kind, long lon
     const CUtensorMapDataType dt = (kind == KUDNN_B200_F32)   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : (kind == KUDNN_B200_F16) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                    : (kind == KUDNN_B200_S8)  ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                                   : (kind == KUDNN_B200_S32) ? CU_TENSOR_MAP_DATA_TYPE_INT32
                                                               : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     cuuint64_t dims[2] = {static_cast<cuuint64_t>(k_total), static_cast<cuuint64_t>(rows)};
     cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld_elems) * es};
@@ -152,13 +153,15 @@ double single_cta_cycles(long long tiles, int splits, long long kb, int bn, int 
 
 // Estimated SM cycles of the kernel of 256 x 512 tiles on `pairs` CTA pairs, and how its work is cut: the whole tiles of the last
 // wave, which would keep only some of the pairs busy, become halves, and the halves of a last wave quarters.
-double wide_cycles(long long m, long long n, long long kb, int pairs, TcPlan *plan)
+double wide_cycles(bool ints, long long m, long long n, long long kb, int pairs, TcPlan *plan)
 {
     // A k-block costs 1024 cycles of MMAs in a whole tile (measured 1.85 times the 640 of a pair's 256 x 256 tile in
     // tc_kernel.cuh, in launches that fill the GPU), and in a half or a quarter what six stages in flight bring in; where K is
     // short the epilogue is the longer part.
-    const double whole_cost = std::max(kb * 1200.0, 16000.0), half_cost = std::max(kb * 740.0, 9000.0);
-    const double quarter_cost = std::max(kb * 670.0, 6000.0);
+    // 8-bit integers are multiplied twice as fast, so that the copies set the pace, and 32-bit results are not drained ahead.
+    const double whole_cost = ints ? kb * 850.0 + 6000.0 : std::max(kb * 1200.0, 16000.0);
+    const double half_cost = ints ? kb * 560.0 + 4000.0 : std::max(kb * 740.0, 9000.0);
+    const double quarter_cost = ints ? kb * 500.0 + 2500.0 : std::max(kb * 670.0, 6000.0);
     const long long tiles_m = (m + 255) / 256, columns = (n + 255) / 256;
     const long long tiles = tiles_m * (columns / 2), odd = tiles_m * (columns % 2);
     const int forced = env_choice("KUDNN_B200_TC_WIDE");
@@ -197,6 +200,11 @@ bool tc_wide_takes(const TcOperands &ops, const EpiParams &epi, TcRows rows)
 {
     const int kind = ops.kind;
     const bool second = epi.res_op != KUDNN_B200_RES_NONE;
+    if (kind == KUDNN_B200_S8) {
+        // (a TMA store does not clip inside 16 bytes)
+        return epi.n % 4 == 0 && ops.batch == 1 && epi.n_mirrors == 0 && epi.beta == 0.0f && !second && epi.c != nullptr && epi.c_sn == 1 && epi.c_sm % 4 == 0 &&
+               (reinterpret_cast<uintptr_t>(epi.c) & 15u) == 0 && (epi.has_bias == 0 || (epi.bias_dtype == KUDNN_B200_S32 && epi.bias_sm == 0));
+    }
     return (kind == KUDNN_B200_F16 || kind == KUDNN_B200_BF16) && ops.batch == 1 && rows == TcRows::kVectors && epi.n_mirrors == 0 &&
            epi.beta == 0.0f && (epi.c == nullptr) == second && epi.c_dtype == kind &&
            (epi.has_bias == 0 || (epi.bias_dtype == kind && epi.bias_sm == 0)) &&
@@ -285,8 +293,9 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     plan->narrow_from = 0;
     // What the shape chosen so far is held against the kernel of 512-column tiles with: the same estimate, but with what a value
     // of its epilogue takes where K is too short to cover it (2048 rows against 1024, n = 9216, k = 256: 10 to 12 us per tile).
-    constexpr double kNarrowPerValue = 0.55;
-    double narrow_cycles = via_smem ? best : single_cta_cycles(ops.batch * tiles_m * ((n + bn - 1) / bn), 1, num_kb, bn, a_rows_single, false, sm_count, kNarrowPerValue);
+    // 32-bit integers leave there 16 bytes of a row at a time: about 28 000 cycles per tile of 4096 x 11008 x 4096.
+    const double narrow_per_value = ints ? 0.85 : 0.55;
+    double narrow_cycles = via_smem ? best : single_cta_cycles(ops.batch * tiles_m * ((n + bn - 1) / bn), 1, num_kb, bn, a_rows_single, false, sm_count, narrow_per_value);
     if (pair) {
         const long long pair_tiles = ((m + 2 * kBM - 1) / (2 * kBM)) * ((n + 255) / 256);
         const long long guess = sm_count / 2;
@@ -296,7 +305,9 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
         const double cycles = 4000.0 + waves * std::max(num_kb * 640.0, epilogue) + epilogue;
         pair = cycles < best || env_choice("KUDNN_B200_TC_PAIR") > 0;
         if (pair) {
-            narrow_cycles = 4000.0 + waves * std::max(num_kb * 640.0, kNarrowPerValue * kBM * 256) + kNarrowPerValue * kBM * 256;
+            const double drain = narrow_per_value * kBM * 256;
+            narrow_cycles = ints ? 4000.0 + num_kb * 640.0 + (waves - 1.0) * std::max(num_kb * 640.0, drain) + 0.5 * drain
+                                 : 4000.0 + waves * std::max(num_kb * 640.0, drain) + drain;
         }
         int clusters = 0;
         if (pair) {
@@ -320,8 +331,8 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     const int forced_wide = env_choice("KUDNN_B200_TC_WIDE");
     if (wide_ok && m > kBM && forced_splits <= 1 && forced_wide != 0 && (env_choice("KUDNN_B200_TC_PAIR") < 0 || forced_wide > 0) &&
         m < (1ll << 31) - 512 && n < (1ll << 31) - 512 && ((m + 255) / 256) * ((n + 127) / 128) < (1ll << 30)) {
-        const int clusters = pair_clusters_of(ops.kind, with_staging, kWideSmem);
-        if (clusters > 0 && (wide_cycles(m, n, num_kb, clusters, plan) < narrow_cycles || forced_wide > 0)) {
+        const int clusters = pair_clusters_of(ops.kind, with_staging, WideShape<KUDNN_B200_F16>::kSmem);
+        if (clusters > 0 && (wide_cycles(ints, m, n, num_kb, clusters, plan) < narrow_cycles || forced_wide > 0)) {
             plan->wide = 1;
             pair = true;
             bn = 256;
@@ -358,7 +369,7 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
     }
     ring = (ring + 1023) / 1024 * 1024;
     plan->ring_bytes = static_cast<int>(ring);
-    plan->smem_bytes = plan->wide ? kWideSmem : static_cast<size_t>(ring + fixed);
+    plan->smem_bytes = plan->wide ? (ints ? WideShape<KUDNN_B200_S8>::kSmem : WideShape<KUDNN_B200_F16>::kSmem) : static_cast<size_t>(ring + fixed);
     if (plan->smem_bytes > static_cast<size_t>(kSmemLimit)) {
         return cudaErrorInvalidValue;
     }
@@ -411,20 +422,22 @@ cudaError_t launch_wide(const TcOperands &ops, const TcPlan &plan, const EpiPara
     p.n_whole = plan.wide_whole;
     p.n_half = plan.wide_half;
     p.num_items = plan.wide_items;
-    p.idesc = make_idesc(ops.kind, 256, 2 * kBM);
-    p.idesc_quarter = make_idesc(ops.kind, 128, 2 * kBM);
+    const bool ints = ops.kind == KUDNN_B200_S8;
+    p.idesc = ints ? make_idesc_i8(ops.a_signed != 0, ops.b_signed != 0, 256, 2 * kBM) : make_idesc(ops.kind, 256, 2 * kBM);
+    p.idesc_quarter = ints ? make_idesc_i8(ops.a_signed != 0, ops.b_signed != 0, 128, 2 * kBM) : make_idesc(ops.kind, 128, 2 * kBM);
     p.b_stable = ops.b_stable ? 1 : 0;
     p.status = status;
     p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimitCycles;
     // the output, written in boxes of 32 rows x 128 bytes
     const bool second = epi.res_op != KUDNN_B200_RES_NONE;
     CUtensorMap out;
-    const cudaError_t e = encode_kmajor(&out, second ? epi.out : epi.c, ops.kind, m, n, second ? epi.out_sm : epi.c_sm, 32);
+    const cudaError_t e = encode_kmajor(&out, second ? epi.out : epi.c, ints ? KUDNN_B200_S32 : ops.kind, m, n, second ? epi.out_sm : epi.c_sm, 32);
     if (e != cudaSuccess) {
         return e;
     }
-    return ops.kind == KUDNN_B200_F16 ? launch_wide_kind<KUDNN_B200_F16>(plan, &out, p, stream)
-                                      : launch_wide_kind<KUDNN_B200_BF16>(plan, &out, p, stream);
+    return ints                        ? launch_wide_kind<KUDNN_B200_S8>(plan, &out, p, stream)
+           : ops.kind == KUDNN_B200_F16 ? launch_wide_kind<KUDNN_B200_F16>(plan, &out, p, stream)
+                                        : launch_wide_kind<KUDNN_B200_BF16>(plan, &out, p, stream);
 }
 
 }  // namespace

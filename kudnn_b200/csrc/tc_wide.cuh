@@ -11,7 +11,7 @@
 //
 // Shape of one CTA (384 threads, persistent, one CTA per SM, clusters of two):
 //   warp 0       one lane loads a k-block: 128 rows of A, 128 rows of B per accumulator (TMA, 128-byte swizzle) into a ring of
-//                four stages (halves and quarters: six)
+//                four stages (halves and quarters: six; 8-bit integers: three, and four)
 //   warp 1       one lane of the leader issues the cta_group::2 MMAs for both CTAs
 //   warps 4..11  epilogue, four warps per accumulator, each with 32 rows of it: out of tensor memory and rounded to 16 bits at
 //                once, which frees the accumulator; the rest of the chain under the next tile's products; then through 4 KiB of
@@ -37,16 +37,20 @@ namespace tc {
 constexpr int kWideThreads = 128 + 32 * kEpiWarps;
 // Registers per thread at launch and in the two parts of the block: 128 * 40 + 256 * 232 = 384 * 168
 constexpr int kWideControlRegs = 40, kWideEpilogueRegs = 232;
-constexpr int kWideStages = 4;
-constexpr int kWideStageBytes = 3 * kABytes;             // A, and B of either accumulator
-constexpr int kWideRing = kWideStages * kWideStageBytes;
-// Halves and quarters, with one B each, see the same memory as a ring of six
-constexpr int kWideSmallStages = 6;
-constexpr int kWideSmallBytes = 2 * kABytes;
-static_assert(kWideSmallStages * kWideSmallBytes == kWideRing, "both rings cover the same memory");
-constexpr int kWideSmem = kWideRing + kStagingBytes + 256;
+constexpr int kWideStageBytes = 3 * kABytes;  // A, and B of either accumulator
+constexpr int kWideSmallBytes = 2 * kABytes;  // halves and quarters, with one B each, see the same memory as a ring of their own
+template <int kKind>
+struct WideShape {
+    // 32-bit results leave tensor memory through shared memory box by box, while the next tile waits for the accumulator: two boxes
+    // per warp there, and a stage less
+    static constexpr int kBoxes = kKind == KUDNN_B200_S8 ? 2 : 1;
+    static constexpr int kStages = kKind == KUDNN_B200_S8 ? 3 : 4;
+    static constexpr int kRing = kStages * kWideStageBytes;
+    static constexpr int kSmallStages = kRing / kWideSmallBytes;
+    static constexpr int kSmem = kRing + kBoxes * kStagingBytes + 256;
+    static_assert(kSmem <= kSmemLimit, "shared memory of the wide kernel");
+};
 constexpr int kWideSkew = 2;                             // k-blocks by which the accumulators run out of step
-static_assert(kWideSmem <= kSmemLimit, "shared memory of the wide kernel");
 
 struct WideParams {
     EpiParams epi;
@@ -274,6 +278,66 @@ __device__ __forceinline__ void wide_finish(const WideParams &p, const CUtensorM
     }
 }
 
+// The same for 8-bit integer products: exact 32-bit sums, a bias of 32-bit integers, clamped to their range; 32 columns at a time,
+// 128 bytes of every row.  `box` is the one of the warp's two boxes that the next store leaves from: only stores alternate them, so
+// that all but the newest have been read when one is used again.
+__device__ __forceinline__ void wide_epilogue_int(const WideParams &p, const CUtensorMap *tmap_out, uint32_t taddr, int row0, int n0,
+                                                  int columns, uint32_t stage, int lane, uint32_t drained, uint32_t &box)
+{
+    const EpiParams &e = p.epi;
+    const uint32_t swz = static_cast<uint32_t>(lane & 7) << 4;
+    uint32_t next[32], cur[32];
+    tmem_load_16_issue(taddr, *reinterpret_cast<uint32_t(*)[16]>(&next[0]));
+    tmem_load_16_issue(taddr + 16u, *reinterpret_cast<uint32_t(*)[16]>(&next[16]));
+#pragma unroll 1
+    for (int c0 = 0; c0 < columns; c0 += 32) {
+        tmem_load_wait16(*reinterpret_cast<uint32_t(*)[16]>(&next[0]));
+        tmem_load_wait16(*reinterpret_cast<uint32_t(*)[16]>(&next[16]));
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            cur[j] = next[j];
+        }
+        if (c0 + 32 < columns) {
+            tmem_load_16_issue(taddr + static_cast<uint32_t>(c0 + 32), *reinterpret_cast<uint32_t(*)[16]>(&next[0]));
+            tmem_load_16_issue(taddr + static_cast<uint32_t>(c0 + 48), *reinterpret_cast<uint32_t(*)[16]>(&next[16]));
+        } else {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive_cluster(drained);
+            }
+        }
+        if (e.has_bias != 0) {
+            const int mine = n0 + c0 + lane < p.n ? static_cast<const int *>(e.bias)[(n0 + c0 + lane) * e.bias_sn] : 0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                int sum;
+                asm("add.sat.s32 %0, %1, %2;" : "=r"(sum) : "r"(static_cast<int>(cur[j])), "r"(__shfl_sync(0xffffffffu, mine, j)));
+                cur[j] = static_cast<uint32_t>(sum);
+            }
+        }
+        if (row0 >= p.m || n0 + c0 >= p.n) {
+            continue;
+        }
+        if (lane == 0) {
+            asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + box + static_cast<uint32_t>(lane * 128) + ((static_cast<uint32_t>(g) << 4) ^ swz)),
+                         "r"(cur[g * 4]), "r"(cur[g * 4 + 1]), "r"(cur[g * 4 + 2]), "r"(cur[g * 4 + 3])
+                         : "memory");
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(tmap_out, stage + box, n0 + c0, row0);
+        }
+        box ^= static_cast<uint32_t>(kWarpStageBytes);
+    }
+}
+
 template <int kKind>
 __global__ void __launch_bounds__(kWideThreads, 1)
     tc_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -281,9 +345,11 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                    const __grid_constant__ WideParams p)
 {
     constexpr int kElemsPerRow = kKind == KUDNN_B200_S8 ? 128 : 64;  // per 128-byte k-block row
+    constexpr int kWideStages = WideShape<kKind>::kStages, kWideSmallStages = WideShape<kKind>::kSmallStages;
+    constexpr int kBoxBytes = WideShape<kKind>::kBoxes * kWarpStageBytes;  // per warp
     extern __shared__ __align__(1024) unsigned char smem[];          // the swizzle pattern repeats every 1024 bytes
-    unsigned char *staging = smem + kWideRing;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(staging + kStagingBytes);
+    unsigned char *staging = smem + WideShape<kKind>::kRing;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(staging + kEpiWarps * kBoxBytes);
     uint64_t *full_bar = bars;
     uint64_t *empty_bar = bars + kWideStages;
     uint64_t *small_full = bars + 2 * kWideStages;
@@ -559,11 +625,11 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         pdl_wait();
         const int quarter = warp & 3;  // tensor-memory lanes [32 * quarter, 32 * quarter + 32)
         const int acc = (warp - 4) / 4;
-        const uint32_t stage = smem_u32(staging + (warp - 4) * kWarpStageBytes);
+        const uint32_t stage = smem_u32(staging + (warp - 4) * kBoxBytes);
         const uint32_t drained = map_to_rank(smem_u32(tmem_empty + acc), 0u);
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * 256);
         const EpiParams &e = p.epi;
-        uint32_t phase = 0;
+        uint32_t phase = 0, box = 0;
         int turn = 0;
         for (int item = first_item; item < p.num_items; item += stride) {
             const WideItem w = wide_item(p, item);
@@ -576,50 +642,56 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             }
             const int n0 = w.n0 + (w.whole ? acc * 256 : 0);
             const int row0 = w.tm * 256 + static_cast<int>(rank) * kBM + quarter * 32;
-            // the bias waits in this warp's box, which the stores of the previous item have left
-            if (lane == 0) {
-                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            if constexpr (kKind != KUDNN_B200_S8) {
+                // the bias waits in this warp's box, which the stores of the previous item have left
+                if (lane == 0) {
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                }
+                __syncwarp();
+                for (int c = lane; c < w.width; c += 32) {
+                    const unsigned short b = e.has_bias == 0 ? static_cast<unsigned short>(0x8000)
+                                             : n0 + c < p.n  ? static_cast<const unsigned short *>(e.bias)[(n0 + c) * e.bias_sn]
+                                                             : static_cast<unsigned short>(0);
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(stage + static_cast<uint32_t>(c * 2)), "h"(b) : "memory");
+                }
+                __syncwarp();
             }
-            __syncwarp();
-            for (int c = lane; c < w.width; c += 32) {
-                const unsigned short b = e.has_bias == 0 ? static_cast<unsigned short>(0x8000)
-                                         : n0 + c < p.n  ? static_cast<const unsigned short *>(e.bias)[(n0 + c) * e.bias_sn]
-                                                         : static_cast<unsigned short>(0);
-                asm volatile("st.shared.u16 [%0], %1;" ::"r"(stage + static_cast<uint32_t>(c * 2)), "h"(b) : "memory");
-            }
-            __syncwarp();
             const bool arrived = __all_sync(0xffffffffu, mbar_wait(tmem_full + acc, phase, abort_flag, p.status, 4, p.wait_limit));
             phase ^= 1u;
             if (!arrived) {
                 break;
             }
             tc_fence_after();
-            uint4 keep[32];
-            if (e.alpha == 1.0f && e.has_bias == 0) {
-                wide_drain<kKind, 0>(e, taddr, w.width, stage, keep);
-            } else if (kKind == KUDNN_B200_F16 && e.half_chain != 0) {
-                wide_drain<kKind, 2>(e, taddr, w.width, stage, keep);
+            if constexpr (kKind == KUDNN_B200_S8) {
+                wide_epilogue_int(p, &tmap_out, taddr, row0, n0, w.width, stage, lane, drained, box);
             } else {
-                wide_drain<kKind, 1>(e, taddr, w.width, stage, keep);
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive_cluster(drained);
-            }
+                uint4 keep[32];
+                if (e.alpha == 1.0f && e.has_bias == 0) {
+                    wide_drain<kKind, 0>(e, taddr, w.width, stage, keep);
+                } else if (kKind == KUDNN_B200_F16 && e.half_chain != 0) {
+                    wide_drain<kKind, 2>(e, taddr, w.width, stage, keep);
+                } else {
+                    wide_drain<kKind, 1>(e, taddr, w.width, stage, keep);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive_cluster(drained);
+                }
 #define KB_WIDE(ACT)                                                                           \
-    if (e.res_op != KUDNN_B200_RES_NONE) {                                                     \
-        wide_finish<ACT, kKind, true>(p, &tmap_out, row0, n0, w.width, stage, lane, keep);    \
-    } else {                                                                                   \
-        wide_finish<ACT, kKind, false>(p, &tmap_out, row0, n0, w.width, stage, lane, keep);   \
-    }
-            switch (e.act) {
-                case KUDNN_B200_ACT_NONE: KB_WIDE(KUDNN_B200_ACT_NONE); break;
-                case KUDNN_B200_ACT_RELU: KB_WIDE(KUDNN_B200_ACT_RELU); break;
-                case KUDNN_B200_ACT_SWISH: KB_WIDE(KUDNN_B200_ACT_SWISH); break;
-                default: KB_WIDE(KUDNN_B200_ACT_GELU_TANH); break;
-            }
+        if (e.res_op != KUDNN_B200_RES_NONE) {                                                     \
+            wide_finish<ACT, kKind, true>(p, &tmap_out, row0, n0, w.width, stage, lane, keep);    \
+        } else {                                                                                   \
+            wide_finish<ACT, kKind, false>(p, &tmap_out, row0, n0, w.width, stage, lane, keep);   \
+        }
+                switch (e.act) {
+                    case KUDNN_B200_ACT_NONE: KB_WIDE(KUDNN_B200_ACT_NONE); break;
+                    case KUDNN_B200_ACT_RELU: KB_WIDE(KUDNN_B200_ACT_RELU); break;
+                    case KUDNN_B200_ACT_SWISH: KB_WIDE(KUDNN_B200_ACT_SWISH); break;
+                    default: KB_WIDE(KUDNN_B200_ACT_GELU_TANH); break;
+                }
 #undef KB_WIDE
+            }
         }
         if (lane == 0) {
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -657,7 +729,7 @@ cudaError_t launch_wide_one(const TcPlan &plan, const void *tmap_out, const Wide
     std::memcpy(&tb, plan.tmap_b, sizeof(tb));
     std::memcpy(&tb64, plan.tmap_b64, sizeof(tb64));
     std::memcpy(&to, tmap_out, sizeof(to));
-    return launch_chained(kernel, dim3(static_cast<unsigned>(plan.grid)), dim3(kWideThreads), kWideSmem, stream, 2u, ta, tb, tb64, to, p);
+    return launch_chained(kernel, dim3(static_cast<unsigned>(plan.grid)), dim3(kWideThreads), WideShape<kKind>::kSmem, stream, 2u, ta, tb, tb64, to, p);
 }
 
 // One translation unit per operand kind (tc_inst_*.cu).
@@ -668,6 +740,7 @@ cudaError_t launch_wide_kind(const TcPlan &plan, const void *tmap_out, const Wid
     cudaError_t launch_wide_kind<KIND>(const TcPlan &plan, const void *tmap_out, const WideParams &p, cudaStream_t stream);
 KB_WIDE_DECLARE(KUDNN_B200_F16)
 KB_WIDE_DECLARE(KUDNN_B200_BF16)
+KB_WIDE_DECLARE(KUDNN_B200_S8)
 #undef KB_WIDE_DECLARE
 
 }  // namespace tc

@@ -265,3 +265,36 @@ def test_wide_tiles_equal_the_narrow_ones(cuda_device, monkeypatch, capfd, dtype
             # alpha * acc + bias is rounded once here and twice there: one unit of the 16-bit value, carried through the chain
             eps = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
             assert torch.allclose(a.float(), b.float(), rtol=2 * eps, atol=2 * eps)
+
+
+@pytest.mark.parametrize("cut,m,n,k", [("1", 129, 512, 128), ("1", 1027, 776, 1096), ("2", 257, 516, 16), ("2", 513, 1032, 640), ("3", 300, 264, 912),
+                                       ("3", 2000, 1160, 272), (None, 4100, 9004, 520), (None, 4100, 9001, 520)])
+@pytest.mark.parametrize("signs", [(kb.S8, kb.S8), (kb.U8, kb.S8)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_wide_tiles_of_integer_products(cuda_device, monkeypatch, capfd, cut, m, n, k, signs, bias):
+    """8-bit integers on tiles of 512 columns: exact, also where the sum with the bias leaves the 32-bit range."""
+    stream = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(41)
+
+    def draw(code, *shape):
+        lo, hi, dt = (-128, 128, torch.int8) if code == kb.S8 else (0, 256, torch.uint8)
+        return torch.randint(lo, hi, shape, generator=gen, device=cuda_device, dtype=torch.int32).to(dt)
+
+    if cut is not None:
+        monkeypatch.setenv("KUDNN_B200_TC_WIDE", cut)
+    monkeypatch.setenv("KUDNN_B200_DEBUG", "1")
+    a, w = draw(signs[0], m, k), draw(signs[1], n, k)
+    side = torch.randint(-2 ** 31, 2 ** 31 - 1, (n,), generator=gen, device=cuda_device, dtype=torch.int64).to(torch.int32) if bias else None
+    pitch = (n + 3) // 4 * 4 + 4
+    lin = kb.Linear(kb.make_desc(m, n, k, signs[0], b_dtype=signs[1], c_dtype=kb.S32, has_bias=bias, bias_dtype=kb.S32, c_strides=(pitch, 1)))
+    lin.force_kernel(kb.KERNEL_TC)
+    lin.prepack(w, stream=stream)
+    c = torch.full((m, pitch), 7, device=cuda_device, dtype=torch.int32)
+    for _ in range(2):
+        lin.run(a, w, c, side, stream=stream)
+    lin.check(stream=stream)
+    want = a.double() @ w.double().T + (side.double() if bias else 0.0)
+    assert torch.equal(c[:, :n], want.clamp(-2.0 ** 31, 2.0 ** 31 - 1).to(torch.int64).to(torch.int32))
+    assert bool((c[:, n:] == 7).all())
+    assert ("256 (CTA pair) x 512" in capfd.readouterr().err) == (n % 4 == 0)  # rows that end inside 16 bytes are left to narrow tiles
