@@ -1509,6 +1509,8 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
         }
         b_dev = h->stage[1].ptr;
     }
+    // from here on the packed copy is being rewritten: until all of it is there it stands for no pointer
+    h->packed_key = nullptr;
     h->plan_valid = false;
     if (d.c_dtype == KUDNN_B200_S32) {
         // 8-bit integer weights: K-major rows with a pitch of a multiple of 16 bytes, what the tensor maps of the

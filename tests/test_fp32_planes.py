@@ -96,3 +96,27 @@ def test_weights_the_planes_do_not_carry(cuda_device, monkeypatch, value):
         lin.check()
         assert lin.last_launches == 2
     assert torch.equal(outs[0].nan_to_num(1.5), outs[1].nan_to_num(1.5))
+
+
+def test_a_pre_pack_that_fails_leaves_no_copy_under_the_old_pointer(cuda_device, monkeypatch):
+    m, n, k = 300, 520, 328
+    a, marked, plain = _draw(cuda_device, m, k), _draw(cuda_device, n, k), _draw(cuda_device, n, k + 1)[:, :k].contiguous()
+    marked[519, 327] = 1e-25
+    stream = torch.cuda.current_stream().cuda_stream
+    want = {}
+    for w in (marked, plain):
+        want[w] = torch.empty((m, n), device=cuda_device)
+        _layer(monkeypatch, "0", m, n, k, w).run(a, w, want[w], stream=stream)
+    lin = _layer(monkeypatch, "1", m, n, k, marked)
+    try:
+        kb.debug_fail_allocation(0)
+        lin.prepack(plain, stream=stream)
+    except kb.KudnnError as err:
+        assert err.status == 3
+    finally:
+        kb.debug_fail_allocation(-1)
+    for w in (marked, plain):
+        c = torch.empty((m, n), device=cuda_device)
+        lin.run(a, w, c, stream=stream)
+        lin.check()
+        assert bool(((c - want[w]).abs() <= 2.0 ** -16 * (a.abs() @ w.abs().T)).all())
