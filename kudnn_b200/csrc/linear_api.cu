@@ -451,6 +451,16 @@ size_t planes_bytes(long long rows, long long k_pad)
     return static_cast<size_t>(rows) * (2 * k_pad * 2 + 4 + 1) + 16;
 }
 
+// Memory that a call does without where there is none: false, and no error is left behind for the launches that follow.
+bool reserve_optional(DeviceBuffer *buf, size_t bytes)
+{
+    if (buf->reserve(bytes) == cudaSuccess) {
+        return true;
+    }
+    (void)cudaGetLastError();
+    return false;
+}
+
 // Whether an fp32 product is worth the planes: they take half of the time of the TF32 form and two more launches, 4 us.  Times of
 // both in us: 512 x 1152 x 1152 23.4 and 24.4, 676 x 1280 x 1152 33 and 31, 1024 x 1152 x 1152 31 and 26, 1195 x 2816 x 1472 66 and
 // 38, 4096 x 4608 x 2304 350 and 185, x 64 57 and 37.  With fewer than 20 tiles of 256 x 256 most pairs would be idle, where the TF32 form cuts K:
@@ -1032,16 +1042,20 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             }
             // fp32, large and pre-packed: fp16 planes, unless a row asks for the TF32 planes, which the device decides
             const int *run_if = nullptr;
-            if (f32 && use_packed && two_d && h->planes_kpad > 0 && kmajor_ready(args.a, d.a_dtype, d.a_sm, d.a_sk, d.m) && kb::planes_take(pr.epi)) {
-                const long long kp = h->planes_kpad, k32 = round_up(d.k, 32);
-                cudaError_t e = sc->planes.reserve(planes_bytes(d.m, kp));
-                if (e == cudaSuccess) e = sc->a.reserve(static_cast<size_t>(d.m) * 3 * k32 * 4);
+            bool planes = f32 && use_packed && two_d && h->planes_kpad > 0 && kmajor_ready(args.a, d.a_dtype, d.a_sm, d.a_sk, d.m) && kb::planes_take(pr.epi);
+            if (planes) {
+                // what both forms need comes first
+                cudaError_t e = sc->a.reserve(static_cast<size_t>(d.m) * 3 * round_up(d.k, 32) * 4);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "packed activations");
                 }
+                planes = reserve_optional(&sc->planes, planes_bytes(d.m, h->planes_kpad));
+            }
+            if (planes) {
+                const long long kp = h->planes_kpad, k32 = round_up(d.k, 32);
                 int *word = nullptr;
                 const kb::PlanesOperand pa = planes_in(sc->planes.ptr, d.m, kp, &word), pb = planes_in(h->b_planes.ptr, d.n, kp);
-                e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
+                cudaError_t e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
                 if (e == cudaSuccess) {
                     e = kb::launch_planes(pa, pb, kp, pr.epi, d.m, d.n, word, static_cast<kb::DeviceStatus *>(h->status.ptr), h->sm_count, stream,
                                           h->wait_limit);
@@ -1599,23 +1613,21 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
         h->packed_ld = ld;
         h->packed_ktotal = kt;
     }
-    // Large fp32 products get the weights as fp16 planes too, if the planes carry every row
+    // Large fp32 products get the weights as fp16 planes too, if the planes carry every row and there is memory for them
     if (d.b_dtype == KUDNN_B200_F32 && planes_worth(d)) {
         const long long kp = round_up(d.k, 64);
-        e = h->b_planes.reserve(planes_bytes(d.n, kp));
-        if (e != cudaSuccess) {
-            return fail_cuda(e, "weight planes");
-        }
-        const kb::PlanesOperand pb = planes_in(h->b_planes.ptr, d.n, kp);
-        e = kb::launch_split_half(h->packed_raw, d.n, d.k, h->packed_ld, pb, kp, stream);
-        std::vector<unsigned char> marks(static_cast<size_t>(d.n));
-        if (e == cudaSuccess) e = cudaMemcpyAsync(marks.data(), pb.flags, marks.size(), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e != cudaSuccess) {
-            return fail_cuda(e, "weight planes");
-        }
-        if (std::all_of(marks.begin(), marks.end(), [](unsigned char f) { return f == 0; })) {
-            h->planes_kpad = kp;
+        if (reserve_optional(&h->b_planes, planes_bytes(d.n, kp))) {
+            const kb::PlanesOperand pb = planes_in(h->b_planes.ptr, d.n, kp);
+            e = kb::launch_split_half(h->packed_raw, d.n, d.k, h->packed_ld, pb, kp, stream);
+            std::vector<unsigned char> marks(static_cast<size_t>(d.n));
+            if (e == cudaSuccess) e = cudaMemcpyAsync(marks.data(), pb.flags, marks.size(), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess) {
+                return fail_cuda(e, "weight planes");
+            }
+            if (std::all_of(marks.begin(), marks.end(), [](unsigned char f) { return f == 0; })) {
+                h->planes_kpad = kp;
+            }
         }
     }
     if (h->planes_kpad == 0) {

@@ -120,3 +120,31 @@ def test_a_pre_pack_that_fails_leaves_no_copy_under_the_old_pointer(cuda_device,
         lin.run(a, w, c, stream=stream)
         lin.check()
         assert bool(((c - want[w]).abs() <= 2.0 ** -16 * (a.abs() @ w.abs().T)).all())
+
+
+@pytest.mark.parametrize("where", ["weights", "activations"])
+def test_without_memory_for_the_planes_the_call_takes_the_tf32_form(cuda_device, monkeypatch, where):
+    m, n, k = 300, 520, 328
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    stream = torch.cuda.current_stream().cuda_stream
+    want, c = (torch.empty((m, n), device=cuda_device) for _ in range(2))
+    _layer(monkeypatch, "0", m, n, k, w).run(a, w, want, stream=stream)
+    monkeypatch.setenv("KUDNN_B200_TC_PLANES", "1")
+    lin = kb.Linear(kb.make_desc(m, n, k, kb.F32))
+    lin.force_kernel(kb.KERNEL_TC)
+    try:
+        if where == "weights":
+            kb.debug_fail_allocation(2)  # the status block, the TF32 planes, these planes
+        lin.prepack(w, stream=stream)
+        if where != "weights":
+            kb.debug_fail_allocation(1)  # the TF32 planes, these planes
+        lin.run(a, w, c, stream=stream)
+    finally:
+        kb.debug_fail_allocation(-1)
+    lin.check()
+    assert bool(((c - want).abs() <= 2.0 ** -16 * (a.abs() @ w.abs().T)).all())
+    # and with memory again, the planes
+    lin.prepack(w, stream=stream)
+    lin.run(a, w, c, stream=stream)
+    lin.check()
+    assert lin.last_launches == 4 and bool(((c - want).abs() <= 2.0 ** -16 * (a.abs() @ w.abs().T)).all())
