@@ -150,7 +150,7 @@ struct PlanesOperand {
 cudaError_t launch_split_half(const void *src, long long rows, long long k, long long s_row, const PlanesOperand &dst, long long k_pad,
                               cudaStream_t stream);
 bool planes_take(const EpiParams &epi);
-// *fallback becomes 1 if any row of a is marked: nothing of c is written then.
+// *fallback becomes 1 if any row of a or b is marked: nothing of c is written then.
 cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long long k_pad, const EpiParams &epi, long long m, long long n,
                           int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles);
 

@@ -1613,8 +1613,10 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
         h->packed_ld = ld;
         h->packed_ktotal = kt;
     }
-    // Large fp32 products get the weights as fp16 planes too, if the planes carry every row and there is memory for them
-    if (d.b_dtype == KUDNN_B200_F32 && planes_worth(d)) {
+    // Large fp32 products get the weights as fp16 planes too, where there is memory for them.  Once made they stay where they are
+    // until unpack or destroy, and every pre-pack writes them anew: graphs hold launches that read them, and these look at the
+    // marks.  Other runs take them only if they carry every row.
+    if (d.b_dtype == KUDNN_B200_F32 && (h->b_planes.ptr != nullptr || planes_worth(d))) {
         const long long kp = round_up(d.k, 64);
         if (reserve_optional(&h->b_planes, planes_bytes(d.n, kp))) {
             const kb::PlanesOperand pb = planes_in(h->b_planes.ptr, d.n, kp);
@@ -1625,13 +1627,10 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
             if (e != cudaSuccess) {
                 return fail_cuda(e, "weight planes");
             }
-            if (std::all_of(marks.begin(), marks.end(), [](unsigned char f) { return f == 0; })) {
+            if (planes_worth(d) && std::all_of(marks.begin(), marks.end(), [](unsigned char f) { return f == 0; })) {
                 h->planes_kpad = kp;
             }
         }
-    }
-    if (h->planes_kpad == 0) {
-        h->b_planes.release();
     }
     // Decode-shaped primitives (m <= 16, 16-bit types) stream the whole weight matrix on every call: they get a
     // second copy in blocks of 8 rows x 64 k, the unit their MMA kernels read, so that a warp's loads are one

@@ -10,7 +10,7 @@
 // SM and 1536 cycles of MMAs.
 //
 // Rows that this form does not carry (elements that are not finite, whose largest lies outside [2^-100, 2^64], or with a nonzero
-// element below 2^-34 of it) are marked by the split; if there is any, all CTAs leave, and the launches that follow compute the
+// element below 2^-34 of it) are marked by the split; if there is any among the activations or the weights, all CTAs leave, and the launches that follow compute the
 // product on TF32 planes (tc_linear_kernel), which otherwise leave at once.
 //
 // Shape of one CTA: as tc_wide_kernel, a ring of three stages, tiles of 256 x 256 (both accumulators), and 256 x 128 for the tiles of
@@ -42,7 +42,7 @@ struct PlanesParams {
     int n_whole, num_items;  // items [0, n_whole) are whole tiles, the rest two to a tile
     unsigned idesc, idesc_half;
     const float *a_scale, *b_scale;  // what a row of the planes has to be multiplied with
-    const unsigned char *flags;      // per row of A: not carried by the planes
+    const unsigned char *a_flags, *b_flags;  // per row: not carried by the planes
     int *fallback;                   // written: whether any is set
     DeviceStatus *status;
     long long wait_limit;
@@ -185,11 +185,16 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     pdl_wait();
     // every CTA comes to the same answer, from the same bytes
     bool marked = false;
-    for (int i = static_cast<int>(threadIdx.x); i < p.m / 4; i += kWideThreads) {
-        marked |= reinterpret_cast<const unsigned *>(p.flags)[i] != 0u;
-    }
-    if (threadIdx.x < static_cast<unsigned>(p.m & 3)) {
-        marked |= p.flags[(p.m & ~3) + threadIdx.x] != 0;
+#pragma unroll
+    for (int op = 0; op < 2; ++op) {
+        const unsigned char *flags = op == 0 ? p.a_flags : p.b_flags;
+        const int rows = op == 0 ? p.m : p.n;
+        for (int i = static_cast<int>(threadIdx.x); i < rows / 4; i += kWideThreads) {
+            marked |= reinterpret_cast<const unsigned *>(flags)[i] != 0u;
+        }
+        if (threadIdx.x < static_cast<unsigned>(rows & 3)) {
+            marked |= flags[(rows & ~3) + threadIdx.x] != 0;
+        }
     }
     const bool fallback = __syncthreads_or(marked ? 1 : 0) != 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -148,3 +148,31 @@ def test_without_memory_for_the_planes_the_call_takes_the_tf32_form(cuda_device,
     lin.run(a, w, c, stream=stream)
     lin.check()
     assert lin.last_launches == 4 and bool(((c - want).abs() <= 2.0 ** -16 * (a.abs() @ w.abs().T)).all())
+
+
+def test_graphs_follow_weights_that_are_pre_packed_again(cuda_device, monkeypatch):
+    """A captured launch on the planes, replayed after the weights changed in place and were pre-packed again: to rows that the
+    planes do not carry, and back."""
+    m, n, k = 300, 520, 328
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    stream = torch.cuda.current_stream().cuda_stream
+    lin = _layer(monkeypatch, "1", m, n, k, w)
+    c, other, want = (torch.empty((m, n), device=cuda_device) for _ in range(3))
+    lin.run(a, w, c, stream=stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        lin.run(a, w, c, stream=torch.cuda.current_stream().cuda_stream)
+    first = w.clone()
+    second = _draw(cuda_device, n, k + 1)[:, :k].contiguous()
+    for source, value in ((first, None), (second, 1e-25), (second, None), (first, 1e30), (first, None)):
+        w.copy_(source)
+        if value is not None:
+            w[519, 327] = value
+        lin.prepack(w, stream=stream)
+        graph.replay()
+        lin.run(a, w, other, stream=stream)
+        lin.check()
+        _layer(monkeypatch, "0", m, n, k, w).run(a, w, want, stream=stream)
+        monkeypatch.setenv("KUDNN_B200_TC_PLANES", "1")
+        for got in (c, other):
+            assert bool(((got - want).abs() <= 2.0 ** -16 * (a.abs() @ w.abs().T)).all())
