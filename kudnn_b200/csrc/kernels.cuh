@@ -139,10 +139,20 @@ cudaError_t launch_split_tf32(const void *src, long long rows, long long k, long
 cudaError_t launch_split_tf32_if(const int *run_if, const void *src, long long rows, long long k, long long s_row, float *dst, long long ldd,
                                  long long k_pad, int sm_count, cudaStream_t stream);
 
-// fp32 operands as two planes of fp16 (tc_planes.cuh): rows of k_pad / 64 blocks of [64 hi | 64 lo], a scale per row, and a byte per
-// row that is set where the planes do not carry the row.
+// fp32 operands as two planes of fp16 (tc_planes.cuh): rows of k_pad / 64 blocks of [64 hi | 64 lo], a scale per row, and a mark per
+// row.  A row that is marked kPlanesLeft has elements too small for the planes: they are zero there and stand in the row's list, in
+// order, the column after the last of them -1.  The planes do not carry rows marked kPlanesNot.  Up to a multiple of 16 rows the marks
+// go on as 0.
+constexpr int kPlanesRest = 8;       // elements in a row's list
+constexpr int kPlanesRestRows = 16;  // rows of both operands whose lists a launch works off; with more it leaves the product alone
+constexpr unsigned char kPlanesLeft = 1, kPlanesNot = 2;
+struct __align__(8) PlanesElement {
+    int k;
+    float x;
+};
 struct PlanesOperand {
     unsigned short *planes;
+    PlanesElement *rest;
     float *scale;
     unsigned char *flags;
 };
@@ -150,7 +160,7 @@ struct PlanesOperand {
 cudaError_t launch_split_half(const void *src, long long rows, long long k, long long s_row, const PlanesOperand &dst, long long k_pad,
                               cudaStream_t stream);
 bool planes_take(const EpiParams &epi);
-// *fallback becomes 1 if any row of a or b is marked: nothing of c is written then.
+// *fallback becomes 1 if a row of a or b is marked kPlanesNot, or more than kPlanesRestRows are marked: nothing of c is written then.
 cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long long k_pad, const EpiParams &epi, long long m, long long n,
                           int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles);
 

@@ -430,25 +430,28 @@ int pack_weights(Handle *h, const void *b_dev, DeviceBuffer *buf, bool with_raw,
     return KUDNN_B200_OK;
 }
 
-// Rows of fp16 planes in one buffer: the planes, a scale per row, a mark per row, and a word for the launches that depend on the marks.
+// Rows of fp16 planes in one buffer: the planes, a list and a mark per row (both on 16 bytes), a word for the launches that depend on the
+// marks, a scale per row.
 kb::PlanesOperand planes_in(void *base, long long rows, long long k_pad, int **word = nullptr)
 {
     kb::PlanesOperand p;
     unsigned char *at = static_cast<unsigned char *>(base);
     p.planes = reinterpret_cast<unsigned short *>(at);
     at += rows * 2 * k_pad * 2;
-    p.scale = reinterpret_cast<float *>(at);
-    at += rows * 4;
+    p.rest = reinterpret_cast<kb::PlanesElement *>(at);
+    at += rows * kb::kPlanesRest * static_cast<long long>(sizeof(kb::PlanesElement));
+    p.flags = at;
+    at += round_up(rows, 16);
     if (word != nullptr) {
         *word = reinterpret_cast<int *>(at);
     }
-    p.flags = at + 16;
+    p.scale = reinterpret_cast<float *>(at + 16);
     return p;
 }
 
 size_t planes_bytes(long long rows, long long k_pad)
 {
-    return static_cast<size_t>(rows) * (2 * k_pad * 2 + 4 + 1) + 16;
+    return static_cast<size_t>(rows) * (2 * k_pad * 2 + kb::kPlanesRest * sizeof(kb::PlanesElement) + 4) + round_up(rows, 16) + 16;
 }
 
 // Memory that a call does without where there is none: false, and no error is left behind for the launches that follow.
@@ -1627,7 +1630,8 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
             if (e != cudaSuccess) {
                 return fail_cuda(e, "weight planes");
             }
-            if (planes_worth(d) && std::all_of(marks.begin(), marks.end(), [](unsigned char f) { return f == 0; })) {
+            if (planes_worth(d) && std::count(marks.begin(), marks.end(), kb::kPlanesNot) == 0 &&
+                std::count(marks.begin(), marks.end(), kb::kPlanesLeft) <= kb::kPlanesRestRows) {
                 h->planes_kpad = kp;
             }
         }

@@ -222,12 +222,20 @@ __global__ void __launch_bounds__(256) split_rows_if_kernel(const int *run_if, c
 // fp32 rows -> two planes of fp16 (see tc_planes.cuh): a CTA per row, eight columns per thread and step.  Bound by memory: the row
 // is read once (rows of up to 8192 columns stay in registers between the search for the largest element and the conversion) and as
 // many bytes are written.
+//
+// The low plane has all of its bits for elements from 2^-14 on after scaling: an error of 2^-37 there, 2^-23 of the element, as in
+// the TF32 planes at any size.  Smaller ones would lose a bit for every factor of two, so they go to the row's list.
 constexpr int kSplitThreads = 128, kSplitHeld = 8;
 
-__global__ void __launch_bounds__(kSplitThreads) split_half_kernel(const float *src_base, long long k, long long s_row, unsigned short *planes,
-                                                                   float *scales, unsigned char *flags, long long k_pad)
+__global__ void __launch_bounds__(kSplitThreads, 6) split_half_kernel(const float *src_base, long long k, long long s_row, const PlanesOperand to,
+                                                                   long long k_pad)
 {
     __shared__ unsigned most[kSplitThreads / 32], least[kSplitThreads / 32];
+    __shared__ int left_out;
+    __shared__ PlanesElement rest[kPlanesRest];
+    if (threadIdx.x == 0) {
+        left_out = 0;
+    }
     pdl_launch_dependents();
     pdl_wait();
     const long long row = blockIdx.x;
@@ -289,14 +297,24 @@ __global__ void __launch_bounds__(kSplitThreads) split_half_kernel(const float *
     // 2^(14 - exponent) and its inverse
     const float up = mx == 0u || !in_range ? 1.0f : __uint_as_float(static_cast<unsigned>(127 + 14 - exponent) << 23);
     const float down = mx == 0u || !in_range ? 1.0f : __uint_as_float(static_cast<unsigned>(127 - 14 + exponent) << 23);
-    if (threadIdx.x == 0) {
-        scales[row] = down;
-        flags[row] = !in_range || (mn != 0xffffffffu && __uint_as_float(mn) * up < 0x1p-20f) ? 1 : 0;
-    }
-    unsigned short *dst = planes + row * 2 * k_pad;
-    auto put = [&](int piece, const float (&v)[8]) {
+    const float smallest = mn != 0xffffffffu && in_range ? __uint_as_float(mn) * up : 1.0f;
+    const bool some_small = smallest < 0x1p-14f;
+    unsigned short *dst = to.planes + row * 2 * k_pad;
+    auto put = [&](int piece, float (&v)[8]) {
         if (piece >= pieces) {
             return;
+        }
+        if (some_small) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (v[i] != 0.0f && fabsf(v[i] * up) < 0x1p-14f) {
+                    const int slot = atomicAdd(&left_out, 1);
+                    if (slot < kPlanesRest) {
+                        rest[slot] = PlanesElement{piece * 8 + i, v[i]};
+                    }
+                    v[i] = 0.0f;
+                }
+            }
         }
         unsigned hi[4], lo[4];
 #pragma unroll
@@ -304,7 +322,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_half_kernel(const float *
             const float x = v[2 * i] * up, y = v[2 * i + 1] * up;
             const __half2 h = __floats2half2_rn(x, y);
             const float2 back = __half22float2(h);
-            const __half2 l = __floats2half2_rn((x - back.x) * 2048.0f, (y - back.y) * 2048.0f);
+            const __half2 l = __floats2half2_rn((x - back.x) * 4096.0f, (y - back.y) * 4096.0f);
             hi[i] = *reinterpret_cast<const unsigned *>(&h);
             lo[i] = *reinterpret_cast<const unsigned *>(&l);
         }
@@ -324,6 +342,32 @@ __global__ void __launch_bounds__(kSplitThreads) split_half_kernel(const float *
             fetch(piece, held[0]);
             put(piece, held[0]);
         }
+    }
+    if (some_small) {
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        to.scale[row] = down;
+        unsigned char mark = !in_range || smallest < 0x1p-20f ? kPlanesNot : 0;
+        if (some_small && mark == 0) {
+            const int count = left_out;
+            mark = count <= kPlanesRest ? kPlanesLeft : kPlanesNot;
+            PlanesElement *list = to.rest + row * kPlanesRest;
+            for (int i = 0; mark == kPlanesLeft && i < count; ++i) {  // by column: the slots were taken in any order
+                int at = 0;
+                for (int j = 0; j < count; ++j) {
+                    at += rest[j].k < rest[i].k ? 1 : 0;
+                }
+                list[at] = rest[i];
+            }
+            if (count < kPlanesRest) {
+                list[count] = PlanesElement{-1, 0.0f};
+            }
+        }
+        to.flags[row] = mark;
+    }
+    if (row == static_cast<long long>(gridDim.x) - 1 && threadIdx.x < static_cast<unsigned>(-gridDim.x & 15u)) {
+        to.flags[row + 1 + threadIdx.x] = 0;
     }
 }
 
@@ -437,7 +481,7 @@ cudaError_t launch_split_half(const void *src, long long rows, long long k, long
                               cudaStream_t stream)
 {
     return launch_chained(split_half_kernel, dim3(static_cast<unsigned>(rows)), dim3(kSplitThreads), 0, stream, 1, static_cast<const float *>(src), k,
-                          s_row, dst.planes, dst.scale, dst.flags, k_pad);
+                          s_row, dst, k_pad);
 }
 
 }  // namespace kb

@@ -49,10 +49,8 @@ cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long l
     p.num_items = p.n_whole + 2 * (tiles - p.n_whole);
     p.idesc = make_idesc(KUDNN_B200_F16, 256, 2 * kBM);
     p.idesc_half = make_idesc(KUDNN_B200_F16, 128, 2 * kBM);
-    p.a_scale = a.scale;
-    p.b_scale = b.scale;
-    p.a_flags = a.flags;
-    p.b_flags = b.flags;
+    p.a = a;
+    p.b = b;
     p.fallback = fallback;
     p.status = status;
     p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimitCycles;

@@ -2,16 +2,19 @@
 //
 // An fp32 matrix product is bound by the tensor pipe, which multiplies TF32 at half the rate of fp16 although both carry 11
 // significant bits.  So every row is scaled by a power of two that takes its largest element to [2^14, 2^15) and written as
-// x = hi + lo / 2^11 with hi = fp16(x) and lo = fp16((x - hi) 2^11) (split_half_kernel): 22 bits of every element down to 2^-28 of the
-// row's largest, and an error below 2^-50 of the largest for the rest.  The products hi.hi go to one accumulator and
-// hi.lo + lo.hi to another; acc0 + acc1 / 2^11, scaled back by row and column, is the sum of the three products that the TF32
+// x = hi + lo / 2^12 with hi = fp16(x) and lo = fp16((x - hi) 2^12) (split_half_kernel): to 2^-23 of every element down to 2^-28 of
+// the row's largest, as the TF32 planes do.  The products hi.hi go to one accumulator and
+// hi.lo + lo.hi to another; acc0 + acc1 / 2^12, scaled back by row and column, is the sum of the three products that the TF32
 // planes add up (the fourth, lo.lo, is 2^-22 relative there and here).  Two accumulators also keep the small products out of the
 // additions to the large one, and a k-block of 64 brings in each operand's planes once instead of one and a half times: 64 KiB per
 // SM and 1536 cycles of MMAs.
 //
-// Rows that this form does not carry (elements that are not finite, whose largest lies outside [2^-100, 2^64], or with a nonzero
-// element below 2^-34 of it) are marked by the split; if there is any among the activations or the weights, all CTAs leave, and the launches that follow compute the
-// product on TF32 planes (tc_linear_kernel), which otherwise leave at once.
+// A normal distribution has one element below 2^-28 of its row's largest in 10^8.  The split leaves up to eight of them per row out of the planes,
+// and the epilogue adds their products in fp32 (planes_add_rest), for up to sixteen rows of activations and weights.
+//
+// Rows that this form does not carry (elements that are not finite, whose largest lies outside [2^-100, 2^64], with a nonzero
+// element below 2^-34 of it, or with more than eight below 2^-28) are marked by the split; if there is any, or lists of more rows than that, among the
+// activations or the weights, all CTAs leave, and the launches that follow compute the product on TF32 planes (tc_linear_kernel), which otherwise leave at once.
 //
 // Shape of one CTA: as tc_wide_kernel, a ring of three stages, tiles of 256 x 256 (both accumulators), and 256 x 128 for the tiles of
 // a last wave that would keep at most half of the pairs busy.
@@ -41,9 +44,8 @@ struct PlanesParams {
     int group_m;
     int n_whole, num_items;  // items [0, n_whole) are whole tiles, the rest two to a tile
     unsigned idesc, idesc_half;
-    const float *a_scale, *b_scale;  // what a row of the planes has to be multiplied with
-    const unsigned char *a_flags, *b_flags;  // per row: not carried by the planes
-    int *fallback;                   // written: whether any is set
+    PlanesOperand a, b;
+    int *fallback;  // written: whether the product is left to the launches that follow
     DeviceStatus *status;
     long long wait_limit;
 };
@@ -93,8 +95,83 @@ __device__ __forceinline__ void planes_drain(float alpha, float row_scale, uint3
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]) : "r"(at + 512));
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float v = fmaf(__uint_as_float(cross[g * 4 + j]), 0x1p-11f, __uint_as_float(main[g * 4 + j]));
+                const float v = fmaf(__uint_as_float(cross[g * 4 + j]), 0x1p-12f, __uint_as_float(main[g * 4 + j]));
                 keep[i * 16 + g * 4 + j] = fmaf(v * row_scale * s[j], alpha, b[j]);
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ float planes_value(const PlanesOperand &o, long long row, int k, int num_kb)
+{
+    const unsigned short *at = o.planes + (row * num_kb + (k >> 6)) * 128 + (k & 63);
+    return fmaf(__half2float(__ushort_as_half(at[64])), 0x1p-12f, __half2float(__ushort_as_half(at[0]))) * o.scale[row];
+}
+
+// What the planes of a row or column leave out, times the other operand's elements; where both leave out the same k, it is added
+// with the column.
+__device__ __forceinline__ void planes_add_rest(const PlanesParams &p, int row0, int n0, int columns, int lane, unsigned marked_rows,
+                                                const unsigned (&marked_columns)[4], float (&keep)[128])
+{
+    const float alpha = p.epi.alpha;
+    const int row = row0 + lane;
+    const bool mine = (marked_rows >> lane & 1u) != 0u;
+#pragma unroll 1
+    for (unsigned left = marked_rows; left != 0u; left &= left - 1u) {
+        const int r = __ffs(left) - 1;
+        const PlanesElement *list = p.a.rest + static_cast<long long>(row0 + r) * kPlanesRest;
+#pragma unroll 1
+        for (int i = 0; i < kPlanesRest; ++i) {
+            const PlanesElement e = list[i];
+            if (e.k < 0) {
+                break;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int col = n0 + q * 32 + lane;
+                const float y = q * 32 < columns && col < p.n ? planes_value(p.b, col, e.k, p.num_kb) : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const float t = e.x * __shfl_sync(0xffffffffu, y, j);
+                    if (lane == r) {
+                        keep[q * 32 + j] = fmaf(t, alpha, keep[q * 32 + j]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll 1
+        for (unsigned left = q == 0 ? marked_columns[0] : q == 1 ? marked_columns[1] : q == 2 ? marked_columns[2] : marked_columns[3]; left != 0u;
+             left &= left - 1u) {
+            const int c = q * 32 + __ffs(left) - 1;
+            const PlanesElement *list = p.b.rest + static_cast<long long>(n0 + c) * kPlanesRest;
+#pragma unroll 1
+            for (int i = 0; i < kPlanesRest; ++i) {
+                const PlanesElement e = list[i];
+                if (e.k < 0) {
+                    break;
+                }
+                float x = 0.0f;
+                if (row < p.m) {
+                    x = planes_value(p.a, row, e.k, p.num_kb);
+#pragma unroll 1
+                    for (int j = 0; mine && j < kPlanesRest; ++j) {
+                        const PlanesElement f = p.a.rest[static_cast<long long>(row) * kPlanesRest + j];
+                        if (f.k < 0) {
+                            break;
+                        }
+                        x = f.k == e.k ? f.x : x;
+                    }
+                }
+                const float t = x * e.x;
+#pragma unroll
+                for (int j = 0; j < 128; ++j) {
+                    if (j == c) {
+                        keep[j] = fmaf(t, alpha, keep[j]);
+                    }
+                }
             }
         }
     }
@@ -149,6 +226,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     uint64_t *tmem_empty = tmem_full + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    int *marked_rows = reinterpret_cast<int *>(tmem_slot + 2);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -166,6 +244,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         mbar_init(tmem_full, 1);
         mbar_init(tmem_empty, 2 * kEpiWarps);
         *abort_flag = 0;
+        *marked_rows = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -183,20 +262,37 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     const int stride = static_cast<int>(gridDim.x >> 1);
     pdl_launch_dependents();  // only now that this CTA holds its tensor memory (see tc_linear_kernel)
     pdl_wait();
-    // every CTA comes to the same answer, from the same bytes
-    bool marked = false;
+    // every CTA comes to the same answer, from the same bytes; both operands' marks are on their way at a time
+    int marked = 0;
+    auto count = [&](unsigned marks) {
+        marked += (marks & 0x02020202u) != 0u ? kPlanesRestRows + 1 : __popc(marks & 0x01010101u);
+        marked = marked < kPlanesRestRows + 1 ? marked : kPlanesRestRows + 1;
+    };
+    for (int i = static_cast<int>(threadIdx.x); i < (p.m + 15) / 16 || i < (p.n + 15) / 16; i += kWideThreads) {
+        uint4 some[2] = {};
 #pragma unroll
-    for (int op = 0; op < 2; ++op) {
-        const unsigned char *flags = op == 0 ? p.a_flags : p.b_flags;
-        const int rows = op == 0 ? p.m : p.n;
-        for (int i = static_cast<int>(threadIdx.x); i < rows / 4; i += kWideThreads) {
-            marked |= reinterpret_cast<const unsigned *>(flags)[i] != 0u;
+        for (int op = 0; op < 2; ++op) {
+            const int rows = op == 0 ? p.m : p.n;
+            const unsigned char *flags = (op == 0 ? p.a.flags : p.b.flags) + static_cast<long long>(i) * 16;
+            if (i < (rows + 15) / 16) {
+                some[op] = *reinterpret_cast<const uint4 *>(flags);
+            }
         }
-        if (threadIdx.x < static_cast<unsigned>(rows & 3)) {
-            marked |= flags[(rows & ~3) + threadIdx.x] != 0;
+#pragma unroll
+        for (int op = 0; op < 2; ++op) {
+            if ((some[op].x | some[op].y | some[op].z | some[op].w) != 0u) {
+                count(some[op].x);
+                count(some[op].y);
+                count(some[op].z);
+                count(some[op].w);
+            }
         }
     }
-    const bool fallback = __syncthreads_or(marked ? 1 : 0) != 0;
+    if (marked != 0) {
+        atomicAdd(marked_rows, marked);
+    }
+    __syncthreads();
+    const bool fallback = *marked_rows > kPlanesRestRows, rest = *marked_rows != 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *p.fallback = fallback ? 1 : 0;
     }
@@ -300,13 +396,22 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             __syncwarp();
             for (int c = lane; c < columns; c += 32) {
                 const bool inside = n0 + c < p.n;
-                const float s = inside ? p.b_scale[n0 + c] : 0.0f;
+                const float s = inside ? p.b.scale[n0 + c] : 0.0f;
                 const float b = e.has_bias == 0 ? -0.0f : inside ? static_cast<const float *>(e.bias)[(n0 + c) * e.bias_sn] : 0.0f;
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + static_cast<uint32_t>(c * 4)), "f"(s) : "memory");
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + 512u + static_cast<uint32_t>(c * 4)), "f"(b) : "memory");
             }
             __syncwarp();
-            const float row_scale = row0 + lane < p.m ? p.a_scale[row0 + lane] : 0.0f;
+            const float row_scale = row0 + lane < p.m ? p.a.scale[row0 + lane] : 0.0f;
+            unsigned marked_row = 0u, marked_column[4] = {};
+            if (rest) {
+                marked_row = __ballot_sync(0xffffffffu, row0 + lane < p.m && p.a.flags[row0 + lane] != 0);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int c = n0 + q * 32 + lane;
+                    marked_column[q] = __ballot_sync(0xffffffffu, q * 32 < columns && c < p.n && p.b.flags[c] != 0);
+                }
+            }
             const bool arrived = __all_sync(0xffffffffu, mbar_wait(tmem_full, phase, abort_flag, p.status, 4, p.wait_limit));
             phase ^= 1u;
             if (!arrived) {
@@ -320,6 +425,9 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive_cluster(drained);
+            }
+            if ((marked_row | marked_column[0] | marked_column[1] | marked_column[2] | marked_column[3]) != 0u) {
+                planes_add_rest(p, row0, n0, columns, lane, marked_row, marked_column, keep);
             }
             switch (e.act) {
                 case KUDNN_B200_ACT_NONE: planes_finish<KUDNN_B200_ACT_NONE>(p, &tmap_out, row0, n0, columns, stage, lane, keep); break;

@@ -176,3 +176,74 @@ def test_graphs_follow_weights_that_are_pre_packed_again(cuda_device, monkeypatc
         monkeypatch.setenv("KUDNN_B200_TC_PLANES", "1")
         for got in (c, other):
             assert bool(((got - want).abs() <= 2.0 ** -16 * (a.abs() @ w.abs().T)).all())
+
+
+def _tail(a, w, form, low):
+    """Every row has one large element that meets zeros, and otherwise only elements of about 2^low of it: `few` of them (the rest
+    of the row zero), or all of the columns."""
+    k = a.shape[1]
+    a, w = a.clamp(-3.0, 3.0), w.clone()
+    sign = torch.where(a < 0.0, -1.0, 1.0)
+    small = sign * (1.0 + 0.9 * torch.rand_like(a)) * 2.0 ** low
+    if form == "few":
+        at = (torch.arange(a.shape[0], device=a.device)[:, None] * 37 + torch.tensor([3, 64, 65, 127, k - 1], device=a.device)) % (k - 2) + 2
+        small = torch.zeros_like(small).scatter(1, at, small.gather(1, at))
+    small[:, :2] = 0.0
+    small[:, 0] = 1.0
+    w[:, 0] = 0.0
+    return small, w
+
+
+@pytest.mark.parametrize("low", [-27, -28, -29, -30, -31, -32, -33, -34])
+@pytest.mark.parametrize("form", ["few", "all"])
+@pytest.mark.parametrize("operand", ["activations", "weights"])
+def test_small_elements_of_a_row_keep_their_bits(cuda_device, monkeypatch, low, form, operand):
+    """Results that only elements far below their row's largest contribute to, against 64 bits and relative to the terms themselves."""
+    m, n, k = 300, 264, 136
+    rows = (0, 31, 32, 130, 255, 256, 299) if operand == "activations" else (0, 63, 64, 127, 128, 200, 263)
+    if form == "all":
+        rows = rows[:2]
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    a[:, 0], w[:, 0] = 0.0, 0.0
+    if operand == "activations":
+        a[list(rows)], w = _tail(a[list(rows)], w, form, low)
+    else:
+        w[list(rows)], a = _tail(w[list(rows)], a, form, low)
+    stream = torch.cuda.current_stream().cuda_stream
+    lin = _layer(monkeypatch, "1", m, n, k, w)
+    c = torch.empty((m, n), device=cuda_device)
+    for _ in range(2):
+        lin.run(a, w, c, stream=stream)
+    lin.check(stream=stream)
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # each operand to 2^-22, the product of the low parts 2^-22, and per 8 columns three additions that cut at 2^-23 of a partial sum
+    bound = (3 * 2.0 ** -22 + (k / 8 * 3 + 8) * 2.0 ** -23) * size
+    if form == "few":
+        # five terms in five k-steps (and as many rounded to fp32 where they are added one by one)
+        part = (list(rows), slice(None)) if operand == "activations" else (slice(None), list(rows))
+        bound[part] = (3 * 2.0 ** -22 + (5 * 3 + 5) * 2.0 ** -23) * size[part]
+    assert bool(((c.double() - want).abs() <= bound).all())
+
+
+def test_small_elements_of_both_operands_meet(cuda_device, monkeypatch):
+    """A row and a column whose largest elements meet zeros, and whose small ones meet each other, once where both are small."""
+    m, n, k = 300, 264, 136
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    a[:, :2], w[:, :2] = 0.0, 0.0
+    a[40], w[70] = 0.0, 0.0
+    a[40, 0], w[70, 1] = 1.0, 1.0
+    a[40, 5], w[70, 5] = 1.7 * 2.0 ** -30, 1.3 * 2.0 ** -31
+    a[40, 100], a[40, 130] = 1.1 * 2.0 ** -33, -1.9 * 2.0 ** -29
+    w[70, 130] = 1.4 * 2.0 ** -32
+    stream = torch.cuda.current_stream().cuda_stream
+    lin = _layer(monkeypatch, "1", m, n, k, w)
+    tf32, c = torch.empty((m, n), device=cuda_device), torch.empty((m, n), device=cuda_device)
+    lin.run(a, w, c, alpha=0.5, stream=stream)
+    lin.check(stream=stream)
+    assert lin.last_launches == 4
+    _layer(monkeypatch, "0", m, n, k, w).run(a, w, tf32, alpha=0.5, stream=stream)
+    want, size = 0.5 * (a.double() @ w.double().T), 0.5 * (a.double().abs() @ w.double().abs().T)
+    # per term: each operand to 2^-22, the low parts' product 2^-22, rounding of the product and of each sum 2^-23
+    assert bool(((c.double() - want).abs()[40, :] <= (3 * 2.0 ** -22 + (3 * 3 + 4) * 2.0 ** -23) * size[40, :]).all())
+    assert bool(((c.double() - want).abs()[:, 70] <= (3 * 2.0 ** -22 + (3 * 3 + 4) * 2.0 ** -23) * size[:, 70]).all())
+    assert float(want[40, 70]) != 0.0 and not torch.equal(c, tf32)
