@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *src_base, 
     *reinterpret_cast<float4 *>(dst + 2 * k_pad) = h;
 }
 
-// The same split of activation rows by CTAs that walk over the rows, and only if *run_if is not 0: the launch that otherwise leaves
-// at once has to be small.
+// The same split of activation rows (contiguous, on 16 bytes) by CTAs that walk over the rows, and only if *run_if is not 0: the
+// launch that otherwise leaves at once has to be small.
 __global__ void __launch_bounds__(256) split_rows_if_kernel(const int *run_if, const float *src_base, long long rows, long long k, long long s_row,
                                                             float *dst_base, long long ldd, long long k_pad)
 {
@@ -209,12 +209,18 @@ __global__ void __launch_bounds__(256) split_rows_if_kernel(const int *run_if, c
     for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
         const float *src = src_base + row * s_row;
         float *dst = dst_base + row * ldd;
-        for (long long kk = threadIdx.x; kk < k_pad; kk += 256) {
-            const float v = kk < k ? src[kk] : 0.0f;
-            const float hi = to_tf32(v);
-            dst[kk] = to_tf32(v - hi);
-            dst[k_pad + kk] = hi;
-            dst[2 * k_pad + kk] = hi;
+        for (long long kk = threadIdx.x * 4; kk < k_pad; kk += 1024) {
+            float4 v;
+            if (kk + 4 <= k) {
+                v = *reinterpret_cast<const float4 *>(src + kk);
+            } else {
+                v = make_float4(kk < k ? src[kk] : 0.0f, kk + 1 < k ? src[kk + 1] : 0.0f, kk + 2 < k ? src[kk + 2] : 0.0f, 0.0f);
+            }
+            const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
+            const float4 l = make_float4(to_tf32(v.x - h.x), to_tf32(v.y - h.y), to_tf32(v.z - h.z), to_tf32(v.w - h.w));
+            *reinterpret_cast<float4 *>(dst + kk) = l;
+            *reinterpret_cast<float4 *>(dst + k_pad + kk) = h;
+            *reinterpret_cast<float4 *>(dst + 2 * k_pad + kk) = h;
         }
     }
 }
@@ -348,7 +354,7 @@ __global__ void __launch_bounds__(kSplitThreads, 6) split_half_kernel(const floa
     }
     if (threadIdx.x == 0) {
         to.scale[row] = down;
-        unsigned char mark = !in_range || smallest < 0x1p-20f ? kPlanesNot : 0;
+        unsigned char mark = !in_range || smallest < 0x1p-46f ? kPlanesNot : 0;
         if (some_small && mark == 0) {
             const int count = left_out;
             mark = count <= kPlanesRest ? kPlanesLeft : kPlanesNot;

@@ -247,3 +247,25 @@ def test_small_elements_of_both_operands_meet(cuda_device, monkeypatch):
     assert bool(((c.double() - want).abs()[40, :] <= (3 * 2.0 ** -22 + (3 * 3 + 4) * 2.0 ** -23) * size[40, :]).all())
     assert bool(((c.double() - want).abs()[:, 70] <= (3 * 2.0 ** -22 + (3 * 3 + 4) * 2.0 ** -23) * size[:, 70]).all())
     assert float(want[40, 70]) != 0.0 and not torch.equal(c, tf32)
+
+
+@pytest.mark.parametrize("operand", ["activations", "weights"])
+@pytest.mark.parametrize("rows,per_row,value,planes", [(1, 1, 1e-10, True), (1, 8, 1e-17, True), (16, 1, 1e-12, True), (17, 1, 1e-12, False), (1, 9, 1e-10, False)])
+def test_a_few_tiny_elements_stay_on_the_planes(cuda_device, monkeypatch, operand, rows, per_row, value, planes):
+    """Beside elements of size one; more rows or elements than the lists take are the TF32 form bit by bit."""
+    m, n, k = 300, 520, 328
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    for x in (a, w):
+        x.copy_(torch.where(x.abs() < 1e-3, torch.full_like(x, 1e-3), x))
+    x = a if operand == "activations" else w
+    for r in range(rows):
+        x[m - 1 - 17 * r, 40 * r % (k - per_row):][:per_row] = value
+    stream = torch.cuda.current_stream().cuda_stream
+    tf32, c = torch.empty((m, n), device=cuda_device), torch.empty((m, n), device=cuda_device)
+    _layer(monkeypatch, "0", m, n, k, w).run(a, w, tf32, stream=stream)
+    lin = _layer(monkeypatch, "1", m, n, k, w)
+    lin.run(a, w, c, stream=stream)
+    lin.check(stream=stream)
+    assert torch.equal(c, tf32) is not planes
+    size = a.double().abs() @ w.double().abs().T
+    assert bool(((c.double() - a.double() @ w.double().T).abs() <= (3 * 2.0 ** -22 + (k / 8 * 3 + 12) * 2.0 ** -23) * size).all())
