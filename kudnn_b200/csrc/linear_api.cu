@@ -130,13 +130,12 @@ struct StreamScratch {
     unsigned long long last_use = 0;
     bool counters_clear = false;  // the arrival counters are zero, or will be when the next launch on the stream starts
     DeviceBuffer partials, counters;  // split-K partial sums and arrival counters of the streaming kernels
-    DeviceBuffer a;                   // packed activations
+    DeviceBuffer a;                   // packed activations; fp32: as fp16 planes, then, for the launches that replace these, as TF32 planes
     DeviceBuffer b;                   // packed weights (when not pre-packed)
     DeviceBuffer q;                   // 8-bit weights widened to fp16 (when not pre-packed)
-    DeviceBuffer planes;              // fp32 activations as fp16 planes, with their scales and marks
     void release()
     {
-        for (DeviceBuffer *buf : {&partials, &counters, &a, &b, &q, &planes}) {
+        for (DeviceBuffer *buf : {&partials, &counters, &a, &b, &q}) {
             buf->release();
         }
     }
@@ -430,9 +429,8 @@ int pack_weights(Handle *h, const void *b_dev, DeviceBuffer *buf, bool with_raw,
     return KUDNN_B200_OK;
 }
 
-// Rows of fp16 planes in one buffer: the planes, a list and a mark per row (both on 16 bytes), a word for the launches that depend on the
-// marks, a scale per row.
-kb::PlanesOperand planes_in(void *base, long long rows, long long k_pad, int **word = nullptr)
+// Rows of fp16 planes in one buffer: the planes, a list and a mark per row (both on 16 bytes), a scale per row.
+kb::PlanesOperand planes_in(void *base, long long rows, long long k_pad)
 {
     kb::PlanesOperand p;
     unsigned char *at = static_cast<unsigned char *>(base);
@@ -442,16 +440,13 @@ kb::PlanesOperand planes_in(void *base, long long rows, long long k_pad, int **w
     at += rows * kb::kPlanesRest * static_cast<long long>(sizeof(kb::PlanesElement));
     p.flags = at;
     at += round_up(rows, 16);
-    if (word != nullptr) {
-        *word = reinterpret_cast<int *>(at);
-    }
-    p.scale = reinterpret_cast<float *>(at + 16);
+    p.scale = reinterpret_cast<float *>(at);
     return p;
 }
 
 size_t planes_bytes(long long rows, long long k_pad)
 {
-    return static_cast<size_t>(rows) * (2 * k_pad * 2 + kb::kPlanesRest * sizeof(kb::PlanesElement) + 4) + round_up(rows, 16) + 16;
+    return static_cast<size_t>(rows) * (2 * k_pad * 2 + kb::kPlanesRest * sizeof(kb::PlanesElement) + 4) + round_up(rows, 16);
 }
 
 // Memory that a call does without where there is none: false, and no error is left behind for the launches that follow.
@@ -1045,20 +1040,18 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
             }
             // fp32, large and pre-packed: fp16 planes, unless a row asks for the TF32 planes, which the device decides
             const int *run_if = nullptr;
-            bool planes = f32 && use_packed && two_d && h->planes_kpad > 0 && kmajor_ready(args.a, d.a_dtype, d.a_sm, d.a_sk, d.m) && kb::planes_take(pr.epi);
-            if (planes) {
-                // what both forms need comes first
-                cudaError_t e = sc->a.reserve(static_cast<size_t>(d.m) * 3 * round_up(d.k, 32) * 4);
+            if (f32 && use_packed && two_d && h->planes_kpad > 0 && kmajor_ready(args.a, d.a_dtype, d.a_sm, d.a_sk, d.m) && kb::planes_take(pr.epi)) {
+                const long long kp = h->planes_kpad, k32 = round_up(d.k, 32);
+                // The TF32 planes are written when the fp16 planes have been read, over them: the memory, and the time to get it
+                // in a first call, of the TF32 form.  The word that decides is behind both.
+                const size_t planes = std::max(round_up(planes_bytes(d.m, kp), 16), d.m * 3 * k32 * 4);
+                cudaError_t e = sc->a.reserve(planes + 16);
                 if (e != cudaSuccess) {
                     return fail_cuda(e, "packed activations");
                 }
-                planes = reserve_optional(&sc->planes, planes_bytes(d.m, h->planes_kpad));
-            }
-            if (planes) {
-                const long long kp = h->planes_kpad, k32 = round_up(d.k, 32);
-                int *word = nullptr;
-                const kb::PlanesOperand pa = planes_in(sc->planes.ptr, d.m, kp, &word), pb = planes_in(h->b_planes.ptr, d.n, kp);
-                cudaError_t e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
+                int *word = reinterpret_cast<int *>(static_cast<char *>(sc->a.ptr) + planes);
+                const kb::PlanesOperand pa = planes_in(sc->a.ptr, d.m, kp), pb = planes_in(h->b_planes.ptr, d.n, kp);
+                e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
                 if (e == cudaSuccess) {
                     e = kb::launch_planes(pa, pb, kp, pr.epi, d.m, d.n, word, static_cast<kb::DeviceStatus *>(h->status.ptr), h->sm_count, stream,
                                           h->wait_limit);
@@ -2094,7 +2087,7 @@ int64_t kudnn_b200_linear_workspace_bytes(kudnn_b200_linear_t h)
     }
     size_t bytes = h->b_packed.bytes + h->b_blocked.bytes + h->b_planes.bytes;
     for (const auto &sc : h->scratch) {
-        bytes += sc->partials.bytes + sc->counters.bytes + sc->a.bytes + sc->b.bytes + sc->planes.bytes;
+        bytes += sc->partials.bytes + sc->counters.bytes + sc->a.bytes + sc->b.bytes;
     }
     return static_cast<int64_t>(bytes);
 }

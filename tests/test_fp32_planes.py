@@ -269,3 +269,17 @@ def test_a_few_tiny_elements_stay_on_the_planes(cuda_device, monkeypatch, operan
     assert torch.equal(c, tf32) is not planes
     size = a.double().abs() @ w.double().abs().T
     assert bool(((c.double() - a.double() @ w.double().T).abs() <= (3 * 2.0 ** -22 + (k / 8 * 3 + 12) * 2.0 ** -23) * size).all())
+
+
+def test_scratch_of_a_run_is_that_of_the_tf32_form(cuda_device, monkeypatch):
+    m, n, k = 1100, 520, 328
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    stream = torch.cuda.current_stream().cuda_stream
+    c, grown = torch.empty((m, n), device=cuda_device), []
+    for planes in "01":
+        lin = _layer(monkeypatch, planes, m, n, k, w)
+        before = lin.workspace_bytes
+        lin.run(a, w, c, stream=stream)
+        lin.check(stream=stream)
+        grown.append(lin.workspace_bytes - before)
+    assert grown[1] <= grown[0] + 16
