@@ -180,7 +180,7 @@ struct kudnn_b200_linear_s {
     unsigned long long scratch_uses = 0;
     DeviceBuffer b_packed;      // pre-packed weights
     DeviceBuffer b_blocked;     // decode-shaped handles: the weights once more in 8-row x 64-k blocks
-    DeviceBuffer b_planes;      // fp32: the weights once more as fp16 planes (tc_planes.cuh), for large products
+    DeviceBuffer b_planes;      // fp32: the weights once more as fp16 planes (tc_planes.cuh), where b_packed has no room for them
     DeviceBuffer stage[6];      // host-pointer staging: a, b, c, bias, res, out
 
     // pre-pack state
@@ -191,7 +191,8 @@ struct kudnn_b200_linear_s {
     long long packed_ld = 0, packed_ktotal = 0;
     long long blocked_kpad = 0;  // columns per row of b_blocked (k rounded up to 256); 0 = no blocked copy
 
-    long long planes_kpad = 0;   // columns per row of b_planes (k rounded up to 64); 0 = no planes
+    void *planes_at = nullptr;   // the fp16 planes of fp32 weights, behind the packed weights or in b_planes, until unpack or destroy
+    long long planes_kpad = 0;   // columns per row of them (k rounded up to 64); 0 = runs don't use them
 
     // tensor-map cache of the last tensor-core launch
     kb::TcPlan tc_plan;
@@ -447,6 +448,12 @@ kb::PlanesOperand planes_in(void *base, long long rows, long long k_pad)
 size_t planes_bytes(long long rows, long long k_pad)
 {
     return static_cast<size_t>(rows) * (2 * k_pad * 2 + kb::kPlanesRest * sizeof(kb::PlanesElement) + 4) + round_up(rows, 16);
+}
+
+// What pack_weights() takes for fp32 weights with their raw plane
+size_t packed_f32_bytes(const kudnn_b200_linear_desc &d)
+{
+    return static_cast<size_t>(d.n) * 4 * round_up(d.k, 32) * 4;
 }
 
 // Memory that a call does without where there is none: false, and no error is left behind for the launches that follow.
@@ -1050,7 +1057,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                     return fail_cuda(e, "packed activations");
                 }
                 int *word = reinterpret_cast<int *>(static_cast<char *>(sc->a.ptr) + planes);
-                const kb::PlanesOperand pa = planes_in(sc->a.ptr, d.m, kp), pb = planes_in(h->b_planes.ptr, d.n, kp);
+                const kb::PlanesOperand pa = planes_in(sc->a.ptr, d.m, kp), pb = planes_in(h->planes_at, d.n, kp);
                 e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
                 if (e == cudaSuccess) {
                     e = kb::launch_planes(pa, pb, kp, pr.epi, d.m, d.n, word, static_cast<kb::DeviceStatus *>(h->status.ptr), h->sm_count, stream,
@@ -1600,6 +1607,10 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
         int launches = 0;
         long long ld = 0, kt = 0;
         const void *raw = nullptr;
+        if (d.b_dtype == KUDNN_B200_F32 && h->b_packed.ptr == nullptr && planes_worth(d)) {
+            // with the fp16 planes behind them: an allocation of any size takes a third of a millisecond, as long as all of the packing
+            (void)reserve_optional(&h->b_packed, packed_f32_bytes(d) + planes_bytes(d.n, round_up(d.k, 64)));
+        }
         rc = pack_weights(h, b_dev, &h->b_packed, true, stream, &ld, &kt, &raw, &launches);
         if (rc != KUDNN_B200_OK) {
             return rc;
@@ -1612,10 +1623,17 @@ int kudnn_b200_linear_prepack(kudnn_b200_linear_t h, const void *b, void *cuda_s
     // Large fp32 products get the weights as fp16 planes too, where there is memory for them.  Once made they stay where they are
     // until unpack or destroy, and every pre-pack writes them anew: graphs hold launches that read them, and these look at the
     // marks.  Other runs take them only if they carry every row.
-    if (d.b_dtype == KUDNN_B200_F32 && (h->b_planes.ptr != nullptr || planes_worth(d))) {
+    if (d.b_dtype == KUDNN_B200_F32 && (h->planes_at != nullptr || planes_worth(d))) {
         const long long kp = round_up(d.k, 64);
-        if (reserve_optional(&h->b_planes, planes_bytes(d.n, kp))) {
-            const kb::PlanesOperand pb = planes_in(h->b_planes.ptr, d.n, kp);
+        if (h->planes_at == nullptr) {
+            if (h->b_packed.bytes >= packed_f32_bytes(d) + planes_bytes(d.n, kp)) {
+                h->planes_at = static_cast<char *>(h->b_packed.ptr) + packed_f32_bytes(d);
+            } else if (reserve_optional(&h->b_planes, planes_bytes(d.n, kp))) {
+                h->planes_at = h->b_planes.ptr;
+            }
+        }
+        if (h->planes_at != nullptr) {
+            const kb::PlanesOperand pb = planes_in(h->planes_at, d.n, kp);
             e = kb::launch_split_half(h->packed_raw, d.n, d.k, h->packed_ld, pb, kp, stream);
             std::vector<unsigned char> marks(static_cast<size_t>(d.n));
             if (e == cudaSuccess) e = cudaMemcpyAsync(marks.data(), pb.flags, marks.size(), cudaMemcpyDeviceToHost, stream);
@@ -2036,6 +2054,7 @@ int kudnn_b200_linear_unpack(kudnn_b200_linear_t h)
         h->b_packed.release();
         h->b_blocked.release();
         h->b_planes.release();
+        h->planes_at = nullptr;
     }
     return KUDNN_B200_OK;
 }

@@ -134,10 +134,10 @@ def test_without_memory_for_the_planes_the_call_takes_the_tf32_form(cuda_device,
     lin.force_kernel(kb.KERNEL_TC)
     try:
         if where == "weights":
-            kb.debug_fail_allocation(2)  # the status block, the TF32 planes, these planes
+            kb.debug_fail_allocation(1)  # the status block, both kinds of planes together, the TF32 planes alone
         lin.prepack(w, stream=stream)
         if where != "weights":
-            kb.debug_fail_allocation(1)  # the TF32 planes, these planes
+            kb.debug_fail_allocation(1)  # one allocation for both kinds of planes, and no other
         lin.run(a, w, c, stream=stream)
     finally:
         kb.debug_fail_allocation(-1)
@@ -283,3 +283,21 @@ def test_scratch_of_a_run_is_that_of_the_tf32_form(cuda_device, monkeypatch):
         lin.check(stream=stream)
         grown.append(lin.workspace_bytes - before)
     assert grown[1] <= grown[0] + 16
+
+
+def test_pre_packing_a_new_primitive_allocates_once(cuda_device, monkeypatch):
+    m, n, k = 300, 520, 328
+    a, w = _draw(cuda_device, m, k), _draw(cuda_device, n, k)
+    stream = torch.cuda.current_stream().cuda_stream
+    c = torch.empty((m, n), device=cuda_device)
+    monkeypatch.setenv("KUDNN_B200_TC_PLANES", "1")
+    lin = kb.Linear(kb.make_desc(m, n, k, kb.F32))
+    lin.force_kernel(kb.KERNEL_TC)
+    try:
+        kb.debug_fail_allocation(2)  # the status block, both kinds of planes: a third would fail, and the fp16 planes be left out
+        lin.prepack(w, stream=stream)
+    finally:
+        kb.debug_fail_allocation(-1)
+    lin.run(a, w, c, stream=stream)
+    lin.check(stream=stream)
+    assert lin.last_launches == 4
