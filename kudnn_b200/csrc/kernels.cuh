@@ -162,7 +162,8 @@ cudaError_t launch_split_half(const void *src, long long rows, long long k, long
 bool planes_take(const EpiParams &epi);
 // *fallback becomes 1 if a row of a or b is marked kPlanesNot, or more than kPlanesRestRows are marked: nothing of c is written then.
 cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long long k_pad, const EpiParams &epi, long long m, long long n,
-                          int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles);
+                          int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles,
+                          int skip_kblock);
 
 // Stand-alone element-wise activation and RMS normalisation (eltwise.cu); device pointers.
 cudaError_t launch_activation(const void *src, int src_dtype, void *dst, int dst_dtype, long long count, int act, float alpha,

@@ -762,7 +762,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 print_plan(h, 1, d);
             }
             cudaError_t e = kb::launch_tc(ops, h->tc_plan, ip.epi, d.m, d.n, static_cast<kb::DeviceStatus *>(h->status.ptr), stream,
-                                          h->wait_limit, -1, nullptr);
+                                          h->wait_limit, h->skip_kblock, nullptr);
             if (e != cudaSuccess) {
                 return fail_cuda(e, "tensor-core kernel launch");
             }
@@ -1061,7 +1061,7 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
                 if (e == cudaSuccess) {
                     e = kb::launch_planes(pa, pb, kp, pr.epi, d.m, d.n, word, static_cast<kb::DeviceStatus *>(h->status.ptr), h->sm_count, stream,
-                                          h->wait_limit);
+                                          h->wait_limit, h->skip_kblock);
                 }
                 if (e == cudaSuccess) {
                     e = kb::launch_split_tf32_if(word, args.a, d.m, d.k, d.a_sm, static_cast<float *>(sc->a.ptr), 3 * k32, k32, h->sm_count, stream);

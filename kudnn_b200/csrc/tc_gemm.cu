@@ -405,7 +405,7 @@ int raster_group(const TcOperands &ops, int tile_rows)
 }
 
 cudaError_t launch_wide(const TcOperands &ops, const TcPlan &plan, const EpiParams &epi, long long m, long long n,
-                        DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles)
+                        DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles, int skip_kblock)
 {
     if (!tc_wide_takes(ops, epi, plan.rows)) {
         return cudaErrorInvalidValue;  // the plan was made for another epilogue
@@ -431,6 +431,7 @@ cudaError_t launch_wide(const TcOperands &ops, const TcPlan &plan, const EpiPara
     p.idesc = ints ? make_idesc_i8(ops.a_signed != 0, ops.b_signed != 0, 256, 2 * kBM) : make_idesc(ops.kind, 256, 2 * kBM);
     p.idesc_quarter = ints ? make_idesc_i8(ops.a_signed != 0, ops.b_signed != 0, 128, 2 * kBM) : make_idesc(ops.kind, 128, 2 * kBM);
     p.b_stable = ops.b_stable ? 1 : 0;
+    p.skip_kb = skip_kblock;
     p.status = status;
     p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimitCycles;
     // the output, written in boxes of 32 rows x 128 bytes
@@ -452,7 +453,7 @@ cudaError_t launch_tc(const TcOperands &ops, const TcPlan &plan, const EpiParams
                       const BatchParams *bp, const int *run_if)
 {
     if (plan.wide) {
-        return run_if != nullptr ? cudaErrorInvalidValue : launch_wide(ops, plan, epi, m, n, status, stream, wait_limit_cycles);
+        return run_if != nullptr ? cudaErrorInvalidValue : launch_wide(ops, plan, epi, m, n, status, stream, wait_limit_cycles, skip_kblock);
     }
     TcParams p;
     p.epi = epi;

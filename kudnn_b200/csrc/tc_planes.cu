@@ -18,7 +18,7 @@ bool planes_take(const EpiParams &epi)
 }
 
 cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long long k_pad, const EpiParams &epi, long long m, long long n,
-                          int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles)
+                          int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles, int skip_kblock)
 {
     if (!tc_available() || !planes_take(epi)) {
         return cudaErrorNotSupported;
@@ -52,6 +52,7 @@ cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long l
     p.a = a;
     p.b = b;
     p.fallback = fallback;
+    p.skip_kb = skip_kblock;
     p.status = status;
     p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimitCycles;
     return launch_chained(tc_planes_kernel, dim3(static_cast<unsigned>(2 * std::min(p.num_items, pairs))), dim3(kWideThreads), kPlanesSmem, stream,

@@ -48,6 +48,7 @@ struct PlanesParams {
     unsigned idesc, idesc_half;
     PlanesOperand a, b;
     int *fallback;  // written: whether the product is left to the launches that follow
+    int skip_kb;    // test hook, as in WideParams
     DeviceStatus *status;
     long long wait_limit;
 };
@@ -321,14 +322,16 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                             alive = false;
                             break;
                         }
-                        if (rank == 0) {
-                            mbar_expect_tx(full_bar + stage, bytes);
+                        if (kb != p.skip_kb || blockIdx.x >= 2 || item != first_item) {
+                            if (rank == 0) {
+                                mbar_expect_tx(full_bar + stage, bytes);
+                            }
+                            const uint32_t at = ring + static_cast<uint32_t>(stage * kPlanesStageBytes), bar = full_at + static_cast<uint32_t>(stage * 8);
+                            tma_load_pair_at(at, &tmap_a, bar, kb * 128, a_row);
+                            tma_load_pair_at(at + kABytes, &tmap_a, bar, kb * 128 + 64, a_row);
+                            tma_load_pair_at(at + 2 * kABytes, map_b, bar, kb * 128, b_row);
+                            tma_load_pair_at(at + 3 * kABytes, map_b, bar, kb * 128 + 64, b_row);
                         }
-                        const uint32_t at = ring + static_cast<uint32_t>(stage * kPlanesStageBytes), bar = full_at + static_cast<uint32_t>(stage * 8);
-                        tma_load_pair_at(at, &tmap_a, bar, kb * 128, a_row);
-                        tma_load_pair_at(at + kABytes, &tmap_a, bar, kb * 128 + 64, a_row);
-                        tma_load_pair_at(at + 2 * kABytes, map_b, bar, kb * 128, b_row);
-                        tma_load_pair_at(at + 3 * kABytes, map_b, bar, kb * 128 + 64, b_row);
                         if (++stage == kPlanesStages) {
                             stage = 0;
                             phase ^= 1u;

@@ -63,6 +63,7 @@ struct WideParams {
     int n_whole, n_half, num_items;
     unsigned idesc, idesc_quarter;
     int b_stable;
+    int skip_kb;  // test hook: the first pair never loads this k-block of its first item; -1 = off
     DeviceStatus *status;
     long long wait_limit;
 };
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 };
                 // weights that only pre-packing writes are on their way before the previous kernel has ended
                 int early = 0;
-                if (p.b_stable != 0) {
+                if (p.b_stable != 0 && p.skip_kb < 0) {
                     const WideItem w = wide_item(p, first_item);
                     const int row = w.n0 + static_cast<int>(rank) * (w.width / 2);
                     const int stages = w.whole ? kWideStages : kWideSmallStages;
@@ -451,12 +452,14 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                             alive = false;
                             break;
                         }
-                        if (early == 0) {
-                            load_b_whole(stage, x, b_row);
-                        } else {
-                            --early;
+                        if (kb != p.skip_kb || blockIdx.x >= 2 || item != first_item) {
+                            if (early == 0) {
+                                load_b_whole(stage, x, b_row);
+                            } else {
+                                --early;
+                            }
+                            tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideStageBytes), &tmap_a, large_at + static_cast<uint32_t>(stage * 8), x, a_row);
                         }
-                        tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideStageBytes), &tmap_a, large_at + static_cast<uint32_t>(stage * 8), x, a_row);
                         if (++stage == kWideStages) {
                             stage = 0;
                             phase ^= 1u;
@@ -484,12 +487,14 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                             alive = false;
                             break;
                         }
-                        if (early == 0) {
-                            load_b_small(map, bytes, stage, x, b_row);
-                        } else {
-                            --early;
+                        if (kb != p.skip_kb || blockIdx.x >= 2 || item != first_item) {
+                            if (early == 0) {
+                                load_b_small(map, bytes, stage, x, b_row);
+                            } else {
+                                --early;
+                            }
+                            tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideSmallBytes), &tmap_a, small_at + static_cast<uint32_t>(stage * 8), x, a_row);
                         }
-                        tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideSmallBytes), &tmap_a, small_at + static_cast<uint32_t>(stage * 8), x, a_row);
                         if (++stage == kWideSmallStages) {
                             stage = 0;
                             phase ^= 1u;
@@ -732,7 +737,7 @@ cudaError_t launch_wide_one(const TcPlan &plan, const void *tmap_out, const Wide
     return launch_chained(kernel, dim3(static_cast<unsigned>(plan.grid)), dim3(kWideThreads), WideShape<kKind>::kSmem, stream, 2u, ta, tb, tb64, to, p);
 }
 
-// One translation unit per operand kind (tc_inst_*.cu).
+// One translation unit per operand kind (tc_wide_*.cu).
 template <int kKind>
 cudaError_t launch_wide_kind(const TcPlan &plan, const void *tmap_out, const WideParams &p, cudaStream_t stream);
 #define KB_WIDE_DECLARE(KIND) \

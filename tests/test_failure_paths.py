@@ -120,3 +120,34 @@ def test_prepacked_weights_follow_an_in_place_update(cuda_device):
     lin.run(d["a"], d["b"], y, d["bias"], stream=stream)
     lin.check(stream=stream)
     helpers.compare(helpers._from_torch(y).reshape(ref3.shape), ref3, desc.c_dtype)
+
+
+@pytest.mark.parametrize("dtype,shape", [(kb.BF16, 1), (kb.F16, 2), (kb.BF16, 3), (kb.S8, 1), (kb.S8, 2), (kb.S8, 3), (kb.F32, 0)])
+def test_waits_that_run_out_on_wide_tiles_and_on_planes(cuda_device, monkeypatch, dtype, shape):
+    """Whole tiles of 512 columns, halves and quarters, and fp16 planes: the first pair never loads k-block 2 of its first tile."""
+    monkeypatch.setenv("KUDNN_B200_TC_WIDE", str(shape))
+    monkeypatch.setenv("KUDNN_B200_TC_PLANES", "1")
+    m, n, k = 600, 1160, 1024
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(dtype * 8 + shape)
+    kind = {kb.F32: torch.float32, kb.F16: torch.float16, kb.BF16: torch.bfloat16, kb.S8: torch.int8}[dtype]
+    # small integers: every form gives the exact sums, which 16 bits hold
+    a, w = (torch.randint(-1, 2, s, generator=gen, device=cuda_device).to(kind) for s in ((m, k), (n, k)))
+    want = (a.double() @ w.double().T)
+    c = torch.zeros((m, n), dtype=torch.int32 if dtype == kb.S8 else kind, device=cuda_device)
+    stream = torch.cuda.current_stream().cuda_stream
+    lin = kb.Linear(kb.make_desc(m, n, k, dtype, b_dtype=kb.S8, c_dtype=kb.S32) if dtype == kb.S8 else kb.make_desc(m, n, k, dtype))
+    lin.force_kernel(kb.KERNEL_TC)
+    lin.prepack(w, stream=stream)
+    for _ in range(2):
+        lin.debug_set_wait(2_000_000, 2)  # about a millisecond
+        lin.run(a, w, c, stream=stream)
+        with pytest.raises(kb.KudnnError) as err:
+            lin.check(stream=stream)
+        assert err.value.status == 5 and "gave up" in str(err.value)
+        lin.debug_set_wait(0, -1)
+        for _ in range(2):
+            c.zero_()
+            lin.run(a, w, c, stream=stream)
+            lin.check(stream=stream)
+            assert torch.equal(c.double(), want)
