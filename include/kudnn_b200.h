@@ -241,10 +241,11 @@ KUDNN_B200_API int kudnn_b200_peer_buffer_close(void *dev_ptr);
 KUDNN_B200_API int kudnn_b200_peer_buffer_destroy(void *dev_ptr);
 
 /* Test hooks (no counterpart in the reference).  set_wait: device-side waits of this handle's tensor-core launches
- * give up after `wait_limit_cycles` SM cycles (0 = the default, about two seconds), and the producer of CTA 0 (of the
- * first CTA pair, on tiles of 512 columns and on fp16 planes) leaves out the loads of k-block `skip_kblock` of its first
- * tile (-1 = never), so that one bounded wait runs out, the kernel drains, frees its tensor memory and the run reports
- * KUDNN_B200_TIMEOUT; nothing faults or hangs.  Pairs on tiles of 256 columns and launches that cut K load all the same.
+ * give up after `wait_limit_cycles` SM cycles (0 = the default, about two seconds), and the producer of CTA 0 leaves
+ * out the loads of k-block `skip_kblock` of its first tile (-1 = never), so that one bounded wait runs out, the
+ * kernel drains, frees its tensor memory and the run reports KUDNN_B200_TIMEOUT; nothing faults or hangs.  On tiles of
+ * 512 columns and on fp16 planes all producers leave out the k-blocks from `skip_kblock` on; pairs on tiles of 256
+ * columns and launches that cut K load all the same.
  * fail_allocation: the nth (0 = next) device allocation the library attempts fails as if the device were out of
  * memory (KUDNN_B200_ALLOC_FAILED); negative = off. */
 KUDNN_B200_API int kudnn_b200_debug_set_wait(kudnn_b200_linear_t handle, long long wait_limit_cycles, int skip_kblock);

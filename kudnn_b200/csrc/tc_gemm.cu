@@ -431,7 +431,7 @@ cudaError_t launch_wide(const TcOperands &ops, const TcPlan &plan, const EpiPara
     p.idesc = ints ? make_idesc_i8(ops.a_signed != 0, ops.b_signed != 0, 256, 2 * kBM) : make_idesc(ops.kind, 256, 2 * kBM);
     p.idesc_quarter = ints ? make_idesc_i8(ops.a_signed != 0, ops.b_signed != 0, 128, 2 * kBM) : make_idesc(ops.kind, 128, 2 * kBM);
     p.b_stable = ops.b_stable ? 1 : 0;
-    p.skip_kb = skip_kblock;
+    p.load_kb = skip_kblock >= 0 ? std::min(skip_kblock, p.num_kb) : p.num_kb;
     p.status = status;
     p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimitCycles;
     // the output, written in boxes of 32 rows x 128 bytes

@@ -52,7 +52,7 @@ cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long l
     p.a = a;
     p.b = b;
     p.fallback = fallback;
-    p.skip_kb = skip_kblock;
+    p.load_kb = skip_kblock >= 0 ? std::min(skip_kblock, p.num_kb) : p.num_kb;
     p.status = status;
     p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimitCycles;
     return launch_chained(tc_planes_kernel, dim3(static_cast<unsigned>(2 * std::min(p.num_items, pairs))), dim3(kWideThreads), kPlanesSmem, stream,

@@ -48,7 +48,7 @@ struct PlanesParams {
     unsigned idesc, idesc_half;
     PlanesOperand a, b;
     int *fallback;  // written: whether the product is left to the launches that follow
-    int skip_kb;    // test hook, as in WideParams
+    int load_kb;    // as in WideParams
     DeviceStatus *status;
     long long wait_limit;
 };
@@ -317,21 +317,19 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                     const int a_row = w.tm * 256 + static_cast<int>(rank) * kBM, b_row = w.n0 + static_cast<int>(rank) * (w.width / 2);
                     const CUtensorMap *map_b = w.width == 256 ? &tmap_b : &tmap_b64;
                     const uint32_t bytes = w.width == 256 ? 8 * kABytes : 6 * kABytes;
-                    for (int kb = 0; kb < p.num_kb; ++kb) {
+                    for (int kb = 0; kb < p.load_kb; ++kb) {
                         if (!mbar_wait(empty_bar + stage, phase ^ 1u, abort_flag, p.status, 1, p.wait_limit)) {
                             alive = false;
                             break;
                         }
-                        if (kb != p.skip_kb || blockIdx.x >= 2 || item != first_item) {
-                            if (rank == 0) {
-                                mbar_expect_tx(full_bar + stage, bytes);
-                            }
-                            const uint32_t at = ring + static_cast<uint32_t>(stage * kPlanesStageBytes), bar = full_at + static_cast<uint32_t>(stage * 8);
-                            tma_load_pair_at(at, &tmap_a, bar, kb * 128, a_row);
-                            tma_load_pair_at(at + kABytes, &tmap_a, bar, kb * 128 + 64, a_row);
-                            tma_load_pair_at(at + 2 * kABytes, map_b, bar, kb * 128, b_row);
-                            tma_load_pair_at(at + 3 * kABytes, map_b, bar, kb * 128 + 64, b_row);
+                        if (rank == 0) {
+                            mbar_expect_tx(full_bar + stage, bytes);
                         }
+                        const uint32_t at = ring + static_cast<uint32_t>(stage * kPlanesStageBytes), bar = full_at + static_cast<uint32_t>(stage * 8);
+                        tma_load_pair_at(at, &tmap_a, bar, kb * 128, a_row);
+                        tma_load_pair_at(at + kABytes, &tmap_a, bar, kb * 128 + 64, a_row);
+                        tma_load_pair_at(at + 2 * kABytes, map_b, bar, kb * 128, b_row);
+                        tma_load_pair_at(at + 3 * kABytes, map_b, bar, kb * 128 + 64, b_row);
                         if (++stage == kPlanesStages) {
                             stage = 0;
                             phase ^= 1u;

@@ -63,7 +63,7 @@ struct WideParams {
     int n_whole, n_half, num_items;
     unsigned idesc, idesc_quarter;
     int b_stable;
-    int skip_kb;  // test hook: the first pair never loads this k-block of its first item; -1 = off
+    int load_kb;  // num_kb, or by the test hook fewer: the k-blocks of an item that are loaded
     DeviceStatus *status;
     long long wait_limit;
 };
@@ -425,11 +425,11 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 };
                 // weights that only pre-packing writes are on their way before the previous kernel has ended
                 int early = 0;
-                if (p.b_stable != 0 && p.skip_kb < 0) {
+                if (p.b_stable != 0) {
                     const WideItem w = wide_item(p, first_item);
                     const int row = w.n0 + static_cast<int>(rank) * (w.width / 2);
                     const int stages = w.whole ? kWideStages : kWideSmallStages;
-                    early = p.num_kb < stages ? p.num_kb : stages;
+                    early = p.load_kb < stages ? p.load_kb : stages;
                     for (int i = 0; i < early; ++i) {
                         if (w.whole) {
                             load_b_whole(i, i * kElemsPerRow, row);
@@ -447,19 +447,17 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                     const WideItem w = wide_item(p, item);
                     const int a_row = w.tm * 256 + static_cast<int>(rank) * kBM, b_row = w.n0 + static_cast<int>(rank) * 128;
                     int x = 0;
-                    for (int kb = 0; kb < p.num_kb; ++kb, x += kElemsPerRow) {
+                    for (int kb = 0; kb < p.load_kb; ++kb, x += kElemsPerRow) {
                         if (!mbar_wait(empty_bar + stage, phase ^ 1u, abort_flag, p.status, 1, p.wait_limit)) {
                             alive = false;
                             break;
                         }
-                        if (kb != p.skip_kb || blockIdx.x >= 2 || item != first_item) {
-                            if (early == 0) {
-                                load_b_whole(stage, x, b_row);
-                            } else {
-                                --early;
-                            }
-                            tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideStageBytes), &tmap_a, large_at + static_cast<uint32_t>(stage * 8), x, a_row);
+                        if (early == 0) {
+                            load_b_whole(stage, x, b_row);
+                        } else {
+                            --early;
                         }
+                        tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideStageBytes), &tmap_a, large_at + static_cast<uint32_t>(stage * 8), x, a_row);
                         if (++stage == kWideStages) {
                             stage = 0;
                             phase ^= 1u;
@@ -482,19 +480,17 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                     const CUtensorMap *map = w.width == 256 ? &tmap_b : &tmap_b64;
                     const uint32_t bytes = w.width == 256 ? 4 * kABytes : 3 * kABytes;
                     int x = 0;
-                    for (int kb = 0; kb < p.num_kb; ++kb, x += kElemsPerRow) {
+                    for (int kb = 0; kb < p.load_kb; ++kb, x += kElemsPerRow) {
                         if (!mbar_wait(small_empty + stage, phase ^ 1u, abort_flag, p.status, 1, p.wait_limit)) {
                             alive = false;
                             break;
                         }
-                        if (kb != p.skip_kb || blockIdx.x >= 2 || item != first_item) {
-                            if (early == 0) {
-                                load_b_small(map, bytes, stage, x, b_row);
-                            } else {
-                                --early;
-                            }
-                            tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideSmallBytes), &tmap_a, small_at + static_cast<uint32_t>(stage * 8), x, a_row);
+                        if (early == 0) {
+                            load_b_small(map, bytes, stage, x, b_row);
+                        } else {
+                            --early;
                         }
+                        tma_load_pair_at(ring + static_cast<uint32_t>(stage * kWideSmallBytes), &tmap_a, small_at + static_cast<uint32_t>(stage * 8), x, a_row);
                         if (++stage == kWideSmallStages) {
                             stage = 0;
                             phase ^= 1u;

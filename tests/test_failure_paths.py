@@ -124,7 +124,7 @@ def test_prepacked_weights_follow_an_in_place_update(cuda_device):
 
 @pytest.mark.parametrize("dtype,shape", [(kb.BF16, 1), (kb.F16, 2), (kb.BF16, 3), (kb.S8, 1), (kb.S8, 2), (kb.S8, 3), (kb.F32, 0)])
 def test_waits_that_run_out_on_wide_tiles_and_on_planes(cuda_device, monkeypatch, dtype, shape):
-    """Whole tiles of 512 columns, halves and quarters, and fp16 planes: the first pair never loads k-block 2 of its first tile."""
+    """Whole tiles of 512 columns, halves and quarters, and fp16 planes: the loads end ahead of k-block 2 of every tile."""
     monkeypatch.setenv("KUDNN_B200_TC_WIDE", str(shape))
     monkeypatch.setenv("KUDNN_B200_TC_PLANES", "1")
     m, n, k = 600, 1160, 1024
