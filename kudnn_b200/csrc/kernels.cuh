@@ -96,6 +96,8 @@ const char *tc_unavailable_reason();
 // boxes of 128 bytes of K x box_rows rows with the 128-byte swizzle; rows and columns out of range read as zero.
 cudaError_t tc_encode_kmajor(void *map128, const void *base, int kind, long long rows, long long k_total, long long ld_elems,
                              int box_rows);
+// How many CTA pairs with this much shared memory run at a time, as many as the GPU's partitions let; 0 if the driver does not say.
+int tc_pair_clusters(int kind, size_t smem_bytes);
 // with_staging: the launch writes output mirrors and needs the epilogue's row staging in shared memory
 // wide_ok: the kernel of 256 x 512 tiles takes this epilogue (tc_wide_takes)
 cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm_count, bool with_staging, TcRows rows,
@@ -162,7 +164,7 @@ cudaError_t launch_split_half(const void *src, long long rows, long long k, long
 bool planes_take(const EpiParams &epi);
 // *fallback becomes 1 if a row of a or b is marked kPlanesNot, or more than kPlanesRestRows are marked: nothing of c is written then.
 cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long long k_pad, const EpiParams &epi, long long m, long long n,
-                          int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles,
+                          int *fallback, DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles,
                           int skip_kblock);
 
 // Stand-alone element-wise activation and RMS normalisation (eltwise.cu); device pointers.

@@ -1060,8 +1060,8 @@ int run_device(Handle *h, const kudnn_b200_linear_desc &d_in, const kudnn_b200_l
                 const kb::PlanesOperand pa = planes_in(sc->a.ptr, d.m, kp), pb = planes_in(h->planes_at, d.n, kp);
                 e = kb::launch_split_half(args.a, d.m, d.k, d.a_sm, pa, kp, stream);
                 if (e == cudaSuccess) {
-                    e = kb::launch_planes(pa, pb, kp, pr.epi, d.m, d.n, word, static_cast<kb::DeviceStatus *>(h->status.ptr), h->sm_count, stream,
-                                          h->wait_limit, h->skip_kblock);
+                    e = kb::launch_planes(pa, pb, kp, pr.epi, d.m, d.n, word, static_cast<kb::DeviceStatus *>(h->status.ptr), stream, h->wait_limit,
+                                          h->skip_kblock);
                 }
                 if (e == cudaSuccess) {
                     e = kb::launch_split_tf32_if(word, args.a, d.m, d.k, d.a_sm, static_cast<float *>(sc->a.ptr), 3 * k32, k32, h->sm_count, stream);

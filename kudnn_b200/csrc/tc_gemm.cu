@@ -133,6 +133,15 @@ int pair_clusters_of(int kind, bool with_staging, size_t smem)
     return clusters;
 }
 
+}  // namespace
+
+int tc_pair_clusters(int kind, size_t smem_bytes)
+{
+    return pair_clusters_of(kind, false, smem_bytes);
+}
+
+namespace {
+
 // Estimated SM cycles of a launch of single CTAs.  A k-block of a tile costs its MMAs (2 cycles per column whatever the
 // operand type) or its operand bytes (about 60 per cycle and SM), whichever is more.
 double single_cta_cycles(long long tiles, int splits, long long kb, int bn, int a_rows, bool via_smem, int sm_count, double per_value = 0.35)

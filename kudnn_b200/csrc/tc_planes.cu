@@ -18,7 +18,7 @@ bool planes_take(const EpiParams &epi)
 }
 
 cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long long k_pad, const EpiParams &epi, long long m, long long n,
-                          int *fallback, DeviceStatus *status, int sm_count, cudaStream_t stream, long long wait_limit_cycles, int skip_kblock)
+                          int *fallback, DeviceStatus *status, cudaStream_t stream, long long wait_limit_cycles, int skip_kblock)
 {
     if (!tc_available() || !planes_take(epi)) {
         return cudaErrorNotSupported;
@@ -42,7 +42,10 @@ cudaError_t launch_planes(const PlanesOperand &a, const PlanesOperand &b, long l
     p.tiles_n = static_cast<int>((n + 255) / 256);
     // the A rows of a raster group (4 bytes per element and row) should stay in L2, as for the other kernels
     p.group_m = static_cast<int>(std::clamp<long long>((64ll << 20) / (256 * 4 * k_pad), 2, kMaxGroupM));
-    const int tiles = p.tiles_m * p.tiles_n, pairs = sm_count / 2;
+    const int tiles = p.tiles_m * p.tiles_n, pairs = tc_pair_clusters(KUDNN_B200_F16, kPlanesSmem);
+    if (pairs <= 0) {
+        return cudaErrorNotSupported;
+    }
     const int left = tiles % pairs;
     // tiles left over after the last full wave, if they would keep at most half of the pairs busy
     p.n_whole = 2 * left <= pairs ? tiles - left : tiles;
