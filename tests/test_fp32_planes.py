@@ -301,3 +301,34 @@ def test_pre_packing_a_new_primitive_allocates_once(cuda_device, monkeypatch):
     lin.run(a, w, c, stream=stream)
     lin.check(stream=stream)
     assert lin.last_launches == 4
+
+
+@pytest.mark.parametrize("n", [2564, 2308])
+@pytest.mark.parametrize("marks", [False, True])
+def test_several_tiles_per_pair(cuda_device, monkeypatch, n, marks):
+    """17 x 11 tiles: two waves on 74 pairs and a third of whole tiles; 17 x 10: the last wave of halves.  Two raster groups, two calls one
+    after the other on other inputs, chosen by size."""
+    monkeypatch.delenv("KUDNN_B200_TC_PLANES", raising=False)
+    m, k = 4100, 264
+    w, side = _draw(cuda_device, n, k), _draw(cuda_device, n)
+    xs = [_draw(cuda_device, m, k), _draw(cuda_device, m, k + 1)[:, :k].contiguous()]
+    for x in xs + [w]:
+        x.copy_(torch.where(x.abs() < 1e-3, torch.full_like(x, 1e-3), x))
+    if marks:
+        xs[0][4099, 77], xs[0][130, 3], w[n - 1, 263] = 1e-11, -2e-10, 3e-9
+    stream = torch.cuda.current_stream().cuda_stream
+    lin = kb.Linear(kb.make_desc(m, n, k, kb.F32, has_bias=True))
+    lin.prepack(w, stream=stream)
+    cs = [torch.full((m, n), 7.0, device=cuda_device) for _ in xs]
+    for x, c in zip(xs, cs):
+        lin.run(x, w, c, side, stream=stream)
+    lin.check(stream=stream)
+    assert lin.last_launches == 4
+    for x, c in zip(xs, cs):
+        want = x.double() @ w.double().T + side.double()
+        error = c.double() - want
+        # every 256 x 128 piece by itself: the operands to 2^-23, and 17 steps of 16 columns, each cut at 2^-23 of the sum so far
+        for r in range(0, m, 256):
+            for j in range(0, n, 128):
+                part = (slice(r, r + 256), slice(j, j + 128))
+                assert float(error[part].norm()) <= (k / 16 + 8) * 2.0 ** -23 * float(want[part].norm())
