@@ -116,7 +116,8 @@ KUDNN_B200_API int kudnn_b200_linear_clone(kudnn_b200_linear_t src, kudnn_b200_l
 KUDNN_B200_API int kudnn_b200_linear_destroy(kudnn_b200_linear_t handle);
 
 /* Pre-packs the weight operand `b` (host or device memory) into the layout the chosen kernel streams (K-major,
- * 16-byte aligned rows; fp32 weights additionally split into TF32 hi/lo planes).  Later runs whose args->b equals
+ * 16-byte aligned rows; fp32 weights as TF32 hi/lo planes and as they are, 16 bytes per element, and those of large products
+ * where memory allows once more as two planes of fp16, 4 bytes per element).  Later runs whose args->b equals
  * `b` use the packed copy and do not read `b` again: the packed copy is recognised by the ADDRESS alone.  After the
  * weights at that address have changed (an in-place update, or a new tensor the allocator placed where the old one
  * was) call prepack again, or kudnn_b200_linear_unpack to go back to reading `b` on every run; otherwise runs keep

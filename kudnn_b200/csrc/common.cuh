@@ -168,9 +168,9 @@ __device__ __forceinline__ float rcp_approx(float v)
 // 1 / (1 + 2^t)
 __device__ __forceinline__ float sigmoid_neg2(float t)
 {
-    // Branch-free and without a clamp: beyond t = 126 the quotient is 0, far below it 1, which are the values of the
-    // reference's clamp of the exponent (src/dnn/src/kernels/vml/vml_sve_la_sigmoid.h:39-48).  Denormals as zero change nothing
-    // here: a power that small vanishes beside the 1.
+    // Branch-free and without a clamp.  The reference clamps the exponent of e at 87 (src/dnn/src/kernels/vml/vml_sve_la_sigmoid.h:39-48)
+    // and so returns at least 1.6e-38; beyond t = 126 (e^87.3) this is 0.  Far below it is 1 as there.  A power so small that it is taken
+    // as zero vanishes beside the 1.
     return rcp_approx(1.0f + ex2_approx(t));
 }
 // 1 / (1 + exp(t)), libm grade
@@ -315,7 +315,8 @@ __device__ __forceinline__ void epilogue_scalar(const EpiParams &p, float acc, l
 }
 
 // ---- programmatic dependent launch
-// The tensor-core kernel, the streaming kernels, simt_small_kernel, pack_rows_kernel and split_rows_kernel let the next kernel
+// The tensor-core kernels (tc_linear_kernel, tc_wide_kernel, tc_planes_kernel), the streaming kernels, simt_small_kernel,
+// pack_rows_kernel, split_rows_kernel, split_rows_if_kernel and split_half_kernel let the next kernel
 // on their stream be set up while they still run, and wait for their predecessor before they touch memory that it may write;
 // what they do earlier (barriers, tensor memory, descriptors, weights in copies that the handle owns) depends on no kernel.  The
 // other kernels of the library do neither.  Takes 2-4 us off a call that follows another one.

@@ -286,10 +286,11 @@ cudaError_t tc_make_plan(const TcOperands &ops, long long m, long long n, int sm
         return cudaErrorInvalidValue;
     }
     // CTA pairs: 256 x 256 tiles over clusters of two, where that is estimated to be faster.  Not for launches
-    // that run for many milliseconds: those are limited by the board's power cap, and the pair shape, which needs
+    // that run for many milliseconds: those are limited by the board's power cap, and this pair shape, which needs
     // fewer cycles, draws enough more power per cycle to end up slower there (bf16 n = 28672, k = 8192, ms per call,
     // pair / single CTA: 4096 rows 1.385 / 1.396, 8192 rows 2.84 / 2.85, 16384 rows 6.10 / 5.96, 32768 rows
-    // 13.3 / 12.4).
+    // 13.3 / 12.4).  The pairs on 256 x 512 tiles below are not held back so: in turn for seconds each, 32768 rows with
+    // SiLU 12.4 to 12.5 ms at 1.10 GHz against 12.9 at 1.25 GHz of single CTAs.
     const double flops = 2.0 * static_cast<double>(m) * static_cast<double>(n) * static_cast<double>(ops.k_total);
     // Batched launches use single CTAs.
     bool pair = n > kBM && m > kBM && (flops < 6.0e12 || env_choice("KUDNN_B200_TC_PAIR") > 0) && ops.batch == 1 &&
@@ -427,8 +428,9 @@ cudaError_t launch_wide(const TcOperands &ops, const TcPlan &plan, const EpiPara
     p.num_kb = static_cast<int>((ops.k_total + elems_per_row - 1) / elems_per_row);
     p.tiles_m = static_cast<int>((m + 255) / 256);
     p.tiles_w = static_cast<int>((n + 255) / 256 / 2);
-    // Taller raster groups for launches of many milliseconds: the rows of B of a tile are then shared by more pairs at a time.  The
-    // 32768-row layer in a loop of seconds under the power cap, 8 / 16 / 32 tile rows per group: 14.3 / 13.2-13.7 / 13.0-13.2 ms.
+    // Taller raster groups for launches of many milliseconds: the rows of B of a tile are then shared by more pairs at a time, although
+    // a group's rows of A (134 MB there) no longer stay in L2.  The 32768-row layer in a loop of seconds under the power cap, on a
+    // warmer GPU than the figures above, 8 / 16 / 32 tile rows per group: 14.3 / 13.2-13.7 / 13.0-13.2 ms.
     // Not for shorter ones: 8192 x 4096 x 4096 in one group of 32 instead of two of 16 gains nothing (1.05 against 1.07 times the
     // 256-column tiles, runs differing by 2 %).
     const bool tall = 2.0 * static_cast<double>(m) * static_cast<double>(n) * static_cast<double>(ops.k_total) >= 6.0e12;

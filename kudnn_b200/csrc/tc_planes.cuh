@@ -9,21 +9,23 @@
 // additions to the large one, and a k-block of 64 brings in each operand's planes once instead of one and a half times: 64 KiB per
 // SM and 1536 cycles of MMAs.
 //
-// A normal distribution has one element below 2^-28 of its row's largest in 10^8.  The split leaves up to eight of them per row out of the planes,
-// and the epilogue adds their products in fp32 (planes_add_rest), for up to sixteen rows of activations and weights.
+// A normal distribution has one element below 2^-28 of its row's largest in 10^8.  The split leaves up to eight of them per row out
+// of the planes, and the epilogue adds their products in fp32 (planes_add_rest), for up to sixteen rows of activations and weights.
 //
 // Rows that this form does not carry (elements that are not finite, whose largest lies outside [2^-100, 2^64], with a nonzero
-// element below 2^-60 of it, or with more than eight below 2^-28) are marked by the split; if there is any, or lists of more rows than that, among the
-// activations or the weights, all CTAs leave, and the launches that follow compute the product on TF32 planes (tc_linear_kernel), which otherwise leave at once.
-// 4096 x 4608 x 2304 in calls one after the other: 188 to 209 us, with one element of 1e-10 205 to 216, left to the TF32 planes 430 to
-// 470, where the TF32 form by itself takes 390 to 420: the split and the marks in vain.
+// element below 2^-60 of it, or with more than eight below 2^-28) are marked by the split; if there is any, or lists of more rows
+// than that, among the activations or the weights, all CTAs leave, and the launches that follow compute the product on TF32 planes
+// (tc_linear_kernel), which otherwise leave at once.  4096 x 4608 x 2304 in calls one after the other: 188 to 209 us, with one
+// element of 1e-10 205 to 216, left to the TF32 planes 430 to 470, where the TF32 form by itself takes 390 to 420: the split and
+// the marks in vain.
 //
 // Shape of one CTA: as tc_wide_kernel, a ring of three stages, tiles of 256 x 256 (both accumulators), and 256 x 128 for the tiles of
 // a last wave that would keep at most half of the pairs busy.
 //
 // Measured against the TF32 form, kernels and splits together, in turn on one GPU: 4096 x 4608 x 2304 350 -> 185 us, 8192 x 5120 x
 // 5120 1715 -> 863 us (1494 TFLOP/s of fp16 products), normwise error against 64 bits 5.4e-6 -> 2.8e-6 and 1.3e-5 -> 6.7e-6: half
-// as many additions, each of which cuts the sum, and none of the small products among them.
+// as many additions, each of which cuts the sum, and none of the small products among them.  The product kernel alone takes 174 us
+// of the first, the tensor pipe busy for 81 % of its cycles, the split 19 us, the two launches that leave at once 5 each (serialised).
 #pragma once
 
 #include "tc_wide.cuh"

@@ -20,9 +20,11 @@
 //
 // Measured against the pairs on 256 x 256 tiles, in turn on one GPU, inputs from memory: 4096 x 11008 x 4096 bf16 with SiLU
 // 276.5 -> 261.4 us, 8192 x 4096 x 4096 fp16 with GELU and a residual 239.6 -> 225.4, 8192 x 8192 x 8192 bf16 840 -> 735,
-// 32768 x 28672 x 8192 with SiLU (single CTAs before) 12.6 -> 11.75 ms, 8192 x 8192 x 512 (epilogue) 181 -> 83.  All but the
+// 32768 x 28672 x 8192 with SiLU (single CTAs before) 12.6 -> 11.75 ms, 8192 x 8192 x 512 (epilogue) 181 -> 83.  On a warmer
+// GPU, where the power cap bites sooner, the gain was 4.6, 7.4 and 4.5 % on the first, second and fourth.  All but the
 // last run under the power cap: leaving out the step between the accumulators costs cycles but no time there, while every
-// instruction left out of the epilogue shows.
+// instruction left out of the epilogue shows.  The 16-bit instances spill (fp16 524 bytes of stores and 1380 of loads, bf16 372
+// and 1388): the 128 registers of a drained accumulator beside two residual pieces and the values at work.
 //
 // Work items, in this order: whole tiles; halves (256 x 256, one accumulator), of which the two accumulators take turns;
 // quarters (256 x 128).  The host cuts the tiles of the last wave so that all pairs end at about the same time.
