@@ -298,3 +298,28 @@ def test_wide_tiles_of_integer_products(cuda_device, monkeypatch, capfd, cut, m,
     assert torch.equal(c[:, :n], want.clamp(-2.0 ** 31, 2.0 ** 31 - 1).to(torch.int64).to(torch.int32))
     assert bool((c[:, n:] == 7).all())
     assert ("256 (CTA pair) x 512" in capfd.readouterr().err) == (n % 4 == 0)  # rows that end inside 16 bytes are left to narrow tiles
+
+
+@pytest.mark.parametrize("kind", [kb.BF16, kb.F16])
+@pytest.mark.parametrize("cut", ["1", "2", "3"])
+@pytest.mark.parametrize("wide_bias", [False, True])
+def test_wide_tiles_round_alpha_times_the_product(cuda_device, monkeypatch, kind, cut, wide_bias):
+    """alpha * acc is rounded to fp32 (to fp16 in the fp16 chain) ahead of the bias, in tiles of any width: the same bits, so that
+    the rows of a call may be cut anywhere."""
+    m, n, k = 1200, 2056, 264
+    dtype = torch.bfloat16 if kind == kb.BF16 else torch.float16
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(43)
+    a, w, side = (torch.randn(s, generator=gen, device=cuda_device).to(dtype) for s in ((m, k), (n, k), (n,)))
+    stream = torch.cuda.current_stream().cuda_stream
+    got = []
+    for wide in ("0", cut):
+        monkeypatch.setenv("KUDNN_B200_TC_WIDE", wide)
+        lin = kb.Linear(kb.make_desc(m, n, k, kind, has_bias=True, bias_dtype=kb.F32 if wide_bias else None, act=kb.ACT_RELU, act_alpha=0.25))
+        lin.force_kernel(kb.KERNEL_TC)
+        lin.prepack(w, stream=stream)
+        c = torch.empty((m, n), device=cuda_device, dtype=dtype)
+        lin.run(a, w, c, side.float() if wide_bias else side, alpha=0.3, stream=stream)
+        lin.check(stream=stream)
+        got.append(c)
+    assert torch.equal(*got)
