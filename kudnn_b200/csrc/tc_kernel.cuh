@@ -208,6 +208,13 @@ __device__ __forceinline__ bool vec_ok(const void *base, int dtype, long long id
     return (addr & 15u) == 0;
 }
 
+// The activation of 16-bit results, the same in every epilogue of these kernels: which of them finishes a value depends on the tiles.
+template <int kAct>
+__device__ __forceinline__ float activation16(float x, float alpha)
+{
+    return kAct == KUDNN_B200_ACT_GELU_TANH ? gelu_tanh_sigmoid(x) : activation<false>(x, kAct, alpha);
+}
+
 // Post-GEMM chain and stores for 8 consecutive columns of one output row, starting at column ni.  Same arithmetic
 // as finish_element(), but organised as passes over the 8 values: every run-time switch (element type, bias,
 // second output) is tested once per pass instead of once per element, which leaves straight-line code with eight
@@ -280,7 +287,7 @@ __device__ __forceinline__ void epilogue_group8(const EpiParams &e, const EpiTen
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                v[j] = activation<kPrecise == 1>(v[j], kAct, e.act_alpha);
+                v[j] = kPrecise == 0 ? activation16<kAct>(v[j], e.act_alpha) : activation<kPrecise == 1>(v[j], kAct, e.act_alpha);
             }
         }
         if (ct == KUDNN_B200_F16) {
@@ -491,7 +498,7 @@ __device__ __forceinline__ uint4 act8_packed(const EpiParams &e, const uint4 &w)
     unpack8<kDt>(w, v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        v[j] = kAct == KUDNN_B200_ACT_GELU_TANH ? gelu_tanh_sigmoid(v[j]) : activation<false>(v[j], kAct, e.act_alpha);
+        v[j] = activation16<kAct>(v[j], e.act_alpha);
     }
     if (kDt == KUDNN_B200_F16) {
         return pack8_rne<kDt>(v);
@@ -591,7 +598,7 @@ __device__ __forceinline__ void chain8(const EpiParams &e, bool has_bias, const 
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                v[j] = activation<kDt == KUDNN_B200_F32>(v[j], kAct, e.act_alpha);
+                v[j] = kDt == KUDNN_B200_F32 ? activation<true>(v[j], kAct, e.act_alpha) : activation16<kAct>(v[j], e.act_alpha);
             }
         }
         if (ct == KUDNN_B200_F16) {

@@ -323,3 +323,28 @@ def test_wide_tiles_round_alpha_times_the_product(cuda_device, monkeypatch, kind
         lin.check(stream=stream)
         got.append(c)
     assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("kind", [kb.BF16, kb.F16])
+@pytest.mark.parametrize("alpha,n,pitch", [(1.0, 2056, 2056), (0.3, 2056, 2056), (1.0, 2052, 2056), (0.3, 2052, 2056), (1.0, 2051, 2051), (1.0, 2052, 2052)])
+def test_gelu_is_the_same_in_every_epilogue(cuda_device, monkeypatch, kind, alpha, n, pitch):
+    """Finished from tensor memory, from shared memory or on wide tiles, in whole vectors, cut ones or value by value: the same bits."""
+    m, k = 1200, 264
+    dtype = torch.bfloat16 if kind == kb.BF16 else torch.float16
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(47)
+    a, w = (torch.randn(s, generator=gen, device=cuda_device).to(dtype) for s in ((m, k), (n, k)))
+    a *= 0.2  # results of a few units, where the forms of the function differ most
+    stream = torch.cuda.current_stream().cuda_stream
+    got = []
+    for pair, wide in (("1", "0"), ("0", "0"), (None, "1")):
+        for name, value in (("KUDNN_B200_TC_PAIR", pair), ("KUDNN_B200_TC_WIDE", wide), ("KUDNN_B200_TC_SPLITS", "1")):
+            monkeypatch.delenv(name, raising=False) if value is None else monkeypatch.setenv(name, value)
+        lin = kb.Linear(kb.make_desc(m, n, k, kind, act=kb.ACT_GELU_TANH, c_strides=(pitch, 1)))
+        lin.force_kernel(kb.KERNEL_TC)
+        lin.prepack(w, stream=stream)
+        c = torch.zeros((m, pitch), device=cuda_device, dtype=dtype)
+        lin.run(a, w, c, alpha=alpha, stream=stream)
+        lin.check(stream=stream)
+        got.append(c)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
