@@ -43,12 +43,13 @@ WORKLOADS = {
                label="Linear+SiLU bf16 M32768 K8192 N28672"),
 }
 
-# DRAM bytes per launch of the dominant kernel, from ncu captures (dram__bytes_read.sum + dram__bytes_write.sum) of
-# reduced cases, scaled to the full launch by the rows processed (null where nothing was captured)
+# DRAM bytes per launch of the dominant kernel, from ncu captures (dram__bytes_read.sum + dram__bytes_write.sum); null where
+# nothing was captured
 NCU_TRAFFIC_BYTES = {
-    # ncu capture of a half-size case (m = 2048): 110.7 MB read + 29.1 MB written; x and y scale with the rows, W does
-    # not, and the part of y still in L2 at kernel end is counted as written
-    "c2": 127.5e6 + 90.2e6,
+    # the launch itself, on 256 x 512 tiles: read + written (part of y is still in L2 at the kernel's end)
+    "c2": 219.0e6 + 81.1e6,
+    # 256 x 512 tiles: read + written
+    "c3": 297.0e6 + 66.0e6,
     # ncu capture of an n = 8192 case: traffic equals the algorithmic bytes within 0.1 % (+3 % for the m = 16 partial
     # sums); scaled to n = 28672 by the rows
     "c4": 471.9e6 + 11.5e6,
@@ -56,11 +57,11 @@ NCU_TRAFFIC_BYTES = {
 
 
 def c5m_traffic_bytes(rows):
-    """DRAM bytes per launch of the tensor-core kernel on `rows` rows of the large prefill layer: ncu capture of an
-    8192-row launch (dram__bytes_read.sum 6.47 GB + dram__bytes_write.sum 0.56 GB), scaled by the rows; the weights are
-    streamed once per group of 4096 rows and rows of x are fetched again for later tile columns, so the traffic grows
-    in proportion to the rows.  The full-size launch is too large to capture."""
-    return 7.03e9 * rows / 8192.0
+    """DRAM bytes per launch of the tensor-core kernel on `rows` rows of the large prefill layer: ncu capture of the whole
+    layer's launch (32768 rows, 256 x 512 tiles: dram__bytes_read.sum 23.67 GB + dram__bytes_write.sum 2.49 GB), scaled by the
+    rows; the weights are streamed once per raster group and rows of x are fetched again for later tile columns, so the
+    traffic grows about in proportion to the rows."""
+    return 26.16e9 * rows / 32768.0
 
 
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
