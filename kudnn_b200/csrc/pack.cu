@@ -306,21 +306,9 @@ __global__ void __launch_bounds__(kSplitThreads, 6) split_half_kernel(const floa
     const float smallest = mn != 0xffffffffu && in_range ? __uint_as_float(mn) * up : 1.0f;
     const bool some_small = smallest < 0x1p-14f;
     unsigned short *dst = to.planes + row * 2 * k_pad;
-    auto put = [&](int piece, float (&v)[8]) {
+    auto put = [&](int piece, const float (&v)[8]) {
         if (piece >= pieces) {
             return;
-        }
-        if (some_small) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (v[i] != 0.0f && fabsf(v[i] * up) < 0x1p-14f) {
-                    const int slot = atomicAdd(&left_out, 1);
-                    if (slot < kPlanesRest) {
-                        rest[slot] = PlanesElement{piece * 8 + i, v[i]};
-                    }
-                    v[i] = 0.0f;
-                }
-            }
         }
         unsigned hi[4], lo[4];
 #pragma unroll
@@ -350,6 +338,23 @@ __global__ void __launch_bounds__(kSplitThreads, 6) split_half_kernel(const floa
         }
     }
     if (some_small) {
+        // rare, and so a pass of its own over the row, now that its planes are written
+        __syncthreads();
+#pragma unroll 1
+        for (int piece = static_cast<int>(threadIdx.x); piece < pieces; piece += kSplitThreads) {
+            fetch(piece, held[0]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (held[0][i] != 0.0f && fabsf(held[0][i] * up) < 0x1p-14f) {
+                    const int slot = atomicAdd(&left_out, 1);
+                    if (slot < kPlanesRest) {
+                        rest[slot] = PlanesElement{piece * 8 + i, held[0][i]};
+                    }
+                    unsigned short *at = dst + (piece >> 3) * 128 + (piece & 7) * 8 + i;
+                    at[0] = at[64] = 0;
+                }
+            }
+        }
         __syncthreads();
     }
     if (threadIdx.x == 0) {
