@@ -466,12 +466,27 @@ bool reserve_optional(DeviceBuffer *buf, size_t bytes)
     return false;
 }
 
+// Whether runs can take the planes at all, given pointers on 16 bytes.
+bool planes_fit(const kudnn_b200_linear_desc &d)
+{
+    kudnn_b200_linear_args args = {};
+    args.alpha = 1.0f;
+    args.c = reinterpret_cast<void *>(16);
+    args.bias = d.has_bias != 0 ? args.c : nullptr;
+    kb::EpiParams epi;
+    fill_epi(d, args, &epi);
+    return kb::planes_take(epi) && kmajor_ready(args.c, d.a_dtype, d.a_sm, d.a_sk, d.m);
+}
+
 // Whether an fp32 product is worth the planes: they take half of the time of the TF32 form and two more launches, 4 us.  Times of
 // both in us: 512 x 1152 x 1152 23.4 and 24.4, 676 x 1280 x 1152 33 and 31, 1024 x 1152 x 1152 31 and 26, 1195 x 2816 x 1472 66 and
 // 38, 4096 x 4608 x 2304 350 and 185, x 64 57 and 37.  With fewer than 20 tiles of 256 x 256 most pairs would be idle, where the TF32 form cuts K:
 // 741 x 1280 x 2816 48 and 51, 620 x 1280 x 4736 60 and 65.
 bool planes_worth(const kudnn_b200_linear_desc &d)
 {
+    if (!planes_fit(d)) {
+        return false;
+    }
     const char *forced = std::getenv("KUDNN_B200_TC_PLANES");
     if (forced != nullptr && *forced != '\0') {
         return *forced != '0';

@@ -332,3 +332,12 @@ def test_several_tiles_per_pair(cuda_device, monkeypatch, n, marks):
             for j in range(0, n, 128):
                 part = (slice(r, r + 256), slice(j, j + 128))
                 assert float(error[part].norm()) <= (k / 16 + 8) * 2.0 ** -23 * float(want[part].norm())
+
+
+@pytest.mark.parametrize("n,desc", [(1030, {}), (1032, dict(res_op=kb.RES_IDENTICAL)), (1032, dict(act=kb.ACT_TANH)), (1032, dict(c_strides=(1, 1100))),
+                                    (1032, dict(has_bias=True, bias_strides=(1, 0))), (1032, dict(a_strides=(1, 1100))), (1032, dict(a_strides=(330, 1)))])
+def test_planes_are_not_packed_where_no_run_takes_them(cuda_device, monkeypatch, n, desc):
+    m, k = 1100, 328
+    w = _draw(cuda_device, n, k)
+    held = [_layer(monkeypatch, planes, m, n, k, w, **desc).workspace_bytes for planes in "01"]
+    assert held[0] == held[1]
