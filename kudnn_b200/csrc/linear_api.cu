@@ -481,7 +481,9 @@ bool planes_fit(const kudnn_b200_linear_desc &d)
 // Whether an fp32 product is worth the planes: they take half of the time of the TF32 form and two more launches, 4 us.  Times of
 // both in us: 512 x 1152 x 1152 23.4 and 24.4, 676 x 1280 x 1152 33 and 31, 1024 x 1152 x 1152 31 and 26, 1195 x 2816 x 1472 66 and
 // 38, 4096 x 4608 x 2304 350 and 185, x 64 57 and 37.  With fewer than 20 tiles of 256 x 256 most pairs would be idle, where the TF32 form cuts K:
-// 741 x 1280 x 2816 48 and 51, 620 x 1280 x 4736 60 and 65.
+// 741 x 1280 x 2816 48 and 51, 620 x 1280 x 4736 60 and 65.  So they would with 20 to 23 tiles whose last rows leave the second
+// half of a tile empty, if K is long: 64 x 5120 x 8192 95 and 104, 32 x 5632 x 8192 99 and 104, 300 x 2560 x 12288 145 and 151, but
+// 100 x 5120 x 2304 42 and 39, 64 x 6144 x 8192 109 and 105, 256 x 5120 x 8192 140 and 106.
 bool planes_worth(const kudnn_b200_linear_desc &d)
 {
     if (!planes_fit(d)) {
@@ -492,7 +494,8 @@ bool planes_worth(const kudnn_b200_linear_desc &d)
         return *forced != '0';
     }
     const long long tiles = ((d.m + 255) / 256) * ((d.n + 255) / 256);
-    return tiles >= 20 && d.k >= 64 && static_cast<double>(d.m) * d.n * d.k >= 1.0e9;
+    const bool half_empty = (d.m + 127) / 128 % 2 != 0;
+    return tiles >= (half_empty && d.k > 4096 ? 24 : 20) && d.k >= 64 && static_cast<double>(d.m) * d.n * d.k >= 1.0e9;
 }
 
 // A batched problem whose weights are shared by all batch entries and whose other tensors are laid out so that

@@ -341,3 +341,20 @@ def test_planes_are_not_packed_where_no_run_takes_them(cuda_device, monkeypatch,
     w = _draw(cuda_device, n, k)
     held = [_layer(monkeypatch, planes, m, n, k, w, **desc).workspace_bytes for planes in "01"]
     assert held[0] == held[1]
+
+
+@pytest.mark.parametrize("m,n,k,planes", [(64, 5120, 8192, False), (64, 5120, 4096, True), (64, 6144, 8192, True), (300, 2560, 8192, False),
+                                          (256, 5120, 8192, True), (385, 2560, 8192, True)])
+def test_few_tiles_that_are_half_empty_stay_on_the_tf32_form_where_k_is_long(cuda_device, monkeypatch, m, n, k, planes):
+    monkeypatch.delenv("KUDNN_B200_TC_PLANES", raising=False)
+    a, w = _draw(cuda_device, m, k).clamp(1e-3, 4.0), _draw(cuda_device, n, k).clamp(-4.0, -1e-3)
+    lin = kb.Linear(kb.make_desc(m, n, k, kb.F32))
+    stream = torch.cuda.current_stream().cuda_stream
+    lin.prepack(w, stream=stream)
+    c = torch.empty((m, n), device=cuda_device)
+    lin.run(a, w, c, stream=stream)
+    lin.check(stream=stream)
+    assert lin.last_launches == (4 if planes else 2)
+    want = a.double() @ w.double().T
+    # all terms have one sign: 3 k / 8 additions at most, each cut at 2^-23 of the sum
+    assert bool(((c.double() - want).abs() <= (3 * 2.0 ** -22 + (k / 8 * 3 + 4) * 2.0 ** -23) * want.abs()).all())
