@@ -11,6 +11,8 @@
 //
 // A normal distribution has one element below 2^-28 of its row's largest in 10^8.  The split leaves up to eight of them per row out
 // of the planes, and the epilogue adds their products in fp32 (planes_add_rest), for up to sixteen rows of activations and weights.
+// A call with lists takes 2 to 4 us more; one without 0.3 to 0.5 us more than without the code (1024 x 2048 x 1536 31.5 -> 32.0), which
+// stands between the drain and the stores of every item: by 32 columns, in a function or a branch of its own it cost as much or more.
 //
 // Rows that this form does not carry (elements that are not finite, whose largest lies outside [2^-100, 2^64], with a nonzero
 // element below 2^-60 of it, or with more than eight below 2^-28) are marked by the split; if there is any, or lists of more rows
